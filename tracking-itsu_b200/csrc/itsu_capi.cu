@@ -81,6 +81,7 @@ struct itsu_context {
   float *phi = nullptr;
   int32_t *trk_count = nullptr, *trk_off = nullptr, *trk_lookup = nullptr;
   float4 *zs = nullptr;
+  int2 *trk_range = nullptr;
   int32_t *clu_seg = nullptr;
   int4 *clu_aux = nullptr;
   int32_t *clu_crowded = nullptr;
@@ -93,7 +94,7 @@ struct itsu_context {
   float *vtx = nullptr;
   // tracklet class
   itsu_tracklet *tracklets = nullptr;
-  float2 *trk_slope = nullptr;  // (tanL, phi) of each tracklet, beside the records
+  uint32_t *trk_key = nullptr;  // (tanL, phi) of each tracklet in fixed point, beside the records
   int32_t *trk_seg_id = nullptr, *cell_count = nullptr, *cell_off = nullptr, *cell_lookup = nullptr, *cell_crowded = nullptr;
   unsigned long long *cell_mask = nullptr;
   // cell class
@@ -330,11 +331,12 @@ Arena arena_of(const itsu_context *ctx)
   a.trk_slots = ctx->trk_slots;
   a.slot_stride = ctx->cap_clusters;
   a.trk_off = ctx->trk_off;
+  a.trk_range = ctx->trk_range;
   a.trk_lookup = ctx->trk_lookup;
   a.trk_seg = ctx->trk_seg;
   a.cell_seginfo = ctx->cell_seginfo;
   a.tracklets = ctx->tracklets;
-  a.trk_slope = ctx->trk_slope;
+  a.trk_key = ctx->trk_key;
   a.trk_seg_id = ctx->trk_seg_id;
   a.cell_count = ctx->cell_count;
   a.cell_mask = ctx->cell_mask;
@@ -404,6 +406,7 @@ itsu_status ensure_clusters(itsu_context *ctx, int64_t n_clusters, int32_t n_eve
     ITSU_CUDA(ctx, alloc(ctx, ctx->phi, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_count, cap + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_off, cap + 1));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->trk_range, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_lookup, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->zs, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->clu_seg, cap));
@@ -440,7 +443,7 @@ itsu_status ensure_tracklets(itsu_context *ctx, int64_t need)
     if (st != ITSU_OK) return st;
     const int64_t cap = grow_to(need);
     ITSU_CUDA(ctx, alloc(ctx, ctx->tracklets, cap));
-    ITSU_CUDA(ctx, alloc(ctx, ctx->trk_slope, cap));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->trk_key, cap + 4));  // read in aligned groups of four
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_seg_id, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_count, cap + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_mask, cap));
@@ -940,11 +943,11 @@ void itsu_context_destroy(itsu_context *ctx)
   if (ctx->twin) itsu_context_destroy(ctx->twin);
   drop_graph(ctx);
   release(ctx->raw); release(ctx->raw_in); release(ctx->raw_track); release(ctx->sorted); release(ctx->tmp); release(ctx->xyzr); release(ctx->phi);
-  release(ctx->trk_count); release(ctx->trk_off); release(ctx->trk_lookup); release(ctx->zs); release(ctx->clu_seg); release(ctx->clu_aux); release(ctx->clu_crowded); release(ctx->trk_slots);
+  release(ctx->trk_count); release(ctx->trk_off); release(ctx->trk_range); release(ctx->trk_lookup); release(ctx->zs); release(ctx->clu_seg); release(ctx->clu_aux); release(ctx->clu_crowded); release(ctx->trk_slots);
   release(ctx->seg_rrange); release(ctx->seg_regular); release(ctx->raw_off);
   release(ctx->layer_off); release(ctx->index_tables); release(ctx->trk_seg); release(ctx->cell_seginfo); release(ctx->cell_seg);
   release(ctx->road_seg); release(ctx->vtx);
-  release(ctx->tracklets); release(ctx->trk_slope); release(ctx->trk_seg_id); release(ctx->cell_count); release(ctx->cell_mask); release(ctx->cell_off); release(ctx->cell_lookup); release(ctx->cell_crowded);
+  release(ctx->tracklets); release(ctx->trk_key); release(ctx->trk_seg_id); release(ctx->cell_count); release(ctx->cell_mask); release(ctx->cell_off); release(ctx->cell_lookup); release(ctx->cell_crowded);
   release(ctx->cells); release(ctx->cell_entries); release(ctx->cell_dca); release(ctx->cell_seg_id); release(ctx->nb_count); release(ctx->nb_off); release(ctx->nb_fill);
   release(ctx->nb_mask);
   release(ctx->road_count); release(ctx->road_off); release(ctx->paths);

@@ -136,6 +136,57 @@ __device__ __forceinline__ bool cell_precut(int layer, float t1_tan_lambda, floa
   return cell_precut_dz(t1_tan_lambda, t1_phi, t2_tan_lambda, t2_phi, c1, vz, kC.cell_max_dz[layer]);
 }
 
+// The cell stage's precut in fixed point: a superset of the cheap cuts above in about three
+// instructions a pair (the cuts themselves take about twenty). A tracklet's key holds its phi in
+// units of 2 pi / 65536 (high half; wraps with the angle) and its tanL in units of 1 / 4096 modulo 16
+// (low half). For a first tracklet, the second ones that can pass lie within |delta phi| < 0.14
+// (1460.3 units) and in an interval of tanL: |delta tanL| < 0.025 (102.4 units) and, because the
+// delta z cut is |B - delta r1 / 2| < max_dz for B = z1 - vz - tanL1 r1 and delta = tanL2 - tanL1,
+// delta within 2 (B +- max_dz) / r1. The margins cover the keys' rounding (half a unit each) and the
+// binary32 rounding of the cuts and of the bounds, relative to the operands (1e-6 of their
+// magnitudes against four roundings of 2^-24). A non-finite tanL never passes the cuts; tanL beyond
+// 2^19 saturates, where neighbouring binary32 values are further apart than the cut. Pairs that pass
+// are tested again exactly; tests/test_cell_window.py checks that none is lost.
+constexpr float kKeyTanUnits = 4096.0f;
+constexpr float kKeyPhiUnits = 10430.3783504704527f;  // 65536 / (2 pi)
+constexpr int kKeyPhiReach = 1463;                    // 0.14 rad in units, the keys' roundings and one to spare
+
+__device__ __forceinline__ uint32_t tracklet_key(float tan_lambda, float phi)
+{
+  return ((uint32_t)__float2int_rn(phi * kKeyPhiUnits) << 16) | ((uint32_t)__float2int_rn(tan_lambda * kKeyTanUnits) & 0xffffu);
+}
+
+struct CellWindow {
+  uint32_t minus_base;  // minus the lowest phi (high half) and the lowest tanL (low half)
+  uint32_t width;       // the reach of each above its lowest
+  bool empty;
+};
+
+__device__ __forceinline__ CellWindow cell_window(float t1_tan_lambda, float t1_phi, float z1, float r1, float vz, float max_dz)
+{
+  float lo = -0.0251f, hi = 0.0251f;
+  if (r1 > 0.01f) {
+    const float z_beam = t1_tan_lambda * r1;
+    const float b = z1 - vz - z_beam;
+    const float reach = max_dz + 1e-5f + 1e-6f * (fabsf(z_beam) + fabsf(z1) + fabsf(vz) + r1);
+    const float scale = __fdividef(2.0f, r1);  // two ulp off at most; the bounds' margin is two units of 1 / 4096 in 0.025
+    lo = fmaxf(lo, (b - reach) * scale);  // fmaxf, fminf: a NaN bound is no bound
+    hi = fminf(hi, (b + reach) * scale);
+  }
+  CellWindow w;
+  w.empty = !(lo <= hi);
+  const int from = __float2int_rd(lo * kKeyTanUnits) - 2, to = __float2int_ru(hi * kKeyTanUnits) + 2;
+  w.minus_base = __vneg2(__vadd2(tracklet_key(t1_tan_lambda, t1_phi), ((uint32_t)-kKeyPhiReach << 16) | ((uint32_t)from & 0xffffu)));
+  w.width = ((uint32_t)(2 * kKeyPhiReach) << 16) | (uint32_t)(to - from);
+  return w;
+}
+
+// Both halves of key - base at most width: one add-and-max on the halves, one compare.
+__device__ __forceinline__ bool cell_window_pass(const CellWindow &w, uint32_t key)
+{
+  return __viaddmax_u16x2(key, w.minus_base, w.width) == w.width;
+}
+
 // Tracker.cxx:175-216: circle-plane normal, radius and DCA of the three clusters. Returns false
 // when the pair is rejected; otherwise fills the unit normal and curvature. dca_out receives the
 // DCA whenever it is computed (-1 when the clusters give no plane).

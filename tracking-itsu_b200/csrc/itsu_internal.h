@@ -114,7 +114,8 @@ struct Arena {
   int32_t *trk_lookup;
   int32_t *trk_seg;
   itsu_tracklet *tracklets;
-  float2 *trk_slope;  // per tracklet its (tanL, phi) again, packed: the cell pass's precut reads only these
+  int2 *trk_range;  // per inner cluster its first tracklet and their number: trk_off's two, in one 8-byte gather
+  uint32_t *trk_key;  // per tracklet its (tanL, phi) in fixed point (tracklet_key): the cell pass's precut reads only these
   int32_t *trk_seg_id;
   int4 *cell_seginfo;  // per tracklet segment, two records: {first cluster of L (-1: no cells), of L+1, of L+2,
                        // first tracklet of L}, {first tracklet of L+1, vertex x, y, z (float bits)}

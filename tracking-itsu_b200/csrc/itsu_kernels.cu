@@ -706,10 +706,23 @@ __device__ __forceinline__ itsu_tracklet make_tracklet(float4 c, float4 d, int32
   return t;
 }
 
+// The record in one 16-byte store (the struct's own alignment of 4 would make it four), and its key.
 __device__ __forceinline__ void store_tracklet(const Arena &a, int64_t out, const itsu_tracklet &t)
 {
-  a.tracklets[out] = t;
-  a.trk_slope[out] = make_float2(t.tan_lambda, t.phi);
+  reinterpret_cast<int4 *>(a.tracklets)[out] =
+      make_int4(t.first_cluster, t.second_cluster, __float_as_int(t.tan_lambda), __float_as_int(t.phi));
+  a.trk_key[out] = tracklet_key(t.tan_lambda, t.phi);
+}
+
+__device__ __forceinline__ itsu_tracklet load_tracklet(const Arena &a, int64_t k)
+{
+  const int4 w = reinterpret_cast<const int4 *>(a.tracklets)[k];
+  itsu_tracklet t;
+  t.first_cluster = w.x;
+  t.second_cluster = w.y;
+  t.tan_lambda = __int_as_float(w.z);
+  t.phi = __int_as_float(w.w);
+  return t;
 }
 
 __device__ __forceinline__ void write_tracklet(const Arena &a, int out, int64_t i_flat, int64_t j_flat, int seg)
@@ -1311,8 +1324,8 @@ __global__ void __launch_bounds__(kGateThreads) k_tracklets_gate(Arena a)
 // Write pass, a warp per 32 consecutive inner clusters: their tracklets form one contiguous range
 // (the scan of the counts), which the warp's lanes fill together: each lane takes the next
 // tracklet of the range, finds its inner cluster (owner) and rank there, reads the outer cluster
-// the count pass kept in that slot, and writes the tracklet (Tracklet.cxx:32-40) and its segment
-// id with coalesced stores; all lanes compute their binary64 azimuths together. Each cluster's
+// the count pass kept in that slot, and writes the tracklet (Tracklet.cxx:32-40), its key and its
+// segment id with coalesced stores; all lanes compute their binary64 azimuths together. Each cluster's
 // tracklets lookup entry is written here too. The tracklets of an inner cluster with more than
 // kTrackletSlots of them (not kept by the count pass) get their segment ids here and the rest
 // from k_tracklets_crowded.
@@ -1332,6 +1345,7 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tracklets_write(Arena a, int
   if (valid) {
     first = a.trk_off[i];
     count = a.trk_off[i + 1] - first;
+    a.trk_range[i] = make_int2(first, count);
     seg = a.clu_seg[i];
     const int e = seg / ITSU_LAYERS, layer = seg % ITSU_LAYERS;
     a.trk_lookup[i] = (layer >= 1 && layer <= ITSU_CELL_LAYERS && count > 0)
@@ -1464,7 +1478,7 @@ __device__ __forceinline__ CellLane cell_lane(const Arena &a, int64_t k, int64_t
   }
   // both loads first: neither depends on the other
   const int sid = a.trk_seg_id[k];
-  const itsu_tracklet t1 = a.tracklets[k];
+  const itsu_tracklet t1 = load_tracklet(a, k);
   s.e = sid / ITSU_TRACKLET_LAYERS;
   s.layer = sid % ITSU_TRACKLET_LAYERS;
   if (s.layer >= ITSU_CELL_LAYERS) {
@@ -1513,103 +1527,200 @@ __device__ __forceinline__ void write_cell(const Arena &a, int64_t out, const Ce
 }
 
 // Count pass: for each first tracklet, a mask of which of its (<= 64) outgoing tracklets make a
-// cell, and their number. Each lane runs the cheap cuts of its own tracklet's outgoing tracklets
-// (Tracker.cxx:155-173) on their (tanL, phi), one independent 8-byte load each; the
-// pairs that pass (about one in eighteen candidates) are then flattened across the warp's lanes so
-// that the circle geometry runs with the lanes converged. Each pair that passes the geometry
-// becomes a cell entry (its tracklets, normal, curvature and DCA) in the warp's current chunk of
-// the entry scratch, so the write pass needs no geometry.
+// cell, and their number. A warp takes a span of 32, 64 or 128 consecutive first tracklets:
+//  1. Precut, a lane per first tracklet, 32 at a time: one unsigned window per lane (cell_window)
+//     against the outgoing tracklets' 4-byte keys, four keys per 16-byte load. About six
+//     instructions a pair; the window is a superset of the exact cheap cuts by the keys'
+//     resolution, and what it lets through (about one pair in eighteen) goes to the warp's queue.
+//  2. Geometry, a lane per queued pair, in rounds of 32 from the queue, so that the rounds are full
+//     (a round per group of 32 first tracklets held 17 pairs on average): the exact cheap cuts
+//     (Tracker.cxx:161-173) on the records, then the circle geometry. Each passing pair becomes a
+//     cell entry (its tracklets, normal, curvature) in the warp's current chunk of the entry
+//     scratch and a bit in its first tracklet's mask, so the write pass needs no geometry.
+//  3. The span's masks, counts and reset lookup entries in coalesced stores.
+// Spans longer than 32 only pay where every warp has many of them; short runs take 32 so that
+// more warps share the work. The grid is one wave of resident blocks (8 of 128 threads at 64
+// registers per SM: blocks beyond that would run as a second, mostly empty wave). Bound by the
+// latency of the gathers (51% of issue slots, 53% of the L1 data pipe): 1.34 ms per 128 central
+// events, 1.78 ms with the cuts evaluated pair by pair in binary32 and a round per 32 tracklets.
 //
-// Runs over the first tracklets of events [e0, e1), or of all events when e1 is 0. Warps hold
-// aligned groups of 32 tracklets (their cells go to one scan tile); a group that straddles the
-// range's ends has its lanes outside the range idle.
-__global__ void __launch_bounds__(kMaxThreads) k_cells_count(Arena a, int32_t e0, int32_t e1)
+// Runs over the first tracklets of events [e0, e1), or of all events when e1 is 0. A span lies in
+// one scan tile; one that straddles the range's ends has its lanes outside the range idle.
+constexpr int kCellThreads = 128;
+constexpr int kCellBlocks = 8;  // resident blocks per SM
+constexpr int kCellGroups = 4;  // groups of 32 first tracklets in the longest span
+constexpr int kCellSpan = 32 * kCellGroups;
+constexpr int kCellQueue = 256;  // queued pairs of a warp (a group of 32 first tracklets has 17 on average)
+static_assert(kScanTile % kCellSpan == 0 && kCellSpan <= 128, "a span lies in one scan tile; its index has 7 bits in a queue item");
+
+struct CellWarp {
+  unsigned long long mask[kCellSpan];  // which outgoing tracklets make cells
+  int2 state[kCellSpan];  // first outgoing tracklet and segment (-1: a crowded outer cluster)
+  uint16_t queue[kCellQueue];  // (first tracklet in the span) | (outgoing tracklet) << 7
+};
+
+// Cells of first tracklet k whose outer cluster has more than kMaxMaskedOut outgoing tracklets, in order on one lane.
+__device__ __forceinline__ int crowded_cells(const Arena &a, int64_t k, int64_t n)
 {
-  __shared__ unsigned long long masks[kMaxThreads / 32][32];
+  const CellLane s = cell_lane(a, k, n);
+  int count = 0;
+  for (int b = 0; b < s.n_out; ++b) {
+    const itsu_tracklet t2 = load_tracklet(a, s.j0 + b);
+    float3 normal;
+    float curvature;
+    count += cell_precut(s.layer, s.t1_tan_lambda, s.t1_phi, t2.tan_lambda, t2.phi, s.c1, s.vz) &&
+             cell_geometry(s.layer, s.c1, s.c2, a.xyzr[s.c3_base + t2.second_cluster], s.vx, s.vy, normal, curvature);
+  }
+  return count;
+}
+
+// The outgoing tracklets of first tracklet k that its window lets through, as a mask.
+__device__ __forceinline__ unsigned long long cell_precut_mask(const Arena &a, uint32_t k, int2 &state)
+{
+  // both loads first: neither depends on the other
+  const int sid = a.trk_seg_id[k];
+  const itsu_tracklet t1 = load_tracklet(a, k);
+  const int layer = sid % ITSU_TRACKLET_LAYERS;
+  state = make_int2(0, sid);
+  if (layer >= ITSU_CELL_LAYERS) {
+    return 0ull;
+  }
+  const int4 A = a.cell_seginfo[2 * sid];
+  if (A.x < 0) {
+    return 0ull;  // the cell layer does not run
+  }
+  const int2 out = a.trk_range[A.y + t1.second_cluster];  // the outer cluster's first outgoing tracklet and their number
+  const int j0 = out.x, n_out = out.y;
+  if (n_out > kMaxMaskedOut) {
+    state.y = -1;  // counted with the span's results
+    return 0ull;
+  }
+  state.x = j0;
+  const float2 c1 = reinterpret_cast<const float2 *>(a.xyzr + A.x + t1.first_cluster)[1];  // z, r
+  const CellWindow w = cell_window(t1.tan_lambda, t1.phi, c1.x, c1.y, __int_as_float(a.cell_seginfo[2 * sid + 1].w), kC.cell_max_dz[layer]);
+  if (w.empty || n_out <= 0) {
+    return 0ull;
+  }
+  // keys in aligned groups of four (the array has room for the last group's overrun): those before
+  // j0 fall off by the shift, those past the end by the last mask
+  const int skip = j0 & 3;
+  const uint4 *keys = reinterpret_cast<const uint4 *>(a.trk_key + (j0 - skip));
+  auto four = [&](uint4 q) {
+    return (cell_window_pass(w, q.x) ? 1u : 0u) | (cell_window_pass(w, q.y) ? 2u : 0u) | (cell_window_pass(w, q.z) ? 4u : 0u) |
+           (cell_window_pass(w, q.w) ? 8u : 0u);
+  };
+  unsigned long long window = four(keys[0]) >> skip;
+#pragma unroll 2
+  for (int at = 4 - skip; at < n_out; at += 4) {
+    window |= (unsigned long long)four(*++keys) << at;
+  }
+  return window & (~0ull >> (kMaxMaskedOut - n_out));
+}
+
+__global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena a, int32_t e0, int32_t e1)
+{
+  __shared__ CellWarp shared[kCellThreads / 32];
   if (capacity_failed(a.status)) {
     return;
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t n = a.status->total[kTracklets];
-  const int64_t t0 = e1 > 0 ? a.trk_seg[(int64_t)e0 * ITSU_TRACKLET_LAYERS] : 0;
-  const int64_t t1 = e1 > 0 ? a.trk_seg[(int64_t)e1 * ITSU_TRACKLET_LAYERS] : n;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  int64_t chunk_pos = 0, chunk_end = 0;  // this warp's reserved cell entries (warp-uniform)
-  for (int64_t base = (t0 & ~int64_t(31)) + ((int64_t)blockIdx.x * (blockDim.x >> 5) + warp) * 32; base < t1;
-       base += warps * 32) {
-    const int64_t k_lane = base + lane;
-    const bool active = k_lane >= t0 && k_lane < t1;
-    const CellLane s = cell_lane(a, active ? k_lane : n, n);
-    const bool big = s.n_out > kMaxMaskedOut;
-    unsigned long long window = 0;  // the outgoing tracklets that pass the cheap cuts
-    if (!big && s.n_out > 0) {
-      const float max_dz = kC.cell_max_dz[s.layer];  // n_out > 0: an active cell layer
-      // (tanL, phi) of the outgoing tracklets, packed 8 bytes each; the window's two 32-bit
-      // halves are filled by two loops (a 64-bit variable shift per candidate costs more)
-      const float2 *tp = a.trk_slope + s.j0;
-      unsigned lo = 0u, hi = 0u;
-      const int n_lo = s.n_out < 32 ? s.n_out : 32;
-#pragma unroll 4
-      for (int q = 0; q < n_lo; ++q) {
-        const float2 t2 = tp[q];
-        lo |= (unsigned)cell_precut_dz(s.t1_tan_lambda, s.t1_phi, t2.x, t2.y, s.c1, s.vz, max_dz) << q;
-      }
-#pragma unroll 4
-      for (int q = 32; q < s.n_out; ++q) {
-        const float2 t2 = tp[q];
-        hi |= (unsigned)cell_precut_dz(s.t1_tan_lambda, s.t1_phi, t2.x, t2.y, s.c1, s.vz, max_dz) << (q - 32);
-      }
-      window = ((unsigned long long)hi << 32) | lo;
-    }
-    masks[warp][lane] = 0ull;
-    int total = 0;
-    const int excl = warp_exclusive_sum(__popcll(window), total);
-    __syncwarp();
-    for (int p0 = 0; p0 < total; p0 += 32) {
-      const int p = p0 + lane;
-      const int owner = owner_of(excl, p);
-      const int r = p - __shfl_sync(0xffffffffu, excl, owner);
-      const unsigned long long wmask = __shfl_sync(0xffffffffu, window, owner);
-      const int32_t j0 = __shfl_sync(0xffffffffu, s.j0, owner);
-      // the circle geometry reads x, y and r of the first two clusters, not z
-      const int32_t c3_base = __shfl_sync(0xffffffffu, s.c3_base, owner);
-      const float4 c1 = make_float4(__shfl_sync(0xffffffffu, s.c1.x, owner), __shfl_sync(0xffffffffu, s.c1.y, owner), 0.0f,
-                                    __shfl_sync(0xffffffffu, s.c1.w, owner));
-      const float4 c2 = make_float4(__shfl_sync(0xffffffffu, s.c2.x, owner), __shfl_sync(0xffffffffu, s.c2.y, owner), 0.0f,
-                                    __shfl_sync(0xffffffffu, s.c2.w, owner));
-      const float vx = __shfl_sync(0xffffffffu, s.vx, owner), vy = __shfl_sync(0xffffffffu, s.vy, owner);
-      const int layer = __shfl_sync(0xffffffffu, s.layer, owner);
-      bool pass = false;
-      int b = 0;
-      int32_t c3 = 0;
-      float3 normal = make_float3(0.0f, 0.0f, 0.0f);
-      float curvature = 0.0f, dca = 0.0f;
-      if (p < total) {
-        {
-          // the owner's r-th passing outgoing tracklet: the r-th set bit of its window, found in
-          // the 32-bit half that holds it
-          const unsigned wlo = (unsigned)wmask;
-          const int plo = __popc(wlo);
-          const bool in_lo = r < plo;
-          unsigned m = in_lo ? wlo : (unsigned)(wmask >> 32);
-          for (int q = in_lo ? r : r - plo; q > 0; --q) {
-            m &= m - 1u;
-          }
-          b = __ffs(m) - 1 + (in_lo ? 0 : 32);
+  const int lane = threadIdx.x & 31;
+  CellWarp &w = shared[threadIdx.x >> 5];
+  // tracklet indices stay below 2^31 (the scan flags larger totals), a span's end below 2^32
+  const uint32_t n = (uint32_t)a.status->total[kTracklets];
+  const uint32_t t0 = e1 > 0 ? (uint32_t)a.trk_seg[(int64_t)e0 * ITSU_TRACKLET_LAYERS] : 0u;
+  const uint32_t t1 = e1 > 0 ? (uint32_t)a.trk_seg[(int64_t)e1 * ITSU_TRACKLET_LAYERS] : n;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t per_warp = (t1 - t0) / (32 * warps);  // groups of 32 a warp would take one by one
+  const int groups = per_warp >= 32 ? kCellGroups : (per_warp >= 8 ? 2 : 1);
+  const uint32_t span = 32 * groups;
+  int64_t chunk_pos = 0;  // this warp's reserved cell entries: the next one, and how many are left (warp-uniform)
+  int chunk_left = 0;
+  for (uint32_t base = (t0 & ~(span - 1)) + (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * span; base < t1; base += warps * span) {
+    int g = 0, queued = 0;
+    unsigned long long window = 0;  // this lane's pairs of group g - 1 not yet queued
+    for (;;) {
+      const unsigned pending = __ballot_sync(0xffffffffu, window != 0);
+      if (pending == 0 && g < groups) {
+        const int at = 32 * g + lane;
+        const uint32_t k = base + at;
+        int2 state = make_int2(0, 0);
+        if (k >= t0 && k < t1) {
+          window = cell_precut_mask(a, k, state);
         }
-        c3 = a.tracklets[j0 + b].second_cluster;
-        pass = cell_geometry(layer, c1, c2, a.xyzr[c3_base + c3], vx, vy, normal, curvature, dca);
+        w.state[at] = state;
+        w.mask[at] = 0ull;
+        ++g;
+        // the group's pairs go to the queue together where they fit
+        int total;
+        const int first = queued + warp_exclusive_sum(__popcll(window), total);
+        if (queued + total <= kCellQueue) {
+          int to = first;
+          for (unsigned m = (unsigned)window; m != 0; m &= m - 1u) {
+            w.queue[to++] = (uint16_t)(at | (__ffs(m) - 1) << 7);
+          }
+          for (unsigned m = (unsigned)(window >> 32); m != 0; m &= m - 1u) {
+            w.queue[to++] = (uint16_t)(at | (__ffs(m) + 31) << 7);
+          }
+          queued += total;
+          window = 0;
+        }
+        if (queued < 32 && g < groups) {
+          continue;
+        }
+      } else if (pending != 0 && queued < 32) {
+        // too many at once (a crowded region): one pair of every lane that has one
+        if (window != 0) {
+          const int b = __ffsll((long long)window) - 1;
+          window &= window - 1ull;
+          w.queue[queued + __popc(pending & ((1u << lane) - 1u))] = (uint16_t)(32 * (g - 1) + lane | b << 7);
+        }
+        queued += __popc(pending);
+      }
+      if (queued == 0) {
+        if (g == groups && __ballot_sync(0xffffffffu, window != 0) == 0) {
+          break;
+        }
+        continue;
+      }
+      __syncwarp();
+      // a round of the last 32 queued pairs (fewer at the span's end)
+      const int m = min(queued, 32);
+      queued -= m;
+      bool pass = false;
+      int b = 0, sid = 0;
+      uint32_t k = 0, j = 0;
+      itsu_tracklet f, s;
+      int4 A, B;
+      float3 normal;
+      float curvature, dca;
+      if (lane < m) {
+        const int item = w.queue[queued + lane];
+        const int at = item & (kCellSpan - 1);
+        b = item >> 7;
+        const int2 state = w.state[at];
+        sid = state.y;
+        k = base + at;
+        j = state.x + b;
+        A = a.cell_seginfo[2 * sid];
+        B = a.cell_seginfo[2 * sid + 1];
+        f = load_tracklet(a, k);
+        s = load_tracklet(a, j);
+        const float4 c1 = a.xyzr[A.x + f.first_cluster];
+        const float4 c2 = a.xyzr[A.y + f.second_cluster];
+        const float4 c3 = a.xyzr[A.z + s.second_cluster];
+        const int layer = sid % ITSU_TRACKLET_LAYERS;
+        pass = cell_precut(layer, f.tan_lambda, f.phi, s.tan_lambda, s.phi, c1, __int_as_float(B.w)) &&
+               cell_geometry(layer, c1, c2, c3, __int_as_float(B.y), __int_as_float(B.z), normal, curvature, dca);
         if (pass) {
-          atomicOr(&masks[warp][owner], 1ull << b);
+          atomicOr(reinterpret_cast<unsigned *>(&w.mask[at]) + (b >> 5), 1u << (b & 31));
         }
       }
       // entries: the passing lanes' slots, contiguous in the warp's chunk
-      const unsigned m = __ballot_sync(0xffffffffu, pass);
-      const int need = __popc(m);
-      const int rank = __popc(m & ((1u << lane) - 1u));
+      const unsigned passed = __ballot_sync(0xffffffffu, pass);
+      const int need = __popc(passed);
+      const int rank = __popc(passed & ((1u << lane) - 1u));
       int64_t slot = chunk_pos + rank;
-      if (need > chunk_end - chunk_pos) {
-        const int room = (int)(chunk_end - chunk_pos);
+      if (need > chunk_left) {
         unsigned long long fresh = 0;
         if (lane == 0) {
           fresh = atomicAdd(reinterpret_cast<unsigned long long *>(&a.status->cell_entries), (unsigned long long)kCellChunk);
@@ -1618,62 +1729,57 @@ __global__ void __launch_bounds__(kMaxThreads) k_cells_count(Arena a, int32_t e0
           }
         }
         const int64_t fresh_base = (int64_t)__shfl_sync(0xffffffffu, fresh, 0);
-        slot = rank < room ? chunk_pos + rank : fresh_base + (rank - room);
-        chunk_pos = fresh_base + (need - room);
-        chunk_end = fresh_base + kCellChunk;
+        slot = rank < chunk_left ? chunk_pos + rank : fresh_base + (rank - chunk_left);
+        chunk_pos = fresh_base + (need - chunk_left);
+        chunk_left += kCellChunk - need;
       } else {
         chunk_pos += need;
+        chunk_left -= need;
       }
       if (pass && slot < a.cap_cell_entries) {
-        // the rest of the cell record, read again (cached since cell_lane) rather than kept in
-        // registers through the pair loops
-        const int64_t t1 = base + owner;
-        const int2 t1_clusters = *reinterpret_cast<const int2 *>(a.tracklets + t1);
-        const int e = a.trk_seg_id[t1] / ITSU_TRACKLET_LAYERS;
-        const int32_t *ts = a.trk_seg + e * ITSU_TRACKLET_LAYERS;
         int4 *dst = reinterpret_cast<int4 *>(a.cell_entries + slot);
-        dst[0] = make_int4((int)t1, b, e * ITSU_CELL_LAYERS + layer, t1_clusters.x);
-        dst[1] = make_int4(t1_clusters.y, c3, (int)(t1 - ts[layer]), j0 + b - ts[layer + 1]);
+        const int e = sid / ITSU_TRACKLET_LAYERS;
+        dst[0] = make_int4((int)k, b, sid - e, f.first_cluster);  // sid - e = 5 e + layer: the cell segment
+        dst[1] = make_int4(f.second_cluster, s.second_cluster, (int)(k - A.w), (int)(j - B.x));
         dst[2] = make_int4(__float_as_int(normal.x), __float_as_int(normal.y), __float_as_int(normal.z), __float_as_int(curvature));
         if (a.mlp) {
           a.cell_dca[slot] = dca;
         }
       }
+      __syncwarp();  // the queue's freed places are refilled
     }
     __syncwarp();
-    int count = __popcll(masks[warp][lane]);
-    if (big) {  // a crowded outer cluster: this lane evaluates its pairs in order
-      count = 0;
-      for (int b = 0; b < s.n_out; ++b) {
-        const itsu_tracklet t2 = a.tracklets[s.j0 + b];
-        float3 normal;
-        float curvature;
-        count += cell_precut(s.layer, s.t1_tan_lambda, s.t1_phi, t2.tan_lambda, t2.phi, s.c1, s.vz) &&
-                 cell_geometry(s.layer, s.c1, s.c2, a.xyzr[s.c3_base + t2.second_cluster], s.vx, s.vy, normal, curvature);
+    // the span's results; its cells go to its scan tile's sum (the cells scan has no reduce pass)
+    int cells = 0;
+    for (uint32_t at = lane; at < span; at += 32) {
+      const uint32_t k = base + at;
+      if (k < t0 || k >= t1) {
+        continue;
       }
-    }
-    // the warp's 32 tracklets lie in one scan tile: their cells go to its sum (the cells scan
-    // has no reduce pass)
-    const int batch_cells = (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
-    if (lane == 0 && batch_cells != 0) {
-      atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[base / kScanTile]), (unsigned long long)batch_cells);
-    }
-    if (active) {
-      a.cell_count[s.k] = count;
-      a.cell_mask[s.k] = big ? 0ull : masks[warp][lane];
-      a.cell_lookup[s.k] = ITSU_UNUSED_INDEX;  // the write pass fills it for tracklets with cells
+      const unsigned long long mask = w.mask[at];
+      const int2 state = w.state[at];
+      const bool big = state.y < 0;
+      const int count = big ? crowded_cells(a, k, n) : __popcll(mask);
+      cells += count;
+      a.cell_count[k] = count;
+      a.cell_mask[k] = mask;
+      a.cell_lookup[k] = ITSU_UNUSED_INDEX;  // the write pass fills it for tracklets with cells
       if (big && count > 0) {
         const unsigned long long q = atomicAdd(reinterpret_cast<unsigned long long *>(&a.status->crowded), 1ull);
         if ((int64_t)q < n) {
-          a.cell_crowded[q] = (int32_t)s.k;
+          a.cell_crowded[q] = (int32_t)k;
         }
       }
     }
-    __syncwarp();
+    cells = (int)__reduce_add_sync(0xffffffffu, (unsigned)cells);
+    if (lane == 0 && cells != 0) {
+      atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[base / kScanTile]), (unsigned long long)cells);
+    }
+    __syncwarp();  // the span's state is refilled next
   }
   // the unused rest of the last chunk is marked empty
-  for (int64_t i = chunk_pos + lane; i < chunk_end && i < a.cap_cell_entries; i += 32) {
-    a.cell_entries[i].t1 = -1;
+  for (int i = lane; i < chunk_left && chunk_pos + i < a.cap_cell_entries; i += 32) {
+    a.cell_entries[chunk_pos + i].t1 = -1;
   }
 }
 
@@ -1709,8 +1815,8 @@ __global__ void __launch_bounds__(kPrefilterThreads) k_cells_prefilter(Arena a)
       const int4 g = reinterpret_cast<const int4 *>(a.cell_entries + i)[1];  // c2, c3, t1 local, t2 local
       const int e = h.z / ITSU_CELL_LAYERS, layer = h.z % ITSU_CELL_LAYERS;
       const int32_t *lo = a.layer_off + e * ITSU_LAYERS;
-      const itsu_tracklet t1 = a.tracklets[h.x];
-      const itsu_tracklet t2 = a.tracklets[a.trk_seg[e * ITSU_TRACKLET_LAYERS + layer + 1] + g.w];
+      const itsu_tracklet t1 = load_tracklet(a, h.x);
+      const itsu_tracklet t2 = load_tracklet(a, a.trk_seg[e * ITSU_TRACKLET_LAYERS + layer + 1] + g.w);
       const float4 c1 = a.xyzr[lo[layer] + h.w];
       const float4 c2 = a.xyzr[lo[layer + 1] + g.x];
       const float4 c3 = a.xyzr[lo[layer + 2] + g.y];
@@ -1807,7 +1913,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_cells_crowded(Arena a)
     int64_t out = first;
     for (int b = 0; b < s.n_out; ++b) {
       const int32_t j = s.j0 + b;
-      const itsu_tracklet t2 = a.tracklets[j];
+      const itsu_tracklet t2 = load_tracklet(a, j);
       float3 normal;
       float curvature;
       if (cell_precut(s.layer, s.t1_tan_lambda, s.t1_phi, t2.tan_lambda, t2.phi, s.c1, s.vz) &&
@@ -2238,10 +2344,15 @@ void step_tracklet_segments(const Arena &a, const Launch &l)
   k_tracklet_segments<<<(a.n_events * ITSU_TRACKLET_LAYERS + kThreads) / kThreads, kThreads, 0, l.stream>>>(a);
 }
 
+void launch_cells_range(const Arena &a, const Launch &l, int32_t e0, int32_t e1)
+{
+  k_cells_count<<<l.num_sms * kCellBlocks, kCellThreads, 0, l.stream>>>(a, e0, e1);
+}
+
 void step_cells_count(const Arena &a, const Launch &l)
 {
   if (l.n_groups == 0 && whole_warps(a, l)) {
-    k_cells_count<<<fixed_grid(l), l.block, 0, l.stream>>>(a, 0, 0);
+    launch_cells_range(a, l, 0, 0);
   }
 }
 
@@ -2257,7 +2368,7 @@ void step_write_count_groups(const Arena &a, const Launch &l)
   for (int g = 0; g < l.n_groups; ++g) {
     launch_write_range(a, l, l.groups[g], l.groups[g + 1]);
     const int32_t e0 = g * l.group_events, e1 = std::min(a.n_events, (g + 1) * l.group_events);
-    k_cells_count<<<fixed_grid(l), l.block, 0, l.stream>>>(a, e0, e1);
+    launch_cells_range(a, l, e0, e1);
   }
 }
 
