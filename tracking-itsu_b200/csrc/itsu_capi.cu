@@ -89,14 +89,14 @@ struct itsu_context {
   // event class
   float2 *seg_rrange = nullptr;
   int32_t *seg_regular = nullptr;
-  int32_t *layer_off = nullptr, *index_tables = nullptr, *trk_seg = nullptr, *cell_seg = nullptr, *road_seg = nullptr;
+  int32_t *layer_off = nullptr, *index_tables = nullptr, *trk_seg = nullptr, *cell_seg = nullptr, *cell_seg_count = nullptr, *road_seg = nullptr;
   int4 *cell_seginfo = nullptr;
   float *vtx = nullptr;
   // tracklet class
   itsu_tracklet *tracklets = nullptr;
   uint32_t *trk_key = nullptr;  // (tanL, phi) of each tracklet in fixed point, beside the records
-  int32_t *trk_seg_id = nullptr, *cell_count = nullptr, *cell_off = nullptr, *cell_lookup = nullptr, *cell_crowded = nullptr;
-  unsigned long long *cell_mask = nullptr;
+  int32_t *trk_seg_id = nullptr, *cell_lookup = nullptr, *cell_span_count = nullptr, *cell_span_off = nullptr;
+  int2 *cell_span = nullptr;
   // cell class
   itsu_cell *cells = nullptr;
   itsu::CellEntry *cell_entries = nullptr;
@@ -338,11 +338,11 @@ Arena arena_of(const itsu_context *ctx)
   a.tracklets = ctx->tracklets;
   a.trk_key = ctx->trk_key;
   a.trk_seg_id = ctx->trk_seg_id;
-  a.cell_count = ctx->cell_count;
-  a.cell_mask = ctx->cell_mask;
-  a.cell_off = ctx->cell_off;
+  a.cell_span = ctx->cell_span;
+  a.cell_span_count = ctx->cell_span_count;
+  a.cell_span_off = ctx->cell_span_off;
+  a.cell_seg_count = ctx->cell_seg_count;
   a.cell_lookup = ctx->cell_lookup;
-  a.cell_crowded = ctx->cell_crowded;
   a.cell_seg = ctx->cell_seg;
   a.cells = ctx->cells;
   a.cell_seg_id = ctx->cell_seg_id;
@@ -426,6 +426,7 @@ itsu_status ensure_clusters(itsu_context *ctx, int64_t n_clusters, int32_t n_eve
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_seg, (int64_t)cap * ITSU_TRACKLET_LAYERS + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_seginfo, (int64_t)cap * ITSU_TRACKLET_LAYERS * 2));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_seg, (int64_t)cap * ITSU_CELL_LAYERS + 1));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->cell_seg_count, (int64_t)cap * ITSU_CELL_LAYERS));
     ITSU_CUDA(ctx, alloc(ctx, ctx->road_seg, (int64_t)cap + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->seg_rrange, (int64_t)cap * ITSU_LAYERS));
     ITSU_CUDA(ctx, alloc(ctx, ctx->seg_regular, (int64_t)cap * ITSU_LAYERS));
@@ -445,25 +446,24 @@ itsu_status ensure_tracklets(itsu_context *ctx, int64_t need)
     ITSU_CUDA(ctx, alloc(ctx, ctx->tracklets, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_key, cap + 4));  // read in aligned groups of four
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_seg_id, cap));
-    ITSU_CUDA(ctx, alloc(ctx, ctx->cell_count, cap + 1));
-    ITSU_CUDA(ctx, alloc(ctx, ctx->cell_mask, cap));
-    ITSU_CUDA(ctx, alloc(ctx, ctx->cell_off, cap + 1));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->cell_span, cap / 32 + 1));  // spans of 32 tracklets or more
+    ITSU_CUDA(ctx, alloc(ctx, ctx->cell_span_count, cap / 32 + 1));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->cell_span_off, cap / 32 + 2));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_lookup, cap));
-    ITSU_CUDA(ctx, alloc(ctx, ctx->cell_crowded, cap));
     ctx->cap_tracklets = cap;
     ctx->generation++;
   }
   return ensure_partials(ctx);
 }
 
-// Entries the cell count pass may reserve beyond the cells it finds: every warp of its grid can
-// leave part of one chunk unused. Sized for the larger of the current launch shape and the
-// largest shape the autotuner tries (16 blocks of 512 threads per SM).
-int64_t cell_entry_slack(const itsu_context *ctx)
+// Entry scratch for an arena of these capacities: the cell count pass reserves a place per pair that
+// its precut lets through (0.54 per tracklet in central events, up to one in pile-up frames) and
+// reports what did not fit. A fixed arena cannot grow it, so it gets room for twice its tracklets,
+// the pairs of crowded events' cells and every short run.
+int64_t cell_places(const itsu_context *ctx)
 {
-  const Tune t = current_tune(ctx);
-  const int64_t warps = std::max<int64_t>((int64_t)t.blocks_per_sm * (t.block / 32), 16 * (512 / 32));
-  return (int64_t)ctx->num_sms * warps * itsu::kCellChunk;
+  const bool fixed = (ctx->flags & ITSU_FLAG_NO_GROW) != 0;
+  return fixed ? 2 * ctx->cap_tracklets + 8 * ctx->cap_cells + (int64_t(5) << 19) : ctx->cap_tracklets / 2 + ctx->cap_cells + (1 << 14);
 }
 
 itsu_status ensure_cell_entries(itsu_context *ctx, int64_t need)
@@ -480,7 +480,8 @@ itsu_status ensure_cell_entries(itsu_context *ctx, int64_t need)
   return ITSU_OK;
 }
 
-itsu_status ensure_cells(itsu_context *ctx, int64_t need)
+// The cell stage's outputs. Not its scratch: after the count pass, growing it would lose the entries.
+itsu_status ensure_cell_outputs(itsu_context *ctx, int64_t need)
 {
   if (need > ctx->cap_cells) {
     itsu_status st = growth_allowed(ctx, "cells", need, ctx->cap_cells);
@@ -498,9 +499,14 @@ itsu_status ensure_cells(itsu_context *ctx, int64_t need)
     ctx->cap_cells = cap;
     ctx->generation++;
   }
-  itsu_status st = ensure_cell_entries(ctx, ctx->cap_cells + cell_entry_slack(ctx));
-  if (st != ITSU_OK) return st;
   return ensure_partials(ctx);
+}
+
+itsu_status ensure_cells(itsu_context *ctx, int64_t need)
+{
+  itsu_status st = ensure_cell_outputs(ctx, need);
+  if (st != ITSU_OK) return st;
+  return ensure_cell_entries(ctx, cell_places(ctx));
 }
 
 itsu_status ensure_neighbours(itsu_context *ctx, int64_t need)
@@ -696,7 +702,7 @@ itsu_status run_all(itsu_context *ctx)
       if ((st = ensure_roads(ctx, (int64_t)(ctx->cap_roads * f))) != ITSU_OK) return st;
     }
     if ((s.flags & itsu::kFlagCapCells) && (st = ensure_cells(ctx, s.total[1])) != ITSU_OK) return st;
-    if ((s.flags & itsu::kFlagCapScratch) && (st = ensure_cell_entries(ctx, s.cell_entries + cell_entry_slack(ctx))) != ITSU_OK) {
+    if ((s.flags & itsu::kFlagCapScratch) && (st = ensure_cell_entries(ctx, s.cell_entries)) != ITSU_OK) {
       return st;
     }
     if ((s.flags & itsu::kFlagCapNeighbours) && (st = ensure_neighbours(ctx, s.total[2])) != ITSU_OK) return st;
@@ -712,10 +718,11 @@ itsu_status stage_count_then_write(itsu_context *ctx, void (*count)(const Arena 
   itsu_status st;
   for (int attempt = 0;; ++attempt) {
     if ((st = clear_flags(ctx)) != ITSU_OK) return st;
-    // the entry reservation, the crowded lists and the tile sums of the tracklet and cell scans
-    // (the count passes add to them) start empty for every count, also a retry
-    ITSU_CUDA(ctx, cudaMemsetAsync(&ctx->d_status->cell_entries, 0, 3 * sizeof(int64_t), ctx->stream));
+    // the entry reservation, the crowded list, the tile sums of the tracklet and cell scans and the
+    // segments' cell counts (the count passes add to them) start empty for every count, also a retry
+    ITSU_CUDA(ctx, cudaMemsetAsync(&ctx->d_status->cell_entries, 0, 4 * sizeof(int64_t), ctx->stream));
     ITSU_CUDA(ctx, cudaMemsetAsync(ctx->scan_partials, 0, sizeof(int64_t) * ctx->cap_partials, ctx->stream));
+    ITSU_CUDA(ctx, cudaMemsetAsync(ctx->cell_seg_count, 0, sizeof(int32_t) * ITSU_CELL_LAYERS * ctx->n_events, ctx->stream));
     count(arena_of(ctx), launch_of(ctx));
     if ((st = check_launch(ctx)) != ITSU_OK) return st;
     if ((st = sync_status(ctx)) != ITSU_OK) return st;
@@ -723,7 +730,7 @@ itsu_status stage_count_then_write(itsu_context *ctx, void (*count)(const Arena 
     // grow it and count again
     if (!(ctx->h_status->flags & itsu::kFlagCapScratch) || (ctx->h_status->flags & itsu::kFlagCountOverflow)) break;
     if (attempt == 4) return fail(ctx, ITSU_ERR_CAPACITY, "cell entry scratch growth did not converge");
-    if ((st = ensure_cell_entries(ctx, ctx->h_status->cell_entries + cell_entry_slack(ctx))) != ITSU_OK) return st;
+    if ((st = ensure_cell_entries(ctx, ctx->h_status->cell_entries)) != ITSU_OK) return st;
   }
   const DevStatus &s = *ctx->h_status;
   if (s.flags & itsu::kFlagCountOverflow) return count_overflow(ctx);
@@ -945,9 +952,9 @@ void itsu_context_destroy(itsu_context *ctx)
   release(ctx->raw); release(ctx->raw_in); release(ctx->raw_track); release(ctx->sorted); release(ctx->tmp); release(ctx->xyzr); release(ctx->phi);
   release(ctx->trk_count); release(ctx->trk_off); release(ctx->trk_range); release(ctx->trk_lookup); release(ctx->zs); release(ctx->clu_seg); release(ctx->clu_aux); release(ctx->clu_crowded); release(ctx->trk_slots);
   release(ctx->seg_rrange); release(ctx->seg_regular); release(ctx->raw_off);
-  release(ctx->layer_off); release(ctx->index_tables); release(ctx->trk_seg); release(ctx->cell_seginfo); release(ctx->cell_seg);
+  release(ctx->layer_off); release(ctx->index_tables); release(ctx->trk_seg); release(ctx->cell_seginfo); release(ctx->cell_seg); release(ctx->cell_seg_count);
   release(ctx->road_seg); release(ctx->vtx);
-  release(ctx->tracklets); release(ctx->trk_key); release(ctx->trk_seg_id); release(ctx->cell_count); release(ctx->cell_mask); release(ctx->cell_off); release(ctx->cell_lookup); release(ctx->cell_crowded);
+  release(ctx->tracklets); release(ctx->trk_key); release(ctx->trk_seg_id); release(ctx->cell_span); release(ctx->cell_span_count); release(ctx->cell_span_off); release(ctx->cell_lookup);
   release(ctx->cells); release(ctx->cell_entries); release(ctx->cell_dca); release(ctx->cell_seg_id); release(ctx->nb_count); release(ctx->nb_off); release(ctx->nb_fill);
   release(ctx->nb_mask);
   release(ctx->road_count); release(ctx->road_off); release(ctx->paths);
@@ -1030,7 +1037,7 @@ itsu_status itsu_compute_layer_cells(itsu_context *ctx)
   if ((st = require_stage(ctx, kTracklets, "itsu_compute_layer_cells")) != ITSU_OK) return st;
   ITSU_CUDA(ctx, cudaSetDevice(ctx->device));
   if ((st = ensure_cells(ctx, 1)) != ITSU_OK) return st;
-  if ((st = stage_count_then_write(ctx, itsu::launch_cells_count, itsu::launch_cells_write, itsu::kCells, ensure_cells)) != ITSU_OK) {
+  if ((st = stage_count_then_write(ctx, itsu::launch_cells_count, itsu::launch_cells_write, itsu::kCells, ensure_cell_outputs)) != ITSU_OK) {
     return st;
   }
   ctx->stage = kCells;
@@ -1689,7 +1696,7 @@ itsu_status run_host_streamed(itsu_context *ctx, const HostClusters &clusters, c
     const DevStatus &s = ctx->h_chunk_status[fail_chunk];
     itsu_status g = ITSU_OK;
     if (g == ITSU_OK && (s.flags & itsu::kFlagCapTracklets)) g = ensure_tracklets(x, s.total[itsu::kTracklets]);
-    if (g == ITSU_OK && (s.flags & itsu::kFlagCapScratch)) g = ensure_cell_entries(x, s.cell_entries + cell_entry_slack(x));
+    if (g == ITSU_OK && (s.flags & itsu::kFlagCapScratch)) g = ensure_cell_entries(x, s.cell_entries);
     if (g == ITSU_OK && (s.flags & itsu::kFlagCapCells)) g = ensure_cells(x, s.total[itsu::kCells]);
     if (g == ITSU_OK && (s.flags & itsu::kFlagCapNeighbours)) g = ensure_neighbours(x, s.total[itsu::kNeighbours]);
     if (g == ITSU_OK && (s.flags & itsu::kFlagCapRoads)) g = ensure_roads(x, s.total[itsu::kRoads]);

@@ -7,7 +7,7 @@
 //   index_tables       E*6 tables of 401 ints (table of layer L+1 at (6e+L)*401)
 //   trk_count/trk_off  tracklets per inner cluster and their exclusive scan (NC+1)
 //   trk_seg[E*6+1]     tracklet segment (e, L) = [trk_seg[6e+L], trk_seg[6e+L+1])
-//   cell_count/off     cells per first tracklet and their scan (T+1); cell_seg[E*5+1]
+//   cell_span_count/off  cells per span of first tracklets and their scan; cell_seg[E*5+1]
 //   nb_count/off       neighbours per next-layer cell and their scan (C+1): CSR over cells
 //   road_count/off     roads per root cell and their scan (C+1); road_seg[E+1]
 #pragma once
@@ -40,7 +40,6 @@ constexpr int kTrackletSlotsPerCluster = 48;  // outer clusters the tracklet cou
 // Any of these stops every later kernel of the run (they check the mask first).
 constexpr int32_t kCapacityMask = kFlagCapTracklets | kFlagCapCells | kFlagCapNeighbours | kFlagCapRoads |
                                   kFlagCountOverflow | kFlagCapScratch | kFlagLaunchShape | kFlagTimeout;
-constexpr int kCellChunk = 64;  // cell entries a warp of the cell count pass reserves at a time
 
 // Totals and requirements of a run, written by the device.
 struct DevStatus {
@@ -49,32 +48,31 @@ struct DevStatus {
   int32_t invalid_event;  // first event with a malformed vertex, INT32_MAX if none
   int32_t pad_;
   int64_t total[4];       // tracklets, cells, neighbours, roads
-  int64_t cell_entries;   // cell entries reserved by the cell count pass (may exceed the scratch)
-  int64_t crowded;        // tracklets the cell count pass listed in cell_crowded
+  int64_t cell_entries;   // places reserved by the cell count pass (may exceed the scratch)
+  int64_t cell_spans;     // spans of first tracklets of the cell count pass
   int64_t trk_crowded;    // inner clusters the tracklet count pass listed in clu_crowded
+  int64_t cell_next;      // spans handed out by the cell count pass's counter
 };
-// The three list counters are reset together before each count pass (one 24-byte memset).
-static_assert(offsetof(DevStatus, crowded) == offsetof(DevStatus, cell_entries) + 8 &&
-                  offsetof(DevStatus, trk_crowded) == offsetof(DevStatus, cell_entries) + 16,
+// The four counters are reset together before each count pass (one 32-byte memset).
+static_assert(offsetof(DevStatus, cell_spans) == offsetof(DevStatus, cell_entries) + 8 &&
+                  offsetof(DevStatus, trk_crowded) == offsetof(DevStatus, cell_entries) + 16 &&
+                  offsetof(DevStatus, cell_next) == offsetof(DevStatus, cell_entries) + 24,
               "status counters");
 
-// A cell as the count pass finds it: its first tracklet (flat) and the outgoing-tracklet bit it
-// came from, and everything the cell record needs: its segment (5 e + L), its three clusters
-// (local to layers L, L+1, L+2), its two tracklets (local to tracklet layers L and L+1), and what
-// its geometry gave. The write pass scatters each entry whose bit survived to cell_off[t1] + (the
-// rank of its bit among the tracklet's set bits) with no other gather; t1 < 0 marks an unused
-// slot. The learned prefilter scores entries in place (the DCA, one of its features, goes to a
-// separate array in that form only).
-struct __align__(16) CellEntry {
-  int32_t t1;
-  int32_t bit;
-  int32_t seg;
-  int32_t c1;
-  int32_t c2, c3;
+// A cell as the count pass finds it: the cell record (its three clusters, local to layers L, L+1,
+// L+2, its two tracklets, local to tracklet layers L and L+1, normal and curvature) with its
+// segment (5 e + L) in the level's place. The write pass copies each entry to its scanned place with
+// no other gather. The learned prefilter scores entries in place (the DCA, one of its features, goes
+// to a separate array in that form only) and marks those it drops.
+struct __align__(8) CellEntry {
+  int32_t c1, c2, c3;
   int32_t t1_local, t2_local;
   float nx, ny, nz, curvature;
+  int32_t segment;
 };
-static_assert(sizeof(CellEntry) == 48, "cell entry layout");
+static_assert(sizeof(CellEntry) == 40 && sizeof(CellEntry) == sizeof(itsu_cell), "cell entry layout");
+constexpr int32_t kEntryUnscored = 1 << 30;  // flag on segment: the prefilter keeps the entry as it is
+constexpr int32_t kEntryDropped = -1;        // in place of segment: not a cell
 
 enum TotalIndex { kTracklets = 0, kCells = 1, kNeighbours = 2, kRoads = 3 };
 
@@ -120,11 +118,10 @@ struct Arena {
   int4 *cell_seginfo;  // per tracklet segment, two records: {first cluster of L (-1: no cells), of L+1, of L+2,
                        // first tracklet of L}, {first tracklet of L+1, vertex x, y, z (float bits)}
   // cells
-  int32_t *cell_count;
-  unsigned long long *cell_mask;  // per first tracklet: which outgoing tracklets make cells
-  int32_t *cell_off;
+  int2 *cell_span;  // per span of first tracklets: its first cell entry and their number
+  int32_t *cell_span_count, *cell_span_off;  // per span: its cells (entries the prefilter kept), and their scan
+  int32_t *cell_seg_count;    // per segment: its cells
   int32_t *cell_lookup;
-  int32_t *cell_crowded;  // tracklets whose outer cluster has more than 64 outgoing tracklets
   int32_t *cell_seg;
   itsu_cell *cells;
   int32_t *cell_seg_id;

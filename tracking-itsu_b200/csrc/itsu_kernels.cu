@@ -9,10 +9,10 @@
 //   tracklets    count: one thread per inner cluster walking the reference's bin window,
 //                z-pruned (Tracker.cxx:45-117); tail: lookup, owners, crowded clusters; write:
 //                a map over tracklets (slope and correctly rounded azimuth)
-//   cells        count: a warp per 32 first tracklets, their outgoing-tracklet pairs flattened
-//                over the lanes, exact cuts, one 32-byte entry per found cell (Tracker.cxx:
-//                120-235); learned form: the prefilter scores the entries; write: the entries
-//                scattered to their scanned slots, then the lookup table
+//   cells        count: the tracklet pairs inside a fixed-point window queued, then the exact cuts
+//                and the geometry, a lane per queued pair, one 40-byte entry per found cell
+//                (Tracker.cxx:120-235); learned form: the prefilter scores the entries; write: the
+//                entries copied to their scanned places, with the lookup table
 //   neighbours   one thread per cell walking the next-layer cells of its outer tracklet; rows
 //                keyed by the next-layer cell, sorted ascending (Tracker.cxx:417-474)
 //   levels       layer-ordered longest-chain DP plus the number of level-decreasing chains
@@ -75,7 +75,8 @@ __global__ void k_status_init(Arena a)
     s->total[k] = 0;
   }
   s->cell_entries = 0;
-  s->crowded = 0;
+  s->cell_spans = 0;
+  s->cell_next = 0;
   s->trk_crowded = 0;
 }
 
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int32_t *__re
 
 int scan_grid(const Launch &l) { return l.num_sms * 4; }
 
-// The four scans of a run: tracklets per cluster, cells per tracklet, neighbours per cell, roads
+// The four scans of a run: tracklets per cluster, cells per span of tracklets, neighbours per cell, roads
 // per cell. The neighbour and road scans are three kernels (tile sums, scan of tile sums, tile
 // scans); the tracklet and cell scans are two, their tile sums added up by the count passes.
 struct ScanArgs {
@@ -252,7 +253,7 @@ ScanArgs scan_args(const Arena &a)
 {
   switch (kWhich) {
   case 0: return ScanArgs{a.trk_count, a.trk_off, nullptr, a.n_clusters, &a.status->total[kTracklets]};
-  case 1: return ScanArgs{a.cell_count, a.cell_off, &a.status->total[kTracklets], 0, &a.status->total[kCells]};
+  case 1: return ScanArgs{a.cell_span_count, a.cell_span_off, &a.status->cell_spans, 0, &a.status->total[kCells]};
   case 2: return ScanArgs{a.nb_count, a.nb_off, &a.status->total[kCells], 0, &a.status->total[kNeighbours]};
   default: return ScanArgs{a.road_count, a.road_off, &a.status->total[kCells], 0, &a.status->total[kRoads]};
   }
@@ -1425,6 +1426,10 @@ __global__ void k_tracklet_segments(Arena a)
       a.scan_partials[t] = 0;
     }
   }
+  // and so do the segments' cell counts
+  for (int64_t s = global_thread(); s < (int64_t)a.n_events * ITSU_CELL_LAYERS; s += grid_threads()) {
+    a.cell_seg_count[s] = 0;
+  }
   const int nseg = a.n_events * ITSU_TRACKLET_LAYERS;
   for (int s = (int)global_thread(); s <= nseg; s += grid_threads()) {
     if (s == nseg) {
@@ -1454,342 +1459,277 @@ __global__ void k_tracklet_segments(Arena a)
 // ------------------------------------------------------------------------------------------
 // (c) cells: TrackerTraits<false>::computeLayerCells (Tracker.cxx:120-235)
 
-// Per-lane state of the warp-parallel cell stage: lane l owns first tracklet k = base + l.
+// Count pass. A warp takes a span of 32, 64 or 128 consecutive first tracklets:
+//  1. Precut, a lane per first tracklet, 32 at a time: one window per lane (cell_window) against the
+//     outgoing tracklets' 4-byte keys, four keys per 16-byte load, about three instructions a pair.
+//     The window is a superset of the exact cheap cuts by the keys' resolution; what it lets through
+//     (about one pair in eighteen) goes to the warp's queue, in the reference's order (first
+//     tracklet, then outgoing tracklet).
+//  2. Geometry, a lane per queued pair, in rounds of 32 in the queue's order (a round per group of 32
+//     first tracklets would hold 17 pairs on average): the exact cheap cuts (Tracker.cxx:161-173) on
+//     the records, then the circle geometry. The passing pairs become the span's cell entries, in
+//     order, from the place reserved for the span on (room for all its pairs).
+// The cells are counted per span (whose scan places them) and per segment (cell_seg): there is no
+// mask, count or offset per tracklet, and the write pass copies entries in order.
+// Bound by the gathers (half of the issue slots and of the L1 data pipe busy). Spans of 128 leave
+// half a round in five empty, but only pay where every warp has many of them. The grid is one wave of
+// resident blocks (9 of 128 threads at 56 registers per SM: a second, part-empty wave would cost
+// almost as much again). 1.13 ms per 128 central events (1.15 at 10 blocks and 48 registers, 1.21 at
+// 8); as two kernels with the pairs listed in global memory 0.75 + 0.75 ms; with masks, counts and
+// lookup entries per first tracklet 1.34 ms, and 0.34 instead of 0.17 ms to place the cells.
+constexpr int kCellThreads = 128;
+constexpr int kCellBlocks = 9;  // resident blocks per SM
+constexpr int kMaxSpan = 128;
+constexpr int kCellQueue = 512;  // queued pairs of a warp (a span of 128 has 68 on average, 250 behind the tracklet gate)
+constexpr int kCellRing = 64;    // of a span whose pairs the queue cannot hold
+static_assert(kMaxSpan <= 128 && kMaxMaskedOut <= 64, "a queue item is 7 bits of span and 6 of outgoing tracklets");
+
+// First tracklets in a span, of a run of n (there are 4736 warps: from 2^21 on each has 3 spans of 128 or more).
+__device__ __forceinline__ uint32_t span_of(uint32_t n) { return n >= (1u << 22) ? 128 : (n >= (1u << 20) ? 64 : 32); }
+
+struct CellWarp {
+  int2 state[kMaxSpan];        // first outgoing tracklet; segment (kCrowded: more than kMaxMaskedOut outgoing tracklets)
+  union {
+    uint16_t queue[kCellQueue];  // (first tracklet in the span) | (outgoing tracklet) << 7
+    uint32_t ring[kCellRing];    // the same, for any number of outgoing tracklets
+  };
+};
+constexpr int kCrowded = 1 << 30;
+
+// A first tracklet's segment, precut window and outgoing tracklets [j0, j0 + n_out) (none: no cell
+// starts with it).
 struct CellLane {
-  int64_t k;
-  int layer, e;
-  float t1_tan_lambda, t1_phi;
-  float4 c1, c2;
-  float vx, vy, vz;
-  int32_t j0, n_out;     // the outgoing tracklets of the tracklet's outer cluster: [j0, j0 + n_out)
-  int32_t c3_base;       // first cluster of layer L + 2
-  int32_t t1_local, t1_first, t1_second, t2_base;  // tracklet index in its layer, its clusters, first tracklet of layer L + 1
+  CellWindow w;
+  int sid, j0, n_out;
 };
 
-__device__ __forceinline__ CellLane cell_lane(const Arena &a, int64_t k, int64_t n)
+__device__ __forceinline__ CellLane cell_lane(const Arena &a, uint32_t k)
 {
   CellLane s;
-  s.k = k;
-  s.n_out = 0;
-  s.layer = ITSU_CELL_LAYERS;
-  s.e = 0;
-  if (k >= n) {
-    return s;
-  }
+  s.j0 = s.n_out = 0;
   // both loads first: neither depends on the other
-  const int sid = a.trk_seg_id[k];
+  s.sid = a.trk_seg_id[k];
   const itsu_tracklet t1 = load_tracklet(a, k);
-  s.e = sid / ITSU_TRACKLET_LAYERS;
-  s.layer = sid % ITSU_TRACKLET_LAYERS;
-  if (s.layer >= ITSU_CELL_LAYERS) {
-    s.layer = ITSU_CELL_LAYERS;
+  const int layer = s.sid % ITSU_TRACKLET_LAYERS;
+  if (layer >= ITSU_CELL_LAYERS) {
     return s;
   }
-  const int4 A = a.cell_seginfo[2 * sid], B = a.cell_seginfo[2 * sid + 1];
+  const int4 A = a.cell_seginfo[2 * s.sid];
   if (A.x < 0) {
-    s.layer = ITSU_CELL_LAYERS;
-    return s;
+    return s;  // the cell layer does not run
   }
-  s.t1_tan_lambda = t1.tan_lambda;
-  s.t1_phi = t1.phi;
-  s.t1_first = t1.first_cluster;
-  s.t1_second = t1.second_cluster;
-  s.c1 = a.xyzr[A.x + t1.first_cluster];
-  const int64_t c2i = A.y + t1.second_cluster;
-  s.c2 = a.xyzr[c2i];
-  s.j0 = a.trk_off[c2i];
-  s.n_out = a.trk_off[c2i + 1] - s.j0;
-  s.vx = __int_as_float(B.y);
-  s.vy = __int_as_float(B.z);
-  s.vz = __int_as_float(B.w);
-  s.c3_base = A.z;
-  s.t1_local = (int32_t)(k - A.w);
-  s.t2_base = B.x;
+  const int2 out = a.trk_range[A.y + t1.second_cluster];  // the outer cluster's first outgoing tracklet and their number
+  const float2 c1 = reinterpret_cast<const float2 *>(a.xyzr + A.x + t1.first_cluster)[1];  // z, r
+  s.w = cell_window(t1.tan_lambda, t1.phi, c1.x, c1.y, __int_as_float(a.cell_seginfo[2 * s.sid + 1].w), kC.cell_max_dz[layer]);
+  s.j0 = out.x;
+  s.n_out = s.w.empty ? 0 : out.y;
   return s;
 }
 
-__device__ __forceinline__ void write_cell(const Arena &a, int64_t out, const CellLane &s, const itsu_tracklet &t2, int32_t j,
-                                           float3 normal, float curvature)
+// Which of a lane's outgoing tracklets (1 to kMaxMaskedOut) pass its window. Keys in aligned groups of
+// four (the array has room for the last group's overrun): those before j0 fall off by the shift,
+// those past the end by the last mask.
+__device__ __forceinline__ unsigned long long cell_precut_mask(const Arena &a, const CellLane &s)
 {
-  itsu_cell cell;
-  cell.first_cluster = s.t1_first;
-  cell.second_cluster = t2.first_cluster;
-  cell.third_cluster = t2.second_cluster;
-  cell.first_tracklet = s.t1_local;
-  cell.second_tracklet = j - s.t2_base;
-  cell.nx = normal.x;
-  cell.ny = normal.y;
-  cell.nz = normal.z;
-  cell.curvature = curvature;
-  cell.level = 1;
-  a.cells[out] = cell;
-  a.cell_seg_id[out] = s.e * ITSU_CELL_LAYERS + s.layer;
-}
-
-// Count pass: for each first tracklet, a mask of which of its (<= 64) outgoing tracklets make a
-// cell, and their number. A warp takes a span of 32, 64 or 128 consecutive first tracklets:
-//  1. Precut, a lane per first tracklet, 32 at a time: one unsigned window per lane (cell_window)
-//     against the outgoing tracklets' 4-byte keys, four keys per 16-byte load. About six
-//     instructions a pair; the window is a superset of the exact cheap cuts by the keys'
-//     resolution, and what it lets through (about one pair in eighteen) goes to the warp's queue.
-//  2. Geometry, a lane per queued pair, in rounds of 32 from the queue, so that the rounds are full
-//     (a round per group of 32 first tracklets held 17 pairs on average): the exact cheap cuts
-//     (Tracker.cxx:161-173) on the records, then the circle geometry. Each passing pair becomes a
-//     cell entry (its tracklets, normal, curvature) in the warp's current chunk of the entry
-//     scratch and a bit in its first tracklet's mask, so the write pass needs no geometry.
-//  3. The span's masks, counts and reset lookup entries in coalesced stores.
-// Spans longer than 32 only pay where every warp has many of them; short runs take 32 so that
-// more warps share the work. The grid is one wave of resident blocks (8 of 128 threads at 64
-// registers per SM: blocks beyond that would run as a second, mostly empty wave). Bound by the
-// latency of the gathers (51% of issue slots, 53% of the L1 data pipe): 1.34 ms per 128 central
-// events, 1.78 ms with the cuts evaluated pair by pair in binary32 and a round per 32 tracklets.
-//
-// Runs over the first tracklets of events [e0, e1), or of all events when e1 is 0. A span lies in
-// one scan tile; one that straddles the range's ends has its lanes outside the range idle.
-constexpr int kCellThreads = 128;
-constexpr int kCellBlocks = 8;  // resident blocks per SM
-constexpr int kCellGroups = 4;  // groups of 32 first tracklets in the longest span
-constexpr int kCellSpan = 32 * kCellGroups;
-constexpr int kCellQueue = 256;  // queued pairs of a warp (a group of 32 first tracklets has 17 on average)
-static_assert(kScanTile % kCellSpan == 0 && kCellSpan <= 128, "a span lies in one scan tile; its index has 7 bits in a queue item");
-
-struct CellWarp {
-  unsigned long long mask[kCellSpan];  // which outgoing tracklets make cells
-  int2 state[kCellSpan];  // first outgoing tracklet and segment (-1: a crowded outer cluster)
-  uint16_t queue[kCellQueue];  // (first tracklet in the span) | (outgoing tracklet) << 7
-};
-
-// Cells of first tracklet k whose outer cluster has more than kMaxMaskedOut outgoing tracklets, in order on one lane.
-__device__ __forceinline__ int crowded_cells(const Arena &a, int64_t k, int64_t n)
-{
-  const CellLane s = cell_lane(a, k, n);
-  int count = 0;
-  for (int b = 0; b < s.n_out; ++b) {
-    const itsu_tracklet t2 = load_tracklet(a, s.j0 + b);
-    float3 normal;
-    float curvature;
-    count += cell_precut(s.layer, s.t1_tan_lambda, s.t1_phi, t2.tan_lambda, t2.phi, s.c1, s.vz) &&
-             cell_geometry(s.layer, s.c1, s.c2, a.xyzr[s.c3_base + t2.second_cluster], s.vx, s.vy, normal, curvature);
-  }
-  return count;
-}
-
-// The outgoing tracklets of first tracklet k that its window lets through, as a mask.
-__device__ __forceinline__ unsigned long long cell_precut_mask(const Arena &a, uint32_t k, int2 &state)
-{
-  // both loads first: neither depends on the other
-  const int sid = a.trk_seg_id[k];
-  const itsu_tracklet t1 = load_tracklet(a, k);
-  const int layer = sid % ITSU_TRACKLET_LAYERS;
-  state = make_int2(0, sid);
-  if (layer >= ITSU_CELL_LAYERS) {
-    return 0ull;
-  }
-  const int4 A = a.cell_seginfo[2 * sid];
-  if (A.x < 0) {
-    return 0ull;  // the cell layer does not run
-  }
-  const int2 out = a.trk_range[A.y + t1.second_cluster];  // the outer cluster's first outgoing tracklet and their number
-  const int j0 = out.x, n_out = out.y;
-  if (n_out > kMaxMaskedOut) {
-    state.y = -1;  // counted with the span's results
-    return 0ull;
-  }
-  state.x = j0;
-  const float2 c1 = reinterpret_cast<const float2 *>(a.xyzr + A.x + t1.first_cluster)[1];  // z, r
-  const CellWindow w = cell_window(t1.tan_lambda, t1.phi, c1.x, c1.y, __int_as_float(a.cell_seginfo[2 * sid + 1].w), kC.cell_max_dz[layer]);
-  if (w.empty || n_out <= 0) {
-    return 0ull;
-  }
-  // keys in aligned groups of four (the array has room for the last group's overrun): those before
-  // j0 fall off by the shift, those past the end by the last mask
-  const int skip = j0 & 3;
-  const uint4 *keys = reinterpret_cast<const uint4 *>(a.trk_key + (j0 - skip));
+  const int skip = s.j0 & 3;
+  const uint4 *keys = reinterpret_cast<const uint4 *>(a.trk_key + (s.j0 - skip));
   auto four = [&](uint4 q) {
-    return (cell_window_pass(w, q.x) ? 1u : 0u) | (cell_window_pass(w, q.y) ? 2u : 0u) | (cell_window_pass(w, q.z) ? 4u : 0u) |
-           (cell_window_pass(w, q.w) ? 8u : 0u);
+    return (cell_window_pass(s.w, q.x) ? 1u : 0u) | (cell_window_pass(s.w, q.y) ? 2u : 0u) | (cell_window_pass(s.w, q.z) ? 4u : 0u) |
+           (cell_window_pass(s.w, q.w) ? 8u : 0u);
   };
-  unsigned long long window = four(keys[0]) >> skip;
+  unsigned long long mask = four(keys[0]) >> skip;
 #pragma unroll 2
-  for (int at = 4 - skip; at < n_out; at += 4) {
-    window |= (unsigned long long)four(*++keys) << at;
+  for (int at = 4 - skip; at < s.n_out; at += 4) {
+    mask |= (unsigned long long)four(*++keys) << at;
   }
-  return window & (~0ull >> (kMaxMaskedOut - n_out));
+  return mask & (~0ull >> (kMaxMaskedOut - s.n_out));
 }
 
-__global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena a, int32_t e0, int32_t e1)
+// Runs over the spans that end among the tracklets of events below e1 and not below e0 (last: to the
+// end of the run): every span is taken once its tracklets are written.
+__global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena a, int32_t e0, int32_t e1, bool last)
 {
   __shared__ CellWarp shared[kCellThreads / 32];
-  if (capacity_failed(a.status)) {
+  // not stopped by its own scratch flag: the reservations add up to what the run needs
+  if ((*(volatile const int32_t *)&a.status->flags & kCapacityMask & ~kFlagCapScratch) != 0) {
     return;
   }
   const int lane = threadIdx.x & 31;
   CellWarp &w = shared[threadIdx.x >> 5];
   // tracklet indices stay below 2^31 (the scan flags larger totals), a span's end below 2^32
   const uint32_t n = (uint32_t)a.status->total[kTracklets];
-  const uint32_t t0 = e1 > 0 ? (uint32_t)a.trk_seg[(int64_t)e0 * ITSU_TRACKLET_LAYERS] : 0u;
-  const uint32_t t1 = e1 > 0 ? (uint32_t)a.trk_seg[(int64_t)e1 * ITSU_TRACKLET_LAYERS] : n;
-  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  const uint32_t per_warp = (t1 - t0) / (32 * warps);  // groups of 32 a warp would take one by one
-  const int groups = per_warp >= 32 ? kCellGroups : (per_warp >= 8 ? 2 : 1);
-  const uint32_t span = 32 * groups;
-  int64_t chunk_pos = 0;  // this warp's reserved cell entries: the next one, and how many are left (warp-uniform)
-  int chunk_left = 0;
-  for (uint32_t base = (t0 & ~(span - 1)) + (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * span; base < t1; base += warps * span) {
-    int g = 0, queued = 0;
-    unsigned long long window = 0;  // this lane's pairs of group g - 1 not yet queued
-    for (;;) {
-      const unsigned pending = __ballot_sync(0xffffffffu, window != 0);
-      if (pending == 0 && g < groups) {
-        const int at = 32 * g + lane;
-        const uint32_t k = base + at;
-        int2 state = make_int2(0, 0);
-        if (k >= t0 && k < t1) {
-          window = cell_precut_mask(a, k, state);
+  const uint32_t span = span_of(n), spans = (n + span - 1) / span;
+  const uint32_t s0 = (uint32_t)a.trk_seg[(int64_t)e0 * ITSU_TRACKLET_LAYERS] / span;
+  const uint32_t s1 = last ? spans : (uint32_t)a.trk_seg[(int64_t)e1 * ITSU_TRACKLET_LAYERS] / span;
+  if (global_thread() == 0) {
+    a.status->cell_spans = spans;
+  }
+  // a whole run's warps take their next spans from a counter (the spans' work differs widely where
+  // most pairs pass, as behind the tracklet gate), asked for while the current one is worked on
+  const uint32_t warps = gridDim.x * (kCellThreads / 32);
+  const bool counter = s0 == 0 && last;
+  uint32_t s_next = 0;
+  for (uint32_t s = s0 + blockIdx.x * (kCellThreads / 32) + (threadIdx.x >> 5); s < s1; s = s_next) {
+    s_next = s + warps;
+    if (counter) {
+      if (lane == 0) {
+        s_next = warps + (uint32_t)atomicAdd(reinterpret_cast<unsigned long long *>(&a.status->cell_next), 1ull);
+      }
+      s_next = __shfl_sync(0xffffffffu, s_next, 0);
+    }
+    const uint32_t base = s * span;
+    int total = 0;
+    bool queued = true;  // the span's pairs are all in the queue
+    for (uint32_t g = 0; g < span; g += 32) {
+      const uint32_t at = g + lane, k = base + at;
+      CellLane p;
+      p.sid = p.j0 = p.n_out = 0;
+      if (k < n) {
+        a.cell_lookup[k] = ITSU_UNUSED_INDEX;  // the write pass fills it for tracklets with cells
+        p = cell_lane(a, k);
+      }
+      const bool crowded = p.n_out > kMaxMaskedOut;
+      w.state[at] = make_int2(p.j0, crowded ? p.sid | kCrowded : p.sid);
+      unsigned long long mask = 0ull;
+      int count = 0;
+      if (crowded) {
+        for (int q = 0; q < p.n_out; ++q) {
+          count += cell_window_pass(p.w, a.trk_key[p.j0 + q]);
         }
-        w.state[at] = state;
-        w.mask[at] = 0ull;
-        ++g;
-        // the group's pairs go to the queue together where they fit
-        int total;
-        const int first = queued + warp_exclusive_sum(__popcll(window), total);
-        if (queued + total <= kCellQueue) {
-          int to = first;
-          for (unsigned m = (unsigned)window; m != 0; m &= m - 1u) {
-            w.queue[to++] = (uint16_t)(at | (__ffs(m) - 1) << 7);
-          }
-          for (unsigned m = (unsigned)(window >> 32); m != 0; m &= m - 1u) {
-            w.queue[to++] = (uint16_t)(at | (__ffs(m) + 31) << 7);
-          }
-          queued += total;
-          window = 0;
+      } else if (p.n_out > 0) {
+        mask = cell_precut_mask(a, p);
+        count = __popcll(mask);
+      }
+      int group_total;
+      int to = total + warp_exclusive_sum(count, group_total);
+      total += group_total;
+      queued = queued && total <= kCellQueue && !__any_sync(0xffffffffu, crowded);
+      if (queued) {
+        for (unsigned m = (unsigned)mask; m != 0; m &= m - 1u) {
+          w.queue[to++] = (uint16_t)(at | (uint32_t)(__ffs(m) - 1) << 7);
         }
-        if (queued < 32 && g < groups) {
+        for (unsigned m = (unsigned)(mask >> 32); m != 0; m &= m - 1u) {
+          w.queue[to++] = (uint16_t)(at | (uint32_t)(__ffs(m) + 31) << 7);
+        }
+      }
+    }
+    int cells = 0;
+    unsigned long long first = 0;
+    if (total > 0) {
+      if (lane == 0) {
+        first = atomicAdd(reinterpret_cast<unsigned long long *>(&a.status->cell_entries), (unsigned long long)total);
+        if ((int64_t)first + total > a.cap_cell_entries) {
+          atomicOr(&a.status->flags, kFlagCapScratch);  // nothing after this pass runs
+        }
+      }
+      first = __shfl_sync(0xffffffffu, first, 0);
+    }
+    if (total > 0 && (int64_t)first + total <= a.cap_cell_entries) {
+      __syncwarp();
+      int head = 0, tail = queued ? total : 0;
+      uint32_t next = queued ? span : 0;  // not queued (a crowded outer cluster, or more pairs than the queue holds):
+      int next_out = 0;                   // the first tracklets' keys are walked again, 32 of one tracklet at a time
+      for (;;) {
+        if (next < span && tail - head < 32) {
+          const uint32_t k = base + next;
+          CellLane p;
+          p.j0 = p.n_out = 0;
+          if (k < n) {
+            p = cell_lane(a, k);
+          }
+          const int q = next_out + lane;
+          const bool listed = q < p.n_out && cell_window_pass(p.w, a.trk_key[p.j0 + q]);
+          const unsigned m = __ballot_sync(0xffffffffu, listed);
+          if (listed) {
+            w.ring[(tail + __popc(m & ((1u << lane) - 1u))) & (kCellRing - 1)] = next | (uint32_t)q << 7;
+          }
+          tail += __popc(m);
+          next_out += 32;
+          if (next_out >= p.n_out) {
+            next_out = 0;
+            ++next;
+          }
+          __syncwarp();
           continue;
         }
-      } else if (pending != 0 && queued < 32) {
-        // too many at once (a crowded region): one pair of every lane that has one
-        if (window != 0) {
-          const int b = __ffsll((long long)window) - 1;
-          window &= window - 1ull;
-          w.queue[queued + __popc(pending & ((1u << lane) - 1u))] = (uint16_t)(32 * (g - 1) + lane | b << 7);
-        }
-        queued += __popc(pending);
-      }
-      if (queued == 0) {
-        if (g == groups && __ballot_sync(0xffffffffu, window != 0) == 0) {
+        const int m = min(tail - head, 32);
+        if (m == 0) {
           break;
         }
-        continue;
-      }
-      __syncwarp();
-      // a round of the last 32 queued pairs (fewer at the span's end)
-      const int m = min(queued, 32);
-      queued -= m;
-      bool pass = false;
-      int b = 0, sid = 0;
-      uint32_t k = 0, j = 0;
-      itsu_tracklet f, s;
-      int4 A, B;
-      float3 normal;
-      float curvature, dca;
-      if (lane < m) {
-        const int item = w.queue[queued + lane];
-        const int at = item & (kCellSpan - 1);
-        b = item >> 7;
-        const int2 state = w.state[at];
-        sid = state.y;
-        k = base + at;
-        j = state.x + b;
-        A = a.cell_seginfo[2 * sid];
-        B = a.cell_seginfo[2 * sid + 1];
-        f = load_tracklet(a, k);
-        s = load_tracklet(a, j);
-        const float4 c1 = a.xyzr[A.x + f.first_cluster];
-        const float4 c2 = a.xyzr[A.y + f.second_cluster];
-        const float4 c3 = a.xyzr[A.z + s.second_cluster];
-        const int layer = sid % ITSU_TRACKLET_LAYERS;
-        pass = cell_precut(layer, f.tan_lambda, f.phi, s.tan_lambda, s.phi, c1, __int_as_float(B.w)) &&
-               cell_geometry(layer, c1, c2, c3, __int_as_float(B.y), __int_as_float(B.z), normal, curvature, dca);
-        if (pass) {
-          atomicOr(reinterpret_cast<unsigned *>(&w.mask[at]) + (b >> 5), 1u << (b & 31));
+        bool pass = false, crowded = false;
+        int sid = 0, segment = 0;
+        uint32_t k = 0, j = 0;
+        itsu_tracklet f, t;
+        int4 A, B;
+        float3 normal;
+        float curvature, dca;
+        if (lane < m) {
+          const uint32_t item = queued ? w.queue[head + lane] : w.ring[(head + lane) & (kCellRing - 1)], at = item & 127u;
+          const int2 state = w.state[at];
+          crowded = (state.y & kCrowded) != 0;
+          sid = state.y & ~kCrowded;
+          k = base + at;
+          j = (uint32_t)state.x + (item >> 7);
+          A = a.cell_seginfo[2 * sid];
+          B = a.cell_seginfo[2 * sid + 1];
+          f = load_tracklet(a, k);
+          t = load_tracklet(a, j);
+          const float4 c1 = a.xyzr[A.x + f.first_cluster];
+          const float4 c2 = a.xyzr[A.y + f.second_cluster];
+          const float4 c3 = a.xyzr[A.z + t.second_cluster];
+          const int e = sid / ITSU_TRACKLET_LAYERS, layer = sid - e * ITSU_TRACKLET_LAYERS;
+          segment = sid - e;  // 5 e + layer
+          pass = cell_precut(layer, f.tan_lambda, f.phi, t.tan_lambda, t.phi, c1, __int_as_float(B.w)) &&
+                 cell_geometry(layer, c1, c2, c3, __int_as_float(B.y), __int_as_float(B.z), normal, curvature, dca);
         }
-      }
-      // entries: the passing lanes' slots, contiguous in the warp's chunk
-      const unsigned passed = __ballot_sync(0xffffffffu, pass);
-      const int need = __popc(passed);
-      const int rank = __popc(passed & ((1u << lane) - 1u));
-      int64_t slot = chunk_pos + rank;
-      if (need > chunk_left) {
-        unsigned long long fresh = 0;
-        if (lane == 0) {
-          fresh = atomicAdd(reinterpret_cast<unsigned long long *>(&a.status->cell_entries), (unsigned long long)kCellChunk);
-          if ((int64_t)fresh + kCellChunk > a.cap_cell_entries) {
-            atomicOr(&a.status->flags, kFlagCapScratch);
+        head += m;
+        const unsigned passed = __ballot_sync(0xffffffffu, pass);
+        const unsigned same = __match_any_sync(0xffffffffu, pass ? segment : -1);
+        if (pass) {
+          const unsigned before = (1u << lane) - 1u;
+          if ((same & before) == 0) {
+            atomicAdd(&a.cell_seg_count[segment], __popc(same));
+          }
+          const int64_t slot = (int64_t)first + cells + __popc(passed & before);
+          int2 *dst = reinterpret_cast<int2 *>(a.cell_entries + slot);
+          dst[0] = make_int2(f.first_cluster, f.second_cluster);
+          dst[1] = make_int2(t.second_cluster, (int)(k - (uint32_t)A.w));
+          dst[2] = make_int2((int)(j - (uint32_t)B.x), __float_as_int(normal.x));
+          dst[3] = make_int2(__float_as_int(normal.y), __float_as_int(normal.z));
+          dst[4] = make_int2(__float_as_int(curvature), crowded ? segment | kEntryUnscored : segment);
+          if (a.mlp) {
+            a.cell_dca[slot] = dca;
           }
         }
-        const int64_t fresh_base = (int64_t)__shfl_sync(0xffffffffu, fresh, 0);
-        slot = rank < chunk_left ? chunk_pos + rank : fresh_base + (rank - chunk_left);
-        chunk_pos = fresh_base + (need - chunk_left);
-        chunk_left += kCellChunk - need;
-      } else {
-        chunk_pos += need;
-        chunk_left -= need;
-      }
-      if (pass && slot < a.cap_cell_entries) {
-        int4 *dst = reinterpret_cast<int4 *>(a.cell_entries + slot);
-        const int e = sid / ITSU_TRACKLET_LAYERS;
-        dst[0] = make_int4((int)k, b, sid - e, f.first_cluster);  // sid - e = 5 e + layer: the cell segment
-        dst[1] = make_int4(f.second_cluster, s.second_cluster, (int)(k - A.w), (int)(j - B.x));
-        dst[2] = make_int4(__float_as_int(normal.x), __float_as_int(normal.y), __float_as_int(normal.z), __float_as_int(curvature));
-        if (a.mlp) {
-          a.cell_dca[slot] = dca;
-        }
-      }
-      __syncwarp();  // the queue's freed places are refilled
-    }
-    __syncwarp();
-    // the span's results; its cells go to its scan tile's sum (the cells scan has no reduce pass)
-    int cells = 0;
-    for (uint32_t at = lane; at < span; at += 32) {
-      const uint32_t k = base + at;
-      if (k < t0 || k >= t1) {
-        continue;
-      }
-      const unsigned long long mask = w.mask[at];
-      const int2 state = w.state[at];
-      const bool big = state.y < 0;
-      const int count = big ? crowded_cells(a, k, n) : __popcll(mask);
-      cells += count;
-      a.cell_count[k] = count;
-      a.cell_mask[k] = mask;
-      a.cell_lookup[k] = ITSU_UNUSED_INDEX;  // the write pass fills it for tracklets with cells
-      if (big && count > 0) {
-        const unsigned long long q = atomicAdd(reinterpret_cast<unsigned long long *>(&a.status->crowded), 1ull);
-        if ((int64_t)q < n) {
-          a.cell_crowded[q] = (int32_t)k;
-        }
+        cells += __popc(passed);
+        __syncwarp();  // the queue's freed places are refilled
       }
     }
-    cells = (int)__reduce_add_sync(0xffffffffu, (unsigned)cells);
-    if (lane == 0 && cells != 0) {
-      atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[base / kScanTile]), (unsigned long long)cells);
+    if (lane == 0) {
+      a.cell_span[s] = make_int2((int)first, cells);
+      a.cell_span_count[s] = cells;
+      if (cells > 0) {
+        atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[s / kScanTile]), (unsigned long long)cells);
+      }
     }
     __syncwarp();  // the span's state is refilled next
   }
-  // the unused rest of the last chunk is marked empty
-  for (int i = lane; i < chunk_left && chunk_pos + i < a.cap_cell_entries; i += 32) {
-    a.cell_entries[chunk_pos + i].t1 = -1;
-  }
 }
 
-// Learned prefilter: scores the count pass's cell entries, 32 per warp on the tensor cores, and
-// drops those whose logit is below the model's threshold from their tracklet's mask and count
-// before the scan. The score and the exact cuts are combined with AND, so scoring only the pairs
-// that passed the cuts (whose geometry also gave the DCA feature) keeps the same cells as scoring
-// every candidate first. A NaN logit keeps its cell. The pairs of a tracklet with more than
-// kMaxMaskedOut outgoing tracklets are counted in order on one lane and are kept unscored.
+// Learned prefilter: scores the cell entries, 32 per warp on the tensor cores, and drops those whose
+// logit is below the model's threshold (entry and counts) before the scan. The score and the exact
+// cuts are combined with AND, so scoring only the pairs that passed the cuts (whose geometry also
+// gave the DCA feature) keeps the same cells as scoring every candidate first. A NaN logit keeps its
+// cell. The pairs of a tracklet with more than kMaxMaskedOut outgoing tracklets are kept unscored.
+// A warp takes consecutive spans and flattens their entries over its lanes, so that the network's
+// tiles are full.
 constexpr int kPrefilterThreads = 256;
+
+// Spans a warp of a pass over the entries takes at a time (a span of 128 has 15 entries in central
+// events, 85 behind the tracklet gate): about `turns` of them for all warps of the grid. The prefilter
+// wants full tiles (2^13 turns), the write pass many stores in flight (2^16: 0.16 ms per 128 central
+// events, 0.18 at 2^13).
+__device__ __forceinline__ int spans_at_a_time(int64_t spans, int64_t turns) { return (int)min((int64_t)32, max((int64_t)1, spans / turns)); }
 
 __global__ void __launch_bounds__(kPrefilterThreads) k_cells_prefilter(Arena a)
 {
@@ -1801,145 +1741,143 @@ __global__ void __launch_bounds__(kPrefilterThreads) k_cells_prefilter(Arena a)
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t reserved = a.status->cell_entries;
-  const int64_t n = reserved < a.cap_cell_entries ? reserved : a.cap_cell_entries;
-  const int64_t tiles = (n + 31) / 32;
-  for (int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp; tile < tiles; tile += (int64_t)gridDim.x * (blockDim.x >> 5)) {
-    const int64_t i = tile * 32 + lane;
-    int4 h = make_int4(-1, 0, 0, 0);
-    if (i < n) {
-      h = reinterpret_cast<const int4 *>(a.cell_entries + i)[0];
-    }
-    float f[kMlpIn];
-    if (h.x >= 0) {
-      const int4 g = reinterpret_cast<const int4 *>(a.cell_entries + i)[1];  // c2, c3, t1 local, t2 local
-      const int e = h.z / ITSU_CELL_LAYERS, layer = h.z % ITSU_CELL_LAYERS;
-      const int32_t *lo = a.layer_off + e * ITSU_LAYERS;
-      const itsu_tracklet t1 = load_tracklet(a, h.x);
-      const itsu_tracklet t2 = load_tracklet(a, a.trk_seg[e * ITSU_TRACKLET_LAYERS + layer + 1] + g.w);
-      const float4 c1 = a.xyzr[lo[layer] + h.w];
-      const float4 c2 = a.xyzr[lo[layer + 1] + g.x];
-      const float4 c3 = a.xyzr[lo[layer + 2] + g.y];
-      pair_features(layer, t1.tan_lambda, t1.phi, t2.tan_lambda, t2.phi, c1, c2, c3, a.vtx[3 * e], a.vtx[3 * e + 1],
-                    a.vtx[3 * e + 2], a.cell_dca[i], f);
-    } else {
-      for (int k = 0; k < kMlpIn; ++k) {
-        f[k] = mlp.mean[k];
+  const int64_t spans = a.status->cell_spans;
+  const int take = spans_at_a_time(spans, 1 << 13);
+  for (int64_t s0 = ((int64_t)blockIdx.x * (kPrefilterThreads / 32) + warp) * take; s0 < spans;
+       s0 += (int64_t)gridDim.x * (kPrefilterThreads / 32) * take) {
+    const int2 in = lane < take && s0 + lane < spans ? a.cell_span[s0 + lane] : make_int2(0, 0);  // first entry, entries
+    int total;
+    const int excl = warp_exclusive_sum(in.y, total);
+    for (int p0 = 0; p0 < total; p0 += 32) {
+      const int p = p0 + lane;
+      const int owner = owner_of(excl, p);
+      const int64_t i = (int64_t)__shfl_sync(0xffffffffu, in.x, owner) + p - __shfl_sync(0xffffffffu, excl, owner);
+      int segment = kEntryUnscored;
+      int2 h0, h1, h2;
+      if (p < total) {
+        const int2 *src = reinterpret_cast<const int2 *>(a.cell_entries + i);
+        h0 = src[0], h1 = src[1], h2 = src[2], segment = src[4].y;
       }
+      float f[kMlpIn];
+      const bool scored = !(segment & kEntryUnscored);
+      if (scored) {
+        const int layer = segment % ITSU_CELL_LAYERS, sid = segment + segment / ITSU_CELL_LAYERS;  // 6 e + layer
+        const int4 A = a.cell_seginfo[2 * sid], B = a.cell_seginfo[2 * sid + 1];
+        const itsu_tracklet t1 = load_tracklet(a, A.w + h1.y);
+        const itsu_tracklet t2 = load_tracklet(a, B.x + h2.x);
+        const float4 c1 = a.xyzr[A.x + h0.x];
+        const float4 c2 = a.xyzr[A.y + h0.y];
+        const float4 c3 = a.xyzr[A.z + h1.x];
+        pair_features(layer, t1.tan_lambda, t1.phi, t2.tan_lambda, t2.phi, c1, c2, c3, __int_as_float(B.y), __int_as_float(B.z),
+                      __int_as_float(B.w), a.cell_dca[i], f);
+      } else {
+        for (int k = 0; k < kMlpIn; ++k) {
+          f[k] = mlp.mean[k];
+        }
+      }
+      feature_row(mlp.mean, mlp.inv_std, f, rows[warp][lane]);
+      __syncwarp();
+      const float logit = mlp_logits_warp<false>(mlp, rows[warp], nullptr);
+      if (scored && logit < mlp.threshold) {
+        a.cell_entries[i].segment = kEntryDropped;
+        atomicSub(&a.cell_span_count[s0 + owner], 1);
+        atomicSub(&a.cell_seg_count[segment], 1);
+        atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[(s0 + owner) / kScanTile]), ~0ull);  // its tile sum - 1
+      }
+      __syncwarp();
     }
-    feature_row(mlp.mean, mlp.inv_std, f, rows[warp][lane]);
-    __syncwarp();
-    const float logit = mlp_logits_warp<false>(mlp, rows[warp], nullptr);
-    if (h.x >= 0 && logit < mlp.threshold) {
-      atomicAnd(&a.cell_mask[h.x], ~(1ull << h.y));
-      atomicSub(&a.cell_count[h.x], 1);
-      atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[h.x / kScanTile]), ~0ull);  // its tile sum - 1
-    }
-    __syncwarp();
   }
 }
 
-// Write pass, part 1: every cell entry whose bit survived goes to its scanned slot, in
-// outgoing-tracklet order within its first tracklet (the rank of its bit in the mask).
-__global__ void __launch_bounds__(kMaxThreads) k_cells_scatter(Arena a)
+// Write pass: a warp takes consecutive spans and flattens their entries over its lanes; in order, they go to the spans' scanned places, which
+// are contiguous (a dropped entry leaves no gap). The first cell of each first tracklet fills its
+// cells lookup entry.
+constexpr int kScatterThreads = 256;
+
+__global__ void __launch_bounds__(kScatterThreads) k_cells_scatter(Arena a)
 {
   if (capacity_failed(a.status)) {
     return;
   }
-  const int64_t reserved = a.status->cell_entries;
-  const int64_t n = reserved < a.cap_cell_entries ? reserved : a.cap_cell_entries;
-  const int64_t stride = grid_threads();
-  constexpr int kPer = 4;  // entries per thread per round, their loads in flight together
-  for (int64_t i0 = global_thread(); i0 < n; i0 += kPer * stride) {
-    int4 h[kPer], g[kPer], q[kPer];
+  const int lane = threadIdx.x & 31;
+  const int64_t spans = a.status->cell_spans;
+  const int take = spans_at_a_time(spans, 1 << 16);
+  for (int64_t s0 = ((int64_t)blockIdx.x * (kScatterThreads / 32) + (threadIdx.x >> 5)) * take; s0 < spans;
+       s0 += (int64_t)gridDim.x * (kScatterThreads / 32) * take) {
+    const int2 in = lane < take && s0 + lane < spans ? a.cell_span[s0 + lane] : make_int2(0, 0);  // first entry, entries
+    int total;
+    const int excl = warp_exclusive_sum(in.y, total);
+    int out0 = a.cell_span_off[s0];
+    int last_t1 = -1, last_segment = -1;  // of the cell before
+    for (int p0 = 0; p0 < total; p0 += 32) {
+      const int p = p0 + lane;
+      const int owner = owner_of(excl, p);
+      const int64_t i = (int64_t)__shfl_sync(0xffffffffu, in.x, owner) + p - __shfl_sync(0xffffffffu, excl, owner);
+      int2 h[5];
+      h[1].y = 0;
+      h[4].y = kEntryDropped;
+      if (p < total) {
+        const int2 *src = reinterpret_cast<const int2 *>(a.cell_entries + i);
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int64_t i = i0 + u * stride;
-      h[u] = make_int4(-1, 0, 0, 0);
-      if (i < n) {
-        const int4 *src = reinterpret_cast<const int4 *>(a.cell_entries + i);
-        h[u] = src[0];  // t1, bit, segment, c1
-        g[u] = src[1];  // c2, c3, t1 local, t2 local
-        q[u] = src[2];  // normal, curvature
+        for (int q = 0; q < 5; ++q) {
+          h[q] = src[q];
+        }
       }
-    }
-    unsigned long long m[kPer];
-    int32_t off[kPer];
+      const bool alive = h[4].y != kEntryDropped;
+      const unsigned living = __ballot_sync(0xffffffffu, alive);
+      if (living == 0) {
+        continue;
+      }
+      const unsigned before = living & ((1u << lane) - 1u);
+      const int out = out0 + __popc(before);
+      const int segment = h[4].y & ~kEntryUnscored, t1 = h[1].y;
+      const int from = before ? 31 - __clz(before) : 0;
+      const int t1_before = __shfl_sync(0xffffffffu, t1, from), segment_before = __shfl_sync(0xffffffffu, segment, from);
+      if (alive) {
+        const bool first = before ? (t1_before != t1 || segment_before != segment) : (last_t1 != t1 || last_segment != segment);
+        const int e = segment / ITSU_CELL_LAYERS, layer = segment % ITSU_CELL_LAYERS;
+        if (first && layer >= 1) {
+          a.cell_lookup[a.trk_seg[e * ITSU_TRACKLET_LAYERS + layer] + t1] = out - a.cell_seg[segment];
+        }
+        int2 *dst = reinterpret_cast<int2 *>(a.cells + out);
+        h[4].y = 1;  // level
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      if (h[u].x >= 0) {
-        m[u] = a.cell_mask[h[u].x];
-        off[u] = a.cell_off[h[u].x];
+        for (int q = 0; q < 5; ++q) {
+          dst[q] = h[q];
+        }
+        a.cell_seg_id[out] = segment;
       }
-    }
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      if (h[u].x < 0 || !((m[u] >> h[u].y) & 1ull)) {
-        continue;  // an unused slot, or a pair removed by the learned prefilter
-      }
-      const int32_t rank = __popcll(m[u] & ((1ull << h[u].y) - 1ull));
-      const int32_t out = off[u] + rank;
-      if (rank == 0 && h[u].z % ITSU_CELL_LAYERS >= 1) {  // the tracklet's first cell: its cells lookup entry
-        a.cell_lookup[h[u].x] = out - a.cell_seg[h[u].z];
-      }
-      int2 *dst = reinterpret_cast<int2 *>(a.cells + out);
-      dst[0] = make_int2(h[u].w, g[u].x);
-      dst[1] = make_int2(g[u].y, g[u].z);
-      dst[2] = make_int2(g[u].w, q[u].x);
-      dst[3] = make_int2(q[u].y, q[u].z);
-      dst[4] = make_int2(q[u].w, 1);
-      a.cell_seg_id[out] = h[u].z;
+      const int to = 31 - __clz(living);
+      last_t1 = __shfl_sync(0xffffffffu, t1, to);
+      last_segment = __shfl_sync(0xffffffffu, segment, to);
+      out0 += __popc(living);
     }
   }
 }
 
-// Write pass, part 2: the tracklets whose outer cluster was too crowded for the pair-parallel
-// count (listed by the count pass; their mask is empty): their cells in order on one lane, and
-// their cells lookup entry.
-__global__ void __launch_bounds__(kMaxThreads) k_cells_crowded(Arena a)
+// cell_seg[5e+L] = first cell of (e, L), from the segments' counts (cells are in segment order), in
+// one block; capacity check of the cell total.
+__global__ void __launch_bounds__(1024) k_cell_segments(Arena a)
 {
-  if (capacity_failed(a.status)) {
-    return;
-  }
-  const int64_t n = a.status->total[kTracklets];
-  const int64_t listed = min(a.status->crowded, n);
-  for (int64_t q = global_thread(); q < listed; q += grid_threads()) {
-    const int32_t k = a.cell_crowded[q];
-    const CellLane s = cell_lane(a, k, n);
-    const int32_t first = a.cell_off[k];
-    if (s.layer >= 1 && s.layer < ITSU_CELL_LAYERS) {
-      a.cell_lookup[k] = first - a.cell_seg[s.e * ITSU_CELL_LAYERS + s.layer];
-    }
-    int64_t out = first;
-    for (int b = 0; b < s.n_out; ++b) {
-      const int32_t j = s.j0 + b;
-      const itsu_tracklet t2 = load_tracklet(a, j);
-      float3 normal;
-      float curvature;
-      if (cell_precut(s.layer, s.t1_tan_lambda, s.t1_phi, t2.tan_lambda, t2.phi, s.c1, s.vz) &&
-          cell_geometry(s.layer, s.c1, s.c2, a.xyzr[s.c3_base + t2.second_cluster], s.vx, s.vy, normal, curvature)) {
-        write_cell(a, out++, s, t2, j, normal, curvature);
-      }
-    }
-  }
-}
-
-__global__ void k_cell_segments(Arena a)
-{
+  __shared__ int64_t warp_totals[33];
   if (capacity_failed(a.status)) {
     return;  // tracklet offsets beyond the arena: nothing downstream runs
   }
   const int nseg = a.n_events * ITSU_CELL_LAYERS;
-  for (int s = (int)global_thread(); s <= nseg; s += grid_threads()) {
-    if (s == nseg) {
-      const int64_t total = a.status->total[kCells];
-      a.cell_seg[s] = (int32_t)total;
-      if (total > a.cap_cells) {
-        atomicOr(&a.status->flags, kFlagCapCells);
-      }
-    } else {
-      const int e = s / ITSU_CELL_LAYERS, layer = s % ITSU_CELL_LAYERS;
-      a.cell_seg[s] = a.cell_off[a.trk_seg[e * ITSU_TRACKLET_LAYERS + layer]];
+  int64_t carry = 0;
+  for (int s0 = 0; s0 < nseg; s0 += (int)blockDim.x) {
+    const int s = s0 + (int)threadIdx.x;
+    int64_t total;
+    const int64_t ex = block_exclusive_scan<int64_t>(s < nseg ? a.cell_seg_count[s] : 0, warp_totals, total);
+    if (s < nseg) {
+      a.cell_seg[s] = (int32_t)(carry + ex);
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) {
+    a.cell_seg[nseg] = (int32_t)carry;
+    if (carry > a.cap_cells) {
+      atomicOr(&a.status->flags, kFlagCapCells);
     }
   }
 }
@@ -1969,10 +1907,14 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbour_reset(Arena a)
 }
 
 // Tracker.cxx:416-474 (findCellsNeighbours): a cell of layer L and the cells of layer L + 1 built
-// on its second tracklet. The count pass evaluates the cut, counts each passing pair in its row
-// and keeps the passing candidates as a mask (rows of up to kMaxMaskedOut candidates); the write
-// pass, after the scan of the counts, fills the rows from the mask (re-evaluating the cut only for
-// cells with more candidates). Row order is restored by k_levels' sort.
+// on its second tracklet (from its cells lookup entry on, as long as they are built on it). The
+// count pass evaluates the cut, counts each passing pair in its row and keeps the passing candidates
+// as a mask (of up to kMaskedRun candidates; a longer run is marked in the top bit); the write pass,
+// after the scan of the counts, fills the rows from the mask (re-evaluating the cut only for the
+// marked cells). Row order is restored by k_levels' sort.
+constexpr int kMaskedRun = 63;
+constexpr unsigned long long kLongRun = 1ull << kMaskedRun;
+
 template <bool kWrite>
 __global__ void __launch_bounds__(kMaxThreads) k_neighbours(Arena a)
 {
@@ -1986,14 +1928,17 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbours(Arena a)
     if (layer >= ITSU_NEIGHBOUR_LAYERS) {
       continue;
     }
+    unsigned long long mask = 0ull;
+    if (kWrite && (mask = a.nb_mask[c]) == 0ull) {
+      continue;
+    }
     const int32_t second = a.cells[c].second_tracklet;
-    const int64_t ft = a.trk_seg[e * ITSU_TRACKLET_LAYERS + layer + 1] + second;
-    const int32_t j0 = a.cell_off[ft], j1 = a.cell_off[ft + 1];
-    const bool masked = j1 - j0 <= kMaxMaskedOut;
-    if (kWrite && masked) {
-      const int32_t c_local = (int32_t)(c - a.cell_seg[e * ITSU_CELL_LAYERS + layer]);
-      for (unsigned long long m = a.nb_mask[c]; m; m &= m - 1ull) {
-        const int32_t j = j0 + __ffsll((long long)m) - 1;
+    const int32_t found = a.cell_lookup[a.trk_seg[e * ITSU_TRACKLET_LAYERS + layer + 1] + second];
+    const int32_t j0 = a.cell_seg[sid + 1] + found, j1 = found < 0 ? j0 : a.cell_seg[sid + 2];
+    const int32_t c_local = (int32_t)(c - a.cell_seg[sid]);
+    if (kWrite && !(mask & kLongRun)) {
+      for (; mask; mask &= mask - 1ull) {
+        const int32_t j = j0 + __ffsll((long long)mask) - 1;
         const int slot = atomicAdd(&a.nb_fill[j], 1);
         a.nb[a.nb_off[j] + slot] = c_local;
       }
@@ -2001,23 +1946,29 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbours(Arena a)
     }
     const itsu_cell cell = a.cells[c];
     const float3 n1 = make_float3(cell.nx, cell.ny, cell.nz);
-    const int32_t c_local = (int32_t)(c - a.cell_seg[e * ITSU_CELL_LAYERS + layer]);
-    unsigned long long mask = 0ull;
     for (int32_t j = j0; j < j1; ++j) {
       const itsu_cell next = a.cells[j];
-      if (neighbour_cut(layer, n1, cell.curvature, make_float3(next.nx, next.ny, next.nz), next.curvature)) {
-        if (kWrite) {
+      if (next.first_tracklet != second) {
+        break;
+      }
+      const bool pass = neighbour_cut(layer, n1, cell.curvature, make_float3(next.nx, next.ny, next.nz), next.curvature);
+      if (kWrite) {
+        if (pass) {
           const int slot = atomicAdd(&a.nb_fill[j], 1);
           a.nb[a.nb_off[j] + slot] = c_local;
-        } else {
+        }
+      } else {
+        if (pass) {
           atomicAdd(&a.nb_count[j], 1);
-          if (masked) {
-            mask |= 1ull << (j - j0);
-          }
+        }
+        if (j - j0 >= kMaskedRun) {
+          mask |= kLongRun;
+        } else if (pass) {
+          mask |= 1ull << (j - j0);
         }
       }
     }
-    if (!kWrite && masked) {
+    if (!kWrite) {
       a.nb_mask[c] = mask;
     }
   }
@@ -2344,22 +2295,23 @@ void step_tracklet_segments(const Arena &a, const Launch &l)
   k_tracklet_segments<<<(a.n_events * ITSU_TRACKLET_LAYERS + kThreads) / kThreads, kThreads, 0, l.stream>>>(a);
 }
 
-void launch_cells_range(const Arena &a, const Launch &l, int32_t e0, int32_t e1)
+void launch_cells_range(const Arena &a, const Launch &l, int32_t e0, int32_t e1, bool last)
 {
-  k_cells_count<<<l.num_sms * kCellBlocks, kCellThreads, 0, l.stream>>>(a, e0, e1);
+  k_cells_count<<<l.num_sms * kCellBlocks, kCellThreads, 0, l.stream>>>(a, e0, e1, last);
 }
 
 void step_cells_count(const Arena &a, const Launch &l)
 {
-  if (l.n_groups == 0 && whole_warps(a, l)) {
-    launch_cells_range(a, l, 0, 0);
+  if (l.n_groups == 0) {
+    launch_cells_range(a, l, 0, a.n_events, true);
   }
 }
 
 // Event groups: the write pass of a group's inner clusters, then the cell count pass of its
 // tracklets, group after group, so that the tracklets a group's count pass gathers were written
 // moments before and are still in L2. Group g's clusters are [groups[g], groups[g + 1]) (multiples
-// of 32 up to the last), its events [g * group_events, (g + 1) * group_events).
+// of 32 up to the last), its events [g * group_events, (g + 1) * group_events). A span that reaches
+// into the next group's tracklets is left to that group.
 void step_write_count_groups(const Arena &a, const Launch &l)
 {
   if (l.n_groups == 0 || !whole_warps(a, l)) {
@@ -2368,7 +2320,7 @@ void step_write_count_groups(const Arena &a, const Launch &l)
   for (int g = 0; g < l.n_groups; ++g) {
     launch_write_range(a, l, l.groups[g], l.groups[g + 1]);
     const int32_t e0 = g * l.group_events, e1 = std::min(a.n_events, (g + 1) * l.group_events);
-    launch_cells_range(a, l, e0, e1);
+    launch_cells_range(a, l, e0, e1, g + 1 == l.n_groups);
   }
 }
 
@@ -2380,14 +2332,9 @@ void step_cells_prefilter(const Arena &a, const Launch &l)
   }
 }
 
-void step_cells_scatter(const Arena &a, const Launch &l) { k_cells_scatter<<<fixed_grid(l), l.block, 0, l.stream>>>(a); }
+void step_cells_scatter(const Arena &a, const Launch &l) { k_cells_scatter<<<l.num_sms * 8, kScatterThreads, 0, l.stream>>>(a); }
 
-void step_cells_crowded(const Arena &a, const Launch &l) { k_cells_crowded<<<l.num_sms, 128, 0, l.stream>>>(a); }
-
-void step_cell_segments(const Arena &a, const Launch &l)
-{
-  k_cell_segments<<<(a.n_events * ITSU_CELL_LAYERS + kThreads) / kThreads, kThreads, 0, l.stream>>>(a);
-}
+void step_cell_segments(const Arena &a, const Launch &l) { k_cell_segments<<<1, 1024, 0, l.stream>>>(a); }
 
 void step_neighbour_reset(const Arena &a, const Launch &l) { k_neighbour_reset<<<fixed_grid(l), l.block, 0, l.stream>>>(a); }
 
@@ -2434,23 +2381,22 @@ const KernelStep kSteps[] = {
     {"scan_apply_cells", step_scan_apply<1>, 0},             // 13
     {"cell_segments", step_cell_segments, 0},                // 14
     {"cells_scatter", step_cells_scatter, 0},                // 15
-    {"cells_crowded", step_cells_crowded, 0},                // 16
-    {"neighbour_reset", step_neighbour_reset, 0},            // 17 (d)
-    {"neighbours_count", step_neighbours<false>, 0},         // 18
-    {"scan_reduce_neighbours", step_scan_reduce<2>, 0},      // 19
-    {"scan_partials_neighbours", step_scan_partials<2>, 0},  // 20
-    {"scan_apply_neighbours", step_scan_apply<2>, 0},        // 21
-    {"neighbour_check", step_neighbour_check, 0},            // 22
-    {"neighbours_write", step_neighbours<true>, 0},          // 23
-    {"levels_1", step_levels<1>, 0},                         // 24
-    {"levels_2", step_levels<2>, 0},                         // 25
-    {"levels_3", step_levels<3>, 0},                         // 26
-    {"levels_4", step_levels<4>, 0},                         // 27
-    {"scan_reduce_roads", step_scan_reduce<3>, 0},           // 28 (e)
-    {"scan_partials_roads", step_scan_partials<3>, 0},       // 29
-    {"scan_apply_roads", step_scan_apply<3>, 0},             // 30
-    {"road_segments", step_road_segments, 0},                // 31
-    {"roads_write", step_roads, 0},                          // 32
+    {"neighbour_reset", step_neighbour_reset, 0},            // 16 (d)
+    {"neighbours_count", step_neighbours<false>, 0},         // 17
+    {"scan_reduce_neighbours", step_scan_reduce<2>, 0},      // 18
+    {"scan_partials_neighbours", step_scan_partials<2>, 0},  // 19
+    {"scan_apply_neighbours", step_scan_apply<2>, 0},        // 20
+    {"neighbour_check", step_neighbour_check, 0},            // 21
+    {"neighbours_write", step_neighbours<true>, 0},          // 22
+    {"levels_1", step_levels<1>, 0},                         // 23
+    {"levels_2", step_levels<2>, 0},                         // 24
+    {"levels_3", step_levels<3>, 0},                         // 25
+    {"levels_4", step_levels<4>, 0},                         // 26
+    {"scan_reduce_roads", step_scan_reduce<3>, 0},           // 27 (e)
+    {"scan_partials_roads", step_scan_partials<3>, 0},       // 28
+    {"scan_apply_roads", step_scan_apply<3>, 0},             // 29
+    {"road_segments", step_road_segments, 0},                // 30
+    {"roads_write", step_roads, 0},                          // 31
 };
 constexpr int kNumSteps = sizeof(kSteps) / sizeof(kSteps[0]);
 
@@ -2519,11 +2465,11 @@ void launch_atan2f(const float *y, const float *x, float *out, int64_t n, int nu
 }
 void launch_tracklets_write(const Arena &a, const Launch &l) { run_steps(7, 8, a, l); }
 void launch_cells_count(const Arena &a, const Launch &l) { run_steps(9, 14, a, l); }
-void launch_cells_write(const Arena &a, const Launch &l) { run_steps(15, 16, a, l); }
-void launch_neighbours_count(const Arena &a, const Launch &l) { run_steps(17, 22, a, l); }
-void launch_neighbours_write(const Arena &a, const Launch &l) { run_steps(23, 27, a, l); }
-void launch_roads_count(const Arena &a, const Launch &l) { run_steps(28, 31, a, l); }
-void launch_roads_write(const Arena &a, const Launch &l) { run_steps(32, 32, a, l); }
+void launch_cells_write(const Arena &a, const Launch &l) { run_steps(15, 15, a, l); }
+void launch_neighbours_count(const Arena &a, const Launch &l) { run_steps(16, 21, a, l); }
+void launch_neighbours_write(const Arena &a, const Launch &l) { run_steps(22, 26, a, l); }
+void launch_roads_count(const Arena &a, const Launch &l) { run_steps(27, 30, a, l); }
+void launch_roads_write(const Arena &a, const Launch &l) { run_steps(31, 31, a, l); }
 
 int kernels_per_run()
 {
