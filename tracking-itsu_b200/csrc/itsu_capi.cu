@@ -76,7 +76,9 @@ struct itsu_context {
   int64_t init_tracklets = 0, init_cells = 0, init_neighbours = 0, init_roads = 0;
 
   // device buffers: cluster class
-  itsu_cluster *raw = nullptr, *sorted = nullptr, *tmp = nullptr;
+  itsu_cluster *raw = nullptr, *sorted = nullptr;
+  float4 *sort_recs = nullptr;
+  uint32_t *sort_index = nullptr;
   float4 *xyzr = nullptr;
   float *phi = nullptr;
   int32_t *trk_count = nullptr, *trk_off = nullptr, *trk_lookup = nullptr;
@@ -117,6 +119,7 @@ struct itsu_context {
   int32_t n_events = 0;
   int64_t n_clusters = 0;
   std::vector<int32_t> h_layer_off;
+  int64_t max_segment = 0;  // clusters of the current run's largest layer
   std::vector<int64_t> group_bounds;  // event groups of the current whole run (whole_run_launch)
   const itsu_cluster *in_raw = nullptr;
   const itsu_cluster_in *in_raw_in = nullptr;  // the 24-byte input records instead of in_raw (compact host calls)
@@ -145,6 +148,7 @@ struct itsu_context {
   bool tuning = false;
   int graph_tune[4] = {0, 0, -1, -1};
   bool graph_prefilter = false;
+  itsu::SortShape graph_sort{};
   bool graph_gate = false;
 
   // streamed host runs (ITSU_FLAG_STREAM_HOST): upload stream, per-chunk events, batch-wide roads
@@ -263,7 +267,18 @@ Launch launch_of(const itsu_context *ctx)
   l.num_sms = ctx->num_sms;
   l.block = t.block;
   l.blocks_per_sm = t.blocks_per_sm;
+  l.max_segment = ctx->max_segment;
   return l;
+}
+
+// Clusters of the largest of the segments whose offsets are off[0 .. n_segments].
+int64_t largest_segment(const int32_t *off, int64_t n_segments)
+{
+  int64_t largest = 0;
+  for (int64_t k = 0; k < n_segments; ++k) {
+    largest = std::max<int64_t>(largest, off[k + 1] - off[k]);
+  }
+  return largest;
 }
 
 // Event groups of a run of n_events events with host layer offsets off[n_events * 7 + 1]: group g
@@ -318,7 +333,9 @@ Arena arena_of(const itsu_context *ctx)
   a.sorted = ctx->sorted;
   a.xyzr = ctx->xyzr;
   a.phi = ctx->phi;
-  a.tmp = ctx->tmp;
+  a.sort_recs = ctx->sort_recs;
+  a.sort_index = ctx->sort_index;
+  a.sort_stride = ctx->cap_clusters;
   a.index_tables = ctx->index_tables;
   a.zs = ctx->zs;
   a.clu_seg = ctx->clu_seg;
@@ -401,7 +418,8 @@ itsu_status ensure_clusters(itsu_context *ctx, int64_t n_clusters, int32_t n_eve
     const int64_t cap = grow_to(n_clusters);
     ITSU_CUDA(ctx, alloc(ctx, ctx->raw, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->sorted, cap));
-    ITSU_CUDA(ctx, alloc(ctx, ctx->tmp, cap));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->sort_recs, 2 * cap));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->sort_index, 4 * cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->xyzr, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->phi, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_count, cap + 1));
@@ -628,7 +646,9 @@ void drop_graph(itsu_context *ctx)
 itsu_status launch_all(itsu_context *ctx)
 {
   const Tune tune = current_tune(ctx);
-  const bool same = ctx->graph && ctx->graph_generation == ctx->generation && ctx->graph_key[0] == ctx->in_raw &&
+  const itsu::SortShape sort = itsu::sort_shape(ctx->n_events, ctx->n_clusters, ctx->max_segment);
+  const bool same = ctx->graph && sort.threads == ctx->graph_sort.threads && sort.ctas == ctx->graph_sort.ctas &&
+                    ctx->graph_generation == ctx->generation && ctx->graph_key[0] == ctx->in_raw &&
                     ctx->graph_tune[0] == tune.block && ctx->graph_tune[1] == tune.blocks_per_sm &&
                     ctx->graph_tune[2] == tune.prune && ctx->graph_tune[3] == tune.group && ctx->graph_prefilter == ctx->prefilter &&
                     ctx->graph_gate == ctx->gate &&
@@ -666,6 +686,7 @@ itsu_status launch_all(itsu_context *ctx)
     ctx->graph_tune[2] = tune.prune;
     ctx->graph_tune[3] = tune.group;
     ctx->graph_prefilter = ctx->prefilter;
+    ctx->graph_sort = sort;
     ctx->graph_gate = ctx->gate;
     ctx->graph_events = ctx->n_events;
     ctx->graph_clusters = ctx->n_clusters;
@@ -787,6 +808,7 @@ itsu_status upload_vertex(itsu_context *ctx, const itsu_cluster *const layers[IT
   ctx->n_events = 1;
   ctx->n_clusters = off[ITSU_LAYERS];
   ctx->h_layer_off = off;
+  ctx->max_segment = *std::max_element(counts, counts + ITSU_LAYERS);
   ctx->in_raw = ctx->raw;
   ctx->in_raw_in = nullptr;
   ctx->in_raw_track = nullptr;
@@ -949,7 +971,7 @@ void itsu_context_destroy(itsu_context *ctx)
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->twin) itsu_context_destroy(ctx->twin);
   drop_graph(ctx);
-  release(ctx->raw); release(ctx->raw_in); release(ctx->raw_track); release(ctx->sorted); release(ctx->tmp); release(ctx->xyzr); release(ctx->phi);
+  release(ctx->raw); release(ctx->raw_in); release(ctx->raw_track); release(ctx->sorted); release(ctx->sort_recs); release(ctx->sort_index); release(ctx->xyzr); release(ctx->phi);
   release(ctx->trk_count); release(ctx->trk_off); release(ctx->trk_range); release(ctx->trk_lookup); release(ctx->zs); release(ctx->clu_seg); release(ctx->clu_aux); release(ctx->clu_crowded); release(ctx->trk_slots);
   release(ctx->seg_rrange); release(ctx->seg_regular); release(ctx->raw_off);
   release(ctx->layer_off); release(ctx->index_tables); release(ctx->trk_seg); release(ctx->cell_seginfo); release(ctx->cell_seg); release(ctx->cell_seg_count);
@@ -1209,6 +1231,7 @@ static itsu_status set_batch(itsu_context *ctx, const itsu_batch *batch)
       if (ctx->h_layer_off[k] < ctx->h_layer_off[k - 1]) return fail(ctx, ITSU_ERR_INVALID, "layer offsets decrease at %zu", k);
     }
   }
+  ctx->max_segment = largest_segment(ctx->h_layer_off.data(), (int64_t)batch->n_events * ITSU_LAYERS);
   ctx->stage = kNone;
   return ITSU_OK;
 }
@@ -1604,6 +1627,7 @@ itsu_status run_host_streamed(itsu_context *ctx, const HostClusters &clusters, c
     Arena arena = arena_of(x);
     arena.mlp = ctx->prefilter ? ctx->d_mlp : nullptr;  // the context's models serve both arenas
     arena.gate = ctx->gate ? ctx->d_gate : nullptr;
+    x->max_segment = largest_segment(layer_offsets + (int64_t)ev[c] * ITSU_LAYERS, (int64_t)x->n_events * ITSU_LAYERS);
     Launch l = launch_of(x);
     std::vector<int64_t> bounds;  // the chunk's event groups (read while its launches are enqueued)
     const int group = current_tune(x).group;
@@ -1742,6 +1766,7 @@ itsu_status batch_run_host(itsu_context *ctx, const HostClusters &clusters, cons
   ctx->in_layer_off = ctx->layer_off;
   ctx->in_vtx = ctx->vtx;
   ctx->h_layer_off.assign(layer_offsets, layer_offsets + (int64_t)n_events * ITSU_LAYERS + 1);
+  ctx->max_segment = largest_segment(layer_offsets, (int64_t)n_events * ITSU_LAYERS);
   if ((st = run_all(ctx)) != ITSU_OK) return st;
   const int64_t total = ctx->h_status->total[itsu::kRoads];
   if (road_offsets) {
@@ -1840,6 +1865,7 @@ itsu_status itsu_frames_run_host(itsu_context *ctx, const itsu_frames *frames, i
   ctx->in_layer_off = ctx->layer_off;
   ctx->in_vtx = ctx->vtx;
   ctx->h_layer_off = run_off;
+  ctx->max_segment = largest_segment(run_off.data(), (int64_t)nv * ITSU_LAYERS);
   if ((st = run_all(ctx)) != ITSU_OK) return st;
   const int64_t n_roads = ctx->h_status->total[itsu::kRoads];
   if (road_offsets) {

@@ -92,7 +92,9 @@ struct Arena {
   itsu_cluster *sorted;
   float4 *xyzr;
   float *phi;
-  itsu_cluster *tmp;
+  float4 *sort_recs;     // clustering scratch: two per cluster, input order: (x, y, z, r), (phi, id, alpha, MC id)
+  uint32_t *sort_index;  // clustering scratch: four arrays of sort_stride words
+  int64_t sort_stride;
   int32_t *index_tables;
   int32_t *clu_seg;  // per sorted cluster: its segment 7e + L (null: not wanted)
   int4 *clu_aux;     // per sorted cluster: id, alpha bits, MC id, bin (the clustering scatters them here)
@@ -162,7 +164,14 @@ struct Launch {
   int n_groups = 0;
   int group_events = 0;
   const int64_t *groups = nullptr;
+  int64_t max_segment = 0;  // clusters of the run's largest layer
 };
+
+// How the clustering is launched.
+struct SortShape {
+  int threads, ctas;
+};
+SortShape sort_shape(int32_t n_events, int64_t n_clusters, int64_t max_segment);
 
 // Stage launchers (asynchronous on l.stream).
 void launch_status_init(const Arena &a, const Launch &l);

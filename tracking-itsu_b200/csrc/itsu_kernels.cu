@@ -21,6 +21,9 @@
 // Capacity overflow never writes out of bounds: the passes check the scanned totals and scratch
 // reservations against the arena capacities, record the requirement and skip; the host grows
 // and re-runs.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <climits>
 
 #include "itsu_device.cuh"
@@ -32,8 +35,6 @@ namespace {
 
 constexpr int kThreads = 256;     // threads per block of the fixed-shape helper kernels
 constexpr int kMaxThreads = 512;  // upper bound of the tunable per-item kernels' block size
-constexpr int kSortThreads = 512;
-constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kBuckets = kTableSize + 1;  // bucket 0: negative bins; bucket b+1: bin b
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
@@ -377,22 +378,61 @@ __device__ __forceinline__ void stage_put(int32_t *stage, int lane, const itsu_c
   }
 }
 
-__global__ void __launch_bounds__(kSortThreads) k_cluster_sort(Arena a)
+// One segment (event, layer) per cluster of CTAs (of one, where a run has segments enough for the
+// chip). Every hit is touched twice: pass 1 reads it in input order and leaves the transformed record
+// (32 bytes) in a.sort_recs, pass 4 gathers the records in sorted order and writes every output,
+// coalesced. Between them, ranking by bucket, by bin and by z works on indices and z values alone,
+// kept in a.sort_index (12 to 16 bytes per hit, written and read within the CTA's turn, so mostly L2
+// hits; kept in shared memory instead they cost a CTA per SM on large segments: 0.37 against 0.30 ms
+// per 64 events of 7000 tracks, 0.41 against 0.42 on 128 of 6000). Bound by the latency of its
+// barrier-separated phases: 0.39 ms per 128 central events at three CTAs of 512 threads (40 registers,
+// some spilled) per SM, 0.41 at two, 0.51 with CTAs of 256; 0.49 with 36-byte records moved through
+// memory and back in input order. 1024 pp events of 60 tracks: 0.048 ms in CTAs of 64 threads, 0.24 in
+// CTAs of 512.
+constexpr size_t sort_shared_bytes(int warps)
 {
-  __shared__ int hist[kSortWarps][kBuckets];
-  __shared__ int bucket_total[kBuckets];
-  __shared__ int bucket_base[kBuckets];
-  __shared__ int32_t stages[kSortWarps][32 * kClusterWords];
+  return sizeof(int) * ((size_t)warps * kBuckets + 3 * kBuckets + 34 + 4 + (size_t)warps * 32 * kClusterWords);
+}
 
-  const int seg = blockIdx.x;
+template <int kThreads_>
+__global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Arena a)
+{
+  constexpr int kWarps = kThreads_ / 32;
+  namespace cg = cooperative_groups;
+  extern __shared__ int shared[];
+  int *const hist_all = shared;  // [kWarps][kBuckets]
+  int *const cta_total = hist_all + kWarps * kBuckets;
+  int *const bucket_total = cta_total + kBuckets;
+  int *const bucket_base = bucket_total + kBuckets;
+  int *const scan_totals = bucket_base + kBuckets;  // [33]
+  int *const s_flags = scan_totals + 34;            // irregular, least r, largest r (float bits), largest bucket
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ctas = (int)cg::this_cluster().num_blocks(), rank = (int)cg::this_cluster().block_rank();
+  const int seg = blockIdx.x / ctas;
   const int e = seg / ITSU_LAYERS, layer = seg % ITSU_LAYERS;
   const int64_t begin = a.layer_off[seg];
   const int n = (int)(a.layer_off[seg + 1] - begin);
   const int64_t raw_begin = a.raw_off ? a.raw_off[seg] : begin;  // frames share raw clusters
   const float vx = a.vtx[3 * e], vy = a.vtx[3 * e + 1], vz = a.vtx[3 * e + 2];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int *const hist = hist_all + warp * kBuckets;
+  int32_t *const stage = s_flags + 4 + warp * 32 * kClusterWords;
 
-  if (tid == 0 && layer == 0) {
+  // by input index: bucket and z; by sorted position: input index (perm), z, and where the cluster
+  // goes in its bin's z-sorted list (in the input z values' place)
+  uint32_t *const perm = a.sort_index + begin;
+  uint32_t *const bucket = perm + a.sort_stride;
+  float *const z_in = reinterpret_cast<float *>(bucket + a.sort_stride);
+  float *const z_at = z_in + a.sort_stride;
+  auto sync_segment = [&]() {
+    if (ctas == 1) {
+      __syncthreads();
+    } else {
+      cg::this_cluster().sync();
+    }
+  };
+
+  if (tid == 0 && layer == 0 && rank == 0) {
     const bool ok = isfinite(vx) && isfinite(vy) && isfinite(vz) && fabsf(vx) <= kMaxAbsCoordinate &&
                     fabsf(vy) <= kMaxAbsCoordinate && fabsf(vz) <= kMaxAbsCoordinate;
     if (!ok) {
@@ -400,16 +440,23 @@ __global__ void __launch_bounds__(kSortThreads) k_cluster_sort(Arena a)
       atomicMin(&a.status->invalid_event, e);
     }
   }
-  for (int k = tid; k < kSortWarps * kBuckets; k += kSortThreads) {
-    (&hist[0][0])[k] = 0;
+  for (int k = tid; k < kWarps * kBuckets; k += kThreads_) {
+    hist_all[k] = 0;
+  }
+  if (tid == 0) {
+    s_flags[0] = 0;
+    s_flags[1] = 0x7f800000;
+    s_flags[2] = 0;
+    s_flags[3] = 0;
   }
   __syncthreads();
 
   // Pass 1: transform every cluster (input order), per-warp bucket histograms. Each warp owns a
   // consecutive input range and moves it through its stage 32 clusters at a time.
-  int32_t *stage = stages[warp];
-  const int chunk = (n + kSortWarps - 1) / kSortWarps;
-  const int wb = min(n, warp * chunk), we = min(n, wb + chunk);
+  const int chunk = (n + ctas * kWarps - 1) / (ctas * kWarps);
+  const int wb = min(n, (rank * kWarps + warp) * chunk), we = min(n, wb + chunk);
+  float4 *const recs = a.sort_recs + 2 * begin;
+  unsigned irregular = 0, rmin = 0x7f800000u, rmax = 0;  // of r's float bits: r >= 0 orders like its bits
   for (int i0 = wb; i0 < we; i0 += 32) {
     const int count = min(32, we - i0);
     itsu_cluster c{};
@@ -425,259 +472,245 @@ __global__ void __launch_bounds__(kSortThreads) k_cluster_sort(Arena a)
         c.alpha = 0.0f;
         c.mc_id = __float_as_int(q.w);
       }
-    } else if (a.raw_in) {
-      // 24-byte input records (x, y, z, id, alpha, MC id): read in 6-word strides, then the stage
-      // is reused for the 36-byte records once every lane has read its own
-      stage_in_words<kClusterInWords>(stage, a.raw_in + raw_begin + i0, count);
-      if (lane < count) {
-        c = stage_get_in(stage, lane);
-      }
-      __syncwarp();
     } else {
-      stage_in(stage, a.raw + raw_begin + i0, count);
-      if (lane < count) {
-        c = stage_get(stage, lane);
+      __syncwarp();  // the stage is refilled
+      if (a.raw_in) {
+        stage_in_words<kClusterInWords>(stage, a.raw_in + raw_begin + i0, count);
+        if (lane < count) {
+          c = stage_get_in(stage, lane);
+        }
+      } else {
+        stage_in(stage, a.raw + raw_begin + i0, count);
+        if (lane < count) {
+          c = stage_get(stage, lane);
+        }
       }
     }
     if (lane < count) {
+      const int i = i0 + lane;
       const Transformed t = transform_cluster(layer, c.x, c.y, c.z, vx, vy);
-      c.phi = t.phi;
-      c.r = t.r;
-      c.bin = t.bin;
       const bool ok = isfinite(c.x) && isfinite(c.y) && isfinite(c.z) && fabsf(c.x) <= kMaxAbsCoordinate &&
                       fabsf(c.y) <= kMaxAbsCoordinate && fabsf(c.z) <= kMaxAbsCoordinate && !(t.r == 0.0f && c.z == vz);
       if (!ok) {
         atomicOr(&a.status->flags, kFlagInvalid);
-        atomicMin(&a.status->invalid_index, (int)(begin + i0 + lane));
+        atomicMin(&a.status->invalid_index, (int)(begin + i));
       }
-      stage_put(stage, lane, c);
-      atomicAdd(&hist[warp][bucket_of(t.bin)], 1);
+      recs[2 * i] = make_float4(c.x, c.y, c.z, t.r);
+      recs[2 * i + 1] = make_float4(t.phi, __int_as_float(c.cluster_id), c.alpha, __int_as_float(c.mc_id));
+      const int zb = z_bin_index(layer, c.z), pb = phi_bin_index(t.phi);
+      irregular |= zb < 0 || zb >= kZBins || pb < 0 || pb >= kPhiBins;
+      rmin = min(rmin, __float_as_uint(t.r));
+      rmax = max(rmax, __float_as_uint(t.r));
+      const int b = bucket_of(t.bin);
+      bucket[i] = (uint32_t)b;
+      z_in[i] = c.z;
+      atomicAdd(&hist[b], 1);
     }
-    stage_out(a.tmp + begin + i0, stage, count);
-    __syncwarp();  // the stage is refilled next
+  }
+  irregular = __reduce_or_sync(0xffffffffu, irregular);
+  rmin = __reduce_min_sync(0xffffffffu, rmin);
+  rmax = __reduce_max_sync(0xffffffffu, rmax);
+  if (lane == 0) {
+    atomicOr(&s_flags[0], (int)irregular);
+    atomicMin(&s_flags[1], (int)rmin);
+    atomicMax(&s_flags[2], (int)rmax);
   }
   __syncthreads();
 
-  // Pass 2: per-bucket prefix over warps, exclusive scan over buckets, index table.
-  for (int b = tid; b < kBuckets; b += kSortThreads) {
+  // Pass 2: per-bucket prefix over warps (and CTAs), exclusive scan over buckets, index table.
+  for (int b = tid; b < kBuckets; b += kThreads_) {
     int s = 0;
-    for (int w = 0; w < kSortWarps; ++w) {
-      const int v = hist[w][b];
-      hist[w][b] = s;
+    for (int w = 0; w < kWarps; ++w) {
+      const int v = hist_all[w * kBuckets + b];
+      hist_all[w * kBuckets + b] = s;
       s += v;
     }
+    cta_total[b] = s;
     bucket_total[b] = s;
   }
-  __syncthreads();
-  if (warp == 0) {
-    constexpr int per = (kBuckets + 31) / 32;
-    const int b0 = lane * per, b1 = min(kBuckets, b0 + per);
-    int local = 0;
-    for (int b = b0; b < b1; ++b) {
-      local += bucket_total[b];
+  sync_segment();
+  int seg_irregular = s_flags[0], seg_rmin = s_flags[1], seg_rmax = s_flags[2];
+  if (ctas > 1) {
+    for (int c = 0; c < ctas; ++c) {
+      const int *other = cg::this_cluster().map_shared_rank(s_flags, c);
+      seg_irregular |= other[0];
+      seg_rmin = min(seg_rmin, other[1]);
+      seg_rmax = max(seg_rmax, other[2]);
     }
-    int inc = local;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, inc, d);
-      if (lane >= d) {
-        inc += t;
+    for (int b = tid; b < kBuckets; b += kThreads_) {
+      int before = 0, all = 0;
+      for (int c = 0; c < ctas; ++c) {
+        const int v = cg::this_cluster().map_shared_rank(cta_total, c)[b];
+        before += c < rank ? v : 0;
+        all += v;
+      }
+      bucket_total[b] = all;
+      for (int w = 0; w < kWarps; ++w) {
+        hist_all[w * kBuckets + b] += before;
       }
     }
-    int run = inc - local;
-    for (int b = b0; b < b1; ++b) {
-      bucket_base[b] = run;
-      run += bucket_total[b];
+    __syncthreads();
+  }
+  int largest = 0;
+  for (int b0 = 0, carry = 0; b0 < kBuckets; b0 += kThreads_) {
+    const int b = b0 + tid;
+    const int v = b < kBuckets ? bucket_total[b] : 0;
+    int total;
+    const int ex = block_exclusive_scan<int>(v, scan_totals, total);
+    if (b < kBuckets) {
+      bucket_base[b] = carry + ex;
+      if (b > 0 && b <= kTableBins) {
+        largest = max(largest, v);
+      }
     }
+    carry += total;
+  }
+  largest = __reduce_max_sync(0xffffffffu, (unsigned)largest);
+  if (lane == 0) {
+    atomicMax(&s_flags[3], largest);
   }
   __syncthreads();
-  for (int b = tid; b < kBuckets; b += kSortThreads) {
-    const int base = bucket_base[b];
-    for (int w = 0; w < kSortWarps; ++w) {
-      hist[w][b] += base;
-    }
-  }
+  largest = s_flags[3];
   if (layer > 0) {
     // table[b] = first sorted index with bin >= b = #clusters with bin < b for b >= 1; table[0] = 0
     // (PrimaryVertexContext.cxx:90-119: negative bins never move the fill cursor off bin 0).
     int32_t *table = a.index_tables + ((int64_t)e * ITSU_TRACKLET_LAYERS + layer - 1) * kTableSize;
-    for (int b = tid; b < kTableSize; b += kSortThreads) {
+    for (int b = rank * kThreads_ + tid; b < kTableSize; b += ctas * kThreads_) {
       table[b] = b == 0 ? 0 : bucket_base[b + 1];
     }
   }
-  __syncthreads();
 
-  // Pass 3: stable scatter. Warps own consecutive input ranges whose bucket offsets were
-  // prefixed in warp order; inside a warp, lanes of equal bucket rank by lane order.
+  // Pass 3: each cluster's sorted position. Warps own consecutive input ranges whose bucket offsets
+  // were prefixed in warp order; inside a warp, lanes of equal bucket rank by lane order.
   for (int i0 = wb; i0 < we; i0 += 32) {
-    const int count = min(32, we - i0);
-    stage_in(stage, a.tmp + begin + i0, count);
-    const bool valid = lane < count;
-    itsu_cluster c;
-    int bucket = -1 - lane;
-    if (valid) {
-      c = stage_get(stage, lane);
-      bucket = bucket_of(c.bin);
-    }
-    const unsigned peers = __match_any_sync(0xffffffffu, bucket);
-    const int rank = __popc(peers & ((1u << lane) - 1u));
+    const int i = i0 + lane;
+    const bool valid = i < we;
+    const int b = valid ? (int)bucket[i] : -1 - lane;
+    const unsigned peers = __match_any_sync(0xffffffffu, b);
+    const int before = __popc(peers & ((1u << lane) - 1u));
     int pos = 0;
     if (valid) {
-      pos = hist[warp][bucket] + rank;
+      pos = bucket_base[b] + hist[b] + before;
+      perm[pos] = (uint32_t)i;
+      z_at[pos] = z_in[i];
     }
     __syncwarp();
-    if (valid && lane == 31 - __clz(peers)) {
-      hist[warp][bucket] += __popc(peers);
+    if (valid && (peers >> lane) == 1u) {  // the highest lane of its bucket
+      hist[b] += before + 1;
     }
     __syncwarp();
-    if (valid) {
-      const int64_t at = begin + pos;
-      a.xyzr[at] = make_float4(c.x, c.y, c.z, c.r);
-      a.phi[at] = c.phi;
-      a.clu_aux[at] = make_int4(c.cluster_id, __float_as_int(c.alpha), c.mc_id, c.bin);
+  }
+  sync_segment();
+
+  // Negative bins share bucket 0 in input order; order them by bin, stably. A bottom-up merge sort of
+  // (bin, input index) between (z_at, perm) and (z_in, bucket), all free for such a layer: in each
+  // round, runs of `width` are merged in pairs, every cluster moving to (its place in its run) + (the
+  // clusters of the partner run that go before it: smaller bins, and for the right run equal bins
+  // too), so ties keep input order. O(m log^2 m) work, for layers with many clusters beyond the z range.
+  const int m = bucket_total[0];
+  if (m > 1) {
+    if (rank == 0) {
+      int *key = reinterpret_cast<int *>(z_at), *key_to = reinterpret_cast<int *>(z_in);
+      uint32_t *idx = perm, *idx_to = bucket;
+      for (int i = tid; i < m; i += kThreads_) {
+        const int from = (int)perm[i];
+        key[i] = bin_index(z_bin_index(layer, recs[2 * from].z), phi_bin_index(recs[2 * from + 1].x));
+      }
+      for (int width = 1; width < m; width *= 2) {
+        __syncthreads();
+        for (int i = tid; i < m; i += kThreads_) {
+          const int run = i / width;
+          const bool left = (run & 1) == 0;
+          const int own_start = run * width;
+          const int other_start = left ? own_start + width : own_start - width;
+          const int other_end = min(other_start + width, m);
+          const int k = key[i];
+          int lo = other_start, hi = max(other_start, other_end);  // an empty partner run: no move
+          while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (key[mid] < k || (!left && key[mid] == k)) {
+              lo = mid + 1;
+            } else {
+              hi = mid;
+            }
+          }
+          const int to = min(own_start, other_start) + (i - own_start) + (lo - other_start);
+          key_to[to] = k;
+          idx_to[to] = idx[i];
+        }
+        int *const t = key;
+        key = key_to;
+        key_to = t;
+        uint32_t *const u = idx;
+        idx = idx_to;
+        idx_to = u;
+      }
+      __syncthreads();
+      if (idx != perm) {
+        for (int i = tid; i < m; i += kThreads_) {
+          perm[i] = idx[i];
+        }
+      }
+    }
+    sync_segment();
+  }
+
+  // The tracklet stage's candidate-pruning index. A layer is regular when every cluster has a z bin
+  // and a phi bin inside the 20 x 20 table (then a bin's column is its clusters' z bin) and no bin
+  // holds more than kMaxPruneBin clusters; for regular layers, each bin's clusters are listed again
+  // sorted by (z, sorted index), with the layer's r range beside. (Layer 0 is never the outer layer
+  // of a tracklet.)
+  const bool regular = a.zs != nullptr && layer > 0 && !seg_irregular && m == 0 && bucket_total[kBuckets - 1] == 0 && largest <= kMaxPruneBin;
+  uint32_t *const z_rank = reinterpret_cast<uint32_t *>(z_in);  // by sorted position
+  if (regular) {
+    for (int pos = rank * kThreads_ + tid; pos < n; pos += ctas * kThreads_) {
+      const int b = (int)bucket[perm[pos]];
+      const int st = bucket_base[b], en = st + bucket_total[b];
+      const float z = z_at[pos];
+      int at = st;
+      for (int j = st; j < en; ++j) {
+        const float zj = z_at[j];
+        at += zj < z || (zj == z && j < pos);
+      }
+      z_rank[pos] = (uint32_t)at;
     }
   }
-  __syncthreads();
-
-  // Pass 3b: the sorted records (reference layout) assembled from the scattered fields, in
-  // output order, through the stages: coalesced stores instead of nine scattered ones per cluster.
-  for (int i0 = warp * 32; i0 < n; i0 += kSortThreads) {
+  if (a.zs != nullptr && layer > 0 && rank == 0 && tid == 0) {
+    // 0: not regular; else the 64-bit words of a pass mask over its largest bin (1, 2 or 4)
+    a.seg_regular[seg] = !regular ? 0 : (largest <= 64 ? 1 : (largest <= 128 ? 2 : kPruneWords));
+    a.seg_rrange[seg] = make_float2(__int_as_float(seg_rmin), __int_as_float(seg_rmax));
+  }
+  // Pass 4: every output in sorted order.
+  for (int i0 = (rank * kWarps + warp) * 32; i0 < n; i0 += ctas * kThreads_) {
     const int count = min(32, n - i0);
+    __syncwarp();  // the stage is refilled
     if (lane < count) {
-      const int64_t at = begin + i0 + lane;
-      const float4 p = a.xyzr[at];
-      const int4 x = a.clu_aux[at];
+      const int pos = i0 + lane;
+      const int64_t at = begin + pos;
+      const int i = (int)perm[pos];
+      const float4 p = recs[2 * i], q = recs[2 * i + 1];
       itsu_cluster c;
       c.x = p.x;
       c.y = p.y;
       c.z = p.z;
-      c.phi = a.phi[at];
+      c.phi = q.x;
       c.r = p.w;
-      c.cluster_id = x.x;
-      c.alpha = __int_as_float(x.y);
-      c.mc_id = x.z;
-      c.bin = x.w;
+      c.cluster_id = __float_as_int(q.y);
+      c.alpha = q.z;
+      c.mc_id = __float_as_int(q.w);
+      c.bin = bin_index(z_bin_index(layer, c.z), phi_bin_index(c.phi));
       stage_put(stage, lane, c);
-      if (a.clu_seg) {
+      if (a.xyzr) {
+        a.xyzr[at] = p;
+        a.phi[at] = c.phi;
+        a.clu_aux[at] = make_int4(c.cluster_id, __float_as_int(c.alpha), c.mc_id, c.bin);
         a.clu_seg[at] = seg;
+      }
+      if (regular) {
+        a.zs[begin + z_rank[pos]] = make_float4(c.z, c.r, c.phi, __int_as_float(pos));
       }
     }
     stage_out(a.sorted + begin + i0, stage, count);
-    __syncwarp();  // the stage is refilled next
-  }
-
-  // Pass 4: negative bins share bucket 0 in input order; order them by bin, stably. A bottom-up
-  // merge sort between the sorted segment and tmp: in each round, runs of `width` are merged in
-  // pairs, every cluster moving to (its place in its run) + (the clusters of the partner run that
-  // go before it: smaller bins, and for the right run equal bins too), so ties keep input order.
-  // O(m log^2 m) work over the block, for layers with many clusters beyond the z range.
-  const int m = bucket_total[0];
-  if (m > 1) {
-    itsu_cluster *src = a.sorted + begin, *dst = a.tmp + begin;
-    for (int width = 1; width < m; width *= 2) {
-      __syncthreads();
-      for (int i = tid; i < m; i += kSortThreads) {
-        const int run = i / width;
-        const bool left = (run & 1) == 0;
-        const int own_start = run * width;
-        const int other_start = left ? own_start + width : own_start - width;
-        const int other_end = min(other_start + width, m);
-        const itsu_cluster c = src[i];
-        int lo = other_start, hi = max(other_start, other_end);  // an empty partner run: no move
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          const int k = src[mid].bin;
-          if (k < c.bin || (!left && k == c.bin)) {
-            lo = mid + 1;
-          } else {
-            hi = mid;
-          }
-        }
-        dst[min(own_start, other_start) + (i - own_start) + (lo - other_start)] = c;
-      }
-      itsu_cluster *t = src;
-      src = dst;
-      dst = t;
-    }
-    __syncthreads();
-    for (int i = tid; i < m; i += kSortThreads) {
-      const itsu_cluster c = src[i];
-      if (src != a.sorted + begin) {
-        a.sorted[begin + i] = c;
-      }
-      a.xyzr[begin + i] = make_float4(c.x, c.y, c.z, c.r);
-      a.phi[begin + i] = c.phi;
-    }
-  }
-
-  // Pass 5: the tracklet stage's candidate-pruning index. A layer is regular when every cluster
-  // has a z bin and a phi bin inside the 20 x 20 table (then a bin's column is its clusters' z
-  // bin) and no bin holds more than kMaxPruneBin clusters; for regular layers, each bin's
-  // clusters are listed again sorted by (z, sorted index), with the layer's r range beside.
-  if (a.zs == nullptr || layer == 0) {
-    return;  // no index wanted, or layer 0 (never the outer layer of a tracklet)
-  }
-  __shared__ int s_irregular;
-  __shared__ int s_rmin, s_rmax;  // float bits; r >= 0 orders like its bits
-  __shared__ int s_largest;       // the largest bin
-  if (tid == 0) {
-    s_irregular = m > 0 || bucket_total[kBuckets - 1] > 0;  // negative bins or bin 400
-    s_rmin = 0x7f800000;
-    s_rmax = 0;
-    s_largest = 0;
-  }
-  __syncthreads();
-  int irregular = 0, rmin = 0x7f800000, rmax = 0;
-  for (int i = tid; i < n; i += kSortThreads) {
-    const float4 c = a.xyzr[begin + i];
-    const int zb = z_bin_index(layer, c.z);
-    const int pb = phi_bin_index(a.phi[begin + i]);
-    irregular |= zb < 0 || zb >= kZBins || pb < 0 || pb >= kPhiBins;
-    rmin = min(rmin, __float_as_int(c.w));
-    rmax = max(rmax, __float_as_int(c.w));
-  }
-  if (irregular) {
-    atomicOr(&s_irregular, 1);
-  }
-  atomicMin(&s_rmin, rmin);
-  atomicMax(&s_rmax, rmax);
-  int largest = 0;
-  for (int b = tid; b < kTableBins; b += kSortThreads) {
-    largest = max(largest, bucket_total[b + 1]);
-  }
-  if (largest > kMaxPruneBin) {
-    atomicOr(&s_irregular, 1);
-  }
-  atomicMax(&s_largest, largest);
-  // each cluster's rank in its bin by (z, sorted index): a warp per bin of at most kMaxPruneBin
-  // (256) clusters, the bin's z values staged in the warp's record stage (free in this pass)
-  static_assert(kMaxPruneBin <= 32 * kClusterWords, "a bin's z values fit a warp's stage");
-  float *zstage = reinterpret_cast<float *>(stage);
-  for (int bin = warp; bin < kTableBins; bin += kSortWarps) {
-    const int st = bucket_base[bin + 1], cnt = bucket_total[bin + 1];
-    if (cnt == 0 || cnt > kMaxPruneBin) {
-      continue;  // warp-uniform
-    }
-    for (int k = lane; k < cnt; k += 32) {
-      zstage[k] = a.xyzr[begin + st + k].z;
-    }
-    __syncwarp();
-    for (int k = lane; k < cnt; k += 32) {
-      const float4 c = a.xyzr[begin + st + k];
-      int rank = 0;
-      for (int j = 0; j < cnt; ++j) {
-        const float zj = zstage[j];
-        rank += zj < c.z || (zj == c.z && j < k);
-      }
-      a.zs[begin + st + rank] = make_float4(c.z, c.w, a.phi[begin + st + k], __int_as_float(st + k));
-    }
-    __syncwarp();  // the stage is refilled for the warp's next bin
-  }
-  __syncthreads();
-  if (tid == 0) {
-    // 0: not regular; else the 64-bit words of a pass mask over its largest bin (1, 2 or 4)
-    a.seg_regular[seg] = s_irregular ? 0 : (s_largest <= 64 ? 1 : (s_largest <= 128 ? 2 : kPruneWords));
-    a.seg_rrange[seg] = make_float2(__int_as_float(s_rmin), __int_as_float(s_rmax));
   }
 }
 
@@ -2211,10 +2244,39 @@ void step_status_init(const Arena &a, const Launch &l)
   k_status_init<<<(unsigned)std::max<int64_t>(blocks, 1), kThreads, 0, l.stream>>>(a);
 }
 
+template <int kThreads_>
+void launch_sort(const Arena &a, const Launch &l, int ctas)
+{
+  const size_t bytes = sort_shared_bytes(kThreads_ / 32);
+  if (bytes > 48 * 1024) {
+    cudaFuncSetAttribute(k_cluster_sort<kThreads_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  }
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3((unsigned)(a.n_events * ITSU_LAYERS * ctas));
+  config.blockDim = dim3(kThreads_);
+  config.dynamicSmemBytes = bytes;
+  config.stream = l.stream;
+  cudaLaunchAttribute cluster{};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = (unsigned)ctas;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  config.attrs = &cluster;
+  config.numAttrs = ctas > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&config, k_cluster_sort<kThreads_>, a);
+}
+
 void step_cluster_sort(const Arena &a, const Launch &l)
 {
-  if (a.n_events > 0) {
-    k_cluster_sort<<<a.n_events * ITSU_LAYERS, kSortThreads, 0, l.stream>>>(a);
+  if (a.n_events <= 0) {
+    return;
+  }
+  const SortShape shape = sort_shape(a.n_events, a.n_clusters, l.max_segment);
+  if (shape.threads == 64) {
+    launch_sort<64>(a, l, shape.ctas);
+  } else if (shape.threads == 256) {
+    launch_sort<256>(a, l, shape.ctas);
+  } else {
+    launch_sort<512>(a, l, shape.ctas);
   }
 }
 
@@ -2408,6 +2470,24 @@ void run_steps(int first, int last, const Arena &a, const Launch &l)
 }
 
 }  // namespace
+
+// The clustering's launch for a run whose largest layer has max_segment clusters (any shape gives the
+// same results). Small layers take small CTAs: the tables' set-up is most of their work. Layers of
+// even size are split over clusters of 2 to 8 CTAs while that makes no more than 1024 of them (about
+// three waves), so that the last wave is not nearly empty; where the sizes differ widely, the large
+// ones only while the chip has room for all of them at once.
+SortShape sort_shape(int32_t n_events, int64_t n_clusters, int64_t max_segment)
+{
+  const int64_t segments = (int64_t)n_events * ITSU_LAYERS;
+  SortShape s;
+  s.threads = max_segment > 1024 ? 512 : (max_segment > 192 ? 256 : 64);
+  s.ctas = 1;
+  const int64_t most = 2 * n_clusters >= segments * max_segment ? 1024 : 296;
+  while (max_segment > 1024 && s.ctas < 8 && 2 * s.ctas * segments <= most) {
+    s.ctas *= 2;
+  }
+  return s;
+}
 
 // Streamed host runs: appends the last run's roads and road offsets to the batch-wide output at
 // event e0. The chunk's first road index is dst_off[e0], written by the previous chunk (or zeroed

@@ -5,8 +5,7 @@
 // pool), or a latency-critical loop where an allocation's implicit device synchronisation is not
 // acceptable. itsu_pvc_initialize_noalloc serves them: the caller passes device inputs and
 // outputs, and the only scratch the kernel needs (the transformed clusters in input order, the
-// coordinate copies the sort writes beside its output, and the status word) lives in the
-// file-scope array below, which every GPU that loads the library holds until the process exits.
+// sort's index arrays, and the status word) lives in the file-scope array below, which every GPU that loads the library holds until the process exits.
 //
 // In host code, itsu_noalloc_scratch names a host-side stand-in, not the device array: its
 // device address is obtained once per device with cudaGetSymbolAddress, with that device current,
@@ -20,6 +19,7 @@
 // at the same time) race on the array.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -34,13 +34,11 @@ namespace {
 constexpr int64_t kMaxClusters = ITSU_NOALLOC_MAX_CLUSTERS;
 constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t n) { return (n + kAlign - 1) / kAlign * kAlign; }
-// layout: DevStatus | transformed clusters | xyzr | phi | per-cluster id, alpha, MC id, bin
+// layout: DevStatus | transformed records | sort index arrays
 constexpr size_t kStatusOff = 0;
-constexpr size_t kTmpOff = align_up(sizeof(itsu::DevStatus));
-constexpr size_t kXyzrOff = kTmpOff + align_up(sizeof(itsu_cluster) * kMaxClusters);
-constexpr size_t kPhiOff = kXyzrOff + align_up(sizeof(float4) * kMaxClusters);
-constexpr size_t kAuxOff = kPhiOff + align_up(sizeof(float) * kMaxClusters);
-constexpr size_t kScratchBytes = kAuxOff + align_up(sizeof(int4) * kMaxClusters);
+constexpr size_t kRecsOff = align_up(sizeof(itsu::DevStatus));
+constexpr size_t kIndexOff = kRecsOff + align_up(2 * sizeof(float4) * kMaxClusters);
+constexpr size_t kScratchBytes = kIndexOff + align_up(4 * sizeof(uint32_t) * kMaxClusters);
 
 static __device__ __align__(256) unsigned char itsu_noalloc_scratch[kScratchBytes];
 
@@ -115,11 +113,13 @@ extern "C" itsu_status itsu_pvc_initialize_noalloc(const itsu_cluster *clusters,
   a.sorted = sorted;
   a.index_tables = index_tables;
   a.status = reinterpret_cast<itsu::DevStatus *>(scratch + kStatusOff);
-  a.tmp = reinterpret_cast<itsu_cluster *>(scratch + kTmpOff);
-  a.xyzr = reinterpret_cast<float4 *>(scratch + kXyzrOff);
-  a.phi = reinterpret_cast<float *>(scratch + kPhiOff);
-  a.clu_aux = reinterpret_cast<int4 *>(scratch + kAuxOff);
-  const itsu::Launch l{stream, 0, 256, 8};
+  a.sort_recs = reinterpret_cast<float4 *>(scratch + kRecsOff);
+  a.sort_index = reinterpret_cast<uint32_t *>(scratch + kIndexOff);
+  a.sort_stride = kMaxClusters;
+  itsu::Launch l{stream, 0, 256, 8};
+  for (int layer = 0; layer < ITSU_LAYERS; ++layer) {
+    l.max_segment = std::max<int64_t>(l.max_segment, off[layer + 1] - off[layer]);
+  }
   itsu::launch_status_init(a, l);
   itsu::launch_cluster_sort(a, l);
   if ((err = cudaGetLastError()) != cudaSuccess) {
