@@ -104,7 +104,7 @@ struct itsu_context {
   itsu::CellEntry *cell_entries = nullptr;
   float *cell_dca = nullptr;
   int64_t cap_cell_entries = 0;
-  int32_t *cell_seg_id = nullptr, *nb_count = nullptr, *nb_off = nullptr, *nb_fill = nullptr, *road_count = nullptr,
+  int32_t *cell_seg_id = nullptr, *nb_count = nullptr, *nb_off = nullptr, *road_count = nullptr,
           *road_off = nullptr;
   int64_t *paths = nullptr;
   unsigned long long *nb_mask = nullptr;  // per cell, its passing candidates (neighbour count pass)
@@ -149,6 +149,7 @@ struct itsu_context {
   int graph_tune[4] = {0, 0, -1, -1};
   bool graph_prefilter = false;
   itsu::SortShape graph_sort{};
+  itsu::LevelShape graph_levels{};
   bool graph_gate = false;
 
   // streamed host runs (ITSU_FLAG_STREAM_HOST): upload stream, per-chunk events, batch-wide roads
@@ -368,7 +369,6 @@ Arena arena_of(const itsu_context *ctx)
   a.cap_cell_entries = ctx->cap_cell_entries;
   a.nb_count = ctx->nb_count;
   a.nb_off = ctx->nb_off;
-  a.nb_fill = ctx->nb_fill;
   a.nb_mask = ctx->nb_mask;
   a.nb = ctx->nb;
   a.paths = ctx->paths;
@@ -379,6 +379,7 @@ Arena arena_of(const itsu_context *ctx)
   a.mlp = ctx->prefilter ? ctx->d_mlp : nullptr;
   a.gate = ctx->gate ? ctx->d_gate : nullptr;
   a.scan_partials = ctx->scan_partials;
+  a.road_partials = ctx->scan_partials + ctx->cap_partials;
   a.status = ctx->d_status;
   a.cap_tracklets = ctx->cap_tracklets;
   a.cap_cells = ctx->cap_cells;
@@ -403,7 +404,7 @@ itsu_status ensure_partials(itsu_context *ctx)
 {
   const int64_t need = std::max({ctx->cap_clusters, ctx->cap_tracklets, ctx->cap_cells}) / 2048 + 2;
   if (need > ctx->cap_partials) {
-    ITSU_CUDA(ctx, alloc(ctx, ctx->scan_partials, need));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->scan_partials, 2 * need));
     ctx->cap_partials = need;
     ctx->generation++;
   }
@@ -509,7 +510,6 @@ itsu_status ensure_cell_outputs(itsu_context *ctx, int64_t need)
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_seg_id, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->nb_count, cap + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->nb_off, cap + 1));
-    ITSU_CUDA(ctx, alloc(ctx, ctx->nb_fill, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->nb_mask, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->paths, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->road_count, cap + 1));
@@ -647,7 +647,9 @@ itsu_status launch_all(itsu_context *ctx)
 {
   const Tune tune = current_tune(ctx);
   const itsu::SortShape sort = itsu::sort_shape(ctx->n_events, ctx->n_clusters, ctx->max_segment);
+  const itsu::LevelShape levels = itsu::level_shape(ctx->max_segment);
   const bool same = ctx->graph && sort.threads == ctx->graph_sort.threads && sort.ctas == ctx->graph_sort.ctas &&
+                    levels.threads == ctx->graph_levels.threads && levels.ctas == ctx->graph_levels.ctas &&
                     ctx->graph_generation == ctx->generation && ctx->graph_key[0] == ctx->in_raw &&
                     ctx->graph_tune[0] == tune.block && ctx->graph_tune[1] == tune.blocks_per_sm &&
                     ctx->graph_tune[2] == tune.prune && ctx->graph_tune[3] == tune.group && ctx->graph_prefilter == ctx->prefilter &&
@@ -687,6 +689,7 @@ itsu_status launch_all(itsu_context *ctx)
     ctx->graph_tune[3] = tune.group;
     ctx->graph_prefilter = ctx->prefilter;
     ctx->graph_sort = sort;
+    ctx->graph_levels = levels;
     ctx->graph_gate = ctx->gate;
     ctx->graph_events = ctx->n_events;
     ctx->graph_clusters = ctx->n_clusters;
@@ -744,7 +747,9 @@ itsu_status stage_count_then_write(itsu_context *ctx, void (*count)(const Arena 
     ITSU_CUDA(ctx, cudaMemsetAsync(&ctx->d_status->cell_entries, 0, 4 * sizeof(int64_t), ctx->stream));
     ITSU_CUDA(ctx, cudaMemsetAsync(ctx->scan_partials, 0, sizeof(int64_t) * ctx->cap_partials, ctx->stream));
     ITSU_CUDA(ctx, cudaMemsetAsync(ctx->cell_seg_count, 0, sizeof(int32_t) * ITSU_CELL_LAYERS * ctx->n_events, ctx->stream));
-    count(arena_of(ctx), launch_of(ctx));
+    Launch l = launch_of(ctx);
+    l.staged = true;
+    count(arena_of(ctx), l);
     if ((st = check_launch(ctx)) != ITSU_OK) return st;
     if ((st = sync_status(ctx)) != ITSU_OK) return st;
     // the cell count pass keeps its entries for the write: if they overflowed their scratch,
@@ -765,7 +770,9 @@ itsu_status stage_count_then_write(itsu_context *ctx, void (*count)(const Arena 
     if ((st = ensure(ctx, s.total[total_index])) != ITSU_OK) return st;
     if ((st = clear_flags(ctx)) != ITSU_OK) return st;
   }
-  write(arena_of(ctx), launch_of(ctx));
+  Launch l = launch_of(ctx);
+  l.staged = true;
+  write(arena_of(ctx), l);
   if ((st = check_launch(ctx)) != ITSU_OK) return st;
   if ((st = sync_status(ctx)) != ITSU_OK) return st;
   if (ctx->h_status->flags & itsu::kCapacityMask) {
@@ -977,7 +984,7 @@ void itsu_context_destroy(itsu_context *ctx)
   release(ctx->layer_off); release(ctx->index_tables); release(ctx->trk_seg); release(ctx->cell_seginfo); release(ctx->cell_seg); release(ctx->cell_seg_count);
   release(ctx->road_seg); release(ctx->vtx);
   release(ctx->tracklets); release(ctx->trk_key); release(ctx->trk_seg_id); release(ctx->cell_span); release(ctx->cell_span_count); release(ctx->cell_span_off); release(ctx->cell_lookup);
-  release(ctx->cells); release(ctx->cell_entries); release(ctx->cell_dca); release(ctx->cell_seg_id); release(ctx->nb_count); release(ctx->nb_off); release(ctx->nb_fill);
+  release(ctx->cells); release(ctx->cell_entries); release(ctx->cell_dca); release(ctx->cell_seg_id); release(ctx->nb_count); release(ctx->nb_off);
   release(ctx->nb_mask);
   release(ctx->road_count); release(ctx->road_off); release(ctx->paths);
   release(ctx->nb); release(ctx->roads); release(ctx->scan_partials); release(ctx->d_status);

@@ -133,7 +133,6 @@ struct Arena {
   // neighbours, levels, roads
   int32_t *nb_count;
   int32_t *nb_off;
-  int32_t *nb_fill;
   unsigned long long *nb_mask;  // per cell of layers 0-3: its candidates that pass the cut (up to 64)
   int32_t *nb;
   int64_t *paths;  // per cell: its chain count and level (chain_word)
@@ -147,6 +146,7 @@ struct Arena {
   const GateDevice *gate;
   // scan scratch and status
   int64_t *scan_partials;
+  int64_t *road_partials;  // tile sums of the road scan (added up in the stage before it)
   DevStatus *status;
   // capacities of the growable outputs
   int64_t cap_tracklets, cap_cells, cap_neighbours, cap_roads;
@@ -165,6 +165,7 @@ struct Launch {
   int group_events = 0;
   const int64_t *groups = nullptr;
   int64_t max_segment = 0;  // clusters of the run's largest layer
+  bool staged = false;      // a stage call, whose outputs may have to grow between its count and its write
 };
 
 // How the clustering is launched.
@@ -172,6 +173,12 @@ struct SortShape {
   int threads, ctas;
 };
 SortShape sort_shape(int32_t n_events, int64_t n_clusters, int64_t max_segment);
+
+// How the level pass is launched.
+struct LevelShape {
+  int threads, ctas;
+};
+LevelShape level_shape(int64_t max_segment);
 
 // Stage launchers (asynchronous on l.stream).
 void launch_status_init(const Arena &a, const Launch &l);
@@ -217,12 +224,12 @@ void launch_report(const ReportArgs &r, cudaStream_t stream, int num_sms);
 // Every kernel of a run, in launch order, with its name (the instrumentation API times them
 // one by one). The stage launchers above enqueue consecutive ranges of this table.
 // KernelStep::learned_only: the forms a step launches in (0: every run)
-enum : int { kPairPrefilterStep = 1, kGateStep = 2, kGroupedStep = 3, kUngroupedStep = 4 };
+enum : int { kPairPrefilterStep = 1, kGateStep = 2, kGroupedStep = 3, kUngroupedStep = 4, kStagedStep = 5 };
 struct KernelStep {
   const char *name;
   void (*launch)(const Arena &, const Launch &);
   int learned_only;  // 0, or the only form that launches it: a learned network's (kPairPrefilterStep, kGateStep),
-                     // runs with event groups (kGroupedStep) or without (kUngroupedStep)
+                     // runs with event groups (kGroupedStep) or without (kUngroupedStep), stage calls (kStagedStep)
 };
 const KernelStep *pipeline_steps(int *count);
 int kernels_per_run();  // kernels one plain run launches (the learned form adds the learned_only steps)

@@ -85,8 +85,7 @@ __global__ void k_status_init(Arena a)
 __global__ void k_flag_bad_launch(DevStatus *s) { atomicOr(&s->flags, kFlagLaunchShape); }
 
 // ------------------------------------------------------------------------------------------
-// exclusive scan of int32 counts (tile sums, scan of tile sums, tile scans; the tracklet and
-// cell count passes fill their scans' tile sums themselves)
+// exclusive scan of int32 counts (the count passes fill the scans' tile sums)
 
 __device__ __forceinline__ int64_t scan_length(const int64_t *n_dev, int64_t n_host) { return n_dev ? *n_dev : n_host; }
 
@@ -131,78 +130,49 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T *warp_totals, T &block_
   return res;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int32_t *__restrict__ in, const int64_t *n_dev,
-                                                             int64_t n_host, int64_t *partials, const DevStatus *status)
-{
-  __shared__ int64_t warp_totals[33];
-  if (capacity_failed(status)) {
-    return;
-  }
-  const int64_t n = scan_length(n_dev, n_host);
-  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-    const int64_t base = t * kScanTile + (int64_t)threadIdx.x * kScanItems;
-    int64_t sum = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      if (base + k < n) {
-        sum += in[base + k];
-      }
-    }
-    int64_t total;
-    block_exclusive_scan<int64_t>(sum, warp_totals, total);
-    if (threadIdx.x == 0) {
-      partials[t] = total;
-    }
-  }
-}
+// One kernel per scan: the count passes have added each tile's counts up (partials), and a block
+// sums the tile sums before its tiles itself (at most a few thousand of them, from L2) instead of
+// taking them from a kernel of its own. The last tile's block checks the total. own_flag: the
+// capacity flag this scan may raise, which must not stop its own later blocks (the offsets are kept
+// when the stage's outputs are grown). kCellSegments: the grid's last block turns the segments' cell
+// counts into cell_seg meanwhile.
+__device__ void cell_segments(const Arena &a, int64_t *warp_totals);
 
-__global__ void __launch_bounds__(1024) k_scan_partials(int64_t *partials, const int64_t *n_dev, int64_t n_host,
-                                                        int32_t *out, int64_t *total_out, DevStatus *status)
+template <bool kCellSegments>
+__global__ void __launch_bounds__(kScanThreads) k_scan(Arena a, const int32_t *__restrict__ in, int32_t *__restrict__ out,
+                                                       const int64_t *n_dev, int64_t n_host, const int64_t *__restrict__ partials,
+                                                       int64_t *total_out, int64_t cap, int32_t own_flag)
 {
   __shared__ int64_t warp_totals[33];
-  if (capacity_failed(status)) {
+  DevStatus *const status = a.status;
+  if ((*(volatile const int32_t *)&status->flags & kCapacityMask & ~own_flag) != 0) {
     return;
   }
-  const int64_t n = scan_length(n_dev, n_host);
-  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  int64_t carry = 0;
-  for (int64_t t0 = 0; t0 < tiles; t0 += blockDim.x) {
-    const int64_t t = t0 + threadIdx.x;
-    const int64_t v = t < tiles ? partials[t] : 0;
-    int64_t total;
-    const int64_t ex = block_exclusive_scan<int64_t>(v, warp_totals, total);
-    if (t < tiles) {
-      partials[t] = carry + ex;
-    }
-    carry += total;
-  }
-  if (threadIdx.x == 0) {
-    *total_out = carry;
-    out[n] = (int32_t)carry;
-    if (carry > INT_MAX) {
-      atomicOr(&status->flags, kFlagCountOverflow);
+  int blocks = gridDim.x;
+  if constexpr (kCellSegments) {
+    --blocks;
+    if ((int)blockIdx.x == blocks) {
+      cell_segments(a, warp_totals);
+      return;
     }
   }
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int32_t *__restrict__ in, int32_t *__restrict__ out,
-                                                            const int64_t *n_dev, int64_t n_host,
-                                                            const int64_t *__restrict__ partials, const DevStatus *status)
-{
-  __shared__ int64_t warp_totals[33];
-  if (capacity_failed(status)) {
-    return;
-  }
   const int64_t n = scan_length(n_dev, n_host);
-  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+  const int64_t tiles = max((n + kScanTile - 1) / kScanTile, (int64_t)1);  // an empty scan has a total too
+  int64_t before = 0, summed = 0;  // the sum of the tiles below `summed`
+  for (int64_t t = blockIdx.x; t < tiles; t += blocks) {
+    int64_t part = 0, total;
+    for (int64_t k = summed + threadIdx.x; k < t; k += kScanThreads) {
+      part += partials[k];
+    }
+    block_exclusive_scan<int64_t>(part, warp_totals, total);
+    before += total;
+    summed = t;
     const int64_t base = t * kScanTile + (int64_t)threadIdx.x * kScanItems;
     int32_t v[kScanItems];
     if (base + kScanItems <= n) {
-      const int4 a = *reinterpret_cast<const int4 *>(in + base);
-      const int4 b = *reinterpret_cast<const int4 *>(in + base + 4);
-      v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+      const int4 p = *reinterpret_cast<const int4 *>(in + base);
+      const int4 q = *reinterpret_cast<const int4 *>(in + base + 4);
+      v[0] = p.x, v[1] = p.y, v[2] = p.z, v[3] = p.w, v[4] = q.x, v[5] = q.y, v[6] = q.z, v[7] = q.w;
     } else {
 #pragma unroll
       for (int k = 0; k < kScanItems; ++k) {
@@ -214,8 +184,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int32_t *__re
     for (int k = 0; k < kScanItems; ++k) {
       sum += v[k];
     }
-    int64_t total;
-    int64_t run = partials[t] + block_exclusive_scan<int64_t>(sum, warp_totals, total);
+    int64_t run = before + block_exclusive_scan<int64_t>(sum, warp_totals, total);
     int32_t o[kScanItems];
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
@@ -233,52 +202,44 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int32_t *__re
         }
       }
     }
+    if (t == tiles - 1 && threadIdx.x == 0) {
+      const int64_t all = before + total;
+      *total_out = all;
+      out[n] = (int32_t)all;
+      if (all > INT_MAX) {
+        atomicOr(&status->flags, kFlagCountOverflow);
+      }
+      if (all > cap) {
+        atomicOr(&status->flags, own_flag);
+      }
+    }
   }
 }
 
 int scan_grid(const Launch &l) { return l.num_sms * 4; }
 
-// The four scans of a run: tracklets per cluster, cells per span of tracklets, neighbours per cell, roads
-// per cell. The neighbour and road scans are three kernels (tile sums, scan of tile sums, tile
-// scans); the tracklet and cell scans are two, their tile sums added up by the count passes.
-struct ScanArgs {
-  const int32_t *in;
-  int32_t *out;
-  const int64_t *n_dev;
-  int64_t n_host;
-  int64_t *total;
-};
-
+// The four scans of a run: tracklets per cluster, cells per span of tracklets, neighbours per cell,
+// roads per cell. The first leaves the check of its capacity to the segment pass.
 template <int kWhich>
-ScanArgs scan_args(const Arena &a)
+void step_scan(const Arena &a, const Launch &l)
 {
   switch (kWhich) {
-  case 0: return ScanArgs{a.trk_count, a.trk_off, nullptr, a.n_clusters, &a.status->total[kTracklets]};
-  case 1: return ScanArgs{a.cell_span_count, a.cell_span_off, &a.status->cell_spans, 0, &a.status->total[kCells]};
-  case 2: return ScanArgs{a.nb_count, a.nb_off, &a.status->total[kCells], 0, &a.status->total[kNeighbours]};
-  default: return ScanArgs{a.road_count, a.road_off, &a.status->total[kCells], 0, &a.status->total[kRoads]};
+  case 0:
+    k_scan<false><<<scan_grid(l), kScanThreads, 0, l.stream>>>(a, a.trk_count, a.trk_off, nullptr, a.n_clusters, a.scan_partials,
+                                                                &a.status->total[kTracklets], INT64_MAX, 0);
+    break;
+  case 1:
+    k_scan<true><<<scan_grid(l), kScanThreads, 0, l.stream>>>(a, a.cell_span_count, a.cell_span_off, &a.status->cell_spans, 0, a.scan_partials,
+                                                               &a.status->total[kCells], a.cap_cells, kFlagCapCells);
+    break;
+  case 2:
+    k_scan<false><<<scan_grid(l), kScanThreads, 0, l.stream>>>(a, a.nb_count, a.nb_off, &a.status->total[kCells], 0, a.scan_partials,
+                                                                &a.status->total[kNeighbours], a.cap_neighbours, kFlagCapNeighbours);
+    break;
+  default:
+    k_scan<false><<<scan_grid(l), kScanThreads, 0, l.stream>>>(a, a.road_count, a.road_off, &a.status->total[kCells], 0, a.road_partials,
+                                                                &a.status->total[kRoads], a.cap_roads, kFlagCapRoads);
   }
-}
-
-template <int kWhich>
-void step_scan_reduce(const Arena &a, const Launch &l)
-{
-  const ScanArgs s = scan_args<kWhich>(a);
-  k_scan_reduce<<<scan_grid(l), kScanThreads, 0, l.stream>>>(s.in, s.n_dev, s.n_host, a.scan_partials, a.status);
-}
-
-template <int kWhich>
-void step_scan_partials(const Arena &a, const Launch &l)
-{
-  const ScanArgs s = scan_args<kWhich>(a);
-  k_scan_partials<<<1, 1024, 0, l.stream>>>(a.scan_partials, s.n_dev, s.n_host, s.out, s.total, a.status);
-}
-
-template <int kWhich>
-void step_scan_apply(const Arena &a, const Launch &l)
-{
-  const ScanArgs s = scan_args<kWhich>(a);
-  k_scan_apply<<<scan_grid(l), kScanThreads, 0, l.stream>>>(s.in, s.out, s.n_dev, s.n_host, a.scan_partials, a.status);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1150,8 +1111,7 @@ __global__ void __launch_bounds__(kCountThreads, kGate ? 5 : 6) k_tracklets_coun
         },
         staged, staged_off);
   }
-  // the warp's 32 clusters lie in one scan tile: their tracklets go to its sum (the tracklet
-  // scan has no reduce pass)
+  // the warp's 32 clusters lie in one scan tile: their tracklets go to its sum
   const int warp_count = (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
   if ((threadIdx.x & 31) == 0 && warp_count != 0) {
     atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[i / kScanTile]), (unsigned long long)warp_count);
@@ -1416,14 +1376,11 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tracklets_write(Arena a, int
   }
 }
 
-// Write pass, part 2: the inner clusters with more than kTrackletSlots tracklets (listed by the
-// count pass, a handful per batch) walk their candidates again and write their tracklets in order.
+// The inner clusters with more than kTrackletSlots tracklets (listed by the count pass, a handful per
+// batch) walk their candidates again and write their tracklets in order.
 template <bool kGate>
-__global__ void __launch_bounds__(kMaxThreads) k_tracklets_crowded(Arena a)
+__device__ __forceinline__ void write_crowded(const Arena &a)
 {
-  if (capacity_failed(a.status)) {
-    return;
-  }
   const int64_t listed = min(a.status->trk_crowded, (int64_t)a.n_clusters);
   for (int64_t q = global_thread(); q < listed; q += grid_threads()) {
     const int64_t i = a.clu_crowded[q];
@@ -1431,6 +1388,16 @@ __global__ void __launch_bounds__(kMaxThreads) k_tracklets_crowded(Arena a)
     int out = a.trk_off[i];
     walk_inner<kGate>(a, s, [&](int j) { write_tracklet(a, out++, i, s.next_begin + j, s.seg); });
   }
+}
+
+// Write pass, part 2, of the stage call (a whole run's segment pass writes them).
+template <bool kGate>
+__global__ void __launch_bounds__(kMaxThreads) k_tracklets_crowded(Arena a)
+{
+  if (capacity_failed(a.status)) {
+    return;
+  }
+  write_crowded<kGate>(a);
 }
 
 // Cell layer L of event e runs only if tracklet layers 0..L+1 are all non-empty
@@ -1450,7 +1417,10 @@ __device__ __forceinline__ bool cells_active(const int32_t *ts, int layer)
 // layers L, L+1, L+2 (the first -1 when cell layer L of the event does not run), the first
 // tracklet of layers L and L+1 and the vertex, so that each first tracklet's setup in the cell
 // count pass is two 16-byte loads of one record instead of a dozen loads of per-event offsets.
-__global__ void k_tracklet_segments(Arena a)
+// crowded: the crowded inner clusters' tracklets too (not in a stage call, whose outputs may still
+// have to grow).
+template <bool kGate>
+__global__ void __launch_bounds__(kCountThreads) k_tracklet_segments(Arena a, bool crowded)
 {
   // the cells scan's tile sums start at zero: the cell count pass adds each warp's cells there
   const int64_t n_trk = a.status->total[kTracklets];
@@ -1486,6 +1456,9 @@ __global__ void k_tracklet_segments(Arena a)
                                               __float_as_int(a.vtx[3 * e + 2]));
       }
     }
+  }
+  if (crowded && n_trk <= a.cap_tracklets && (*(volatile const int32_t *)&a.status->flags & kFlagCountOverflow) == 0) {
+    write_crowded<kGate>(a);
   }
 }
 
@@ -1824,14 +1797,37 @@ __global__ void __launch_bounds__(kPrefilterThreads) k_cells_prefilter(Arena a)
 
 // Write pass: a warp takes consecutive spans and flattens their entries over its lanes; in order, they go to the spans' scanned places, which
 // are contiguous (a dropped entry leaves no gap). The first cell of each first tracklet fills its
-// cells lookup entry.
+// cells lookup entry, and each cell's state of the stages after is reset (the neighbour scan's tile
+// sums too).
 constexpr int kScatterThreads = 256;
+
+// A cell's CA level and its number of level-decreasing chains down to layer 0, in one word
+// (chains << 3 | level; levels are 1..5 and chain counts are capped at INT_MAX), of layers 1 to 4; the
+// cells of layer 0 all have level 1 and one chain.
+__device__ __forceinline__ int64_t chain_word(int64_t paths, int level) { return (paths << 3) | level; }
+__device__ __forceinline__ int chain_level(int64_t w) { return (int)(w & 7); }
+__device__ __forceinline__ int64_t chain_paths(int64_t w) { return w >> 3; }
+
+// A cell's state of the neighbour and road stages before they run.
+__device__ __forceinline__ void reset_cell(const Arena &a, int64_t c)
+{
+  a.nb_count[c] = 0;
+  a.road_count[c] = 0;
+}
+
+__device__ __forceinline__ void zero_tiles(int64_t *partials, int64_t n)
+{
+  for (int64_t t = global_thread(); t < (n + kScanTile - 1) / kScanTile; t += grid_threads()) {
+    partials[t] = 0;
+  }
+}
 
 __global__ void __launch_bounds__(kScatterThreads) k_cells_scatter(Arena a)
 {
   if (capacity_failed(a.status)) {
     return;
   }
+  zero_tiles(a.scan_partials, a.status->total[kCells]);
   const int lane = threadIdx.x & 31;
   const int64_t spans = a.status->cell_spans;
   const int take = spans_at_a_time(spans, 1 << 16);
@@ -1879,6 +1875,7 @@ __global__ void __launch_bounds__(kScatterThreads) k_cells_scatter(Arena a)
           dst[q] = h[q];
         }
         a.cell_seg_id[out] = segment;
+        reset_cell(a, out);
       }
       const int to = 31 - __clz(living);
       last_t1 = __shfl_sync(0xffffffffu, t1, to);
@@ -1888,43 +1885,41 @@ __global__ void __launch_bounds__(kScatterThreads) k_cells_scatter(Arena a)
   }
 }
 
-// cell_seg[5e+L] = first cell of (e, L), from the segments' counts (cells are in segment order), in
-// one block; capacity check of the cell total.
-__global__ void __launch_bounds__(1024) k_cell_segments(Arena a)
+// cell_seg[5e+L] = first cell of (e, L), from the segments' counts (cells are in segment order), by
+// one block.
+__device__ void cell_segments(const Arena &a, int64_t *warp_totals)
 {
-  __shared__ int64_t warp_totals[33];
-  if (capacity_failed(a.status)) {
-    return;  // tracklet offsets beyond the arena: nothing downstream runs
-  }
+  constexpr int kPer = 4;
   const int nseg = a.n_events * ITSU_CELL_LAYERS;
   int64_t carry = 0;
-  for (int s0 = 0; s0 < nseg; s0 += (int)blockDim.x) {
-    const int s = s0 + (int)threadIdx.x;
-    int64_t total;
-    const int64_t ex = block_exclusive_scan<int64_t>(s < nseg ? a.cell_seg_count[s] : 0, warp_totals, total);
-    if (s < nseg) {
-      a.cell_seg[s] = (int32_t)(carry + ex);
+  for (int s0 = 0; s0 < nseg; s0 += kPer * (int)blockDim.x) {
+    const int s = s0 + kPer * (int)threadIdx.x;
+    int32_t v[kPer];
+    int64_t sum = 0, total;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      v[k] = s + k < nseg ? a.cell_seg_count[s + k] : 0;
+      sum += v[k];
+    }
+    int64_t run = carry + block_exclusive_scan<int64_t>(sum, warp_totals, total);
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      if (s + k < nseg) {
+        a.cell_seg[s + k] = (int32_t)run;
+      }
+      run += v[k];
     }
     carry += total;
   }
   if (threadIdx.x == 0) {
     a.cell_seg[nseg] = (int32_t)carry;
-    if (carry > a.cap_cells) {
-      atomicOr(&a.status->flags, kFlagCapCells);
-    }
   }
 }
 
 // ------------------------------------------------------------------------------------------
 // (d) neighbours and CA levels: Tracker<IsGPU>::findCellsNeighbours (Tracker.cxx:417-474)
 
-// Per-cell state of the neighbour and road stages, reset so that the stage can be re-run.
-// A cell's CA level and its number of level-decreasing chains down to layer 0, in one word
-// (chains << 3 | level; levels are 1..5 and chain counts are capped at INT_MAX).
-__device__ __forceinline__ int64_t chain_word(int64_t paths, int level) { return (paths << 3) | level; }
-__device__ __forceinline__ int chain_level(int64_t w) { return (int)(w & 7); }
-__device__ __forceinline__ int64_t chain_paths(int64_t w) { return w >> 3; }
-
+// Stage call only: the cells' state again, so that the stage can be re-run.
 __global__ void __launch_bounds__(kMaxThreads) k_neighbour_reset(Arena a)
 {
   if (capacity_failed(a.status)) {
@@ -1932,10 +1927,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbour_reset(Arena a)
   }
   const int64_t n = a.status->total[kCells];
   for (int64_t c = global_thread(); c < n; c += grid_threads()) {
-    a.nb_count[c] = 0;
-    a.nb_fill[c] = 0;
-    a.road_count[c] = 0;
-    a.paths[c] = a.cell_seg_id[c] % ITSU_CELL_LAYERS == 0 ? chain_word(1, 1) : 0;  // layer 0: one chain, level 1
+    reset_cell(a, c);
   }
 }
 
@@ -1944,7 +1936,19 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbour_reset(Arena a)
 // count pass evaluates the cut, counts each passing pair in its row and keeps the passing candidates
 // as a mask (of up to kMaskedRun candidates; a longer run is marked in the top bit); the write pass,
 // after the scan of the counts, fills the rows from the mask (re-evaluating the cut only for the
-// marked cells). Row order is restored by k_levels' sort.
+// marked cells), counting the counts down to zero. Row order is restored by k_levels' sort.
+// Adds count to the tile sum of item `at`: one atomic for the lanes that are here together and whose
+// items lie in one tile.
+__device__ __forceinline__ void add_to_tile(int64_t *partials, int64_t at, int count)
+{
+  const unsigned tile = (unsigned)(at / kScanTile);
+  const unsigned peers = __match_any_sync(__activemask(), tile);
+  count = (int)__reduce_add_sync(peers, (unsigned)count);
+  if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) {
+    atomicAdd(reinterpret_cast<unsigned long long *>(&partials[tile]), (unsigned long long)count);
+  }
+}
+
 constexpr int kMaskedRun = 63;
 constexpr unsigned long long kLongRun = 1ull << kMaskedRun;
 
@@ -1955,6 +1959,9 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbours(Arena a)
     return;
   }
   const int64_t n = a.status->total[kCells];
+  if (kWrite) {
+    zero_tiles(a.road_partials, n);  // the level pass adds each tile's roads
+  }
   for (int64_t c = global_thread(); c < n; c += grid_threads()) {
     const int sid = a.cell_seg_id[c];
     const int e = sid / ITSU_CELL_LAYERS, layer = sid % ITSU_CELL_LAYERS;
@@ -1972,13 +1979,14 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbours(Arena a)
     if (kWrite && !(mask & kLongRun)) {
       for (; mask; mask &= mask - 1ull) {
         const int32_t j = j0 + __ffsll((long long)mask) - 1;
-        const int slot = atomicAdd(&a.nb_fill[j], 1);
+        const int slot = atomicSub(&a.nb_count[j], 1) - 1;
         a.nb[a.nb_off[j] + slot] = c_local;
       }
       continue;
     }
     const itsu_cell cell = a.cells[c];
     const float3 n1 = make_float3(cell.nx, cell.ny, cell.nz);
+    int links = 0;  // to cells of j0's scan tile
     for (int32_t j = j0; j < j1; ++j) {
       const itsu_cell next = a.cells[j];
       if (next.first_tracklet != second) {
@@ -1987,12 +1995,17 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbours(Arena a)
       const bool pass = neighbour_cut(layer, n1, cell.curvature, make_float3(next.nx, next.ny, next.nz), next.curvature);
       if (kWrite) {
         if (pass) {
-          const int slot = atomicAdd(&a.nb_fill[j], 1);
+          const int slot = atomicSub(&a.nb_count[j], 1) - 1;
           a.nb[a.nb_off[j] + slot] = c_local;
         }
       } else {
         if (pass) {
           atomicAdd(&a.nb_count[j], 1);
+          if (j / kScanTile == j0 / kScanTile) {
+            ++links;
+          } else {
+            atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[j / kScanTile]), 1ull);
+          }
         }
         if (j - j0 >= kMaskedRun) {
           mask |= kLongRun;
@@ -2003,14 +2016,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbours(Arena a)
     }
     if (!kWrite) {
       a.nb_mask[c] = mask;
+      if (links > 0) {
+        add_to_tile(a.scan_partials, j0, links);
+      }
     }
-  }
-}
-
-__global__ void k_neighbour_check(Arena a)
-{
-  if (global_thread() == 0 && !capacity_failed(a.status) && a.status->total[kNeighbours] > a.cap_neighbours) {
-    atomicOr(&a.status->flags, kFlagCapNeighbours);
   }
 }
 
@@ -2020,7 +2029,7 @@ __device__ __forceinline__ void level_of(const Arena &a, int64_t c, int64_t prev
 {
   const int32_t b = a.nb_off[c], en = a.nb_off[c + 1];
   int32_t *row = a.nb + b;
-  const int len = en - b;
+  int len = en - b;
   for (int p = 1; p < len; ++p) {
     const int32_t v = row[p];
     int q = p - 1;
@@ -2031,11 +2040,16 @@ __device__ __forceinline__ void level_of(const Arena &a, int64_t c, int64_t prev
     row[q + 1] = v;
   }
   int level = 1;
+  int64_t paths = 0;
+  bool overflow = false;
+  if (layer == 1) {  // every neighbour has level 1 and one chain
+    level = len > 0 ? 2 : 1;
+    paths = len;
+    len = 0;
+  }
   for (int p = 0; p < len; ++p) {
     level = max(level, chain_level(a.paths[prev_base + row[p]]) + 1);
   }
-  int64_t paths = 0;
-  bool overflow = false;
   for (int p = 0; p < len; ++p) {
     const int64_t w = a.paths[prev_base + row[p]];
     if (chain_level(w) == level - 1) {
@@ -2050,53 +2064,47 @@ __device__ __forceinline__ void level_of(const Arena &a, int64_t c, int64_t prev
   a.paths[c] = chain_word(paths, level);
   if (layer == ITSU_CELL_LAYERS - 1 && level == kCellsMinLevel) {
     a.road_count[c] = (int32_t)paths;
+    if (paths > 0) {
+      add_to_tile(a.road_partials, c, (int)paths);
+    }
     if (overflow) {
       atomicOr(&a.status->flags, kFlagCountOverflow);
     }
   }
 }
 
-// Rows of layer `layer` cells: sort ascending (the reference pushes in cell order), then the
-// level (Tracker.cxx:463-468: 1 + the highest neighbour level) and the number of
-// level-decreasing chains down to layer 0 (the roads a level-5 cell starts, Tracker.cxx:477-571).
-// The blocks of grid row y take the layer's cells of events y, y + gridDim.y, ... (each event's
-// cells of a layer are one range).
-__global__ void __launch_bounds__(kMaxThreads) k_levels(Arena a, int layer)
+// Layer by layer from 1: rows sorted ascending (the reference pushes in cell order), then the level
+// (Tracker.cxx:463-468: 1 + the highest neighbour level) and the number of level-decreasing chains
+// down to layer 0 (the roads a level-5 cell starts, Tracker.cxx:477-571). A cluster of CTAs per event
+// (events beyond the grid in turn), which meet after each layer: one launch in place of four.
+template <int kThreads_>
+__global__ void __launch_bounds__(kThreads_) k_levels(Arena a)
 {
+  namespace cg = cooperative_groups;
+  const int ctas = (int)cg::this_cluster().num_blocks(), rank = (int)cg::this_cluster().block_rank();
   if (capacity_failed(a.status)) {
-    return;
+    return;  // a thread that finds a count overflow of this pass here leaves; the barriers wait for the others only
   }
-  for (int e = blockIdx.y; e < a.n_events; e += gridDim.y) {
+  for (int e = blockIdx.x / ctas; e < a.n_events; e += gridDim.x / ctas) {
     const int32_t *cs = a.cell_seg + e * ITSU_CELL_LAYERS;
-    const int64_t prev_base = cs[layer - 1];
-    for (int64_t c = cs[layer] + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < cs[layer + 1];
-         c += (int64_t)gridDim.x * blockDim.x) {
-      level_of(a, c, prev_base, layer);
+    for (int layer = 1; layer < ITSU_CELL_LAYERS; ++layer) {
+      const int64_t prev_base = cs[layer - 1];
+      for (int64_t c = cs[layer] + rank * kThreads_ + (int)threadIdx.x; c < cs[layer + 1]; c += ctas * kThreads_) {
+        level_of(a, c, prev_base, layer);
+      }
+      if (layer < ITSU_CELL_LAYERS - 1) {
+        if (ctas == 1) {
+          __syncthreads();
+        } else {
+          cg::this_cluster().sync();
+        }
+      }
     }
   }
 }
 
 // ------------------------------------------------------------------------------------------
 // (e) roads: Tracker<IsGPU>::findTracks / traverseCellsTree / computeMontecarloLabels
-
-__global__ void k_road_segments(Arena a)
-{
-  if (capacity_failed(a.status)) {
-    return;
-  }
-  const int nseg = a.n_events;
-  for (int s = (int)global_thread(); s <= nseg; s += grid_threads()) {
-    if (s == nseg) {
-      const int64_t total = a.status->total[kRoads];
-      a.road_seg[s] = (int32_t)total;
-      if (total > a.cap_roads) {
-        atomicOr(&a.status->flags, kFlagCapRoads);
-      }
-    } else {
-      a.road_seg[s] = a.road_off[a.cell_seg[s * ITSU_CELL_LAYERS + ITSU_CELL_LAYERS - 1]];
-    }
-  }
-}
 
 // A sorted cluster's MC id, from its 16-byte auxiliary record (the batch's 36-byte sorted records
 // are twice the footprint, and the road vote's gathers hit L2 less often there).
@@ -2126,6 +2134,12 @@ __global__ void __launch_bounds__(kMaxThreads) k_roads(Arena a)
     const int32_t *cs = a.cell_seg + e * ITSU_CELL_LAYERS;
     const int32_t *lo = a.layer_off + e * ITSU_LAYERS;
     const int64_t n = cs[ITSU_CELL_LAYERS];  // the event's last cell + 1
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the event's first road
+      a.road_seg[e] = a.road_off[cs[ITSU_CELL_LAYERS - 1]];
+      if (e == a.n_events - 1) {
+        a.road_seg[e + 1] = (int32_t)a.status->total[kRoads];
+      }
+    }
     for (int64_t base = cs[ITSU_CELL_LAYERS - 1] + warp * 32; base < n; base += warps * 32) {
       const int64_t c = base + lane;
       int32_t first = 0, count = 0;
@@ -2152,7 +2166,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_roads(Arena a)
         int level = kCellsMinLevel;
         bool found = true;
 #pragma unroll
-        for (int l = ITSU_CELL_LAYERS - 1; l >= 1; --l) {
+        for (int l = ITSU_CELL_LAYERS - 1; l >= 2; --l) {
           const int32_t j1 = a.nb_off[flat + 1];
           bool down = false;
           cur[l - 1] = 0;
@@ -2173,6 +2187,12 @@ __global__ void __launch_bounds__(kMaxThreads) k_roads(Arena a)
           }
           found = found && down;
           --level;
+        }
+        {  // layer 1 to 0: every neighbour has one chain
+          const int32_t j0 = a.nb_off[flat], j1 = a.nb_off[flat + 1];
+          const bool down = found && k < j1 - j0;
+          cur[0] = down ? a.nb[j0 + k] : 0;
+          found = down;
         }
         if (!found) {  // only when a chain count was capped (the count overflow flag is set)
           atomicOr(&a.status->flags, kFlagCountOverflow);
@@ -2244,6 +2264,24 @@ void step_status_init(const Arena &a, const Launch &l)
   k_status_init<<<(unsigned)std::max<int64_t>(blocks, 1), kThreads, 0, l.stream>>>(a);
 }
 
+// A launch of `ctas` CTAs per cluster (1: no cluster).
+template <typename... Args>
+void launch_clusters(void (*kernel)(Args...), int64_t clusters, int ctas, int threads, size_t bytes, cudaStream_t stream, Args... args)
+{
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3((unsigned)(clusters * ctas));
+  config.blockDim = dim3((unsigned)threads);
+  config.dynamicSmemBytes = bytes;
+  config.stream = stream;
+  cudaLaunchAttribute cluster{};
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = (unsigned)ctas;
+  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+  config.attrs = &cluster;
+  config.numAttrs = ctas > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&config, kernel, args...);
+}
+
 template <int kThreads_>
 void launch_sort(const Arena &a, const Launch &l, int ctas)
 {
@@ -2251,18 +2289,7 @@ void launch_sort(const Arena &a, const Launch &l, int ctas)
   if (bytes > 48 * 1024) {
     cudaFuncSetAttribute(k_cluster_sort<kThreads_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   }
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3((unsigned)(a.n_events * ITSU_LAYERS * ctas));
-  config.blockDim = dim3(kThreads_);
-  config.dynamicSmemBytes = bytes;
-  config.stream = l.stream;
-  cudaLaunchAttribute cluster{};
-  cluster.id = cudaLaunchAttributeClusterDimension;
-  cluster.val.clusterDim.x = (unsigned)ctas;
-  cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-  config.attrs = &cluster;
-  config.numAttrs = ctas > 1 ? 1 : 0;
-  cudaLaunchKernelEx(&config, k_cluster_sort<kThreads_>, a);
+  launch_clusters(k_cluster_sort<kThreads_>, (int64_t)a.n_events * ITSU_LAYERS, ctas, kThreads_, bytes, l.stream, a);
 }
 
 void step_cluster_sort(const Arena &a, const Launch &l)
@@ -2343,8 +2370,12 @@ void step_tracklets_write(const Arena &a, const Launch &l)
   }
 }
 
+// A whole run's crowded clusters are written by the segment pass.
 void step_tracklets_crowded(const Arena &a, const Launch &l)
 {
+  if (!l.staged) {
+    return;
+  }
   if (a.gate) {
     k_tracklets_crowded<true><<<l.num_sms, 128, 0, l.stream>>>(a);
   } else {
@@ -2354,7 +2385,11 @@ void step_tracklets_crowded(const Arena &a, const Launch &l)
 
 void step_tracklet_segments(const Arena &a, const Launch &l)
 {
-  k_tracklet_segments<<<(a.n_events * ITSU_TRACKLET_LAYERS + kThreads) / kThreads, kThreads, 0, l.stream>>>(a);
+  if (a.gate) {
+    k_tracklet_segments<true><<<l.num_sms, 128, 0, l.stream>>>(a, !l.staged);
+  } else {
+    k_tracklet_segments<false><<<l.num_sms, 128, 0, l.stream>>>(a, !l.staged);
+  }
 }
 
 void launch_cells_range(const Arena &a, const Launch &l, int32_t e0, int32_t e1, bool last)
@@ -2396,32 +2431,37 @@ void step_cells_prefilter(const Arena &a, const Launch &l)
 
 void step_cells_scatter(const Arena &a, const Launch &l) { k_cells_scatter<<<l.num_sms * 8, kScatterThreads, 0, l.stream>>>(a); }
 
-void step_cell_segments(const Arena &a, const Launch &l) { k_cell_segments<<<1, 1024, 0, l.stream>>>(a); }
-
-void step_neighbour_reset(const Arena &a, const Launch &l) { k_neighbour_reset<<<fixed_grid(l), l.block, 0, l.stream>>>(a); }
+void step_neighbour_reset(const Arena &a, const Launch &l)
+{
+  if (l.staged) {
+    k_neighbour_reset<<<fixed_grid(l), l.block, 0, l.stream>>>(a);
+  }
+}
 
 template <bool kWrite>
 void step_neighbours(const Arena &a, const Launch &l) { k_neighbours<kWrite><<<fixed_grid(l), l.block, 0, l.stream>>>(a); }
 
-void step_neighbour_check(const Arena &a, const Launch &l) { k_neighbour_check<<<1, 32, 0, l.stream>>>(a); }
-
-template <int kLayer>
+// Threads for about half of the cells of the largest event's largest layer (a layer of hits has about
+// 1.3 cells per hit), so that a layer takes one or two rounds.
 void step_levels(const Arena &a, const Launch &l)
 {
-  if (a.n_events > 0) {
-    k_levels<<<event_grid(a, l), l.block, 0, l.stream>>>(a, kLayer);
+  if (a.n_events <= 0) {
+    return;
   }
-}
-
-void step_road_segments(const Arena &a, const Launch &l)
-{
-  k_road_segments<<<(a.n_events + kThreads) / kThreads, kThreads, 0, l.stream>>>(a);
+  const LevelShape shape = level_shape(l.max_segment);
+  if (shape.threads == 128) {
+    launch_clusters(k_levels<128>, a.n_events, 1, 128, 0, l.stream, a);
+  } else {
+    launch_clusters(k_levels<512>, a.n_events, shape.ctas, 512, 0, l.stream, a);
+  }
 }
 
 void step_roads(const Arena &a, const Launch &l)
 {
   if (a.n_events > 0) {
     k_roads<<<event_grid(a, l), l.block, 0, l.stream>>>(a);
+  } else {
+    cudaMemsetAsync(a.road_seg, 0, sizeof(int32_t), l.stream);  // no road offsets but the end
   }
 }
 
@@ -2431,34 +2471,22 @@ const KernelStep kSteps[] = {
     {"cluster_sort", step_cluster_sort, 0},                  // 1  (a)
     {"tracklets_count", step_tracklets_count, 0},            // 2  (b)
     {"tracklets_gate", step_tracklets_gate, kGateStep},      // 3  (learned form with the gate)
-    {"scan_partials_tracklets", step_scan_partials<0>, 0},   // 4
-    {"scan_apply_tracklets", step_scan_apply<0>, 0},         // 5
-    {"tracklet_segments", step_tracklet_segments, 0},        // 6
-    {"tracklets_crowded", step_tracklets_crowded, 0},        // 7
-    {"tracklets_write", step_tracklets_write, kUngroupedStep},  // 8
-    {"cells_count", step_cells_count, kUngroupedStep},       // 9  (c)
-    {"write_count_by_event_group", step_write_count_groups, kGroupedStep},  // 10 (tracklet write + cell count per group)
-    {"cells_prefilter", step_cells_prefilter, kPairPrefilterStep},  // 11 (learned form with the pair prefilter)
-    {"scan_partials_cells", step_scan_partials<1>, 0},       // 12
-    {"scan_apply_cells", step_scan_apply<1>, 0},             // 13
-    {"cell_segments", step_cell_segments, 0},                // 14
-    {"cells_scatter", step_cells_scatter, 0},                // 15
-    {"neighbour_reset", step_neighbour_reset, 0},            // 16 (d)
-    {"neighbours_count", step_neighbours<false>, 0},         // 17
-    {"scan_reduce_neighbours", step_scan_reduce<2>, 0},      // 18
-    {"scan_partials_neighbours", step_scan_partials<2>, 0},  // 19
-    {"scan_apply_neighbours", step_scan_apply<2>, 0},        // 20
-    {"neighbour_check", step_neighbour_check, 0},            // 21
-    {"neighbours_write", step_neighbours<true>, 0},          // 22
-    {"levels_1", step_levels<1>, 0},                         // 23
-    {"levels_2", step_levels<2>, 0},                         // 24
-    {"levels_3", step_levels<3>, 0},                         // 25
-    {"levels_4", step_levels<4>, 0},                         // 26
-    {"scan_reduce_roads", step_scan_reduce<3>, 0},           // 27 (e)
-    {"scan_partials_roads", step_scan_partials<3>, 0},       // 28
-    {"scan_apply_roads", step_scan_apply<3>, 0},             // 29
-    {"road_segments", step_road_segments, 0},                // 30
-    {"roads_write", step_roads, 0},                          // 31
+    {"scan_tracklets", step_scan<0>, 0},                     // 4
+    {"tracklet_segments", step_tracklet_segments, 0},        // 5  (and a whole run's crowded clusters)
+    {"tracklets_crowded", step_tracklets_crowded, kStagedStep},  // 6
+    {"tracklets_write", step_tracklets_write, kUngroupedStep},  // 7
+    {"cells_count", step_cells_count, kUngroupedStep},       // 8  (c)
+    {"write_count_by_event_group", step_write_count_groups, kGroupedStep},  // 9 (tracklet write + cell count per group)
+    {"cells_prefilter", step_cells_prefilter, kPairPrefilterStep},  // 10 (learned form with the pair prefilter)
+    {"scan_cells", step_scan<1>, 0},                         // 11 (and the cell segments)
+    {"cells_scatter", step_cells_scatter, 0},                // 12
+    {"neighbour_reset", step_neighbour_reset, kStagedStep},  // 13 (d)
+    {"neighbours_count", step_neighbours<false>, 0},         // 14
+    {"scan_neighbours", step_scan<2>, 0},                    // 15
+    {"neighbours_write", step_neighbours<true>, 0},          // 16
+    {"levels", step_levels, 0},                              // 17
+    {"scan_roads", step_scan<3>, 0},                         // 18 (e)
+    {"roads_write", step_roads, 0},                          // 19
 };
 constexpr int kNumSteps = sizeof(kSteps) / sizeof(kSteps[0]);
 
@@ -2484,6 +2512,18 @@ SortShape sort_shape(int32_t n_events, int64_t n_clusters, int64_t max_segment)
   s.ctas = 1;
   const int64_t most = 2 * n_clusters >= segments * max_segment ? 1024 : 296;
   while (max_segment > 1024 && s.ctas < 8 && 2 * s.ctas * segments <= most) {
+    s.ctas *= 2;
+  }
+  return s;
+}
+
+// The level pass's launch for a run whose largest layer has max_segment clusters.
+LevelShape level_shape(int64_t max_segment)
+{
+  LevelShape s;
+  s.threads = max_segment > 192 ? 512 : 128;
+  s.ctas = 1;
+  while (s.threads == 512 && s.ctas < 8 && 3 * max_segment > 4 * 512 * s.ctas) {
     s.ctas *= 2;
   }
   return s;
@@ -2535,7 +2575,7 @@ const KernelStep *pipeline_steps(int *count)
 
 void launch_status_init(const Arena &a, const Launch &l) { run_steps(0, 0, a, l); }
 void launch_cluster_sort(const Arena &a, const Launch &l) { run_steps(1, 1, a, l); }
-void launch_tracklets_count(const Arena &a, const Launch &l) { run_steps(2, 6, a, l); }
+void launch_tracklets_count(const Arena &a, const Launch &l) { run_steps(2, 5, a, l); }
 
 void launch_atan2f(const float *y, const float *x, float *out, int64_t n, int num_sms, cudaStream_t stream)
 {
@@ -2543,13 +2583,13 @@ void launch_atan2f(const float *y, const float *x, float *out, int64_t n, int nu
     k_atan2f<<<num_sms * 4, 256, 0, stream>>>(y, x, out, n);
   }
 }
-void launch_tracklets_write(const Arena &a, const Launch &l) { run_steps(7, 8, a, l); }
-void launch_cells_count(const Arena &a, const Launch &l) { run_steps(9, 14, a, l); }
-void launch_cells_write(const Arena &a, const Launch &l) { run_steps(15, 15, a, l); }
-void launch_neighbours_count(const Arena &a, const Launch &l) { run_steps(16, 21, a, l); }
-void launch_neighbours_write(const Arena &a, const Launch &l) { run_steps(22, 26, a, l); }
-void launch_roads_count(const Arena &a, const Launch &l) { run_steps(27, 30, a, l); }
-void launch_roads_write(const Arena &a, const Launch &l) { run_steps(31, 31, a, l); }
+void launch_tracklets_write(const Arena &a, const Launch &l) { run_steps(6, 7, a, l); }
+void launch_cells_count(const Arena &a, const Launch &l) { run_steps(8, 11, a, l); }
+void launch_cells_write(const Arena &a, const Launch &l) { run_steps(12, 12, a, l); }
+void launch_neighbours_count(const Arena &a, const Launch &l) { run_steps(13, 15, a, l); }
+void launch_neighbours_write(const Arena &a, const Launch &l) { run_steps(16, 17, a, l); }
+void launch_roads_count(const Arena &a, const Launch &l) { run_steps(18, 18, a, l); }
+void launch_roads_write(const Arena &a, const Launch &l) { run_steps(19, 19, a, l); }
 
 int kernels_per_run()
 {
