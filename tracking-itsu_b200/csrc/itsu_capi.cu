@@ -26,6 +26,7 @@
 
 using itsu::Arena;
 using itsu::DevStatus;
+using itsu::EventSegments;
 using itsu::Launch;
 
 namespace {
@@ -50,6 +51,14 @@ struct Tune {
 };
 constexpr int kBands = 32;
 
+// Before the raw clusters' buffer: a vertex's 8 layer offsets and its coordinates.
+constexpr int64_t kRawHead = 64;
+static_assert(sizeof(int32_t) * (ITSU_LAYERS + 1) + sizeof(float) * 3 <= kRawHead, "a vertex's head");
+
+constexpr int kPieces = 4;
+constexpr size_t kPiece = 256 << 10;
+constexpr size_t kPinned = kPieces * kPiece;
+
 // Band of a run: log2 of its mean cluster count per event.
 int band_of(int64_t n_clusters, int32_t n_events)
 {
@@ -61,6 +70,26 @@ int band_of(int64_t n_clusters, int32_t n_events)
   return band;
 }
 }  // namespace
+
+// All that the launches of a whole run depend on.
+struct RunKey {
+  const void *inputs[6] = {};
+  int64_t n_clusters = -1;
+  int32_t n_events = -1;
+  uint64_t generation = 0;
+  int tune[4] = {};
+  bool prefilter = false, gate = false;
+  itsu::SortShape sort{};
+  itsu::LevelShape levels{};
+
+  bool operator==(const RunKey &k) const
+  {
+    return std::equal(inputs, inputs + 6, k.inputs) && n_clusters == k.n_clusters && n_events == k.n_events &&
+           generation == k.generation && std::equal(tune, tune + 4, k.tune) && prefilter == k.prefilter && gate == k.gate &&
+           sort.threads == k.sort.threads && sort.ctas == k.sort.ctas && levels.threads == k.levels.threads &&
+           levels.ctas == k.levels.ctas;
+  }
+};
 
 struct itsu_context {
   int device = 0;
@@ -111,9 +140,17 @@ struct itsu_context {
   // neighbour and road classes
   int32_t *nb = nullptr;
   itsu_road *roads = nullptr;
+  // a vertex's inputs on the device: offsets and coordinates in the head before the raw clusters
+  unsigned char *raw_head = nullptr;
+  // pinned buffer of the per-vertex calls: their inputs' way up (in kPieces pieces, each with the event
+  // of its last copy) and small events' lists' way down
+  unsigned char *h_pinned = nullptr;
+  cudaEvent_t piece_sent[kPieces] = {};
+  bool pinned_busy = false;  // copies from it may be in flight
   int64_t *scan_partials = nullptr;
   DevStatus *d_status = nullptr;
   DevStatus *h_status = nullptr;
+  EventSegments *d_segments = nullptr, *h_segments = nullptr;  // one event's, for the result calls
 
   // current run
   int32_t n_events = 0;
@@ -134,23 +171,16 @@ struct itsu_context {
   const float *in_vtx = nullptr;
   int stage = kNone;
 
-  // CUDA graph of the whole batch sequence
+  // CUDA graph of the whole run, and the last run's key with the number of times it came in a row
   cudaGraphExec_t graph = nullptr;
-  uint64_t graph_generation = 0;
+  RunKey graph_key, last_key;
+  int last_key_runs = 0;
   uint64_t generation = 1;  // bumped whenever a buffer is reallocated
-  const void *graph_key[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  int32_t graph_events = -1;
-  int64_t graph_clusters = -1;
 
   // launch shapes per multiplicity band, and the candidate under test while tuning
   Tune tunes[kBands];
   Tune override_tune;
   bool tuning = false;
-  int graph_tune[4] = {0, 0, -1, -1};
-  bool graph_prefilter = false;
-  itsu::SortShape graph_sort{};
-  itsu::LevelShape graph_levels{};
-  bool graph_gate = false;
 
   // streamed host runs (ITSU_FLAG_STREAM_HOST): upload stream, per-chunk events, batch-wide roads
   cudaStream_t copy_stream = nullptr;   // uploads
@@ -417,7 +447,8 @@ itsu_status ensure_clusters(itsu_context *ctx, int64_t n_clusters, int32_t n_eve
     itsu_status st = growth_allowed(ctx, "clusters", n_clusters, ctx->cap_clusters);
     if (st != ITSU_OK) return st;
     const int64_t cap = grow_to(n_clusters);
-    ITSU_CUDA(ctx, alloc(ctx, ctx->raw, cap));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->raw_head, kRawHead + (int64_t)sizeof(itsu_cluster) * cap));
+    ctx->raw = reinterpret_cast<itsu_cluster *>(ctx->raw_head + kRawHead);
     ITSU_CUDA(ctx, alloc(ctx, ctx->sorted, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->sort_recs, 2 * cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->sort_index, 4 * cap));
@@ -581,6 +612,7 @@ itsu_status sync_status(itsu_context *ctx)
 {
   ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(DevStatus), cudaMemcpyDeviceToHost, ctx->stream));
   ITSU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  ctx->pinned_busy = false;
   if (ctx->h_status->flags & itsu::kFlagLaunchShape) {
     return fail(ctx, ITSU_ERR_INVALID, "launch shape: the per-item passes need a block size that is a multiple of 32");
   }
@@ -641,24 +673,42 @@ void drop_graph(itsu_context *ctx)
   }
 }
 
-// Launches the whole sequence, through a CUDA graph that is re-captured when the inputs,
-// sizes or arena buffers change.
-itsu_status launch_all(itsu_context *ctx)
+RunKey run_key(const itsu_context *ctx)
 {
   const Tune tune = current_tune(ctx);
-  const itsu::SortShape sort = itsu::sort_shape(ctx->n_events, ctx->n_clusters, ctx->max_segment);
-  const itsu::LevelShape levels = itsu::level_shape(ctx->max_segment);
-  const bool same = ctx->graph && sort.threads == ctx->graph_sort.threads && sort.ctas == ctx->graph_sort.ctas &&
-                    levels.threads == ctx->graph_levels.threads && levels.ctas == ctx->graph_levels.ctas &&
-                    ctx->graph_generation == ctx->generation && ctx->graph_key[0] == ctx->in_raw &&
-                    ctx->graph_tune[0] == tune.block && ctx->graph_tune[1] == tune.blocks_per_sm &&
-                    ctx->graph_tune[2] == tune.prune && ctx->graph_tune[3] == tune.group && ctx->graph_prefilter == ctx->prefilter &&
-                    ctx->graph_gate == ctx->gate &&
-                    ctx->graph_key[1] == ctx->in_layer_off && ctx->graph_key[2] == ctx->in_vtx &&
-                    ctx->graph_key[3] == ctx->in_raw_off && ctx->graph_key[4] == ctx->in_raw_in &&
-                    ctx->graph_key[5] == ctx->in_raw_track &&
-                    ctx->graph_events == ctx->n_events && ctx->graph_clusters == ctx->n_clusters;
-  if (!same) {
+  RunKey k;
+  const void *inputs[6] = {ctx->in_raw, ctx->in_raw_in, ctx->in_raw_track, ctx->in_raw_off, ctx->in_layer_off, ctx->in_vtx};
+  std::copy(inputs, inputs + 6, k.inputs);
+  k.n_clusters = ctx->n_clusters;
+  k.n_events = ctx->n_events;
+  k.generation = ctx->generation;
+  k.tune[0] = tune.block;
+  k.tune[1] = tune.blocks_per_sm;
+  k.tune[2] = tune.prune;
+  k.tune[3] = tune.group;
+  k.prefilter = ctx->prefilter;
+  k.gate = ctx->gate;
+  k.sort = itsu::sort_shape(ctx->n_events, ctx->n_clusters, ctx->max_segment);
+  k.levels = itsu::level_shape(ctx->max_segment);
+  return k;
+}
+
+// Launches the whole sequence: kernel by kernel for inputs that were not the last ones (a graph costs
+// several runs of a small event to make, and events of other sizes need another), through a CUDA graph
+// from the third run in a row on (a caller that asks for the road count and then for the roads runs
+// its inputs twice).
+itsu_status launch_all(itsu_context *ctx)
+{
+  constexpr int kRunsBeforeGraph = 2;
+  const RunKey key = run_key(ctx);
+  if (!(ctx->graph && key == ctx->graph_key)) {
+    ctx->last_key_runs = key == ctx->last_key ? ctx->last_key_runs + 1 : 1;
+    ctx->last_key = key;
+    if (ctx->last_key_runs <= kRunsBeforeGraph) {
+      enqueue_all(ctx);
+      ITSU_CUDA(ctx, cudaGetLastError());
+      return ITSU_OK;
+    }
     drop_graph(ctx);
     cudaGraph_t g = nullptr;
     ITSU_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
@@ -676,23 +726,7 @@ itsu_status launch_all(itsu_context *ctx)
       ctx->graph = nullptr;
       return fail(ctx, ITSU_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(inst_err));
     }
-    ctx->graph_generation = ctx->generation;
-    ctx->graph_key[0] = ctx->in_raw;
-    ctx->graph_key[1] = ctx->in_layer_off;
-    ctx->graph_key[2] = ctx->in_vtx;
-    ctx->graph_key[3] = ctx->in_raw_off;
-    ctx->graph_key[4] = ctx->in_raw_in;
-    ctx->graph_key[5] = ctx->in_raw_track;
-    ctx->graph_tune[0] = tune.block;
-    ctx->graph_tune[1] = tune.blocks_per_sm;
-    ctx->graph_tune[2] = tune.prune;
-    ctx->graph_tune[3] = tune.group;
-    ctx->graph_prefilter = ctx->prefilter;
-    ctx->graph_sort = sort;
-    ctx->graph_levels = levels;
-    ctx->graph_gate = ctx->gate;
-    ctx->graph_events = ctx->n_events;
-    ctx->graph_clusters = ctx->n_clusters;
+    ctx->graph_key = key;
   }
   ITSU_CUDA(ctx, cudaGraphLaunch(ctx->graph, ctx->stream));
   return ITSU_OK;
@@ -790,6 +824,20 @@ itsu_status require_stage(itsu_context *ctx, int stage, const char *what)
   return ITSU_OK;
 }
 
+// The pinned buffer, with no copy of an earlier call (one that ended in an error) in flight from it.
+itsu_status ensure_pinned(itsu_context *ctx)
+{
+  if (!ctx->h_pinned) ITSU_CUDA(ctx, cudaMallocHost((void **)&ctx->h_pinned, kPinned));
+  for (cudaEvent_t &e : ctx->piece_sent) {
+    if (!e) ITSU_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
+  if (ctx->pinned_busy) {
+    ITSU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    ctx->pinned_busy = false;
+  }
+  return ITSU_OK;
+}
+
 // Host inputs of one vertex -> device arena.
 itsu_status upload_vertex(itsu_context *ctx, const itsu_cluster *const layers[ITSU_LAYERS], const int32_t counts[ITSU_LAYERS],
                           const float vertex[3])
@@ -804,14 +852,37 @@ itsu_status upload_vertex(itsu_context *ctx, const itsu_cluster *const layers[IT
   }
   itsu_status st;
   if ((st = ensure_clusters(ctx, off[ITSU_LAYERS], 1)) != ITSU_OK) return st;
-  for (int l = 0; l < ITSU_LAYERS; ++l) {
-    if (counts[l] > 0) {
-      ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->raw + off[l], layers[l], sizeof(itsu_cluster) * counts[l], cudaMemcpyHostToDevice,
-                                     ctx->stream));
+  if ((st = ensure_pinned(ctx)) != ITSU_OK) return st;
+  // the head and the layers as one run of bytes, gathered a piece at a time: one copy for small events;
+  // the copies of larger ones run while the next piece is gathered
+  unsigned char head[kRawHead] = {};
+  std::memcpy(head, off.data(), sizeof(int32_t) * off.size());
+  std::memcpy(head + sizeof(int32_t) * off.size(), vertex, sizeof(float) * 3);
+  ctx->pinned_busy = true;
+  size_t sent = 0, filled = 0;  // bytes of the run that are copied, and gathered
+  auto send = [&]() -> itsu_status {
+    const int piece = (int)(sent / kPiece) % kPieces;
+    ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->raw_head + sent, ctx->h_pinned + piece * kPiece, filled - sent, cudaMemcpyHostToDevice, ctx->stream));
+    ITSU_CUDA(ctx, cudaEventRecord(ctx->piece_sent[piece], ctx->stream));
+    sent = filled;
+    return ITSU_OK;
+  };
+  for (int l = -1; l < ITSU_LAYERS; ++l) {
+    const unsigned char *src = l < 0 ? head : reinterpret_cast<const unsigned char *>(layers[l]);
+    size_t left = l < 0 ? kRawHead : sizeof(itsu_cluster) * (size_t)counts[l];
+    while (left > 0) {
+      if (filled == sent && filled >= kPinned) {  // a piece used before
+        ITSU_CUDA(ctx, cudaEventSynchronize(ctx->piece_sent[(filled / kPiece) % kPieces]));
+      }
+      const size_t take = std::min(left, sent + kPiece - filled);
+      std::memcpy(ctx->h_pinned + filled % kPinned, src, take);
+      src += take;
+      left -= take;
+      filled += take;
+      if (filled == sent + kPiece && (st = send()) != ITSU_OK) return st;
     }
   }
-  ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->layer_off, off.data(), sizeof(int32_t) * off.size(), cudaMemcpyHostToDevice, ctx->stream));
-  ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->vtx, vertex, sizeof(float) * 3, cudaMemcpyHostToDevice, ctx->stream));
+  if (filled > sent && (st = send()) != ITSU_OK) return st;
   ctx->n_events = 1;
   ctx->n_clusters = off[ITSU_LAYERS];
   ctx->h_layer_off = off;
@@ -820,9 +891,44 @@ itsu_status upload_vertex(itsu_context *ctx, const itsu_cluster *const layers[IT
   ctx->in_raw_in = nullptr;
   ctx->in_raw_track = nullptr;
   ctx->in_raw_off = nullptr;
-  ctx->in_layer_off = ctx->layer_off;
-  ctx->in_vtx = ctx->vtx;
+  ctx->in_layer_off = reinterpret_cast<const int32_t *>(ctx->raw_head);
+  ctx->in_vtx = reinterpret_cast<const float *>(ctx->raw_head + sizeof(int32_t) * (ITSU_LAYERS + 1));
   ctx->stage = kNone;
+  return ITSU_OK;
+}
+
+// An event's lists on their way to the caller's memory. Up to kPinned bytes go through the pinned buffer
+// with one wait for all, in place of a staged copy of the driver's for each; what does not fit goes
+// directly.
+struct Download {
+  void *dst;
+  size_t at, bytes;
+};
+using Downloads = std::vector<Download>;
+
+template <typename T>
+itsu_status copy_list(itsu_context *ctx, Downloads &lists, T *dst, const T *src, int64_t count)
+{
+  if (!dst || count <= 0) return ITSU_OK;
+  const size_t bytes = sizeof(T) * (size_t)count;
+  const size_t at = lists.empty() ? 0 : (lists.back().at + lists.back().bytes + 15) / 16 * 16;
+  if (at + bytes > kPinned) {
+    ITSU_CUDA(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    return ITSU_OK;
+  }
+  itsu_status st;
+  if (lists.empty() && (st = ensure_pinned(ctx)) != ITSU_OK) return st;
+  ctx->pinned_busy = true;
+  ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->h_pinned + at, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+  lists.push_back(Download{dst, at, bytes});
+  return ITSU_OK;
+}
+
+itsu_status finish_downloads(itsu_context *ctx, const Downloads &lists)
+{
+  ITSU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  ctx->pinned_busy = false;
+  for (const Download &d : lists) std::memcpy(d.dst, ctx->h_pinned + d.at, d.bytes);
   return ITSU_OK;
 }
 
@@ -835,36 +941,20 @@ itsu_status copy_range(itsu_context *ctx, T *dst, const T *src, int64_t count)
   return ITSU_OK;
 }
 
-struct EventSegments {
-  int32_t lo[ITSU_LAYERS + 1];
-  int32_t ts[ITSU_TRACKLET_LAYERS + 1];
-  int32_t cs[ITSU_CELL_LAYERS + 1];
-  int32_t rs[2];
-  int32_t nbo[ITSU_CELL_LAYERS + 1];  // nb_off at cs[0..5]
-};
-
 itsu_status event_segments(itsu_context *ctx, int32_t e, EventSegments &seg)
 {
   if (e < 0 || e >= ctx->n_events) return fail(ctx, ITSU_ERR_INVALID, "event %d out of range", e);
   // Only the segments of stages that have run exist: the others read as empty.
   std::memset(&seg, 0, sizeof seg);
-  std::memcpy(seg.lo, ctx->h_layer_off.data() + (int64_t)e * ITSU_LAYERS, sizeof seg.lo);
   if (ctx->stage >= kTracklets) {
-    ITSU_CUDA(ctx, cudaMemcpyAsync(seg.ts, ctx->trk_seg + (int64_t)e * ITSU_TRACKLET_LAYERS, sizeof seg.ts, cudaMemcpyDeviceToHost, ctx->stream));
-  }
-  if (ctx->stage >= kCells) {
-    ITSU_CUDA(ctx, cudaMemcpyAsync(seg.cs, ctx->cell_seg + (int64_t)e * ITSU_CELL_LAYERS, sizeof seg.cs, cudaMemcpyDeviceToHost, ctx->stream));
-  }
-  if (ctx->stage >= kRoads) {
-    ITSU_CUDA(ctx, cudaMemcpyAsync(seg.rs, ctx->road_seg + e, sizeof seg.rs, cudaMemcpyDeviceToHost, ctx->stream));
-  }
-  ITSU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (ctx->stage >= kNeighbours) {
-    for (int l = 0; l <= ITSU_CELL_LAYERS; ++l) {
-      ITSU_CUDA(ctx, cudaMemcpyAsync(&seg.nbo[l], ctx->nb_off + seg.cs[l], sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-    }
+    itsu::launch_event_segments(arena_of(ctx), e, ctx->stage >= kCells, ctx->stage >= kNeighbours, ctx->stage >= kRoads,
+                                ctx->d_segments, ctx->stream);
+    ITSU_CUDA(ctx, cudaGetLastError());
+    ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->h_segments, ctx->d_segments, sizeof seg, cudaMemcpyDeviceToHost, ctx->stream));
     ITSU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    seg = *ctx->h_segments;
   }
+  std::memcpy(seg.lo, ctx->h_layer_off.data() + (int64_t)e * ITSU_LAYERS, sizeof seg.lo);
   return ITSU_OK;
 }
 
@@ -951,6 +1041,8 @@ itsu_status itsu_context_create(const itsu_config *cfg, itsu_context **out)
     if ((err = cudaMalloc((void **)&ctx->d_status, sizeof(DevStatus))) != cudaSuccess) break;
     if ((err = cudaMallocHost((void **)&ctx->h_status, sizeof(DevStatus))) != cudaSuccess) break;
     std::memset(ctx->h_status, 0, sizeof(DevStatus));
+    if ((err = cudaMalloc((void **)&ctx->d_segments, sizeof(EventSegments))) != cudaSuccess) break;
+    if ((err = cudaMallocHost((void **)&ctx->h_segments, sizeof(EventSegments))) != cudaSuccess) break;
     if (c.max_clusters > 0 || c.max_events > 0) {
       ctx->stage = -1;  // initial allocation: allowed even with ITSU_FLAG_NO_GROW
       if ((st = ensure_clusters(ctx, c.max_clusters, c.max_events)) != ITSU_OK) break;
@@ -978,7 +1070,7 @@ void itsu_context_destroy(itsu_context *ctx)
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->twin) itsu_context_destroy(ctx->twin);
   drop_graph(ctx);
-  release(ctx->raw); release(ctx->raw_in); release(ctx->raw_track); release(ctx->sorted); release(ctx->sort_recs); release(ctx->sort_index); release(ctx->xyzr); release(ctx->phi);
+  release(ctx->raw_head); release(ctx->raw_in); release(ctx->raw_track); release(ctx->sorted); release(ctx->sort_recs); release(ctx->sort_index); release(ctx->xyzr); release(ctx->phi);
   release(ctx->trk_count); release(ctx->trk_off); release(ctx->trk_range); release(ctx->trk_lookup); release(ctx->zs); release(ctx->clu_seg); release(ctx->clu_aux); release(ctx->clu_crowded); release(ctx->trk_slots);
   release(ctx->seg_rrange); release(ctx->seg_regular); release(ctx->raw_off);
   release(ctx->layer_off); release(ctx->index_tables); release(ctx->trk_seg); release(ctx->cell_seginfo); release(ctx->cell_seg); release(ctx->cell_seg_count);
@@ -1000,6 +1092,12 @@ void itsu_context_destroy(itsu_context *ctx)
     if (e) cudaEventDestroy(e);
   }
   if (ctx->h_road_end) cudaFreeHost(ctx->h_road_end);
+  if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
+  for (cudaEvent_t &e : ctx->piece_sent) {
+    if (e) cudaEventDestroy(e);
+  }
+  release(ctx->d_segments);
+  if (ctx->h_segments) cudaFreeHost(ctx->h_segments);
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   if (ctx->d2h_stream) cudaStreamDestroy(ctx->d2h_stream);
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
@@ -1129,21 +1227,23 @@ itsu_status itsu_copy_results(itsu_context *ctx, int32_t event, const itsu_resul
   if ((st = event_segments(ctx, event, s)) != ITSU_OK) return st;
   itsu_counts n;
   counts_from(ctx, s, &n);
+  Downloads lists;
+  lists.reserve(64);
   for (int l = 0; l < ITSU_LAYERS; ++l) {
-    if ((st = copy_range(ctx, out->clusters[l], ctx->sorted + s.lo[l], n.clusters[l])) != ITSU_OK) return st;
+    if ((st = copy_list(ctx, lists, out->clusters[l], ctx->sorted + s.lo[l], n.clusters[l])) != ITSU_OK) return st;
   }
   for (int l = 0; l < ITSU_TRACKLET_LAYERS; ++l) {
-    if ((st = copy_range(ctx, out->index_tables[l], ctx->index_tables + ((int64_t)event * ITSU_TRACKLET_LAYERS + l) * ITSU_INDEX_TABLE_SIZE,
+    if ((st = copy_list(ctx, lists, out->index_tables[l], ctx->index_tables + ((int64_t)event * ITSU_TRACKLET_LAYERS + l) * ITSU_INDEX_TABLE_SIZE,
                          ITSU_INDEX_TABLE_SIZE)) != ITSU_OK) {
       return st;
     }
   }
   if (ctx->stage >= kTracklets) {
     for (int l = 0; l < ITSU_TRACKLET_LAYERS; ++l) {
-      if ((st = copy_range(ctx, out->tracklets[l], ctx->tracklets + s.ts[l], n.tracklets[l])) != ITSU_OK) return st;
+      if ((st = copy_list(ctx, lists, out->tracklets[l], ctx->tracklets + s.ts[l], n.tracklets[l])) != ITSU_OK) return st;
     }
     for (int l = 0; l < ITSU_CELL_LAYERS; ++l) {
-      if ((st = copy_range(ctx, out->tracklets_lookup[l], ctx->trk_lookup + s.lo[l + 1], n.clusters[l + 1])) != ITSU_OK) return st;
+      if ((st = copy_list(ctx, lists, out->tracklets_lookup[l], ctx->trk_lookup + s.lo[l + 1], n.clusters[l + 1])) != ITSU_OK) return st;
     }
   } else {
     for (int l = 0; l < ITSU_CELL_LAYERS; ++l) {
@@ -1152,10 +1252,10 @@ itsu_status itsu_copy_results(itsu_context *ctx, int32_t event, const itsu_resul
   }
   if (ctx->stage >= kCells) {
     for (int l = 0; l < ITSU_CELL_LAYERS; ++l) {
-      if ((st = copy_range(ctx, out->cells[l], ctx->cells + s.cs[l], n.cells[l])) != ITSU_OK) return st;
+      if ((st = copy_list(ctx, lists, out->cells[l], ctx->cells + s.cs[l], n.cells[l])) != ITSU_OK) return st;
     }
     for (int l = 0; l < ITSU_NEIGHBOUR_LAYERS; ++l) {
-      if ((st = copy_range(ctx, out->cells_lookup[l], ctx->cell_lookup + s.ts[l + 1], n.tracklets[l + 1])) != ITSU_OK) return st;
+      if ((st = copy_list(ctx, lists, out->cells_lookup[l], ctx->cell_lookup + s.ts[l + 1], n.tracklets[l + 1])) != ITSU_OK) return st;
     }
   } else {
     for (int l = 0; l < ITSU_NEIGHBOUR_LAYERS; ++l) {  // no cells yet: every lookup entry unused
@@ -1164,8 +1264,8 @@ itsu_status itsu_copy_results(itsu_context *ctx, int32_t event, const itsu_resul
   }
   if (ctx->stage >= kNeighbours) {
     for (int l = 0; l < ITSU_NEIGHBOUR_LAYERS; ++l) {
-      if ((st = copy_range(ctx, out->neighbour_offsets[l], ctx->nb_off + s.cs[l + 1], (int64_t)n.cells[l + 1] + 1)) != ITSU_OK) return st;
-      if ((st = copy_range(ctx, out->neighbours[l], ctx->nb + s.nbo[l + 1], n.neighbours[l])) != ITSU_OK) return st;
+      if ((st = copy_list(ctx, lists, out->neighbour_offsets[l], ctx->nb_off + s.cs[l + 1], (int64_t)n.cells[l + 1] + 1)) != ITSU_OK) return st;
+      if ((st = copy_list(ctx, lists, out->neighbours[l], ctx->nb + s.nbo[l + 1], n.neighbours[l])) != ITSU_OK) return st;
     }
   } else {
     for (int l = 0; l < ITSU_NEIGHBOUR_LAYERS; ++l) {  // no neighbours yet: empty rows
@@ -1173,9 +1273,9 @@ itsu_status itsu_copy_results(itsu_context *ctx, int32_t event, const itsu_resul
     }
   }
   if (ctx->stage >= kRoads) {
-    if ((st = copy_range(ctx, out->roads, ctx->roads + s.rs[0], n.roads)) != ITSU_OK) return st;
+    if ((st = copy_list(ctx, lists, out->roads, (const itsu_road *)ctx->roads + s.rs[0], n.roads)) != ITSU_OK) return st;
   }
-  ITSU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if ((st = finish_downloads(ctx, lists)) != ITSU_OK) return st;
   if (ctx->stage >= kNeighbours) {
     for (int l = 0; l < ITSU_NEIGHBOUR_LAYERS; ++l) {  // rebase the CSR rows to this layer
       if (out->neighbour_offsets[l]) {
@@ -1200,8 +1300,9 @@ itsu_status itsu_clusters_to_tracks(itsu_context *ctx, const itsu_cluster *const
   if (roads_count) *roads_count = (int32_t)total;
   if (roads) {
     if (total > roads_capacity) return fail(ctx, ITSU_ERR_CAPACITY, "%lld roads do not fit the %d given", (long long)total, roads_capacity);
-    if ((st = copy_range(ctx, roads, (const itsu_road *)ctx->roads, total)) != ITSU_OK) return st;
-    ITSU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    Downloads lists;
+    if ((st = copy_list(ctx, lists, roads, (const itsu_road *)ctx->roads, total)) != ITSU_OK) return st;
+    if ((st = finish_downloads(ctx, lists)) != ITSU_OK) return st;
   }
   return ITSU_OK;
 }

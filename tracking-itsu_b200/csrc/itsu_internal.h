@@ -193,6 +193,18 @@ void launch_neighbours_write(const Arena &a, const Launch &l);
 void launch_roads_count(const Arena &a, const Launch &l);
 void launch_roads_write(const Arena &a, const Launch &l);
 
+// One event's segments, for the calls that return its lists: clusters, tracklets, cells per layer, its
+// roads, and where the neighbour rows of each cell layer start.
+struct EventSegments {
+  int32_t lo[ITSU_LAYERS + 1];
+  int32_t ts[ITSU_TRACKLET_LAYERS + 1];
+  int32_t cs[ITSU_CELL_LAYERS + 1];
+  int32_t rs[2];
+  int32_t nbo[ITSU_CELL_LAYERS + 1];  // nb_off at cs[0..5]
+};
+// Fills *out but for lo; what has not run (cells, neighbours, roads) as zeros.
+void launch_event_segments(const Arena &a, int32_t e, bool cells, bool neighbours, bool roads, EventSegments *out, cudaStream_t stream);
+
 // Streamed host runs: append the last run's roads and road offsets at event e0 of the batch-wide
 // output, and snapshot its status.
 void launch_append_roads(const Arena &a, const Launch &l, itsu_road *dst, int32_t *dst_off, int32_t e0, int64_t cap,

@@ -216,7 +216,16 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Arena a, const int32_t *_
   }
 }
 
-int scan_grid(const Launch &l) { return l.num_sms * 4; }
+// Blocks of a grid-stride kernel: those of a full grid, or what about `items` items need. The counts
+// are on the device; the host goes by the clusters (10 tracklets and 2 cells each are the arena's first
+// sizes, above what any workload here has), and any grid gives the same results. A pp event's kernels
+// took 5.5 us each with full grids of idle blocks.
+unsigned blocks_for(int64_t full, int64_t items, int64_t per_block)
+{
+  return (unsigned)std::max<int64_t>(1, std::min(full, (items + per_block - 1) / per_block));
+}
+int64_t likely_tracklets(const Arena &a) { return 10 * a.n_clusters; }
+int64_t likely_cells(const Arena &a) { return 2 * a.n_clusters; }
 
 // The four scans of a run: tracklets per cluster, cells per span of tracklets, neighbours per cell,
 // roads per cell. The first leaves the check of its capacity to the segment pass.
@@ -225,19 +234,19 @@ void step_scan(const Arena &a, const Launch &l)
 {
   switch (kWhich) {
   case 0:
-    k_scan<false><<<scan_grid(l), kScanThreads, 0, l.stream>>>(a, a.trk_count, a.trk_off, nullptr, a.n_clusters, a.scan_partials,
+    k_scan<false><<<blocks_for(l.num_sms * 4, a.n_clusters, kScanTile), kScanThreads, 0, l.stream>>>(a, a.trk_count, a.trk_off, nullptr, a.n_clusters, a.scan_partials,
                                                                 &a.status->total[kTracklets], INT64_MAX, 0);
     break;
   case 1:
-    k_scan<true><<<scan_grid(l), kScanThreads, 0, l.stream>>>(a, a.cell_span_count, a.cell_span_off, &a.status->cell_spans, 0, a.scan_partials,
+    k_scan<true><<<blocks_for(l.num_sms * 4, likely_tracklets(a) / 32, kScanTile) + 1, kScanThreads, 0, l.stream>>>(a, a.cell_span_count, a.cell_span_off, &a.status->cell_spans, 0, a.scan_partials,
                                                                &a.status->total[kCells], a.cap_cells, kFlagCapCells);
     break;
   case 2:
-    k_scan<false><<<scan_grid(l), kScanThreads, 0, l.stream>>>(a, a.nb_count, a.nb_off, &a.status->total[kCells], 0, a.scan_partials,
+    k_scan<false><<<blocks_for(l.num_sms * 4, likely_cells(a), kScanTile), kScanThreads, 0, l.stream>>>(a, a.nb_count, a.nb_off, &a.status->total[kCells], 0, a.scan_partials,
                                                                 &a.status->total[kNeighbours], a.cap_neighbours, kFlagCapNeighbours);
     break;
   default:
-    k_scan<false><<<scan_grid(l), kScanThreads, 0, l.stream>>>(a, a.road_count, a.road_off, &a.status->total[kCells], 0, a.road_partials,
+    k_scan<false><<<blocks_for(l.num_sms * 4, likely_cells(a), kScanTile), kScanThreads, 0, l.stream>>>(a, a.road_count, a.road_off, &a.status->total[kCells], 0, a.road_partials,
                                                                 &a.status->total[kRoads], a.cap_roads, kFlagCapRoads);
   }
 }
@@ -2254,7 +2263,8 @@ int fixed_grid(const Launch &l) { return l.num_sms * l.blocks_per_sm; }
 dim3 event_grid(const Arena &a, const Launch &l)
 {
   const int rows = std::min(a.n_events, 65535);
-  return dim3((unsigned)std::max(1, (fixed_grid(l) + rows - 1) / rows), (unsigned)rows);
+  const int64_t full = std::max(1, (fixed_grid(l) + rows - 1) / rows);
+  return dim3(blocks_for(full, likely_cells(a) / std::max(rows, 1), l.block), (unsigned)rows);
 }
 
 void step_status_init(const Arena &a, const Launch &l)
@@ -2383,18 +2393,21 @@ void step_tracklets_crowded(const Arena &a, const Launch &l)
   }
 }
 
+// Blocks for the segments, and for the crowded clusters of larger runs.
+unsigned segment_blocks(const Arena &a, const Launch &l) { return blocks_for(l.num_sms, a.n_events * ITSU_TRACKLET_LAYERS + a.n_clusters / 32, 128); }
+
 void step_tracklet_segments(const Arena &a, const Launch &l)
 {
   if (a.gate) {
-    k_tracklet_segments<true><<<l.num_sms, 128, 0, l.stream>>>(a, !l.staged);
+    k_tracklet_segments<true><<<segment_blocks(a, l), 128, 0, l.stream>>>(a, !l.staged);
   } else {
-    k_tracklet_segments<false><<<l.num_sms, 128, 0, l.stream>>>(a, !l.staged);
+    k_tracklet_segments<false><<<segment_blocks(a, l), 128, 0, l.stream>>>(a, !l.staged);
   }
 }
 
 void launch_cells_range(const Arena &a, const Launch &l, int32_t e0, int32_t e1, bool last)
 {
-  k_cells_count<<<l.num_sms * kCellBlocks, kCellThreads, 0, l.stream>>>(a, e0, e1, last);
+  k_cells_count<<<blocks_for(l.num_sms * kCellBlocks, likely_tracklets(a), kCellThreads), kCellThreads, 0, l.stream>>>(a, e0, e1, last);
 }
 
 void step_cells_count(const Arena &a, const Launch &l)
@@ -2429,7 +2442,7 @@ void step_cells_prefilter(const Arena &a, const Launch &l)
   }
 }
 
-void step_cells_scatter(const Arena &a, const Launch &l) { k_cells_scatter<<<l.num_sms * 8, kScatterThreads, 0, l.stream>>>(a); }
+void step_cells_scatter(const Arena &a, const Launch &l) { k_cells_scatter<<<blocks_for(l.num_sms * 8, likely_tracklets(a) / 32, kScatterThreads / 32), kScatterThreads, 0, l.stream>>>(a); }
 
 void step_neighbour_reset(const Arena &a, const Launch &l)
 {
@@ -2439,7 +2452,7 @@ void step_neighbour_reset(const Arena &a, const Launch &l)
 }
 
 template <bool kWrite>
-void step_neighbours(const Arena &a, const Launch &l) { k_neighbours<kWrite><<<fixed_grid(l), l.block, 0, l.stream>>>(a); }
+void step_neighbours(const Arena &a, const Launch &l) { k_neighbours<kWrite><<<blocks_for(fixed_grid(l), likely_cells(a), l.block), l.block, 0, l.stream>>>(a); }
 
 // Threads for about half of the cells of the largest event's largest layer (a layer of hits has about
 // 1.3 cells per hit), so that a layer takes one or two rounds.
@@ -2542,8 +2555,10 @@ __global__ void k_append_roads(Arena a, itsu_road *dst, int32_t *dst_off, int32_
   const bool fits = base + total <= cap;
   const int64_t tid = global_thread(), threads = grid_threads();
   if (ok && fits) {
-    for (int64_t r = tid; r < total; r += threads) {
-      dst[base + r] = a.roads[r];
+    const int4 *from = reinterpret_cast<const int4 *>(a.roads);  // 32-byte records, two 16-byte words each
+    int4 *to = reinterpret_cast<int4 *>(dst + base);
+    for (int64_t r = tid; r < 2 * total; r += threads) {
+      to[r] = from[r];
     }
     for (int64_t e = tid + 1; e <= a.n_events; e += threads) {
       dst_off[e0 + e] = (int32_t)(base + a.road_seg[e]);
@@ -2560,6 +2575,27 @@ __global__ void k_append_roads(Arena a, itsu_road *dst, int32_t *dst_off, int32_
     }
     *snap = st;
   }
+}
+
+__global__ void k_event_segments(Arena a, int32_t e, bool cells, bool neighbours, bool roads, EventSegments *out)
+{
+  const int k = threadIdx.x;
+  if (k <= ITSU_TRACKLET_LAYERS) {
+    out->ts[k] = a.trk_seg[(int64_t)e * ITSU_TRACKLET_LAYERS + k];
+  }
+  if (k <= ITSU_CELL_LAYERS) {
+    const int32_t c = cells ? a.cell_seg[(int64_t)e * ITSU_CELL_LAYERS + k] : 0;
+    out->cs[k] = c;
+    out->nbo[k] = neighbours ? a.nb_off[c] : 0;
+  }
+  if (k < 2) {
+    out->rs[k] = roads ? a.road_seg[e + k] : 0;
+  }
+}
+
+void launch_event_segments(const Arena &a, int32_t e, bool cells, bool neighbours, bool roads, EventSegments *out, cudaStream_t stream)
+{
+  k_event_segments<<<1, 32, 0, stream>>>(a, e, cells, neighbours, roads, out);
 }
 
 void launch_append_roads(const Arena &a, const Launch &l, itsu_road *dst, int32_t *dst_off, int32_t e0, int64_t cap, DevStatus *snap)

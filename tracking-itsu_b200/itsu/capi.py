@@ -429,11 +429,16 @@ class Context:
         """Whole path for one vertex in one call; returns its roads."""
         keep, ptrs, counts, v = self._layer_args(layers, vertex)
         n = ctypes.c_int32()
-        self._check(self.lib.itsu_clusters_to_tracks(self.h, ptrs, counts, v, None, 0, ctypes.byref(n)))
-        roads = np.zeros(n.value, ROAD_DTYPE)
-        self._check(self.lib.itsu_clusters_to_tracks(self.h, ptrs, counts, v, _ptr(roads), n.value, ctypes.byref(n)))
-        roads["pad"] = 0
-        return roads
+        # room for one road per cluster first: central events have one per six, small ones one per two
+        room = sum(counts) + 64
+        while True:
+            roads = np.empty(room, ROAD_DTYPE)
+            st = self.lib.itsu_clusters_to_tracks(self.h, ptrs, counts, v, _ptr(roads), room, ctypes.byref(n))
+            if st != ERR_CAPACITY or n.value <= room:
+                break
+            room, n.value = n.value, 0  # they did not fit: again with room for all
+        self._check(st)
+        return roads[: n.value].copy()
 
     # ---- batches ----
     def memory_usage(self) -> dict:
