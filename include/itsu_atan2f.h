@@ -17,14 +17,17 @@
  *     <= 30 significant bits and their exponents are at most two apart), |u| <= 1/64 + 2^-20, and
  *     atan(u) is a 6-term Taylor polynomial. Octant reconstruction uses pi/2 - a and pi - a.
  *     The relative error is below 2^-48; the result is returned when the interval
- *     [a - 2^-44 a, a + 2^-44 a] does not contain a binary32 rounding boundary.
+ *     [a - 2^-44 a, a + 2^-44 a] does not contain a binary32 rounding boundary (read off the 29 bits of
+ *     a below a binary32 significand).
  *  2. Otherwise (about 2e-6 of inputs) the same reduction is re-evaluated in double-double
  *     arithmetic (Dekker's exact product and Knuth's two-sum) with a 10-term series
  *     (relative error ~2^-100) and rounded with the low word deciding exact midpoints.
- * Only IEEE binary64 +, -, *, / and conversions are used. On the device every one of them is
- * an explicitly rounded intrinsic (__dadd_rn, ...), so nvcc cannot contract them into FMAs;
- * host code must be compiled without FP contraction (-ffp-contract=off), as the library's
- * build does. The tables atan(k/32), pi, pi/2 and 1/(2m+1) are double-double values computed
+ * The host uses IEEE binary64 +, -, *, / and conversions only. The device's fast path uses fused
+ * multiply-adds and a Newton-Raphson quotient in their place: its low bits differ, but whatever passes
+ * the rounding test is the correctly rounded value on either side, and the rest takes the slow path,
+ * whose every operation is an explicitly rounded intrinsic (__dadd_rn, ...) on the device, so that nvcc
+ * cannot contract them; host code must be compiled without FP contraction (-ffp-contract=off), as the
+ * library's build does. The tables atan(k/32), pi, pi/2 and 1/(2m+1) are double-double values computed
  * with 300-bit mpmath.
  */
 #ifndef ITSU_ATAN2F_H
@@ -46,7 +49,6 @@
 #define ITSU_DDIV(a, b) __ddiv_rn((a), (b))
 #define ITSU_D2F(a) __double2float_rn(a)
 #define ITSU_D2I_RZ(a) __double2int_rz(a)
-#define ITSU_FDIV(a, b) __fdiv_rn((a), (b))
 #define ITSU_FMUL(a, b) __fmul_rn((a), (b))
 #define ITSU_FADD(a, b) __fadd_rn((a), (b))
 #define ITSU_F2I_RZ(a) __float2int_rz(a)
@@ -57,7 +59,6 @@
 #define ITSU_DDIV(a, b) ((a) / (b))
 #define ITSU_D2F(a) ((float)(a))
 #define ITSU_D2I_RZ(a) ((int)(a))
-#define ITSU_FDIV(a, b) ((a) / (b))
 #define ITSU_FMUL(a, b) ((a) * (b))
 #define ITSU_FADD(a, b) ((a) + (b))
 #define ITSU_F2I_RZ(a) ((int)(a))
@@ -272,6 +273,116 @@ ITSU_CR_FN float itsu_cr_dd_to_float(itsu_cr_dd a)
   return f;
 }
 
+/* a b + c of the fast path: one rounding on the device, two (without contraction) on the host. Both keep
+ * the fast path's error below 2^-48; where the product is exact they agree. */
+ITSU_CR_FN double itsu_cr_mul_add(double a, double b, double c)
+{
+#if defined(__CUDA_ARCH__)
+  return __fma_rn(a, b, c);
+#else
+  return a * b + c;
+#endif
+}
+
+/* num / den of the fast path, for den in binary32's range: on the device a reciprocal estimate, two
+ * Newton-Raphson steps on it and one on the quotient (relative error below 2^-51; no branches, where the
+ * correctly rounded division has one). */
+ITSU_CR_FN double itsu_cr_divide(double num, double den)
+{
+#if defined(__CUDA_ARCH__)
+  double r, q;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(den));
+  r = __fma_rn(r, __fma_rn(-den, r, 1.0), r);
+  r = __fma_rn(r, __fma_rn(-den, r, 1.0), r);
+  q = __dmul_rn(num, r);
+  return __fma_rn(__fma_rn(-den, q, num), r, q);
+#else
+  return num / den;
+#endif
+}
+
+/* num / den within two units of the last place. k, which it picks, only has to be near: host and device
+ * may reduce by different k and round the same value. */
+ITSU_CR_FN float itsu_cr_quotient(float num, float den)
+{
+#if defined(__CUDA_ARCH__)
+  return den > 1e-30f && den < 1e30f ? __fdividef(num, den) : __fdiv_rn(num, den);
+#else
+  return num / den;
+#endif
+}
+
+/* Whether every value within 2^-44 a of a rounds to the same binary32 value as a > 0 does. For a in
+ * binary32's normal range the rounding boundaries are the values whose 29 bits below a binary32
+ * significand are 1 followed by zeros; 2^-44 a is less than 2^9 units of a's last place, so the test is
+ * that those bits are further than that from the boundary (a value across a power of two below a is no
+ * boundary: 2^-44 a does not reach it from there). */
+ITSU_CR_FN int itsu_cr_rounds_safely(double a)
+{
+  uint32_t low, high;
+#if defined(__CUDA_ARCH__)
+  low = (uint32_t)__double2loint(a);
+  high = (uint32_t)__double2hiint(a);
+#else
+  uint64_t bits;
+  memcpy(&bits, &a, sizeof bits);
+  low = (uint32_t)bits;
+  high = (uint32_t)(bits >> 32);
+#endif
+  /* the distance from the boundary is at least 512: low - (boundary - 511) is 1023 or more, modulo 2^29 */
+  return ((low - 0x0ffffe01u) & 0x1fffffffu) >= 1023u && high >= 0x38100000u; /* a >= 2^-126 */
+}
+
+/* The reduction of the fast path re-evaluated in double-double: |atan2| from num / den near k / 32, with
+ * the octant. On the device a function of its own: about one call in 500,000 comes here, and inlined it
+ * took the registers of every caller. */
+#if defined(__CUDACC__)
+static __host__ __device__ __noinline__
+#else
+static inline
+#endif
+    float
+    itsu_cr_slow_path(double num, double den, int k, int swap, int xneg)
+{
+#if defined(ITSU_CR_SLOW_PATH_HOOK)
+  ITSU_CR_SLOW_PATH_HOOK;
+#endif
+  const double c = ITSU_DMUL((double)k, 0.03125);
+  itsu_cr_dd dn, dden, du, ds, dp, dc, dr;
+  int m;
+  dn.hi = ITSU_DSUB(num, ITSU_DMUL(c, den)); /* exact */
+  dn.lo = 0.0;
+  dden = itsu_cr_two_sum(den, ITSU_DMUL(c, num)); /* the product is exact */
+  du = itsu_cr_dd_div(dn, dden);
+  ds = itsu_cr_dd_mul(du, du);
+  dp.hi = itsu_cr_inv_odd[9][0];
+  dp.lo = itsu_cr_inv_odd[9][1];
+  dp = itsu_cr_dd_neg(dp); /* (-1)^9 / 19 */
+  for (m = 8; m >= 0; --m) {
+    dc.hi = itsu_cr_inv_odd[m][0];
+    dc.lo = itsu_cr_inv_odd[m][1];
+    if (m & 1) {
+      dc = itsu_cr_dd_neg(dc);
+    }
+    dp = itsu_cr_dd_add(dc, itsu_cr_dd_mul(ds, dp));
+  }
+  dr = itsu_cr_dd_mul(du, dp);
+  dc.hi = itsu_cr_atan_k32[k][0];
+  dc.lo = itsu_cr_atan_k32[k][1];
+  dr = itsu_cr_dd_add(dc, dr);
+  if (swap) {
+    dc.hi = ITSU_CR_PIO2_HI;
+    dc.lo = ITSU_CR_PIO2_LO;
+    dr = itsu_cr_dd_add(dc, itsu_cr_dd_neg(dr));
+  }
+  if (xneg) {
+    dc.hi = ITSU_CR_PI_HI;
+    dc.lo = ITSU_CR_PI_LO;
+    dr = itsu_cr_dd_add(dc, itsu_cr_dd_neg(dr));
+  }
+  return itsu_cr_dd_to_float(dr);
+}
+
 /* Correctly rounded atan2 for binary32 arguments (C99 Annex F special cases). */
 ITSU_CR_FN float itsu_atan2f(float y, float x)
 {
@@ -309,24 +420,21 @@ ITSU_CR_FN float itsu_atan2f(float y, float x)
     const int swap = ayf > axf;
     const float numf = swap ? axf : ayf, denf = swap ? ayf : axf;
     const double num = (double)numf, den = (double)denf;
-    /* k = round(32 t) from a binary32 quotient: |32 t - k| <= 1/2 + 2^-19, which keeps |u| within
-     * 1/64 + 2^-20 and the numerator below exact (both products have <= 30 significant bits and
-     * exponents at most two apart). */
-    const float tf = ITSU_FDIV(numf, denf);
+    /* k = round(32 t) from a binary32 quotient within two units of its last place: |32 t - k| <=
+     * 1/2 + 2^-16, which keeps |u| within 1/64 + 2^-20 and the numerator below exact (both products are
+     * multiples of 2^-5 of den's last place below 2^30 of them). */
+    const float tf = itsu_cr_quotient(numf, denf);
     const int k = ITSU_F2I_RZ(ITSU_FADD(ITSU_FMUL(tf, 32.0f), 0.5f));
     const double c = ITSU_DMUL((double)k, 0.03125);
-    const double nn = ITSU_DSUB(num, ITSU_DMUL(c, den)); /* exact */
-    const double cn = ITSU_DMUL(c, num);                 /* exact */
-    const double u = ITSU_DDIV(nn, ITSU_DADD(den, cn));
+    const double nn = itsu_cr_mul_add(-c, den, num); /* exact, product and sum */
+    const double u = itsu_cr_divide(nn, itsu_cr_mul_add(c, num, den));
     const double s = ITSU_DMUL(u, u);
-    double p = ITSU_DMUL(s, -0x1.745d1745d1746p-4); /* -1/11 */
-    double a, e, mlo, mhi, fd;
-    uint32_t fb;
-    p = ITSU_DMUL(s, ITSU_DADD(0x1.c71c71c71c71cp-4, p));  /* 1/9 */
-    p = ITSU_DMUL(s, ITSU_DADD(-0x1.2492492492492p-3, p)); /* -1/7 */
-    p = ITSU_DMUL(s, ITSU_DADD(0x1.999999999999ap-3, p));  /* 1/5 */
-    p = ITSU_DMUL(s, ITSU_DADD(-0x1.5555555555555p-2, p)); /* -1/3 */
-    p = ITSU_DADD(u, ITSU_DMUL(u, p));
+    double p = itsu_cr_mul_add(s, -0x1.745d1745d1746p-4, 0x1.c71c71c71c71cp-4); /* -1/11, 1/9 */
+    double a;
+    p = itsu_cr_mul_add(s, p, -0x1.2492492492492p-3); /* -1/7 */
+    p = itsu_cr_mul_add(s, p, 0x1.999999999999ap-3);  /* 1/5 */
+    p = itsu_cr_mul_add(s, p, -0x1.5555555555555p-2); /* -1/3 */
+    p = itsu_cr_mul_add(u, ITSU_DMUL(s, p), u);
     a = ITSU_DADD(itsu_cr_atan_k32[k][0], p);
     if (swap) {
       a = ITSU_DSUB(ITSU_CR_PIO2_HI, a);
@@ -335,55 +443,12 @@ ITSU_CR_FN float itsu_atan2f(float y, float x)
       a = ITSU_DSUB(ITSU_CR_PI_HI, a);
     }
     res = ITSU_D2F(a);
-    fd = (double)res;
-    fb = itsu_cr_f2u(res);
-    mhi = ITSU_DMUL(ITSU_DADD(fd, (double)itsu_cr_u2f(fb + 1u)), 0.5);
-    mlo = fb == 0u ? -(double)itsu_cr_u2f(1u) : ITSU_DMUL(ITSU_DADD(fd, (double)itsu_cr_u2f(fb - 1u)), 0.5);
-    e = ITSU_DMUL(a, 0x1.0p-44);
-    if (ITSU_DSUB(a, e) > mlo && ITSU_DADD(a, e) < mhi) {
+    if (itsu_cr_rounds_safely(a)) {
       return yneg ? -res : res;
     }
 
-    /* Slow path: the same reduction in double-double. */
-    {
-#if defined(ITSU_CR_SLOW_PATH_HOOK)
-      ITSU_CR_SLOW_PATH_HOOK;
-#endif
-      itsu_cr_dd dn, dden, du, ds, dp, dc, dr;
-      int m;
-      dn.hi = nn;
-      dn.lo = 0.0;
-      dden = itsu_cr_two_sum(den, cn);
-      du = itsu_cr_dd_div(dn, dden);
-      ds = itsu_cr_dd_mul(du, du);
-      dp.hi = itsu_cr_inv_odd[9][0];
-      dp.lo = itsu_cr_inv_odd[9][1];
-      dp = itsu_cr_dd_neg(dp); /* (-1)^9 / 19 */
-      for (m = 8; m >= 0; --m) {
-        dc.hi = itsu_cr_inv_odd[m][0];
-        dc.lo = itsu_cr_inv_odd[m][1];
-        if (m & 1) {
-          dc = itsu_cr_dd_neg(dc);
-        }
-        dp = itsu_cr_dd_add(dc, itsu_cr_dd_mul(ds, dp));
-      }
-      dr = itsu_cr_dd_mul(du, dp);
-      dc.hi = itsu_cr_atan_k32[k][0];
-      dc.lo = itsu_cr_atan_k32[k][1];
-      dr = itsu_cr_dd_add(dc, dr);
-      if (swap) {
-        dc.hi = ITSU_CR_PIO2_HI;
-        dc.lo = ITSU_CR_PIO2_LO;
-        dr = itsu_cr_dd_add(dc, itsu_cr_dd_neg(dr));
-      }
-      if (xneg) {
-        dc.hi = ITSU_CR_PI_HI;
-        dc.lo = ITSU_CR_PI_LO;
-        dr = itsu_cr_dd_add(dc, itsu_cr_dd_neg(dr));
-      }
-      res = itsu_cr_dd_to_float(dr);
-      return yneg ? -res : res;
-    }
+    res = itsu_cr_slow_path(num, den, k, swap, xneg);
+    return yneg ? -res : res;
   }
 }
 

@@ -733,6 +733,7 @@ __device__ __forceinline__ void write_tracklet(const Arena &a, int out, int64_t 
 {
   store_tracklet(a, out, make_tracklet(a.xyzr[i_flat], a.xyzr[j_flat], (int32_t)(i_flat - a.layer_off[seg]),
                                        (int32_t)(j_flat - a.layer_off[seg + 1])));
+  a.trk_seg_id[out] = seg - seg / ITSU_LAYERS;  // 7 e + L to 6 e + L
 }
 
 constexpr int kTrackletSlots = kTrackletSlotsPerCluster;
@@ -1137,12 +1138,6 @@ __global__ void __launch_bounds__(kCountThreads, kGate ? 5 : 6) k_tracklets_coun
   }
 }
 
-__device__ __forceinline__ float4 shfl4(float4 v, int src)
-{
-  return make_float4(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
-                     __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
-}
-
 __device__ __forceinline__ int warp_exclusive_sum(int v, int &total)
 {
   const int lane = threadIdx.x & 31;
@@ -1324,28 +1319,40 @@ __global__ void __launch_bounds__(kGateThreads) k_tracklets_gate(Arena a)
   }
 }
 
-// Write pass, a warp per 32 consecutive inner clusters: their tracklets form one contiguous range
-// (the scan of the counts), which the warp's lanes fill together: each lane takes the next
-// tracklet of the range, finds its inner cluster (owner) and rank there, reads the outer cluster
-// the count pass kept in that slot, and writes the tracklet (Tracklet.cxx:32-40), its key and its
-// segment id with coalesced stores; all lanes compute their binary64 azimuths together. Each cluster's
-// tracklets lookup entry is written here too. The tracklets of an inner cluster with more than
-// kTrackletSlots of them (not kept by the count pass) get their segment ids here and the rest
-// from k_tracklets_crowded.
+// Write pass, a warp per 32 consecutive inner clusters: the warp's lanes fill their clusters' tracklets
+// together, each taking the next one: it finds its inner cluster (owner) and rank there, reads the
+// outer cluster the count pass kept in that slot, and writes the tracklet (Tracklet.cxx:32-40), its key
+// and its segment id with coalesced stores; all lanes compute their binary64 azimuths together. What a
+// tracklet needs of its owner stands in shared memory. Each cluster's tracklets lookup entry is
+// written here too. The tracklets of an inner cluster with more than kTrackletSlots of them (not kept
+// by the count pass) come from write_crowded.
 // Runs over the inner clusters [c0, c1) (c0 a multiple of 32, so that warps hold whole aligned
 // groups of 32 clusters): all of them, or one event group's share of them.
-__global__ void __launch_bounds__(kMaxThreads, 2) k_tracklets_write(Arena a, int64_t c0, int64_t c1)  // 64 registers: 4 blocks of 256 per SM
+// Bound by the slots' and outer clusters' gathers with the azimuth's issue: 0.50 ms per 128 central
+// events at five blocks per SM (48 registers), 0.55 at six (the slots' lines, which a warp comes back
+// to, leave L1 too soon) or four; 0.58 with the owners' values in shuffles, the correctly rounded
+// division and the azimuth's double-double path inlined. Slots of a cluster side by side: 0.56.
+constexpr int kWriteThreads = 256;
+constexpr int kWriteBlocks = 5;  // resident blocks per SM
+
+struct WriteWarp {
+  float4 c[32];
+  int4 owner[32];  // first tracklet less the lanes' prefix, the prefix, cluster in its layer, first cluster of the next layer
+  int32_t sid[32];
+};
+
+__global__ void __launch_bounds__(kWriteThreads, kWriteBlocks) k_tracklets_write(Arena a, int64_t c0, int64_t c1)
 {
+  __shared__ WriteWarp shared[kWriteThreads / 32];
   if (capacity_failed(a.status)) {
     return;
   }
+  WriteWarp &w = shared[threadIdx.x >> 5];
   const int64_t i = c0 + global_thread();
   const int lane = threadIdx.x & 31;
-  const bool valid = i < c1;
-  int32_t first = 0, count = 0, local = 0, next_begin = 0;
+  int32_t first = 0, count = 0;
   int seg = 0, sid = 0;
-  float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  if (valid) {
+  if (i < c1) {
     first = a.trk_off[i];
     count = a.trk_off[i + 1] - first;
     a.trk_range[i] = make_int2(first, count);
@@ -1355,32 +1362,29 @@ __global__ void __launch_bounds__(kMaxThreads, 2) k_tracklets_write(Arena a, int
                           ? first - a.trk_seg[e * ITSU_TRACKLET_LAYERS + layer]
                           : ITSU_UNUSED_INDEX;
     sid = e * ITSU_TRACKLET_LAYERS + layer;
-    if (count > 0) {
-      c = a.xyzr[i];
-      local = (int32_t)(i - a.layer_off[seg]);
-      next_begin = a.layer_off[seg + 1];
+    if (count > kTrackletSlots) {
+      count = 0;
     }
   }
   int total = 0;
   const int excl = warp_exclusive_sum(count, total);
-  const int32_t base = __shfl_sync(0xffffffffu, first, 0);
-  const int64_t i0 = i - lane;
+  if (count > 0) {
+    w.c[lane] = a.xyzr[i];
+    w.owner[lane] = make_int4(first - excl, excl, (int32_t)(i - a.layer_off[seg]), a.layer_off[seg + 1]);
+    w.sid[lane] = sid;
+  }
+  __syncwarp();
+  const int32_t *slots = a.trk_slots + (i - lane);
   for (int p0 = 0; p0 < total; p0 += 32) {
     const int p = p0 + lane;
     const int owner = owner_of(excl, p);
-    const int rank = p - __shfl_sync(0xffffffffu, excl, owner);
-    const int owner_sid = __shfl_sync(0xffffffffu, sid, owner);
-    const int owner_count = __shfl_sync(0xffffffffu, count, owner);
-    const int32_t owner_local = __shfl_sync(0xffffffffu, local, owner);
-    const int32_t owner_next = __shfl_sync(0xffffffffu, next_begin, owner);
-    const float4 oc = shfl4(c, owner);
     if (p < total) {
-      a.trk_seg_id[base + p] = owner_sid;
-      if (owner_count <= kTrackletSlots) {
-        const int32_t j = a.trk_slots[(int64_t)rank * a.slot_stride + i0 + owner];
-        const float4 d = a.xyzr[owner_next + j];
-        store_tracklet(a, base + p, make_tracklet(oc, d, owner_local, j));
-      }
+      const int4 o = w.owner[owner];
+      const int32_t j = slots[(int64_t)(p - o.y) * a.slot_stride + owner];
+      const float4 d = a.xyzr[o.w + j];
+      const int32_t out = o.x + p;
+      a.trk_seg_id[out] = w.sid[owner];
+      store_tracklet(a, out, make_tracklet(w.c[owner], d, o.z, j));
     }
   }
 }
@@ -2366,9 +2370,9 @@ void step_tracklets_gate(const Arena &a, const Launch &l)
 
 void launch_write_range(const Arena &a, const Launch &l, int64_t c0, int64_t c1)
 {
-  const int64_t blocks = (c1 - c0 + l.block - 1) / l.block;
+  const int64_t blocks = (c1 - c0 + kWriteThreads - 1) / kWriteThreads;
   if (blocks > 0) {
-    k_tracklets_write<<<(unsigned)blocks, l.block, 0, l.stream>>>(a, c0, c1);
+    k_tracklets_write<<<(unsigned)blocks, kWriteThreads, 0, l.stream>>>(a, c0, c1);
   }
 }
 
