@@ -429,8 +429,8 @@ class Context:
         """Whole path for one vertex in one call; returns its roads."""
         keep, ptrs, counts, v = self._layer_args(layers, vertex)
         n = ctypes.c_int32()
-        # room for one road per cluster first: central events have one per six, small ones one per two
-        room = sum(counts) + 64
+        # room for two roads per cluster first: central events have one per six clusters, tiny ones up to two each
+        room = 2 * sum(counts) + 1024
         while True:
             roads = np.empty(room, ROAD_DTYPE)
             st = self.lib.itsu_clusters_to_tracks(self.h, ptrs, counts, v, _ptr(roads), room, ctypes.byref(n))
