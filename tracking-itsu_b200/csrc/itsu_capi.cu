@@ -126,7 +126,7 @@ struct itsu_context {
   // tracklet class
   itsu_tracklet *tracklets = nullptr;
   uint32_t *trk_key = nullptr;  // (tanL, phi) of each tracklet in fixed point, beside the records
-  int32_t *trk_seg_id = nullptr, *cell_lookup = nullptr, *cell_span_count = nullptr, *cell_span_off = nullptr;
+  int32_t *trk_seg32 = nullptr, *cell_lookup = nullptr, *cell_span_count = nullptr, *cell_span_off = nullptr;
   int2 *cell_span = nullptr;
   // cell class
   itsu_cell *cells = nullptr;
@@ -385,7 +385,7 @@ Arena arena_of(const itsu_context *ctx)
   a.cell_seginfo = ctx->cell_seginfo;
   a.tracklets = ctx->tracklets;
   a.trk_key = ctx->trk_key;
-  a.trk_seg_id = ctx->trk_seg_id;
+  a.trk_seg32 = ctx->trk_seg32;
   a.cell_span = ctx->cell_span;
   a.cell_span_count = ctx->cell_span_count;
   a.cell_span_off = ctx->cell_span_off;
@@ -495,7 +495,7 @@ itsu_status ensure_tracklets(itsu_context *ctx, int64_t need)
     const int64_t cap = grow_to(need);
     ITSU_CUDA(ctx, alloc(ctx, ctx->tracklets, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_key, cap + 4));  // read in aligned groups of four
-    ITSU_CUDA(ctx, alloc(ctx, ctx->trk_seg_id, cap));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->trk_seg32, cap / 32 + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_span, cap / 32 + 1));  // spans of 32 tracklets or more
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_span_count, cap / 32 + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_span_off, cap / 32 + 2));
@@ -1075,7 +1075,7 @@ void itsu_context_destroy(itsu_context *ctx)
   release(ctx->seg_rrange); release(ctx->seg_regular); release(ctx->raw_off);
   release(ctx->layer_off); release(ctx->index_tables); release(ctx->trk_seg); release(ctx->cell_seginfo); release(ctx->cell_seg); release(ctx->cell_seg_count);
   release(ctx->road_seg); release(ctx->vtx);
-  release(ctx->tracklets); release(ctx->trk_key); release(ctx->trk_seg_id); release(ctx->cell_span); release(ctx->cell_span_count); release(ctx->cell_span_off); release(ctx->cell_lookup);
+  release(ctx->tracklets); release(ctx->trk_key); release(ctx->trk_seg32); release(ctx->cell_span); release(ctx->cell_span_count); release(ctx->cell_span_off); release(ctx->cell_lookup);
   release(ctx->cells); release(ctx->cell_entries); release(ctx->cell_dca); release(ctx->cell_seg_id); release(ctx->nb_count); release(ctx->nb_off);
   release(ctx->nb_mask);
   release(ctx->road_count); release(ctx->road_off); release(ctx->paths);

@@ -116,7 +116,7 @@ struct Arena {
   itsu_tracklet *tracklets;
   int2 *trk_range;  // per inner cluster its first tracklet and their number: trk_off's two, in one 8-byte gather
   uint32_t *trk_key;  // per tracklet its (tanL, phi) in fixed point (tracklet_key): the cell pass's precut reads only these
-  int32_t *trk_seg_id;
+  int32_t *trk_seg32;  // the segment (6e + L) of every 32nd tracklet
   int4 *cell_seginfo;  // per tracklet segment, two records: {first cluster of L (-1: no cells), of L+1, of L+2,
                        // first tracklet of L}, {first tracklet of L+1, vertex x, y, z (float bits)}
   // cells
@@ -151,6 +151,30 @@ struct Arena {
   // capacities of the growable outputs
   int64_t cap_tracklets, cap_cells, cap_neighbours, cap_roads;
 };
+
+#if defined(__CUDACC__)
+// The segment (6e + L) of tracklet k: from the 32nd tracklet before it on, almost always the same one
+// (an id per tracklet took 4 bytes of each to write and to read).
+__device__ __forceinline__ int tracklet_segment(const Arena &a, int64_t k)
+{
+  int s = a.trk_seg32[k / 32];
+  if (k >= a.trk_seg[s + 1]) {
+    // steps that double, then halve: a batch may hold any number of empty events in a row
+    const int end = a.n_events * ITSU_TRACKLET_LAYERS;
+    int step = 1;
+    while (s + step < end && a.trk_seg[s + step] <= k) {
+      s += step;
+      step *= 2;
+    }
+    for (; step > 0; step /= 2) {
+      if (s + step < end && a.trk_seg[s + step] <= k) {
+        s += step;
+      }
+    }
+  }
+  return s;
+}
+#endif
 
 // Launch geometry shared by the grid-stride kernels.
 struct Launch {

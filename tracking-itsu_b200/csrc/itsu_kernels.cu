@@ -736,7 +736,9 @@ __device__ __forceinline__ void write_tracklet(const Arena &a, int out, int64_t 
 {
   store_tracklet(a, out, make_tracklet(a.xyzr[i_flat], a.xyzr[j_flat], (int32_t)(i_flat - a.layer_off[seg]),
                                        (int32_t)(j_flat - a.layer_off[seg + 1])));
-  a.trk_seg_id[out] = seg - seg / ITSU_LAYERS;  // 7 e + L to 6 e + L
+  if (out % 32 == 0) {
+    a.trk_seg32[out / 32] = seg - seg / ITSU_LAYERS;  // 7 e + L to 6 e + L
+  }
 }
 
 constexpr int kTrackletSlots = kTrackletSlotsPerCluster;
@@ -1324,15 +1326,15 @@ __global__ void __launch_bounds__(kGateThreads) k_tracklets_gate(Arena a)
 
 // Write pass, a warp per 32 consecutive inner clusters: the warp's lanes fill their clusters' tracklets
 // together, each taking the next one: it finds its inner cluster (owner) and rank there, reads the
-// outer cluster the count pass kept in that slot, and writes the tracklet (Tracklet.cxx:32-40), its key
-// and its segment id with coalesced stores; all lanes compute their binary64 azimuths together. What a
+// outer cluster the count pass kept in that slot, and writes the tracklet (Tracklet.cxx:32-40) and its
+// key with coalesced stores; all lanes compute their binary64 azimuths together. What a
 // tracklet needs of its owner stands in shared memory. Each cluster's tracklets lookup entry is
-// written here too. The tracklets of an inner cluster with more than kTrackletSlots of them (not kept
-// by the count pass) come from write_crowded.
+// written here too, and the segment of every 32nd tracklet. The tracklets of an inner cluster with
+// more than kTrackletSlots of them (not kept by the count pass) come from write_crowded.
 // Runs over the inner clusters [c0, c1) (c0 a multiple of 32, so that warps hold whole aligned
 // groups of 32 clusters): all of them, or one event group's share of them.
-// Bound by the slots' and outer clusters' gathers with the azimuth's issue: 0.50 ms per 128 central
-// events at five blocks per SM (48 registers), 0.55 at six (the slots' lines, which a warp comes back
+// Bound by the slots' and outer clusters' gathers with the azimuth's issue: 0.475 ms per 128 central
+// events (0.488 with a segment id per tracklet; the figures below before the prefetch): 0.50 at five blocks per SM (48 registers), 0.55 at six (the slots' lines, which a warp comes back
 // to, leave L1 too soon) or four; 0.58 with the owners' values in shuffles, the correctly rounded
 // division and the azimuth's double-double path inlined. Slots of a cluster side by side: 0.56.
 constexpr int kWriteThreads = 256;
@@ -1403,7 +1405,9 @@ __global__ void __launch_bounds__(kWriteThreads, kWriteBlocks) k_tracklets_write
       const int32_t j = slots[(int64_t)(p - o.y) * a.slot_stride + owner];
       const float4 d = a.xyzr[o.w + j];
       const int32_t out = o.x + p;
-      a.trk_seg_id[out] = w.sid[owner];
+      if (out % 32 == 0) {
+        a.trk_seg32[out / 32] = w.sid[owner];
+      }
       store_tracklet(a, out, make_tracklet(w.c[owner], d, o.z, j));
     }
   }
@@ -1513,9 +1517,10 @@ __global__ void __launch_bounds__(kCountThreads) k_tracklet_segments(Arena a, bo
 // Bound by the gathers (half of the issue slots and of the L1 data pipe busy). Spans of 128 leave
 // half a round in five empty, but only pay where every warp has many of them. The grid is one wave of
 // resident blocks (9 of 128 threads at 56 registers per SM: a second, part-empty wave would cost
-// almost as much again). 1.13 ms per 128 central events (1.15 at 10 blocks and 48 registers, 1.21 at
-// 8); as two kernels with the pairs listed in global memory 0.75 + 0.75 ms; with masks, counts and
-// lookup entries per first tracklet 1.34 ms, and 0.34 instead of 0.17 ms to place the cells.
+// almost as much again). 1.03 ms per 128 central events; before the prefetch 1.13 (1.15 at 10 blocks
+// and 48 registers, 1.21 at 8); as two kernels with the pairs listed in global memory 0.75 + 0.75 ms;
+// with masks, counts and lookup entries per first tracklet 1.34 ms, and 0.34 instead of 0.17 ms to
+// place the cells.
 constexpr int kCellThreads = 128;
 constexpr int kCellBlocks = 9;  // resident blocks per SM
 constexpr int kMaxSpan = 128;
@@ -1547,7 +1552,7 @@ __device__ __forceinline__ CellLane cell_lane(const Arena &a, uint32_t k)
   CellLane s;
   s.j0 = s.n_out = 0;
   // both loads first: neither depends on the other
-  s.sid = a.trk_seg_id[k];
+  s.sid = tracklet_segment(a, k);
   const itsu_tracklet t1 = load_tracklet(a, k);
   const int layer = s.sid % ITSU_TRACKLET_LAYERS;
   if (layer >= ITSU_CELL_LAYERS) {
@@ -1616,16 +1621,14 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
       }
       s_next = __shfl_sync(0xffffffffu, s_next, 0);
     }
-    // The next span's records, segment ids and keys on their way into L2, a 128-byte line per lane.
+    // The next span's records and keys on their way into L2, a 128-byte line per lane.
     // That span is a round of all warps ahead (two central events), so its data, as first and as
     // outgoing tracklets, is there when its event's spans are worked on (1.125 ms without).
     {
       const int64_t next = (int64_t)s_next * span;
-      const void *line = lane < 16 ? (const void *)(a.tracklets + next + lane * 8)
-                                   : (lane < 20 ? (const void *)(a.trk_seg_id + next + (lane - 16) * 32)
-                                                : (const void *)(a.trk_key + next + (lane - 20) * 32));
-      const uint32_t at = lane < 16 ? lane * 8 : (lane < 20 ? lane - 16 : lane - 20) * 32;
-      if (lane < 24 && at < span && next + at < n) {
+      const void *line = lane < 16 ? (const void *)(a.tracklets + next + lane * 8) : (const void *)(a.trk_key + next + (lane - 16) * 32);
+      const uint32_t at = lane < 16 ? lane * 8 : (lane - 16) * 32;
+      if (lane < 20 && at < span && next + at < n) {
         prefetch_line(line);
       }
     }

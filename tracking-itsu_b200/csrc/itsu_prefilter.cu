@@ -173,7 +173,7 @@ __global__ void k_export_tracklets(Arena a, itsu_gate_samples out)
     if (!out.features) {
       continue;
     }
-    const int sid = a.trk_seg_id[k];
+    const int sid = tracklet_segment(a, k);
     const int e = sid / ITSU_TRACKLET_LAYERS, layer = sid % ITSU_TRACKLET_LAYERS;
     const itsu_tracklet t = a.tracklets[k];
     const int32_t *lo = a.layer_off + e * ITSU_LAYERS;
