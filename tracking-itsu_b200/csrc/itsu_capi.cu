@@ -111,7 +111,7 @@ struct itsu_context {
   float4 *xyzr = nullptr;
   float *phi = nullptr;
   int32_t *trk_count = nullptr, *trk_off = nullptr, *trk_lookup = nullptr;
-  float4 *zs = nullptr;
+  uint32_t *clu_key = nullptr;
   int2 *trk_range = nullptr;
   int32_t *clu_seg = nullptr;
   int4 *clu_aux = nullptr;
@@ -368,7 +368,7 @@ Arena arena_of(const itsu_context *ctx)
   a.sort_index = ctx->sort_index;
   a.sort_stride = ctx->cap_clusters;
   a.index_tables = ctx->index_tables;
-  a.zs = ctx->zs;
+  a.clu_key = ctx->clu_key;
   a.clu_seg = ctx->clu_seg;
   a.clu_aux = ctx->clu_aux;
   a.clu_crowded = ctx->clu_crowded;
@@ -458,7 +458,7 @@ itsu_status ensure_clusters(itsu_context *ctx, int64_t n_clusters, int32_t n_eve
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_off, cap + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_range, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_lookup, cap));
-    ITSU_CUDA(ctx, alloc(ctx, ctx->zs, cap));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->clu_key, cap + 4));
     ITSU_CUDA(ctx, alloc(ctx, ctx->clu_seg, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->clu_aux, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->clu_crowded, cap));
@@ -615,9 +615,6 @@ itsu_status sync_status(itsu_context *ctx)
   ctx->pinned_busy = false;
   if (ctx->h_status->flags & itsu::kFlagLaunchShape) {
     return fail(ctx, ITSU_ERR_INVALID, "launch shape: the per-item passes need a block size that is a multiple of 32");
-  }
-  if (ctx->h_status->flags & itsu::kFlagTimeout) {
-    return fail(ctx, ITSU_ERR_TIMEOUT, "a bounded device wait (a shared-memory bulk copy) gave up");
   }
   return ITSU_OK;
 }
@@ -1071,7 +1068,7 @@ void itsu_context_destroy(itsu_context *ctx)
   if (ctx->twin) itsu_context_destroy(ctx->twin);
   drop_graph(ctx);
   release(ctx->raw_head); release(ctx->raw_in); release(ctx->raw_track); release(ctx->sorted); release(ctx->sort_recs); release(ctx->sort_index); release(ctx->xyzr); release(ctx->phi);
-  release(ctx->trk_count); release(ctx->trk_off); release(ctx->trk_range); release(ctx->trk_lookup); release(ctx->zs); release(ctx->clu_seg); release(ctx->clu_aux); release(ctx->clu_crowded); release(ctx->trk_slots);
+  release(ctx->trk_count); release(ctx->trk_off); release(ctx->trk_range); release(ctx->trk_lookup); release(ctx->clu_key); release(ctx->clu_seg); release(ctx->clu_aux); release(ctx->clu_crowded); release(ctx->trk_slots);
   release(ctx->seg_rrange); release(ctx->seg_regular); release(ctx->raw_off);
   release(ctx->layer_off); release(ctx->index_tables); release(ctx->trk_seg); release(ctx->cell_seginfo); release(ctx->cell_seg); release(ctx->cell_seg_count);
   release(ctx->road_seg); release(ctx->vtx);
@@ -2023,7 +2020,7 @@ itsu_status itsu_autotune(itsu_context *ctx, int32_t repeats, itsu_tune *best)
   ITSU_CUDA(ctx, cudaEventCreate(&e1));
   Tune winner;
   winner.ms = 1e30f;
-  const int blocks[] = {64, 128, 256, 512}, per_sm[] = {4, 8, 16}, prunes[] = {1, 2, 0}, groups[] = {0, 8, 16, 32};
+  const int blocks[] = {64, 128, 256, 512}, per_sm[] = {4, 8, 16}, prunes[] = {1, 0}, groups[] = {0, 8, 16, 32};
   ctx->tuning = true;
   cudaError_t err = cudaSuccess;
   for (int b : blocks) {

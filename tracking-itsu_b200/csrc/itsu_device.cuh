@@ -156,9 +156,27 @@ __device__ __forceinline__ uint32_t tracklet_key(float tan_lambda, float phi)
   return ((uint32_t)__float2int_rn(phi * kKeyPhiUnits) << 16) | ((uint32_t)__float2int_rn(tan_lambda * kKeyTanUnits) & 0xffffu);
 }
 
-struct CellWindow {
-  uint32_t minus_base;  // minus the lowest phi (high half) and the lowest tanL (low half)
+// A window over keys of two 16-bit halves, each wrapping on its own.
+struct KeyWindow {
+  uint32_t minus_base;  // minus the lowest of each half
   uint32_t width;       // the reach of each above its lowest
+};
+
+// Both halves of key - base at most width: one add-and-max on the halves, one compare.
+__device__ __forceinline__ bool key_window_pass(const KeyWindow &w, uint32_t key)
+{
+  return __viaddmax_u16x2(key, w.minus_base, w.width) == w.width;
+}
+
+// Which of four keys pass, as bits.
+__device__ __forceinline__ unsigned key_window_four(const KeyWindow &w, uint4 q)
+{
+  return (key_window_pass(w, q.x) ? 1u : 0u) | (key_window_pass(w, q.y) ? 2u : 0u) | (key_window_pass(w, q.z) ? 4u : 0u) |
+         (key_window_pass(w, q.w) ? 8u : 0u);
+}
+
+struct CellWindow {
+  KeyWindow keys;  // phi (high half) and tanL (low half)
   bool empty;
 };
 
@@ -176,15 +194,37 @@ __device__ __forceinline__ CellWindow cell_window(float t1_tan_lambda, float t1_
   CellWindow w;
   w.empty = !(lo <= hi);
   const int from = __float2int_rd(lo * kKeyTanUnits) - 2, to = __float2int_ru(hi * kKeyTanUnits) + 2;
-  w.minus_base = __vneg2(__vadd2(tracklet_key(t1_tan_lambda, t1_phi), ((uint32_t)-kKeyPhiReach << 16) | ((uint32_t)from & 0xffffu)));
-  w.width = ((uint32_t)(2 * kKeyPhiReach) << 16) | (uint32_t)(to - from);
+  w.keys.minus_base = __vneg2(__vadd2(tracklet_key(t1_tan_lambda, t1_phi), ((uint32_t)-kKeyPhiReach << 16) | ((uint32_t)from & 0xffffu)));
+  w.keys.width = ((uint32_t)(2 * kKeyPhiReach) << 16) | (uint32_t)(to - from);
   return w;
 }
 
-// Both halves of key - base at most width: one add-and-max on the halves, one compare.
-__device__ __forceinline__ bool cell_window_pass(const CellWindow &w, uint32_t key)
+// The tracklet walk's window in the same form, on clusters: a cluster's key holds its phi (high half,
+// as above) and its z in 65536ths of its layer's length (low half, clamped at the ends). The clusters
+// that can pass the cut lie within reach of phi1 (at most 0.3 rad: the units, the keys' roundings and
+// one to spare) and in [zlo, zhi]; the z half is monotone in z, so that interval needs no margin for
+// the keys (one is taken). Passing clusters are tested again exactly; tests/test_tracklet_window.py
+// checks that none is lost.
+constexpr float kKeyZPerBin = 3276.8f;  // 65536 / 20
+
+__device__ __forceinline__ int cluster_key_z(int layer, float z)
 {
-  return __viaddmax_u16x2(key, w.minus_base, w.width) == w.width;
+  return __float2int_rd((z + kC.z_half[layer]) * (kC.inv_z_bin[layer] * kKeyZPerBin));
+}
+
+__device__ __forceinline__ uint32_t cluster_key(int layer, float z, float phi)
+{
+  return ((uint32_t)__float2int_rn(phi * kKeyPhiUnits) << 16) | (uint32_t)min(max(cluster_key_z(layer, z), 0), 65535);
+}
+
+__device__ __forceinline__ KeyWindow tracklet_window(int layer, float phi1, float reach, float zlo, float zhi)
+{
+  const int spread = __float2int_ru(fmaxf(reach, 0.0f) * kKeyPhiUnits) + 2;
+  const int from = min(max(cluster_key_z(layer, zlo), 1), 65535) - 1, to = min(max(cluster_key_z(layer, zhi), 0), 65534) + 1;
+  KeyWindow w;
+  w.minus_base = __vneg2(((uint32_t)(__float2int_rn(phi1 * kKeyPhiUnits) - spread) << 16) | (uint32_t)from);
+  w.width = ((uint32_t)(2 * spread) << 16) | (uint32_t)(to - from);
+  return w;
 }
 
 // Tracker.cxx:175-216: circle-plane normal, radius and DCA of the three clusters. Returns false

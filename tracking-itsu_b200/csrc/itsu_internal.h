@@ -34,12 +34,11 @@ enum : int32_t {
   kFlagCountOverflow = 32,
   kFlagCapScratch = 64,  // the cell entries of the count pass exceed their scratch
   kFlagLaunchShape = 128,  // a per-item pass was given a block size that is not whole warps (nothing ran)
-  kFlagTimeout = 256,      // a bounded device wait gave up (the run's results are not used)
 };
 constexpr int kTrackletSlotsPerCluster = 48;  // outer clusters the tracklet count pass keeps per inner cluster
 // Any of these stops every later kernel of the run (they check the mask first).
 constexpr int32_t kCapacityMask = kFlagCapTracklets | kFlagCapCells | kFlagCapNeighbours | kFlagCapRoads |
-                                  kFlagCountOverflow | kFlagCapScratch | kFlagLaunchShape | kFlagTimeout;
+                                  kFlagCountOverflow | kFlagCapScratch | kFlagLaunchShape;
 
 // Totals and requirements of a run, written by the device.
 struct DevStatus {
@@ -99,13 +98,11 @@ struct Arena {
   int32_t *clu_seg;  // per sorted cluster: its segment 7e + L (null: not wanted)
   int4 *clu_aux;     // per sorted cluster: id, alpha bits, MC id, bin (the clustering scatters them here)
   int32_t *clu_crowded;  // inner clusters with more than kTrackletSlotsPerCluster tracklets (count pass list)
-  // candidate-pruning index (null: not built): per bin, the bin's clusters sorted by (z, index),
-  // each with its r and phi for the cut;
-  // per (event, layer) the r range of its clusters and whether all its bins are regular
-  float4 *zs;  // (z, r, phi, sorted index as int bits)
+  // for pruning the tracklet walk (null: not wanted), with each (event, layer)'s r range and regularity
+  uint32_t *clu_key;  // phi and z of each sorted cluster (cluster_key)
   float2 *seg_rrange;
-  int32_t *seg_regular;  // per segment: 0 if not regular, else the pass-mask words its largest bin needs
-  int32_t prune_tracklets;  // use the index: 0 no, 1 yes, 2 yes, from a shared-memory copy (tuning knob; results are identical)
+  int32_t *seg_regular;  // per segment: whether every cluster lies in its bin of the 20 x 20 table
+  int32_t prune_tracklets;  // 0: walk every row whole (tuning knob; results are identical)
   // tracklets
   int32_t *trk_count;
   int32_t *trk_slots;  // slot n of inner cluster i at n * slot_stride + i: the outer clusters of its first tracklets

@@ -44,9 +44,6 @@ constexpr int kScanTile = kScanThreads * kScanItems;
 // multiples of 32, checked at launch) over tiles of a whole number of warps.
 static_assert(kScanTile % 32 == 0, "a warp's 32 items lie in one scan tile");
 constexpr float kMaxAbsCoordinate = 1.0e6f;
-constexpr int kMaxPruneBin = 256;  // larger bins disable pruning for their layer
-constexpr int kPruneWords = kMaxPruneBin / 64;  // a pruned column's passes: a mask of this many 64-bit words
-static_assert(kMaxPruneBin % 64 == 0, "a pruned column's passes are whole 64-bit words");
 
 __device__ __forceinline__ bool capacity_failed(const DevStatus *s) { return (*(volatile const int32_t *)&s->flags & kCapacityMask) != 0; }
 
@@ -354,13 +351,13 @@ __device__ __forceinline__ void stage_put(int32_t *stage, int lane, const itsu_c
 // One segment (event, layer) per cluster of CTAs (of one, where a run has segments enough for the
 // chip). Every hit is touched twice: pass 1 reads it in input order and leaves the transformed record
 // (32 bytes) in a.sort_recs, pass 4 gathers the records in sorted order and writes every output,
-// coalesced. Between them, ranking by bucket, by bin and by z works on indices and z values alone,
-// kept in a.sort_index (12 to 16 bytes per hit, written and read within the CTA's turn, so mostly L2
-// hits; kept in shared memory instead they cost a CTA per SM on large segments: 0.37 against 0.30 ms
-// per 64 events of 7000 tracks, 0.41 against 0.42 on 128 of 6000). Bound by the latency of its
-// barrier-separated phases: 0.39 ms per 128 central events at three CTAs of 512 threads (40 registers,
-// some spilled) per SM, 0.41 at two, 0.51 with CTAs of 256; 0.49 with 36-byte records moved through
-// memory and back in input order. 1024 pp events of 60 tracks: 0.048 ms in CTAs of 64 threads, 0.24 in
+// coalesced. Between them, ranking by bucket and by bin works on indices alone, kept in a.sort_index
+// (8 bytes per hit, written and read within the CTA's turn, so mostly L2 hits; kept in shared memory
+// instead they cost a CTA per SM on large segments: 0.37 against 0.30 ms per 64 events of 7000
+// tracks). Bound by the latency of its barrier-separated phases: 0.30 ms per 128 central events; 0.39
+// when it also listed each bin's clusters by z for the tracklet walk, and then 0.41 at two CTAs of 512
+// threads per SM in place of three, 0.51 with CTAs of 256, 0.49 with 36-byte records moved through
+// memory and back in input order. 1024 pp events of 60 tracks: 0.044 ms in CTAs of 64 threads, 0.24 in
 // CTAs of 512.
 constexpr size_t sort_shared_bytes(int warps)
 {
@@ -378,7 +375,7 @@ __global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Ar
   int *const bucket_total = cta_total + kBuckets;
   int *const bucket_base = bucket_total + kBuckets;
   int *const scan_totals = bucket_base + kBuckets;  // [33]
-  int *const s_flags = scan_totals + 34;            // irregular, least r, largest r (float bits), largest bucket
+  int *const s_flags = scan_totals + 34;            // irregular, least r, largest r (float bits)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ctas = (int)cg::this_cluster().num_blocks(), rank = (int)cg::this_cluster().block_rank();
@@ -391,12 +388,9 @@ __global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Ar
   int *const hist = hist_all + warp * kBuckets;
   int32_t *const stage = s_flags + 4 + warp * 32 * kClusterWords;
 
-  // by input index: bucket and z; by sorted position: input index (perm), z, and where the cluster
-  // goes in its bin's z-sorted list (in the input z values' place)
+  // by input index: bucket; by sorted position: input index (perm)
   uint32_t *const perm = a.sort_index + begin;
   uint32_t *const bucket = perm + a.sort_stride;
-  float *const z_in = reinterpret_cast<float *>(bucket + a.sort_stride);
-  float *const z_at = z_in + a.sort_stride;
   auto sync_segment = [&]() {
     if (ctas == 1) {
       __syncthreads();
@@ -420,7 +414,6 @@ __global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Ar
     s_flags[0] = 0;
     s_flags[1] = 0x7f800000;
     s_flags[2] = 0;
-    s_flags[3] = 0;
   }
   __syncthreads();
 
@@ -476,7 +469,6 @@ __global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Ar
       rmax = max(rmax, __float_as_uint(t.r));
       const int b = bucket_of(t.bin);
       bucket[i] = (uint32_t)b;
-      z_in[i] = c.z;
       atomicAdd(&hist[b], 1);
     }
   }
@@ -524,7 +516,6 @@ __global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Ar
     }
     __syncthreads();
   }
-  int largest = 0;
   for (int b0 = 0, carry = 0; b0 < kBuckets; b0 += kThreads_) {
     const int b = b0 + tid;
     const int v = b < kBuckets ? bucket_total[b] : 0;
@@ -532,18 +523,10 @@ __global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Ar
     const int ex = block_exclusive_scan<int>(v, scan_totals, total);
     if (b < kBuckets) {
       bucket_base[b] = carry + ex;
-      if (b > 0 && b <= kTableBins) {
-        largest = max(largest, v);
-      }
     }
     carry += total;
   }
-  largest = __reduce_max_sync(0xffffffffu, (unsigned)largest);
-  if (lane == 0) {
-    atomicMax(&s_flags[3], largest);
-  }
   __syncthreads();
-  largest = s_flags[3];
   if (layer > 0) {
     // table[b] = first sorted index with bin >= b = #clusters with bin < b for b >= 1; table[0] = 0
     // (PrimaryVertexContext.cxx:90-119: negative bins never move the fill cursor off bin 0).
@@ -565,7 +548,6 @@ __global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Ar
     if (valid) {
       pos = bucket_base[b] + hist[b] + before;
       perm[pos] = (uint32_t)i;
-      z_at[pos] = z_in[i];
     }
     __syncwarp();
     if (valid && (peers >> lane) == 1u) {  // the highest lane of its bucket
@@ -576,14 +558,14 @@ __global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Ar
   sync_segment();
 
   // Negative bins share bucket 0 in input order; order them by bin, stably. A bottom-up merge sort of
-  // (bin, input index) between (z_at, perm) and (z_in, bucket), all free for such a layer: in each
+  // (bin, input index) between two pairs of arrays: in each
   // round, runs of `width` are merged in pairs, every cluster moving to (its place in its run) + (the
   // clusters of the partner run that go before it: smaller bins, and for the right run equal bins
   // too), so ties keep input order. O(m log^2 m) work, for layers with many clusters beyond the z range.
   const int m = bucket_total[0];
   if (m > 1) {
     if (rank == 0) {
-      int *key = reinterpret_cast<int *>(z_at), *key_to = reinterpret_cast<int *>(z_in);
+      int *key = reinterpret_cast<int *>(bucket + a.sort_stride), *key_to = key + a.sort_stride;
       uint32_t *idx = perm, *idx_to = bucket;
       for (int i = tid; i < m; i += kThreads_) {
         const int from = (int)perm[i];
@@ -628,29 +610,11 @@ __global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Ar
     sync_segment();
   }
 
-  // The tracklet stage's candidate-pruning index. A layer is regular when every cluster has a z bin
-  // and a phi bin inside the 20 x 20 table (then a bin's column is its clusters' z bin) and no bin
-  // holds more than kMaxPruneBin clusters; for regular layers, each bin's clusters are listed again
-  // sorted by (z, sorted index), with the layer's r range beside. (Layer 0 is never the outer layer
-  // of a tracklet.)
-  const bool regular = a.zs != nullptr && layer > 0 && !seg_irregular && m == 0 && bucket_total[kBuckets - 1] == 0 && largest <= kMaxPruneBin;
-  uint32_t *const z_rank = reinterpret_cast<uint32_t *>(z_in);  // by sorted position
-  if (regular) {
-    for (int pos = rank * kThreads_ + tid; pos < n; pos += ctas * kThreads_) {
-      const int b = (int)bucket[perm[pos]];
-      const int st = bucket_base[b], en = st + bucket_total[b];
-      const float z = z_at[pos];
-      int at = st;
-      for (int j = st; j < en; ++j) {
-        const float zj = z_at[j];
-        at += zj < z || (zj == z && j < pos);
-      }
-      z_rank[pos] = (uint32_t)at;
-    }
-  }
-  if (a.zs != nullptr && layer > 0 && rank == 0 && tid == 0) {
-    // 0: not regular; else the 64-bit words of a pass mask over its largest bin (1, 2 or 4)
-    a.seg_regular[seg] = !regular ? 0 : (largest <= 64 ? 1 : (largest <= 128 ? 2 : kPruneWords));
+  // What lets the tracklet stage prune: a layer is regular when every cluster has a z bin and a phi bin
+  // inside the 20 x 20 table (then a bin's column is its clusters' z bin). Its r range stands beside.
+  // (Layer 0 is never the outer layer of a tracklet.)
+  if (a.clu_key != nullptr && layer > 0 && rank == 0 && tid == 0) {
+    a.seg_regular[seg] = !seg_irregular && m == 0 && bucket_total[kBuckets - 1] == 0;
     a.seg_rrange[seg] = make_float2(__int_as_float(seg_rmin), __int_as_float(seg_rmax));
   }
   // Pass 4: every output in sorted order.
@@ -678,9 +642,7 @@ __global__ void __launch_bounds__(kThreads_, 1536 / kThreads_) k_cluster_sort(Ar
         a.phi[at] = c.phi;
         a.clu_aux[at] = make_int4(c.cluster_id, __float_as_int(c.alpha), c.mc_id, c.bin);
         a.clu_seg[at] = seg;
-      }
-      if (regular) {
-        a.zs[begin + z_rank[pos]] = make_float4(c.z, c.r, c.phi, __int_as_float(pos));
+        a.clu_key[at] = cluster_key(layer, c.z, c.phi);
       }
     }
     stage_out(a.sorted + begin + i0, stage, count);
@@ -742,6 +704,7 @@ __device__ __forceinline__ void write_tracklet(const Arena &a, int out, int64_t 
 }
 
 constexpr int kTrackletSlots = kTrackletSlotsPerCluster;
+constexpr int kMaskKeys = 32;  // keys of the walk's window a mask holds (64: 0.72 in place of 0.66 ms per 128 central events)
 constexpr int kMaxMaskedOut = 64;  // out-degrees up to this are evaluated pair-parallel with a pass mask
 
 // The reference's candidate sequence of one inner cluster (Tracker.cxx:73-113), calling
@@ -750,13 +713,13 @@ constexpr int kMaxMaskedOut = 64;  // out-degrees up to this are evaluated pair-
 // row's first bin through the first cluster at or after the window's end (inclusive bound, with
 // the P1/P5 guards).
 //
-// On a regular next layer the row is walked through the pruning index instead, which is exact:
-// a pass needs |P - z2| < dz with P = (tanL (r2 - r1) + z1) in binary32, P is monotone in r2, so
-// every passing z2 lies within [P(rmin) - dz, P(rmax) + dz] (widened by 1e-3 cm for the rounding
-// of the bounds); only the z bins of the row that meet that interval can hold passes, and in each
-// such bin only the clusters listed there between the two z values. Their passes are put back
-// into index order before on_pass. The row's last candidate (the inclusive bound, past the
-// window's z bins) is always evaluated. Irregular layers take the reference walk.
+// On a regular next layer the row is pruned, which is exact: a pass needs |P - z2| < dz with
+// P = (tanL (r2 - r1) + z1) in binary32, P is monotone in r2, so every passing z2 lies within
+// [P(rmin) - dz, P(rmax) + dz] (widened by 1e-3 cm for the rounding of the bounds); only the z bins of
+// the row that meet that interval can hold passes, and of their clusters (consecutive ones) those
+// whose 4-byte keys lie in the window (TrackletWindow, a superset of the cut) are tested. The row's
+// last candidate (the inclusive bound, past the window's z bins) is always evaluated. Irregular layers
+// take the reference walk.
 struct TrackletProbe {
   float4 c;      // inner cluster (x, y, z, r)
   float phi1, tan_lambda, max_dz;
@@ -780,103 +743,10 @@ struct TrackletProbe {
   template <bool kGate>
   __device__ __forceinline__ bool pass(int j) const
   {
-    const float4 d = xyzr[j];
-    return pass<kGate>(d.z, d.w, phi[j]);
+    const float2 d = reinterpret_cast<const float2 *>(xyzr + j)[1];  // z, r
+    return pass<kGate>(d.x, d.y, phi[j]);
   }
 };
-
-// win_row, win_rows: the phi rows whose candidates are walked (win_rows = kPhiBins: every row); of
-// the other rows only the bound candidate is tested (the first cluster of the first bin after the
-// row's last z column: past empty bins it can lie in any later row).
-template <int kWords, bool kGate, typename OnPass>
-__device__ __forceinline__ void walk_candidates(const int32_t *table, int n_next, int4 rect, int layer, const TrackletProbe &probe,
-                                                bool prune, float zlo, float zhi, const float4 *zs, int zs_off,
-                                                int win_row, int win_rows, OnPass &&on_pass)
-{
-  // zs[k - zs_off] is the k-th entry of the next layer's z-sorted bin lists (zs_off > 0: a staged
-  // copy in shared memory that starts at entry zs_off)
-  static_assert(kWords >= 1 && kWords <= kPruneWords, "mask words");
-  int phi_bins = rect.w - rect.y + 1;
-  if (phi_bins < 0) {
-    phi_bins += kPhiBins;
-  }
-  const int zb_lo = prune ? max(rect.x, z_bin_index(layer + 1, zlo)) : 0;
-  const int zb_top = prune ? z_bin_index(layer + 1, zhi) : 0;  // clusters of higher z bins have z > zhi
-  const int zb_hi = prune ? min(rect.z, zb_top) : -1;
-  for (int phi_bin = rect.y, phi_count = 0; phi_count < phi_bins;
-       phi_bin = (phi_bin + 1 == kPhiBins) ? 0 : phi_bin + 1, ++phi_count) {
-    const int first_bin = bin_index(rect.x, phi_bin);
-    const int max_bin = min(first_bin + rect.z - rect.x + 1, kTableBins);  // P5
-    const bool walk_row = win_rows >= kPhiBins ||
-                          (phi_bin < kPhiBins && (phi_bin - win_row + kPhiBins) % kPhiBins < win_rows);
-    if (prune && phi_bin < kPhiBins) {
-      for (int col = zb_lo; walk_row && col <= zb_hi; ++col) {
-        const int bin = phi_bin * kPhiBins + col;
-        const int k0 = table[bin], k1 = table[bin + 1];
-        int lo = k0, hi = k1;  // first listed cluster with z >= zlo
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          if (zs[mid - zs_off].x < zlo) {
-            lo = mid + 1;
-          } else {
-            hi = mid;
-          }
-        }
-        // a pruned column holds at most 64 * kWords clusters (the layer's largest bin chose
-        // kWords): its passes as a mask over their positions in the column, in registers,
-        // emitted in index order
-        unsigned long long hit[kWords];
-#pragma unroll
-        for (int w = 0; w < kWords; ++w) {
-          hit[w] = 0ull;
-        }
-        for (int k = lo; k < k1; ++k) {
-          const float4 q = zs[k - zs_off];  // z, r, phi and the sorted index of the k-th cluster by z
-          if (!(q.x <= zhi)) {
-            break;
-          }
-          if (probe.pass<kGate>(q.x, q.y, q.z)) {
-            const int pos = __float_as_int(q.w) - k0;
-            const unsigned long long bit = 1ull << (pos & 63);
-            if constexpr (kWords == 1) {
-              hit[0] |= bit;  // a single-word layer's columns hold at most 64 clusters
-            } else {
-#pragma unroll
-              for (int w = 0; w < kWords; ++w) {
-                hit[w] |= (pos >> 6) == w ? bit : 0ull;
-              }
-            }
-          }
-        }
-#pragma unroll
-        for (int w = 0; w < kWords; ++w) {
-          while (hit[w]) {
-            const int b = __ffsll((long long)hit[w]) - 1;
-            hit[w] &= hit[w] - 1ull;
-            on_pass(k0 + 64 * w + b);
-          }
-        }
-      }
-      // The inclusive bound's candidate (P1: inside the layer): the first cluster of bin
-      // max_bin, the row's next z column. When that bin is not empty and its z column lies
-      // beyond zhi's (z bins are monotone in z; a regular layer's clusters sit in exactly their
-      // bins), the candidate's z exceeds zhi and it fails the Δz cut: it is not read.
-      const int x = table[max_bin];
-      const bool beyond = rect.z + 1 < kZBins && rect.z + 1 > zb_top && table[max_bin + 1] > x;
-      if (!beyond && x < n_next && probe.pass<kGate>(x)) {
-        on_pass(x);
-      }
-    } else {
-      const int first_row = table[first_bin];
-      const int last_row = min(table[max_bin], n_next - 1);  // inclusive bound, P1
-      for (int j = walk_row ? first_row : last_row; j <= last_row; ++j) {
-        if (probe.pass<kGate>(j) && (walk_row || j == table[max_bin])) {
-          on_pass(j);
-        }
-      }
-    }
-  }
-}
 
 // The walk state of one inner cluster i (flat index): whether its layer runs the tracklet
 // stage, and the probe, window and pruning bounds of its candidate walk.
@@ -887,8 +757,8 @@ struct InnerCluster {
   int4 rect;
   TrackletProbe probe;
   bool prune;
-  int words;
-  float zlo, zhi;
+  int zb_lo, zb_hi, zb_top;  // the z bins walked of a row; clusters of bins above zb_top have z beyond the cut
+  KeyWindow window;
   const int32_t *table;
   int n_next;
   int64_t next_begin;
@@ -945,161 +815,111 @@ __device__ __forceinline__ InnerCluster inner_cluster(const Arena &a, int64_t i)
   s.probe.phi = a.phi + s.next_begin;
   s.probe.max_dz = kC.trk_max_dz[s.layer];
   const int next_seg = s.seg + 1;
-  s.words = a.seg_regular[next_seg];  // 0: not regular, else the mask words its largest bin needs
+  const bool regular = a.prune_tracklets != 0 && a.seg_regular[next_seg] != 0;
   s.win_row = 0;
   s.win_rows = kPhiBins;
+  float half = s.probe.max_dz, reach = kPhiCoordinateCut;
   if constexpr (kGate) {
     s.probe.win = gate_window(*a.gate, s.layer, s.probe.c, s.probe.phi1, vz);
-    if (s.words != 0 && s.probe.win.dphi + 1e-3f < kPhiCoordinateCut) {  // a wider window narrows nothing
-      window_rows(s.probe.phi1, s.probe.win.dphi + 1e-3f, &s.win_row, &s.win_rows);
+    if (regular && s.probe.win.dphi + 1e-3f < kPhiCoordinateCut) {  // a wider window narrows nothing
+      reach = s.probe.win.dphi + 1e-3f;
+      window_rows(s.probe.phi1, reach, &s.win_row, &s.win_rows);
     }
+    half = fminf(half, s.probe.win.dz + 1e-3f);
   }
-  s.prune = a.prune_tracklets && s.words != 0;
-  s.zlo = s.zhi = 0;
-  if (s.prune) {
+  s.prune = regular;
+  if (regular) {
     const float2 rr = a.seg_rrange[next_seg];
     const float p1 = s.probe.tan_lambda * (rr.x - s.probe.c.w) + s.probe.c.z;
     const float p2 = s.probe.tan_lambda * (rr.y - s.probe.c.w) + s.probe.c.z;
-    const float half = kGate ? fminf(s.probe.max_dz, s.probe.win.dz + 1e-3f) : s.probe.max_dz;
-    s.zlo = fminf(p1, p2) - half - 1e-3f;
-    s.zhi = fmaxf(p1, p2) + half + 1e-3f;
-    s.prune = isfinite(s.zlo) && isfinite(s.zhi);
+    const float zlo = fminf(p1, p2) - half - 1e-3f, zhi = fmaxf(p1, p2) + half + 1e-3f;
+    s.prune = isfinite(zlo) && isfinite(zhi);
+    s.zb_lo = max(s.rect.x, z_bin_index(s.layer + 1, zlo));
+    s.zb_top = z_bin_index(s.layer + 1, zhi);
+    s.zb_hi = min(s.rect.z, s.zb_top);
+    s.window = tracklet_window(s.layer + 1, s.probe.phi1, reach, zlo, zhi);
   }
   s.table = a.index_tables + ((int64_t)s.e * ITSU_TRACKLET_LAYERS + s.layer) * kTableSize;
   s.n_next = lo[s.layer + 2] - lo[s.layer + 1];
   return s;
 }
 
-// staged: the block's copy in shared memory of the next layer's z-sorted entries from staged_off on
-// (null: read them from global memory)
+// win_row, win_rows: the phi rows whose candidates are walked (win_rows = kPhiBins: every row); of
+// the other rows only the bound candidate is tested (the first cluster of the first bin after the
+// row's last z column: past empty bins it can lie in any later row).
 template <bool kGate, typename OnPass>
-__device__ __forceinline__ void walk_inner(const Arena &a, const InnerCluster &s, OnPass &&on_pass,
-                                           const float4 *staged = nullptr, int staged_off = 0)
+__device__ __forceinline__ void walk_inner(const Arena &a, const InnerCluster &s, OnPass &&on_pass)
 {
-  const float4 *zs = staged ? staged : a.zs + s.next_begin;
-  const int off = staged ? staged_off : 0;
-  if (s.words <= 1) {  // unpruned, or bins of at most 64 clusters
-    walk_candidates<1, kGate>(s.table, s.n_next, s.rect, s.layer, s.probe, s.prune, s.zlo, s.zhi, zs, off, s.win_row,
-                              s.win_rows, on_pass);
-  } else if (s.words == 2) {
-    walk_candidates<2, kGate>(s.table, s.n_next, s.rect, s.layer, s.probe, s.prune, s.zlo, s.zhi, zs, off, s.win_row,
-                              s.win_rows, on_pass);
-  } else {
-    walk_candidates<kPruneWords, kGate>(s.table, s.n_next, s.rect, s.layer, s.probe, s.prune, s.zlo, s.zhi, zs, off,
-                                        s.win_row, s.win_rows, on_pass);
+  const int4 rect = s.rect;
+  int phi_bins = rect.w - rect.y + 1;
+  if (phi_bins < 0) {
+    phi_bins += kPhiBins;
   }
-}
-
-// ---- bulk copies into shared memory (cp.async.bulk, this GPU's memory, no multicast) ----
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count)
-{
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(bar)), "r"(count) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// One bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) from global to shared
-// memory, completing on `bar` (the calling thread also arrives on it, expecting those bytes).
-__device__ __forceinline__ void bulk_copy_to_shared(void *dst, const void *src, unsigned bytes, uint64_t *bar)
-{
-  const unsigned b = (unsigned)__cvta_generic_to_shared(bar);
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src), "r"(bytes), "r"(b)
-               : "memory");
-}
-
-// Waits for phase `parity` of `bar` to complete, at most `limit` tries; false if it did not.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, int limit)
-{
-  const unsigned b = (unsigned)__cvta_generic_to_shared(bar);
-  for (int t = 0; t < limit; ++t) {
-    unsigned done;
-    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-                 : "=r"(done)
-                 : "r"(b), "r"(parity)
-                 : "memory");
-    if (done) {
-      return true;
-    }
-  }
-  return false;
-}
-
-constexpr int kStageEntries = 2048;  // the staged walk's shared copy: up to 2048 entries (32 KB) per block
-constexpr int kStageRows = 4;        // and up to 4 phi rows of the next layer
-constexpr int kWaitTries = 1 << 20;  // bounded waits: each try_wait suspends for a bounded time
-
-// The staged walk's set-up, block-wide: when every walking thread of the block walks pruned rows
-// of the same next layer, without a wrap around phi, and their rows (at most kStageRows) hold at
-// most kStageEntries entries, one bulk copy brings those entries into shared memory. Returns the
-// first staged entry's index in the layer (its *staged_count entries), or -1 with nothing staged.
-// A copy that does not complete within the bounded wait sets the timeout flag.
-__device__ int stage_rows(const Arena &a, const InnerCluster &s, float4 *stage, uint64_t *bar, int *staged_count)
-{
-  __shared__ int s_lo, s_hi, s_seg, s_ok, s_k0, s_m;
-  if (threadIdx.x == 0) {
-    s_lo = kPhiBins;
-    s_hi = -1;
-    s_seg = -1;
-    s_ok = 1;
-  }
-  __syncthreads();
-  if (s.walk) {
-    if (!s.prune || s.rect.y > s.rect.w) {
-      atomicAnd(&s_ok, 0);  // unpruned, or a window that wraps around phi
-    }
-    atomicMin(&s_lo, s.rect.y);
-    atomicMax(&s_hi, s.rect.w);
-    atomicMax(&s_seg, s.seg + 1);
-  }
-  __syncthreads();
-  if (s.walk && s.seg + 1 != s_seg) {
-    atomicAnd(&s_ok, 0);  // more than one next layer
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s_m = 0;
-    s_k0 = -1;
-    if (s_ok && s_hi >= s_lo && s_hi - s_lo < kStageRows) {
-      const int e = s_seg / ITSU_LAYERS, next_layer = s_seg % ITSU_LAYERS;
-      const int32_t *table = a.index_tables + ((int64_t)e * ITSU_TRACKLET_LAYERS + next_layer - 1) * kTableSize;
-      const int k0 = table[s_lo * kPhiBins], k1 = table[min((s_hi + 1) * kPhiBins, kTableBins)];
-      if (k1 > k0 && k1 - k0 <= kStageEntries) {
-        s_k0 = k0;
-        s_m = k1 - k0;
-        mbar_init(bar, 1);
-        bulk_copy_to_shared(stage, a.zs + a.layer_off[s_seg] + k0, (unsigned)(s_m * sizeof(float4)), bar);
+  for (int phi_bin = rect.y, phi_count = 0; phi_count < phi_bins;
+       phi_bin = (phi_bin + 1 == kPhiBins) ? 0 : phi_bin + 1, ++phi_count) {
+    const int first_bin = bin_index(rect.x, phi_bin);
+    const int max_bin = min(first_bin + rect.z - rect.x + 1, kTableBins);  // P5
+    const bool walk_row = s.win_rows >= kPhiBins ||
+                          (phi_bin < kPhiBins && (phi_bin - s.win_row + kPhiBins) % kPhiBins < s.win_rows);
+    if (s.prune && phi_bin < kPhiBins) {
+      if (walk_row && s.zb_lo <= s.zb_hi) {
+        const int k0 = s.table[phi_bin * kZBins + s.zb_lo], k1 = s.table[phi_bin * kZBins + s.zb_hi + 1];
+        // the keys in aligned groups of four (the array has room for the last group's overrun), a mask
+        // of kMaskKeys at a time
+        const int skip = (int)((s.next_begin + k0) & 3);
+        const uint4 *keys = reinterpret_cast<const uint4 *>(a.clu_key + (s.next_begin + k0 - skip));
+        for (int at = k0 - skip; at < k1; at += kMaskKeys, keys += kMaskKeys / 4) {
+          const int n = min(kMaskKeys, k1 - at);
+          uint32_t mask = 0;
+#pragma unroll 2
+          for (int b = 0; b < n; b += 4) {
+            mask |= key_window_four(s.window, keys[b / 4]) << b;
+          }
+          if (at < k0) {
+            mask &= ~0u << skip;
+          }
+          mask &= ~0u >> (kMaskKeys - n);
+          while (mask) {
+            const int j = at + __ffs((int)mask) - 1;
+            mask &= mask - 1;
+            if (s.probe.template pass<kGate>(j)) {
+              on_pass(j);
+            }
+          }
+        }
+      }
+      // The inclusive bound's candidate (P1: inside the layer): the first cluster of bin
+      // max_bin, the row's next z column. When that bin is not empty and its z column lies
+      // beyond zhi's (z bins are monotone in z; a regular layer's clusters sit in exactly their
+      // bins), the candidate's z exceeds zhi and it fails the dz cut: it is not read.
+      const int x = s.table[max_bin];
+      const bool beyond = rect.z + 1 < kZBins && rect.z + 1 > s.zb_top && s.table[max_bin + 1] > x;
+      if (!beyond && x < s.n_next && s.probe.template pass<kGate>(x)) {
+        on_pass(x);
+      }
+    } else {
+      const int first_row = s.table[first_bin];
+      const int last_row = min(s.table[max_bin], s.n_next - 1);  // inclusive bound, P1
+      for (int j = walk_row ? first_row : last_row; j <= last_row; ++j) {
+        if (s.probe.template pass<kGate>(j) && (walk_row || j == s.table[max_bin])) {
+          on_pass(j);
+        }
       }
     }
   }
-  __syncthreads();
-  if (s_k0 < 0) {
-    return -1;
-  }
-  if (!mbar_wait(bar, 0, kWaitTries)) {
-    atomicOr(&a.status->flags, kFlagTimeout);
-    mbar_wait(bar, 0, kWaitTries);  // the copy may still land: wait once more before leaving
-    return -1;
-  }
-  *staged_count = s_m;
-  return s_k0;
 }
 
 constexpr int kCountThreads = 256;
 
 // Count pass, one thread per inner cluster: the number of tracklets, and the outer clusters of
-// the first kTrackletSlots of them in emission order. kStaged: the block's walks read the next
-// layer's z-sorted entries from a shared-memory copy made by one bulk copy (stage_rows), where
-// they allow it. kGate: the learned form's first stage (inner_cluster). At most kCountThreads
-// threads per block; measured per 128 events: the plain instantiation at 40 registers (6 blocks
-// per SM) 0.64 ms, at 48 0.66, at 54 0.72; the learned one at 48 (5 blocks) 0.39 ms, at 56 0.43.
-template <bool kStaged, bool kGate>
+// the first kTrackletSlots of them in emission order. kGate: the learned form's first stage
+// (inner_cluster). At most kCountThreads threads per block. Bound by issue, half of it lost to lanes
+// whose candidates end at different times: 0.66 ms per 128 central events; with a walk of z-sorted
+// lists (a binary search per bin and passes put back into index order) 0.62, but 0.09 ms more in the
+// clustering.
+template <bool kGate>
 __global__ void __launch_bounds__(kCountThreads, kGate ? 5 : 6) k_tracklets_count(Arena a)
 {
-  extern __shared__ float4 stage[];  // kStaged: kStageEntries entries
-  __shared__ uint64_t bar;
   const int64_t i = global_thread();
   const bool valid = i < a.n_clusters;
   int count = 0;
@@ -1108,23 +928,13 @@ __global__ void __launch_bounds__(kCountThreads, kGate ? 5 : 6) k_tracklets_coun
   if (valid) {
     s = inner_cluster<kGate>(a, i);
   }
-  const float4 *staged = nullptr;
-  int staged_off = 0;
-  if constexpr (kStaged) {
-    int m = 0;
-    staged_off = stage_rows(a, s, stage, &bar, &m);
-    staged = staged_off >= 0 ? stage : nullptr;
-  }
-  if (s.walk && !(a.status->flags & kFlagTimeout)) {
-    walk_inner<kGate>(
-        a, s,
-        [&](int j) {
-          if (count < kTrackletSlots) {
-            a.trk_slots[count * a.slot_stride + i] = j;
-          }
-          ++count;
-        },
-        staged, staged_off);
+  if (s.walk) {
+    walk_inner<kGate>(a, s, [&](int j) {
+      if (count < kTrackletSlots) {
+        a.trk_slots[count * a.slot_stride + i] = j;
+      }
+      ++count;
+    });
   }
   // the warp's 32 clusters lie in one scan tile: their tracklets go to its sum
   const int warp_count = (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
@@ -1577,14 +1387,10 @@ __device__ __forceinline__ unsigned long long cell_precut_mask(const Arena &a, c
 {
   const int skip = s.j0 & 3;
   const uint4 *keys = reinterpret_cast<const uint4 *>(a.trk_key + (s.j0 - skip));
-  auto four = [&](uint4 q) {
-    return (cell_window_pass(s.w, q.x) ? 1u : 0u) | (cell_window_pass(s.w, q.y) ? 2u : 0u) | (cell_window_pass(s.w, q.z) ? 4u : 0u) |
-           (cell_window_pass(s.w, q.w) ? 8u : 0u);
-  };
-  unsigned long long mask = four(keys[0]) >> skip;
+  unsigned long long mask = key_window_four(s.w.keys, keys[0]) >> skip;
 #pragma unroll 2
   for (int at = 4 - skip; at < s.n_out; at += 4) {
-    mask |= (unsigned long long)four(*++keys) << at;
+    mask |= (unsigned long long)key_window_four(s.w.keys, *++keys) << at;
   }
   return mask & (~0ull >> (kMaxMaskedOut - s.n_out));
 }
@@ -1649,7 +1455,7 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
       int count = 0;
       if (crowded) {
         for (int q = 0; q < p.n_out; ++q) {
-          count += cell_window_pass(p.w, a.trk_key[p.j0 + q]);
+          count += key_window_pass(p.w.keys, a.trk_key[p.j0 + q]);
         }
       } else if (p.n_out > 0) {
         mask = cell_precut_mask(a, p);
@@ -1693,7 +1499,7 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
             p = cell_lane(a, k);
           }
           const int q = next_out + lane;
-          const bool listed = q < p.n_out && cell_window_pass(p.w, a.trk_key[p.j0 + q]);
+          const bool listed = q < p.n_out && key_window_pass(p.w.keys, a.trk_key[p.j0 + q]);
           const unsigned m = __ballot_sync(0xffffffffu, listed);
           if (listed) {
             w.ring[(tail + __popc(m & ((1u << lane) - 1u))) & (kCellRing - 1)] = next | (uint32_t)q << 7;
@@ -2376,21 +2182,14 @@ void step_tracklets_count(const Arena &a, const Launch &l)
   if (blocks <= 0) {
     return;
   }
-  const size_t stage_bytes = kStageEntries * sizeof(float4);
   // the count pass takes at most kCountThreads threads per block (any whole warps give the same
   // results)
   const int block = std::min(l.block, kCountThreads);
   const unsigned grid = (unsigned)((a.n_clusters + block - 1) / block);
-  if (a.prune_tracklets == 2) {  // the staged walk (tuning knob; results are identical)
-    if (a.gate) {
-      k_tracklets_count<true, true><<<grid, block, stage_bytes, l.stream>>>(a);
-    } else {
-      k_tracklets_count<true, false><<<grid, block, stage_bytes, l.stream>>>(a);
-    }
-  } else if (a.gate) {
-    k_tracklets_count<false, true><<<grid, block, 0, l.stream>>>(a);
+  if (a.gate) {
+    k_tracklets_count<true><<<grid, block, 0, l.stream>>>(a);
   } else {
-    k_tracklets_count<false, false><<<grid, block, 0, l.stream>>>(a);
+    k_tracklets_count<false><<<grid, block, 0, l.stream>>>(a);
   }
 }
 
