@@ -704,7 +704,7 @@ __device__ __forceinline__ void write_tracklet(const Arena &a, int out, int64_t 
 }
 
 constexpr int kTrackletSlots = kTrackletSlotsPerCluster;
-constexpr int kMaskKeys = 32;  // keys of the walk's window a mask holds (64: 0.72 in place of 0.66 ms per 128 central events)
+constexpr int kMaskKeys = 32;  // keys of the walk's window a mask holds (of 64: 0.72 in place of 0.66 ms per 128 central events)
 constexpr int kMaxMaskedOut = 64;  // out-degrees up to this are evaluated pair-parallel with a pass mask
 
 // The reference's candidate sequence of one inner cluster (Tracker.cxx:73-113), calling
@@ -870,8 +870,8 @@ __device__ __forceinline__ void walk_inner(const Arena &a, const InnerCluster &s
         const uint4 *keys = reinterpret_cast<const uint4 *>(a.clu_key + (s.next_begin + k0 - skip));
         for (int at = k0 - skip; at < k1; at += kMaskKeys, keys += kMaskKeys / 4) {
           const int n = min(kMaskKeys, k1 - at);
+          // (the compiler's own unrolling: of 1, 2, 4 and 8 it is slower, 0.65 to 0.76 ms per 128 central events)
           uint32_t mask = 0;
-#pragma unroll 2
           for (int b = 0; b < n; b += 4) {
             mask |= key_window_four(s.window, keys[b / 4]) << b;
           }
@@ -913,10 +913,11 @@ constexpr int kCountThreads = 256;
 
 // Count pass, one thread per inner cluster: the number of tracklets, and the outer clusters of
 // the first kTrackletSlots of them in emission order. kGate: the learned form's first stage
-// (inner_cluster). At most kCountThreads threads per block. Bound by issue, half of it lost to lanes
-// whose candidates end at different times: 0.66 ms per 128 central events; with a walk of z-sorted
-// lists (a binary search per bin and passes put back into index order) 0.62, but 0.09 ms more in the
-// clustering.
+// (inner_cluster). At most kCountThreads threads per block. Bound by the integer pipe, half of whose
+// work is lost to lanes whose candidates end at different times: 0.59 ms per 128 central events (0.63
+// at five blocks per SM); with a walk of z-sorted lists (a binary search per bin and passes put back
+// into index order) 0.62, and 0.09 ms more in the clustering; with the candidates of all lanes queued
+// and the cut in full rounds 0.74.
 template <bool kGate>
 __global__ void __launch_bounds__(kCountThreads, kGate ? 5 : 6) k_tracklets_count(Arena a)
 {
