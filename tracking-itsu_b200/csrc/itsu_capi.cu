@@ -211,6 +211,8 @@ struct itsu_context {
   // learned tracklet gate: its FP32 master and device model, and whether the learned form uses it
   itsu_gate_model *d_gate_master = nullptr;
   itsu::GateDevice *d_gate = nullptr;
+  float *train = nullptr;  // training workspace (train_scratch)
+  size_t train_floats = 0;
   bool has_gate = false;
   bool gate = false;
   bool prefilter = false;
@@ -1078,7 +1080,7 @@ void itsu_context_destroy(itsu_context *ctx)
   release(ctx->road_count); release(ctx->road_off); release(ctx->paths);
   release(ctx->nb); release(ctx->roads); release(ctx->scan_partials); release(ctx->d_status);
   release(ctx->d_master); release(ctx->d_mlp);
-  release(ctx->d_gate_master); release(ctx->d_gate);
+  release(ctx->d_gate_master); release(ctx->d_gate); release(ctx->train);
   release(ctx->report_scratch); release(ctx->chunk_off); release(ctx->roads_all); release(ctx->road_off_all); release(ctx->chunk_status);
   if (ctx->h_chunk_status) cudaFreeHost(ctx->h_chunk_status);
   if (ctx->h_chunk_off) cudaFreeHost(ctx->h_chunk_off);
@@ -2255,12 +2257,6 @@ std::vector<uint16_t> bf16_weights(const Model &m)
   return out;
 }
 
-template <typename T>
-struct DeviceScratch {  // a temporary device allocation freed on scope exit
-  T *p = nullptr;
-  ~DeviceScratch() { if (p) cudaFree(p); }
-};
-
 template <class Model>
 itsu_status require_net(itsu_context *ctx, const char *what)
 {
@@ -2422,6 +2418,18 @@ itsu_status net_score(itsu_context *ctx, const float *features, int64_t n, float
   return ITSU_OK;
 }
 
+// The context's training workspace, of n floats at least. Its calls end with the stream idle.
+cudaError_t train_scratch(itsu_context *ctx, size_t n)
+{
+  if (n <= ctx->train_floats) return cudaSuccess;
+  cudaFree(ctx->train);
+  ctx->train = nullptr;
+  ctx->train_floats = 0;
+  const cudaError_t e = cudaMalloc((void **)&ctx->train, sizeof(float) * n);
+  if (e == cudaSuccess) ctx->train_floats = n;
+  return e;
+}
+
 template <class Model>
 itsu_status net_train(itsu_context *ctx, const float *features, const uint8_t *labels, int64_t n, const itsu_train_config *cfg,
                       float *losses, const char *what)
@@ -2437,14 +2445,11 @@ itsu_status net_train(itsu_context *ctx, const float *features, const uint8_t *l
   if (!aligned16(features)) return fail(ctx, ITSU_ERR_INVALID, "%s: features must be 16-byte aligned", what);
   ITSU_CUDA(ctx, cudaSetDevice(ctx->device));
   const int blocks = itsu::mlp_gradient_blocks(cfg->batch);
-  DeviceScratch<float> partials, m, v, loss;
-  ITSU_CUDA(ctx, cudaMalloc((void **)&partials.p, sizeof(float) * blocks * N::kParams));
-  ITSU_CUDA(ctx, cudaMalloc((void **)&m.p, sizeof(float) * N::kParams));
-  ITSU_CUDA(ctx, cudaMalloc((void **)&v.p, sizeof(float) * N::kParams));
-  ITSU_CUDA(ctx, cudaMalloc((void **)&loss.p, sizeof(float) * std::max<int64_t>(cfg->steps, 1)));
-  ITSU_CUDA(ctx, cudaMemsetAsync(m.p, 0, sizeof(float) * N::kParams, ctx->stream));
-  ITSU_CUDA(ctx, cudaMemsetAsync(v.p, 0, sizeof(float) * N::kParams, ctx->stream));
-  ITSU_CUDA(ctx, cudaMemsetAsync(loss.p, 0, sizeof(float) * std::max<int64_t>(cfg->steps, 1), ctx->stream));
+  // the partials, then m, v and the losses
+  const size_t n_partials = (size_t)blocks * N::kParams, n_rest = 2 * (size_t)N::kParams + std::max<int64_t>(cfg->steps, 1);
+  ITSU_CUDA(ctx, train_scratch(ctx, n_partials + n_rest));
+  float *const partials = ctx->train, *const m = partials + n_partials, *const v = m + N::kParams, *const loss = v + N::kParams;
+  ITSU_CUDA(ctx, cudaMemsetAsync(m, 0, sizeof(float) * n_rest, ctx->stream));
   double b1t = 1.0, b2t = 1.0;
   for (int64_t step = 0; step < cfg->steps; ++step) {
     // cosine decay from lr to lr_final
@@ -2452,15 +2457,15 @@ itsu_status net_train(itsu_context *ctx, const float *features, const uint8_t *l
     const float lr = (float)(cfg->lr_final + 0.5 * (cfg->lr - cfg->lr_final) * (1.0 + std::cos(3.14159265358979323846 * frac)));
     b1t *= cfg->beta1;
     b2t *= cfg->beta2;
-    itsu::launch_mlp_gradient(N::device(ctx), features, labels, n, cfg->batch, false, cfg->seed, step, cfg->pos_weight, partials.p,
-                              loss.p + step, ctx->stream);
-    itsu::launch_mlp_adam(N::master(ctx), partials.p, blocks, m.p, v.p, lr, cfg->beta1, cfg->beta2, cfg->eps, cfg->weight_decay,
+    itsu::launch_mlp_gradient(N::device(ctx), features, labels, n, cfg->batch, false, cfg->seed, step, cfg->pos_weight, partials,
+                              loss + step, ctx->stream);
+    itsu::launch_mlp_adam(N::master(ctx), partials, blocks, m, v, lr, cfg->beta1, cfg->beta2, cfg->eps, cfg->weight_decay,
                           (float)(1.0 - b1t), (float)(1.0 - b2t), N::device(ctx), ctx->stream);
     if ((step & 1023) == 0) ITSU_CUDA(ctx, cudaGetLastError());
   }
   ITSU_CUDA(ctx, cudaGetLastError());
   if (losses && cfg->steps > 0) {
-    ITSU_CUDA(ctx, cudaMemcpyAsync(losses, loss.p, sizeof(float) * cfg->steps, cudaMemcpyDeviceToHost, ctx->stream));
+    ITSU_CUDA(ctx, cudaMemcpyAsync(losses, loss, sizeof(float) * cfg->steps, cudaMemcpyDeviceToHost, ctx->stream));
   }
   ITSU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   return ITSU_OK;
@@ -2478,22 +2483,17 @@ itsu_status net_gradient(itsu_context *ctx, const float *features, const uint8_t
   ITSU_CUDA(ctx, cudaSetDevice(ctx->device));
   const int32_t batch = (int32_t)n;
   const int blocks = itsu::mlp_gradient_blocks(batch);
-  DeviceScratch<float> partials, loss;
-  ITSU_CUDA(ctx, cudaMalloc((void **)&partials.p, sizeof(float) * blocks * N::kParams));
-  ITSU_CUDA(ctx, cudaMalloc((void **)&loss.p, sizeof(float)));
-  ITSU_CUDA(ctx, cudaMemsetAsync(loss.p, 0, sizeof(float), ctx->stream));
-  itsu::launch_mlp_gradient(N::device(ctx), features, labels, n, batch, true, 0, 0, pos_weight, partials.p, loss.p, ctx->stream);
+  // the partials, then the sums and the loss
+  ITSU_CUDA(ctx, train_scratch(ctx, (size_t)(blocks + 1) * N::kParams + 1));
+  float *const partials = ctx->train, *const sums = partials + (size_t)blocks * N::kParams, *const loss = sums + N::kParams;
+  ITSU_CUDA(ctx, cudaMemsetAsync(loss, 0, sizeof(float), ctx->stream));
+  itsu::launch_mlp_gradient(N::device(ctx), features, labels, n, batch, true, 0, 0, pos_weight, partials, loss, ctx->stream);
+  itsu::launch_mlp_gradient_sum(partials, blocks, N::kParams, sums, ctx->stream);
   ITSU_CUDA(ctx, cudaGetLastError());
-  std::vector<float> h((size_t)blocks * N::kParams);
   float l = 0.0f;
-  ITSU_CUDA(ctx, cudaMemcpyAsync(h.data(), partials.p, sizeof(float) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));
-  ITSU_CUDA(ctx, cudaMemcpyAsync(&l, loss.p, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
+  ITSU_CUDA(ctx, cudaMemcpyAsync(grad, sums, sizeof(float) * N::kParams, cudaMemcpyDeviceToHost, ctx->stream));
+  ITSU_CUDA(ctx, cudaMemcpyAsync(&l, loss, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
   ITSU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  for (int i = 0; i < N::kParams; ++i) {
-    double sum = 0.0;
-    for (int b = 0; b < blocks; ++b) sum += h[(size_t)b * N::kParams + i];
-    grad[i] = (float)sum;
-  }
   if (loss_out) *loss_out = l;
   return ITSU_OK;
 }

@@ -292,7 +292,8 @@ void launch_mlp_gradient(const GateDevice *model, const float *features, const u
                          bool sequential, uint64_t seed, int64_t step, float pos_weight, float *grad_partials, float *loss,
                          cudaStream_t stream);
 int mlp_gradient_blocks(int32_t batch);
-int mlp_max_gradient_blocks();
+// grad[params] = the blocks' partials added up in 64 bits (params: the pair's or the gate's).
+void launch_mlp_gradient_sum(const float *grad_partials, int blocks, int params, float *grad, cudaStream_t stream);
 // One Adam step on the master parameters from the summed partials, then publishes the device model.
 void launch_mlp_adam(itsu_prefilter_model *master, const float *grad_partials, int blocks, float *m, float *v, float lr,
                      float beta1, float beta2, float eps, float weight_decay, float bias1, float bias2, MlpDevice *model,

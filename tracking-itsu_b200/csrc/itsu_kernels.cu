@@ -1639,7 +1639,7 @@ __global__ void __launch_bounds__(kPrefilterThreads) k_cells_prefilter(Arena a)
       }
       feature_row(mlp.mean, mlp.inv_std, f, rows[warp][lane]);
       __syncwarp();
-      const float logit = mlp_logits_warp<false>(mlp, rows[warp], nullptr);
+      const float logit = mlp_logits_warp(mlp, rows[warp]);
       if (scored && logit < mlp.threshold) {
         a.cell_entries[i].segment = kEntryDropped;
         atomicSub(&a.cell_span_count[s0 + owner], 1);

@@ -61,7 +61,7 @@ constexpr int kSmpPitch = 40;  // transposed [unit][sample] operands (32 used)
 
 // A network as the device keeps it in global memory.
 template <int H>
-struct MlpDeviceT {
+struct __align__(16) MlpDeviceT {
   __nv_bfloat16 w1[H][kMlpIn];  // [out][in]
   __nv_bfloat16 w2[H][H];       // [out][in]
   __nv_bfloat16 w3[H];
@@ -95,23 +95,24 @@ struct __align__(16) MlpSmemT {
 using MlpSmem = MlpSmemT<kMlpHidden>;
 using GateSmem = MlpSmemT<kGateHidden>;
 
-// Block-cooperative copy of a network into shared memory (the caller synchronises the block).
+// Block-cooperative copy of a network into shared memory, rows in 16-byte pieces (the caller
+// synchronises the block).
 template <int H>
 __device__ __forceinline__ void load_mlp(MlpSmemT<H> &s, const MlpDeviceT<H> &g)
 {
-  constexpr int P = MlpSmemT<H>::kPitch;
-  const __nv_bfloat16 zero = __float2bfloat16_rn(0.0f);
-  for (int i = threadIdx.x; i < H * kRowPitch; i += blockDim.x) {
-    const int r = i / kRowPitch, c = i % kRowPitch;
-    s.w1[r][c] = c < kMlpIn ? g.w1[r][c] : zero;
+  constexpr int kPieces = H / 8 + 1;  // of a row of W2 or W3 and its padding
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < H * (kRowPitch / 8); i += blockDim.x) {
+    const int r = i / (kRowPitch / 8), c = i % (kRowPitch / 8);
+    reinterpret_cast<uint4 *>(s.w1[r])[c] = c == 0 ? *reinterpret_cast<const uint4 *>(g.w1[r]) : zero;
   }
-  for (int i = threadIdx.x; i < H * P; i += blockDim.x) {
-    const int r = i / P, c = i % P;
-    s.w2[r][c] = c < H ? g.w2[r][c] : zero;
+  for (int i = threadIdx.x; i < H * kPieces; i += blockDim.x) {
+    const int r = i / kPieces, c = i % kPieces;
+    reinterpret_cast<uint4 *>(s.w2[r])[c] = c < H / 8 ? reinterpret_cast<const uint4 *>(g.w2[r])[c] : zero;
   }
-  for (int i = threadIdx.x; i < 8 * P; i += blockDim.x) {
-    const int r = i / P, c = i % P;
-    s.w3[r][c] = (r == 0 && c < H) ? g.w3[c] : zero;
+  for (int i = threadIdx.x; i < 8 * kPieces; i += blockDim.x) {
+    const int r = i / kPieces, c = i % kPieces;
+    reinterpret_cast<uint4 *>(s.w3[r])[c] = (r == 0 && c < H / 8) ? reinterpret_cast<const uint4 *>(g.w3)[c] : zero;
   }
   for (int i = threadIdx.x; i < H; i += blockDim.x) {
     s.b1[i] = g.b1[i];
@@ -207,6 +208,16 @@ __device__ __forceinline__ void mma_bf16(float d[4], const uint32_t a[4], uint32
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// Four 8 x 8 BF16 matrices from shared memory, transposed: lane 8 q + r gives the address of row r of
+// matrix q; each register then holds (row 2t, column g), (row 2t + 1, column g) of its matrix.
+__device__ __forceinline__ void ldmatrix_t(uint32_t r[4], const __nv_bfloat16 *row)
+{
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(row))
+               : "memory");
+}
+
 // Fragment layout of m16n8k16 (g = lane / 4, t = lane % 4): A registers hold (row g, k 2t..2t+1),
 // (row g+8, k 2t..), (row g, k 2t+8..), (row g+8, k 2t+8..); B registers hold (k 2t..2t+1, col g)
 // and (k 2t+8.., col g); D holds (row g, col 2t), (row g, col 2t+1), (row g+8, col 2t), (row g+8,
@@ -234,20 +245,11 @@ __device__ __forceinline__ float act_grad(float x)
   }
 }
 
-// Where the training pass keeps a 32-sample tile's intermediate values.
-template <int H>
-struct MlpTraceT {
-  float (*a1)[H + 1];               // [sample][unit] layer-1 pre-activations
-  float (*a2)[H + 1];               // [sample][unit] layer-2 pre-activations
-  __nv_bfloat16 (*h1t)[kSmpPitch];  // [unit][sample] layer-1 activations (BF16, as the next MMA sees them)
-};
-using MlpTrace = MlpTraceT<kMlpHidden>;
-
 // Forward pass of rows 16 mt .. 16 mt + 15 of a 32-row tile; returns the logits of rows g and
 // g + 8 of the tile in lo / hi (valid in lanes with t == 0). All lanes of the warp take part.
-template <bool kTrace, int H, bool kRelu>
+template <int H, bool kRelu>
 __device__ __forceinline__ void mlp_forward_m16(const MlpSmemT<H> &m, const __nv_bfloat16 (*rows)[kRowPitch], int mt, float &lo,
-                                                float &hi, const MlpTraceT<H> *trace)
+                                                float &hi)
 {
   constexpr int NT = H / 8, KT = H / 16;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -272,18 +274,6 @@ __device__ __forceinline__ void mlp_forward_m16(const MlpSmemT<H> &m, const __nv
     const uint32_t bottom = pack_bf16(act<kRelu>(c[2]), act<kRelu>(c[3]));
     hk[nt >> 1][(nt & 1) * 2 + 0] = top;
     hk[nt >> 1][(nt & 1) * 2 + 1] = bottom;
-    if constexpr (kTrace) {
-      trace->a1[r0][col] = c[0];
-      trace->a1[r0][col + 1] = c[1];
-      trace->a1[r1][col] = c[2];
-      trace->a1[r1][col + 1] = c[3];
-      const __nv_bfloat162 tv = *reinterpret_cast<const __nv_bfloat162 *>(&top);
-      const __nv_bfloat162 bv = *reinterpret_cast<const __nv_bfloat162 *>(&bottom);
-      trace->h1t[col][r0] = tv.x;
-      trace->h1t[col + 1][r0] = tv.y;
-      trace->h1t[col][r1] = bv.x;
-      trace->h1t[col + 1][r1] = bv.y;
-    }
   }
   // layer 2: [16 x H] x [H x H]
   float h2[NT][4];
@@ -309,12 +299,6 @@ __device__ __forceinline__ void mlp_forward_m16(const MlpSmemT<H> &m, const __nv
       const int col = nt * 8 + 2 * t;
       const float v0 = h2[nt][0] + m.b2[col], v1 = h2[nt][1] + m.b2[col + 1];
       const float v2 = h2[nt][2] + m.b2[col], v3 = h2[nt][3] + m.b2[col + 1];
-      if constexpr (kTrace) {
-        trace->a2[r0][col] = v0;
-        trace->a2[r0][col + 1] = v1;
-        trace->a2[r1][col] = v2;
-        trace->a2[r1][col + 1] = v3;
-      }
       ak[half * 2 + 0] = pack_bf16(act<kRelu>(v0), act<kRelu>(v1));
       ak[half * 2 + 1] = pack_bf16(act<kRelu>(v2), act<kRelu>(v3));
     }
@@ -324,22 +308,16 @@ __device__ __forceinline__ void mlp_forward_m16(const MlpSmemT<H> &m, const __nv
   hi = o[2] + m.b3;
 }
 
-template <class T>
-struct NoDeduce {
-  using type = T;
-};
-
 // Logits of the 32 rows of a tile; lane l gets row l's. All lanes of the warp take part.
-template <bool kTrace, int H = kMlpHidden, bool kRelu = false>
-__device__ __forceinline__ float mlp_logits_warp(const MlpSmemT<H> &m, const __nv_bfloat16 (*rows)[kRowPitch],
-                                                 const typename NoDeduce<MlpTraceT<H>>::type *trace)
+template <int H = kMlpHidden, bool kRelu = false>
+__device__ __forceinline__ float mlp_logits_warp(const MlpSmemT<H> &m, const __nv_bfloat16 (*rows)[kRowPitch])
 {
   const int lane = threadIdx.x & 31;
   float mine = 0.0f;
 #pragma unroll 1
   for (int mt = 0; mt < 2; ++mt) {
     float lo, hi;
-    mlp_forward_m16<kTrace, H, kRelu>(m, rows, mt, lo, hi, trace);
+    mlp_forward_m16<H, kRelu>(m, rows, mt, lo, hi);
     // row r of this m-tile sits in lane 4 (r mod 8), in lo for r < 8 and hi otherwise
     const int src = (lane & 7) << 2;
     lo = __shfl_sync(0xffffffffu, lo, src);

@@ -23,9 +23,8 @@ namespace itsu {
 namespace {
 
 constexpr int kTrainWarps = 4;
-constexpr int kMaxGradBlocks = 64;  // per-block gradient partials the Adam step reduces
-
-__device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+constexpr int kTrainSamples = 16 * kTrainWarps;  // a block's tile
+constexpr int kMaxGradBlocks = 2 * 148;          // two per SM; each leaves a gradient partial
 
 __device__ __forceinline__ uint64_t splitmix64(uint64_t x)
 {
@@ -249,7 +248,7 @@ __global__ void __launch_bounds__(kScoreThreads) k_mlp_score(const MlpDeviceT<H>
     }
     feature_row(mlp.mean, mlp.inv_std, f, rows[warp][lane]);
     __syncwarp();
-    const float logit = mlp_logits_warp<false, H, kRelu>(mlp, rows[warp], nullptr);
+    const float logit = mlp_logits_warp<H, kRelu>(mlp, rows[warp]);
     if (row < n) {
       logits[row] = logit;
     }
@@ -259,236 +258,319 @@ __global__ void __launch_bounds__(kScoreThreads) k_mlp_score(const MlpDeviceT<H>
 
 // ---- training: minibatch gradient ----
 
-// One warp's 32-sample tile of the training pass of an 8 -> H -> H -> 1 network.
-template <int H>
-struct TrainWarp {
-  static constexpr int kPitch = MlpShape<H>::kHidPitch;
-  __nv_bfloat16 x[32][kRowPitch];     // standardised inputs [sample][feature] (A of layer 1)
-  __nv_bfloat16 xt[8][kSmpPitch];     // the same, [feature][sample] (B of dW1)
-  float a1[32][H + 1];                // layer-1 pre-activations, then dL/da1
-  float a2[32][H + 1];                // layer-2 pre-activations, then dL/da2
-  __nv_bfloat16 h1t[H][kSmpPitch];    // layer-1 activations [unit][sample] (B of dW2)
-  __nv_bfloat16 d2[32][kPitch];       // dL/da2 [sample][unit] (A of dh1)
-  __nv_bfloat16 d2t[H][kSmpPitch];    // dL/da2 [unit][sample] (A of dW2)
-  __nv_bfloat16 d1t[H][kSmpPitch];    // dL/da1 [unit][sample] (A of dW1)
-  float dz[32];                       // dL/dlogit
-};
-
+// A block's tile of the training pass of an 8 -> H -> H -> 1 network, [sample][unit], as the weight
+// gradients' operands, and what each warp's samples add to the sums over samples.
 template <int H>
 struct __align__(16) TrainBlock {
+  static constexpr int kPitch = MlpShape<H>::kHidPitch;
   MlpSmemT<H> mlp;
-  __nv_bfloat16 w2t[H][MlpShape<H>::kHidPitch];  // W2 transposed [in][out] (B of dh1)
-  float grad[MlpShape<H>::kParams];
-  TrainWarp<H> warps[kTrainWarps];
+  __align__(16) __nv_bfloat16 x[kTrainSamples][kRowPitch];  // standardised inputs
+  __nv_bfloat16 h1[kTrainSamples][kPitch];                  // layer-1 activations
+  __nv_bfloat16 d2[kTrainSamples][kPitch];                  // dL/da2
+  __nv_bfloat16 d1[kTrainSamples][kPitch];                  // dL/da1
+  float unit[kTrainWarps][3][H];                            // dL/dW3, dL/db2, dL/db1
+  float b3[kTrainWarps];
 };
 
+// Gradient of the loss over a batch. A block takes tiles of 64 samples. A warp has 16 of them, as the
+// rows of one MMA, and keeps their forward and backward pass in registers, one layer's output
+// fragments being the next one's operand; then the block's warps share out the rows of dL/dW2 and
+// dL/dW1, contractions over all 64 samples, whose accumulators stay in registers over the block's
+// tiles, like the sums over samples (biases, W3, loss). Each block writes its partial gradient.
+// Bound by the latency of one tile's chain (a batch of 8192 is 128 tiles, one per SM) and of the
+// network's load: 13 us per batch of 8192, 0.075 ms per 262,144 samples; 38 us and 0.79 ms with 32
+// samples per warp passed through shared memory and gradients summed by shared-memory atomics.
 template <int H, bool kRelu>
-__global__ void __launch_bounds__(kTrainWarps * 32) k_mlp_gradient(const MlpDeviceT<H> *model, const float *features,
-                                                                   const uint8_t *labels, int64_t n, int32_t batch,
-                                                                   int32_t sequential, uint64_t seed, int64_t step,
-                                                                   float pos_weight, float *grad_partials, float *loss)
+__global__ void __launch_bounds__(kTrainWarps * 32, 2) k_mlp_gradient(const MlpDeviceT<H> *model, const float *features,
+                                                                      const uint8_t *labels, int64_t n, int32_t batch,
+                                                                      int32_t sequential, uint64_t seed, int64_t step,
+                                                                      float pos_weight, float *grad_partials, float *loss)
 {
   using S = MlpShape<H>;
-  constexpr int NT = H / 8, KT = H / 16, P = S::kHidPitch;
+  constexpr int NT = H / 8, KT = H / 16;
+  constexpr int kRowTiles = (KT + kTrainWarps - 1) / kTrainWarps;  // of dL/dW2 and dL/dW1 per warp
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TrainBlock<H> &B = *reinterpret_cast<TrainBlock<H> *>(smem_raw);
-  load_mlp(B.mlp, *model);
-  for (int i = threadIdx.x; i < H * P; i += blockDim.x) {
-    const int r = i / P, c = i % P;
-    B.w2t[r][c] = c < H ? model->w2[c][r] : __float2bfloat16_rn(0.0f);
-  }
-  for (int i = threadIdx.x; i < S::kParams; i += blockDim.x) {
-    B.grad[i] = 0.0f;
-  }
-  __syncthreads();
   const MlpSmemT<H> &M = B.mlp;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  TrainWarp<H> &W = B.warps[warp];
-  const float inv_batch = 1.0f / (float)batch;
-  const int64_t tiles = (batch + 31) / 32;
-  for (int64_t tile = (int64_t)blockIdx.x * kTrainWarps + warp; tile < tiles; tile += (int64_t)gridDim.x * kTrainWarps) {
-    // 1. the tile's samples
-    const int64_t k = tile * 32 + lane;
-    const bool valid = k < batch;
-    float f[kMlpIn];
-    float y = 0.0f;
-    if (valid) {
+  // half a sample of the warp's in a tile, and its label: two lanes per sample
+  float4 half_row = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float y = 0.0f;
+  auto fetch = [&](int64_t tile) {
+    const int64_t k = tile * kTrainSamples + warp * 16 + (lane >> 1);
+    if (k < batch) {
       const int64_t idx = sequential ? k : (int64_t)(splitmix64(seed + (uint64_t)step * 0x632BE59BD9B4E019ull + (uint64_t)k) % (uint64_t)n);
-      const float4 *src = reinterpret_cast<const float4 *>(features + idx * kMlpIn);
-      const float4 u = src[0], v = src[1];
-      f[0] = u.x, f[1] = u.y, f[2] = u.z, f[3] = u.w, f[4] = v.x, f[5] = v.y, f[6] = v.z, f[7] = v.w;
+      half_row = reinterpret_cast<const float4 *>(features + idx * kMlpIn)[lane & 1];
       y = labels[idx] ? 1.0f : 0.0f;
-    } else {
-      for (int q = 0; q < kMlpIn; ++q) {
-        f[q] = M.mean[q];
-      }
     }
-    feature_row(M.mean, M.inv_std, f, W.x[lane]);
-    for (int q = 0; q < kMlpIn; ++q) {
-      W.xt[q][lane] = W.x[lane][q];
-    }
-    __syncwarp();
-    // 2. forward, keeping the pre-activations and the layer-1 activations
-    const MlpTraceT<H> trace{W.a1, W.a2, W.h1t};
-    const float z = mlp_logits_warp<true, H, kRelu>(M, W.x, &trace);
-    // 3. loss and dL/dz: weighted binary cross-entropy of sigmoid(z), averaged over the batch
-    const float wgt = valid ? (y > 0.0f ? pos_weight : 1.0f) : 0.0f;
-    const float prob = 1.0f / (1.0f + expf(-z));
-    W.dz[lane] = wgt * (prob - y) * inv_batch;
-    float l = wgt * (fmaxf(z, 0.0f) - z * y + log1pf(expf(-fabsf(z)))) * inv_batch;
-    float dzsum = W.dz[lane];
-    for (int o = 16; o > 0; o >>= 1) {
-      l += __shfl_xor_sync(0xffffffffu, l, o);
-      dzsum += __shfl_xor_sync(0xffffffffu, dzsum, o);
-    }
-    if (lane == 0) {
-      atomicAdd(loss, l);
-      atomicAdd(&B.grad[S::kOffB3], dzsum);
-    }
-    __syncwarp();
-    // 4. dW3 (lane owns units lane and lane + 32)
-    for (int jj = lane; jj < H; jj += 32) {
-      float acc = 0.0f;
-      for (int s2 = 0; s2 < 32; ++s2) {
-        acc += W.dz[s2] * bf16r(act<kRelu>(W.a2[s2][jj]));
-      }
-      atomicAdd(&B.grad[S::kOffW3 + jj], acc);
-    }
-    __syncwarp();
-    // 5. dL/da2 (lane owns sample lane)
+  };
+  fetch(blockIdx.x);  // under way while the network is loaded
+  load_mlp(B.mlp, *model);
+  __syncthreads();
+  const int mq = lane >> 3, mr = lane & 7;  // the matrix and row whose address the lane gives to ldmatrix_t
+  const int r0 = warp * 16 + g, r1 = r0 + 8;
+  const float inv_batch = 1.0f / (float)batch;
+  float dw2[kRowTiles][NT][4] = {}, dw1[kRowTiles][4] = {};
+  float dw3[NT][2] = {}, db2[NT][2] = {}, db1[NT][2] = {};  // of columns nt * 8 + 2t, + 1: rows r0 and r1 of every tile
+  float db3 = 0.0f, loss_sum = 0.0f;
+  const int64_t tiles = ((int64_t)batch + kTrainSamples - 1) / kTrainSamples;
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    // 1. the warp's samples as MMA rows
+    const bool valid = tile * kTrainSamples + warp * 16 + (lane >> 1) < batch;
     {
-      const float dz = W.dz[lane];
-      for (int j = 0; j < H; ++j) {
-        const float d = dz * __bfloat162float(M.w3[0][j]) * act_grad<kRelu>(W.a2[lane][j]);
-        W.a2[lane][j] = d;
-        const __nv_bfloat16 db = __float2bfloat16_rn(d);
-        W.d2[lane][j] = db;
-        W.d2t[j][lane] = db;
-      }
+      const int half = lane & 1;
+      const float4 u = half_row;
+      const float *mean = M.mean + 4 * half, *inv_std = M.inv_std + 4 * half;
+      uint2 *const row = reinterpret_cast<uint2 *>(B.x[warp * 16 + (lane >> 1)]);
+      row[half] = valid ? make_uint2(pack_bf16((u.x - mean[0]) * inv_std[0], (u.y - mean[1]) * inv_std[1]),
+                                     pack_bf16((u.z - mean[2]) * inv_std[2], (u.w - mean[3]) * inv_std[3]))
+                        : make_uint2(0, 0);
+      row[2 + half] = make_uint2(0, 0);
     }
+    const float weight = valid ? (y > 0.0f ? pos_weight : 1.0f) : 0.0f;
+    const float y0 = __shfl_sync(0xffffffffu, y, 2 * g), y1 = __shfl_sync(0xffffffffu, y, 2 * g + 16);
+    const float weight0 = __shfl_sync(0xffffffffu, weight, 2 * g), weight1 = __shfl_sync(0xffffffffu, weight, 2 * g + 16);
     __syncwarp();
-    for (int jj = lane; jj < H; jj += 32) {
-      float acc = 0.0f;
-      for (int s2 = 0; s2 < 32; ++s2) {
-        acc += W.a2[s2][jj];
+    // 2. forward, keeping the activations' derivatives
+    uint32_t a[4], h1[KT][4], h2[KT][4];
+    float e1[NT][4], e2[NT][4];
+    a[0] = ld32(&B.x[r0][2 * t]);
+    a[1] = ld32(&B.x[r1][2 * t]);
+    a[2] = ld32(&B.x[r0][2 * t + 8]);
+    a[3] = ld32(&B.x[r1][2 * t + 8]);
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const int col = nt * 8 + 2 * t;
+      float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      mma_bf16(c, a, ld32(&M.w1[nt * 8 + g][2 * t]), ld32(&M.w1[nt * 8 + g][2 * t + 8]));
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        c[q] += M.b1[col + (q & 1)];
+        e1[nt][q] = act_grad<kRelu>(c[q]);
+        c[q] = act<kRelu>(c[q]);
       }
-      atomicAdd(&B.grad[S::kOffB2 + jj], acc);
+      const uint32_t top = pack_bf16(c[0], c[1]), bottom = pack_bf16(c[2], c[3]);
+      h1[nt >> 1][(nt & 1) * 2 + 0] = top;
+      h1[nt >> 1][(nt & 1) * 2 + 1] = bottom;
+      *reinterpret_cast<uint32_t *>(&B.h1[r0][col]) = top;
+      *reinterpret_cast<uint32_t *>(&B.h1[r1][col]) = bottom;
     }
-    // 6. dW2 = dL/da2^T h1: [H j x 32 s] x [32 s x H i]
-    for (int mt = 0; mt < KT; ++mt) {
-      float acc[NT][4];
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
-      }
-#pragma unroll
-      for (int kk = 0; kk < 2; ++kk) {
-        uint32_t a[4];
-        a[0] = ld32(&W.d2t[16 * mt + g][16 * kk + 2 * t]);
-        a[1] = ld32(&W.d2t[16 * mt + g + 8][16 * kk + 2 * t]);
-        a[2] = ld32(&W.d2t[16 * mt + g][16 * kk + 2 * t + 8]);
-        a[3] = ld32(&W.d2t[16 * mt + g + 8][16 * kk + 2 * t + 8]);
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-          mma_bf16(acc[nt], a, ld32(&W.h1t[nt * 8 + g][16 * kk + 2 * t]), ld32(&W.h1t[nt * 8 + g][16 * kk + 2 * t + 8]));
-        }
-      }
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        float *row0 = &B.grad[S::kOffW2 + (16 * mt + g) * H + nt * 8 + 2 * t];
-        float *row1 = row0 + 8 * H;
-        atomicAdd(row0, acc[nt][0]);
-        atomicAdd(row0 + 1, acc[nt][1]);
-        atomicAdd(row1, acc[nt][2]);
-        atomicAdd(row1 + 1, acc[nt][3]);
-      }
-    }
-    // 7. dL/da1 = (dL/da2 W2) * act'(a1): [32 s x H j] x [H j x H i]
-    for (int mt = 0; mt < 2; ++mt) {
-      float acc[NT][4];
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
-      }
+    for (int nt = 0; nt < NT; ++nt) {
+      const int col = nt * 8 + 2 * t;
+      float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
       for (int kk = 0; kk < KT; ++kk) {
-        uint32_t a[4];
-        a[0] = ld32(&W.d2[16 * mt + g][16 * kk + 2 * t]);
-        a[1] = ld32(&W.d2[16 * mt + g + 8][16 * kk + 2 * t]);
-        a[2] = ld32(&W.d2[16 * mt + g][16 * kk + 2 * t + 8]);
-        a[3] = ld32(&W.d2[16 * mt + g + 8][16 * kk + 2 * t + 8]);
+        mma_bf16(c, h1[kk], ld32(&M.w2[nt * 8 + g][16 * kk + 2 * t]), ld32(&M.w2[nt * 8 + g][16 * kk + 2 * t + 8]));
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        c[q] += M.b2[col + (q & 1)];
+        e2[nt][q] = act_grad<kRelu>(c[q]);
+        c[q] = act<kRelu>(c[q]);
+      }
+      h2[nt >> 1][(nt & 1) * 2 + 0] = pack_bf16(c[0], c[1]);
+      h2[nt >> 1][(nt & 1) * 2 + 1] = pack_bf16(c[2], c[3]);
+    }
+    float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int kk = 0; kk < KT; ++kk) {
+      mma_bf16(o, h2[kk], ld32(&M.w3[g][16 * kk + 2 * t]), ld32(&M.w3[g][16 * kk + 2 * t + 8]));
+    }
+    // 3. loss and dL/dz: weighted binary cross-entropy of sigmoid(z), averaged over the batch; the
+    // logits of rows r0 and r1 stand in the quad's first lane
+    const float z0 = __shfl_sync(0xffffffffu, o[0] + M.b3, lane & ~3), z1 = __shfl_sync(0xffffffffu, o[2] + M.b3, lane & ~3);
+    const float dz0 = weight0 * (1.0f / (1.0f + expf(-z0)) - y0) * inv_batch, dz1 = weight1 * (1.0f / (1.0f + expf(-z1)) - y1) * inv_batch;
+    if (t == 0) {
+      loss_sum += weight0 * (fmaxf(z0, 0.0f) - z0 * y0 + log1pf(expf(-fabsf(z0)))) * inv_batch;
+      loss_sum += weight1 * (fmaxf(z1, 0.0f) - z1 * y1 + log1pf(expf(-fabsf(z1)))) * inv_batch;
+      db3 += dz0 + dz1;
+    }
+    // 4. dL/dW3, dL/da2
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const int col = nt * 8 + 2 * t;
+      const __nv_bfloat162 top = *reinterpret_cast<const __nv_bfloat162 *>(&h2[nt >> 1][(nt & 1) * 2 + 0]);
+      const __nv_bfloat162 bottom = *reinterpret_cast<const __nv_bfloat162 *>(&h2[nt >> 1][(nt & 1) * 2 + 1]);
+      dw3[nt][0] += dz0 * __bfloat162float(top.x) + dz1 * __bfloat162float(bottom.x);
+      dw3[nt][1] += dz0 * __bfloat162float(top.y) + dz1 * __bfloat162float(bottom.y);
+      const float w0 = __bfloat162float(M.w3[0][col]), w1 = __bfloat162float(M.w3[0][col + 1]);
+      const float d0 = dz0 * w0 * e2[nt][0], d1 = dz0 * w1 * e2[nt][1], d2 = dz1 * w0 * e2[nt][2], d3 = dz1 * w1 * e2[nt][3];
+      db2[nt][0] += d0 + d2;
+      db2[nt][1] += d1 + d3;
+      const uint32_t d_top = pack_bf16(d0, d1), d_bottom = pack_bf16(d2, d3);
+      h2[nt >> 1][(nt & 1) * 2 + 0] = d_top;  // from here on dL/da2
+      h2[nt >> 1][(nt & 1) * 2 + 1] = d_bottom;
+      *reinterpret_cast<uint32_t *>(&B.d2[r0][col]) = d_top;
+      *reinterpret_cast<uint32_t *>(&B.d2[r1][col]) = d_bottom;
+    }
+    // 5. dL/da1 = (dL/da2 W2) * act'(a1): [16 s x H j] x [H j x H i]
+#pragma unroll
+    for (int nt = 0; nt < NT; nt += 2) {
+      float c[2][4] = {};
+#pragma unroll
+      for (int kk = 0; kk < KT; ++kk) {
+        uint32_t w[4];
+        ldmatrix_t(w, &M.w2[16 * kk + (mq & 1) * 8 + mr][(nt + (mq >> 1)) * 8]);
+        mma_bf16(c[0], h2[kk], w[0], w[1]);
+        mma_bf16(c[1], h2[kk], w[2], w[3]);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int col = (nt + h) * 8 + 2 * t;
+        const float d0 = c[h][0] * e1[nt + h][0], d1 = c[h][1] * e1[nt + h][1], d2 = c[h][2] * e1[nt + h][2], d3 = c[h][3] * e1[nt + h][3];
+        db1[nt + h][0] += d0 + d2;
+        db1[nt + h][1] += d1 + d3;
+        *reinterpret_cast<uint32_t *>(&B.d1[r0][col]) = pack_bf16(d0, d1);
+        *reinterpret_cast<uint32_t *>(&B.d1[r1][col]) = pack_bf16(d2, d3);
+      }
+    }
+    __syncthreads();
+    // 6. dL/dW2 = dL/da2^T h1: [H j x 64 s] x [64 s x H i], dL/dW1 = dL/da1^T x: [H i x 64 s] x [64 s x 8 f]
+#pragma unroll
+    for (int m = 0; m < kRowTiles; ++m) {
+      const int mt = warp + m * kTrainWarps;
+      if (mt < KT) {
+#pragma unroll
+        for (int kk = 0; kk < kTrainSamples / 16; ++kk) {
+          uint32_t d[4], b[4];
+          ldmatrix_t(d, &B.d2[16 * kk + (mq >> 1) * 8 + mr][16 * mt + (mq & 1) * 8]);
+#pragma unroll
+          for (int nt = 0; nt < NT; nt += 2) {
+            ldmatrix_t(b, &B.h1[16 * kk + (mq & 1) * 8 + mr][(nt + (mq >> 1)) * 8]);
+            mma_bf16(dw2[m][nt], d, b[0], b[1]);
+            mma_bf16(dw2[m][nt + 1], d, b[2], b[3]);
+          }
+          ldmatrix_t(d, &B.d1[16 * kk + (mq >> 1) * 8 + mr][16 * mt + (mq & 1) * 8]);
+          ldmatrix_t(b, &B.x[16 * kk + (mq & 1) * 8 + mr][0]);
+          mma_bf16(dw1[m], d, b[0], b[1]);
+        }
+      }
+    }
+    fetch(tile + gridDim.x);
+    __syncthreads();  // the tile is refilled
+  }
+  // The block's partial gradient.
+  float *out = grad_partials + (int64_t)blockIdx.x * S::kParams;
+#pragma unroll
+  for (int m = 0; m < kRowTiles; ++m) {
+    const int mt = warp + m * kTrainWarps;
+    if (mt < KT) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int row = 16 * mt + g + 8 * h;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-          mma_bf16(acc[nt], a, ld32(&B.w2t[nt * 8 + g][16 * kk + 2 * t]), ld32(&B.w2t[nt * 8 + g][16 * kk + 2 * t + 8]));
+          out[S::kOffW2 + row * H + nt * 8 + 2 * t] = dw2[m][nt][2 * h];
+          out[S::kOffW2 + row * H + nt * 8 + 2 * t + 1] = dw2[m][nt][2 * h + 1];
         }
-      }
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int s2 = 16 * mt + g + (q >> 1) * 8, i = nt * 8 + 2 * t + (q & 1);
-          const float d = acc[nt][q] * act_grad<kRelu>(W.a1[s2][i]);
-          W.a1[s2][i] = d;
-          W.d1t[i][s2] = __float2bfloat16_rn(d);
-        }
+        out[S::kOffW1 + row * kMlpIn + 2 * t] = dw1[m][2 * h];
+        out[S::kOffW1 + row * kMlpIn + 2 * t + 1] = dw1[m][2 * h + 1];
       }
     }
-    __syncwarp();
-    for (int jj = lane; jj < H; jj += 32) {
-      float acc = 0.0f;
-      for (int s2 = 0; s2 < 32; ++s2) {
-        acc += W.a1[s2][jj];
-      }
-      atomicAdd(&B.grad[S::kOffB1 + jj], acc);
-    }
-    // 8. dW1 = dL/da1^T x: [H i x 32 s] x [32 s x 8 f]
-    for (int mt = 0; mt < KT; ++mt) {
-      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  }
 #pragma unroll
-      for (int kk = 0; kk < 2; ++kk) {
-        uint32_t a[4];
-        a[0] = ld32(&W.d1t[16 * mt + g][16 * kk + 2 * t]);
-        a[1] = ld32(&W.d1t[16 * mt + g + 8][16 * kk + 2 * t]);
-        a[2] = ld32(&W.d1t[16 * mt + g][16 * kk + 2 * t + 8]);
-        a[3] = ld32(&W.d1t[16 * mt + g + 8][16 * kk + 2 * t + 8]);
-        mma_bf16(acc, a, ld32(&W.xt[g][16 * kk + 2 * t]), ld32(&W.xt[g][16 * kk + 2 * t + 8]));
+  for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      float s3 = dw3[nt][q], s2 = db2[nt][q], s1 = db1[nt][q];
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) {
+        s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
       }
-      float *row0 = &B.grad[S::kOffW1 + (16 * mt + g) * kMlpIn + 2 * t];
-      float *row1 = row0 + 8 * kMlpIn;
-      atomicAdd(row0, acc[0]);
-      atomicAdd(row0 + 1, acc[1]);
-      atomicAdd(row1, acc[2]);
-      atomicAdd(row1 + 1, acc[3]);
+      if (g == 0) {
+        const int col = nt * 8 + 2 * t + q;
+        B.unit[warp][0][col] = s3;
+        B.unit[warp][1][col] = s2;
+        B.unit[warp][2][col] = s1;
+      }
     }
-    __syncwarp();
+  }
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {  // the quads' first lanes
+    db3 += __shfl_xor_sync(0xffffffffu, db3, o);
+    loss_sum += __shfl_xor_sync(0xffffffffu, loss_sum, o);
+  }
+  if (lane == 0) {
+    B.b3[warp] = db3;
+    atomicAdd(loss, loss_sum);
   }
   __syncthreads();
-  float *out = grad_partials + (int64_t)blockIdx.x * S::kParams;
-  for (int i = threadIdx.x; i < S::kParams; i += blockDim.x) {
-    out[i] = B.grad[i];
+  for (int i = threadIdx.x; i < 3 * H + 1; i += blockDim.x) {
+    float sum = 0.0f;
+    for (int w = 0; w < kTrainWarps; ++w) {
+      sum += i < 3 * H ? B.unit[w][i / H][i % H] : B.b3[w];
+    }
+    const int to = i < H ? S::kOffW3 + i : (i < 2 * H ? S::kOffB2 + i - H : (i < 3 * H ? S::kOffB1 + i - 2 * H : S::kOffB3));
+    out[to] = sum;
+  }
+}
+
+// A parameter's partials, one of kSumSlices threads per slice of the blocks: the sum is in the first
+// slice's thread. 32 parameters per block of threads, so that a warp reads consecutive ones.
+constexpr int kSumSlices = 8;
+
+template <class T, int kParams>
+__device__ __forceinline__ T sum_partials(const float *grad_partials, int blocks, int i, T (*part)[32])
+{
+  const int slice = threadIdx.x / 32, at = threadIdx.x % 32;
+  T sum = 0;
+  if (i < kParams) {
+#pragma unroll 16
+    for (int b = slice; b < blocks; b += kSumSlices) {
+      sum += grad_partials[(int64_t)b * kParams + i];
+    }
+  }
+  part[slice][at] = sum;
+  __syncthreads();
+  if (slice == 0) {
+    for (int s = 1; s < kSumSlices; ++s) {
+      sum += part[s][at];
+    }
+  }
+  return sum;
+}
+
+template <int H>
+__global__ void __launch_bounds__(32 * kSumSlices) k_mlp_gradient_sum(const float *grad_partials, int blocks, float *grad)
+{
+  __shared__ double part[kSumSlices][32];
+  const int i = blockIdx.x * 32 + threadIdx.x % 32;
+  const double sum = sum_partials<double, MlpShape<H>::kParams>(grad_partials, blocks, i, part);
+  if (threadIdx.x < 32 && i < MlpShape<H>::kParams) {
+    grad[i] = (float)sum;
   }
 }
 
 // ---- Adam ----
 
+// One step on the sum of the partials (32 parameters per block; 4 us, 6 with a thread per parameter
+// that adds up all partials).
 template <int H>
-__global__ void k_mlp_adam(float *master, const float *grad_partials, int blocks, float *m, float *v, float lr, float beta1,
-                           float beta2, float eps, float weight_decay, float bias1, float bias2, MlpDeviceT<H> *model)
+__global__ void __launch_bounds__(32 * kSumSlices) k_mlp_adam(float *master, const float *grad_partials, int blocks, float *m, float *v,
+                                                              float lr, float beta1, float beta2, float eps, float weight_decay,
+                                                              float bias1, float bias2, MlpDeviceT<H> *model)
 {
   using S = MlpShape<H>;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= S::kParams) {
+  __shared__ float part[kSumSlices][32];
+  const int i = blockIdx.x * 32 + threadIdx.x % 32;
+  const bool own = threadIdx.x < 32 && i < S::kParams;
+  float m0 = 0.0f, v0 = 0.0f, w = 0.0f;  // under way with the partials
+  if (own) {
+    m0 = m[i];
+    v0 = v[i];
+    w = master[i];
+  }
+  const float gsum = sum_partials<float, S::kParams>(grad_partials, blocks, i, part);
+  if (!own) {
     return;
   }
-  float gsum = 0.0f;
-  for (int b = 0; b < blocks; ++b) {
-    gsum += grad_partials[(int64_t)b * S::kParams + i];
-  }
-  const float mm = beta1 * m[i] + (1.0f - beta1) * gsum;
-  const float vv = beta2 * v[i] + (1.0f - beta2) * gsum * gsum;
+  const float mm = beta1 * m0 + (1.0f - beta1) * gsum;
+  const float vv = beta2 * v0 + (1.0f - beta2) * gsum * gsum;
   m[i] = mm;
   v[i] = vv;
-  float w = master[i];
   const bool is_weight = i < S::kOffB1 || (i >= S::kOffW2 && i < S::kOffB2) || (i >= S::kOffW3 && i < S::kOffB3);
   if (is_weight) {
     w -= lr * weight_decay * w;
@@ -500,8 +582,7 @@ __global__ void k_mlp_adam(float *master, const float *grad_partials, int blocks
 
 int gradient_blocks(int32_t batch)
 {
-  const int64_t tiles = ((int64_t)batch + 31) / 32;
-  const int64_t blocks = (tiles + kTrainWarps - 1) / kTrainWarps;
+  const int64_t blocks = ((int64_t)batch + kTrainSamples - 1) / kTrainSamples;
   return (int)(blocks < kMaxGradBlocks ? (blocks > 0 ? blocks : 1) : kMaxGradBlocks);
 }
 
@@ -526,8 +607,7 @@ template <int H, bool kRelu>
 void gradient_net(const MlpDeviceT<H> *model, const float *features, const uint8_t *labels, int64_t n, int32_t batch, bool sequential,
                   uint64_t seed, int64_t step, float pos_weight, float *grad_partials, float *loss, cudaStream_t stream)
 {
-  // per device and cheap: set before every launch (training runs outside graph capture)
-  cudaFuncSetAttribute(k_mlp_gradient<H, kRelu>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainBlock<H>));
+  static_assert(sizeof(TrainBlock<H>) <= 48 * 1024, "within the default limit");
   k_mlp_gradient<H, kRelu><<<gradient_blocks(batch), kTrainWarps * 32, sizeof(TrainBlock<H>), stream>>>(
       model, features, labels, n, batch, sequential ? 1 : 0, seed, step, pos_weight, grad_partials, loss);
 }
@@ -540,7 +620,15 @@ static_assert(sizeof(itsu_gate_model) == sizeof(float) * (kGateParams + 2 * kMlp
 size_t mlp_device_bytes() { return sizeof(MlpDevice); }
 size_t gate_device_bytes() { return sizeof(GateDevice); }
 int mlp_gradient_blocks(int32_t batch) { return gradient_blocks(batch); }
-int mlp_max_gradient_blocks() { return kMaxGradBlocks; }
+
+void launch_mlp_gradient_sum(const float *grad_partials, int blocks, int params, float *grad, cudaStream_t stream)
+{
+  if (params == kMlpParams) {
+    k_mlp_gradient_sum<kMlpHidden><<<(kMlpParams + 31) / 32, 32 * kSumSlices, 0, stream>>>(grad_partials, blocks, grad);
+  } else {
+    k_mlp_gradient_sum<kGateHidden><<<(kGateParams + 31) / 32, 32 * kSumSlices, 0, stream>>>(grad_partials, blocks, grad);
+  }
+}
 
 void launch_mlp_publish(const itsu_prefilter_model *master, MlpDevice *model, cudaStream_t stream)
 {
@@ -595,15 +683,15 @@ void launch_mlp_adam(itsu_prefilter_model *master, const float *grad_partials, i
                      float beta1, float beta2, float eps, float weight_decay, float bias1, float bias2, MlpDevice *model,
                      cudaStream_t stream)
 {
-  k_mlp_adam<kMlpHidden><<<(kMlpParams + 255) / 256, 256, 0, stream>>>(&master->w1[0][0], grad_partials, blocks, m, v, lr,
-                                                                       beta1, beta2, eps, weight_decay, bias1, bias2, model);
+  k_mlp_adam<kMlpHidden><<<(kMlpParams + 31) / 32, 32 * kSumSlices, 0, stream>>>(&master->w1[0][0], grad_partials, blocks, m, v, lr,
+                                                                                 beta1, beta2, eps, weight_decay, bias1, bias2, model);
 }
 
 void launch_mlp_adam(itsu_gate_model *master, const float *grad_partials, int blocks, float *m, float *v, float lr, float beta1,
                      float beta2, float eps, float weight_decay, float bias1, float bias2, GateDevice *model, cudaStream_t stream)
 {
-  k_mlp_adam<kGateHidden><<<(kGateParams + 255) / 256, 256, 0, stream>>>(&master->w1[0][0], grad_partials, blocks, m, v, lr,
-                                                                         beta1, beta2, eps, weight_decay, bias1, bias2, model);
+  k_mlp_adam<kGateHidden><<<(kGateParams + 31) / 32, 32 * kSumSlices, 0, stream>>>(&master->w1[0][0], grad_partials, blocks, m, v, lr,
+                                                                                   beta1, beta2, eps, weight_decay, bias1, bias2, model);
 }
 
 }  // namespace itsu
