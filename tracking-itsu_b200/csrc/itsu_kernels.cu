@@ -1584,16 +1584,14 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
 // gave the DCA feature) keeps the same cells as scoring every candidate first. A NaN logit keeps its
 // cell. The pairs of a tracklet with more than kMaxMaskedOut outgoing tracklets are kept unscored.
 // A warp takes consecutive spans and flattens their entries over its lanes, so that the network's
-// tiles are full.
-constexpr int kPrefilterThreads = 256;
+// tiles are full: about three times in all, the same number for every warp (one wave of blocks, 24
+// warps per SM). Bound by the network's activations: 0.154 ms per 32 central events; 0.175 in blocks
+// of 256 threads with 2^13 turns shared out unevenly.
+constexpr int kPrefilterThreads = 128;
+constexpr int kPrefilterBlocks = 6;  // resident blocks per SM, by registers
+constexpr int kPrefilterTurns = 3;
 
-// Spans a warp of a pass over the entries takes at a time (a span of 128 has 15 entries in central
-// events, 85 behind the tracklet gate): about `turns` of them for all warps of the grid. The prefilter
-// wants full tiles (2^13 turns), the write pass many stores in flight (2^16: 0.16 ms per 128 central
-// events, 0.18 at 2^13).
-__device__ __forceinline__ int spans_at_a_time(int64_t spans, int64_t turns) { return (int)min((int64_t)32, max((int64_t)1, spans / turns)); }
-
-__global__ void __launch_bounds__(kPrefilterThreads) k_cells_prefilter(Arena a)
+__global__ void __launch_bounds__(kPrefilterThreads, kPrefilterBlocks) k_cells_prefilter(Arena a)
 {
   __shared__ MlpSmem mlp;
   __shared__ __align__(16) __nv_bfloat16 rows[kPrefilterThreads / 32][32][kRowPitch];
@@ -1604,7 +1602,8 @@ __global__ void __launch_bounds__(kPrefilterThreads) k_cells_prefilter(Arena a)
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t spans = a.status->cell_spans;
-  const int take = spans_at_a_time(spans, 1 << 13);
+  const int64_t turns = (int64_t)gridDim.x * (kPrefilterThreads / 32) * kPrefilterTurns;
+  const int take = (int)min((int64_t)32, (spans + turns - 1) / turns);  // spans at a time
   for (int64_t s0 = ((int64_t)blockIdx.x * (kPrefilterThreads / 32) + warp) * take; s0 < spans;
        s0 += (int64_t)gridDim.x * (kPrefilterThreads / 32) * take) {
     const int2 in = lane < take && s0 + lane < spans ? a.cell_span[s0 + lane] : make_int2(0, 0);  // first entry, entries
@@ -1651,11 +1650,14 @@ __global__ void __launch_bounds__(kPrefilterThreads) k_cells_prefilter(Arena a)
   }
 }
 
-// Write pass: a warp takes consecutive spans and flattens their entries over its lanes; in order, they go to the spans' scanned places, which
-// are contiguous (a dropped entry leaves no gap). The first cell of each first tracklet fills its
-// cells lookup entry, and each cell's state of the stages after is reset (the neighbour scan's tile
-// sums too).
+// Write pass: a warp takes consecutive spans (a span of 128 has 15 entries in central events, 85 behind
+// the tracklet gate) and flattens their entries over its lanes; in order, they go to the spans' scanned
+// places, which are contiguous (a dropped entry leaves no gap). The first cell of each first tracklet
+// fills its cells lookup entry, and each cell's state of the stages after is reset (the neighbour
+// scan's tile sums too). Many turns keep many stores in flight (0.18 ms per 128 central events; with
+// 2^13 turns 0.20; with the next turn's entries prefetched 0.20).
 constexpr int kScatterThreads = 256;
+constexpr int64_t kScatterTurns = 1 << 16;
 
 // A cell's CA level and its number of level-decreasing chains down to layer 0, in one word
 // (chains << 3 | level; levels are 1..5 and chain counts are capped at INT_MAX), of layers 1 to 4; the
@@ -1686,7 +1688,7 @@ __global__ void __launch_bounds__(kScatterThreads) k_cells_scatter(Arena a)
   zero_tiles(a.scan_partials, a.status->total[kCells]);
   const int lane = threadIdx.x & 31;
   const int64_t spans = a.status->cell_spans;
-  const int take = spans_at_a_time(spans, 1 << 16);
+  const int take = (int)min((int64_t)32, max((int64_t)1, spans / kScatterTurns));  // spans at a time
   for (int64_t s0 = ((int64_t)blockIdx.x * (kScatterThreads / 32) + (threadIdx.x >> 5)) * take; s0 < spans;
        s0 += (int64_t)gridDim.x * (kScatterThreads / 32) * take) {
     const int2 in = lane < take && s0 + lane < spans ? a.cell_span[s0 + lane] : make_int2(0, 0);  // first entry, entries
@@ -2278,7 +2280,7 @@ void step_write_count_groups(const Arena &a, const Launch &l)
 void step_cells_prefilter(const Arena &a, const Launch &l)
 {
   if (a.mlp) {
-    k_cells_prefilter<<<l.num_sms * 3, kPrefilterThreads, 0, l.stream>>>(a);  // one wave (3 blocks per SM by registers)
+    k_cells_prefilter<<<l.num_sms * kPrefilterBlocks, kPrefilterThreads, 0, l.stream>>>(a);
   }
 }
 
