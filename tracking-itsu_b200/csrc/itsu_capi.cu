@@ -5,8 +5,8 @@
 // findTracks / computeMontecarloLabels) and are synchronous like the reference GPU backend
 // (src/CA/gpu/cuda/Tracker.cu synchronises after every stage). Each stage counts, scans, and
 // sizes its outputs exactly before writing them (two-pass sizing). The whole-path and batch
-// entry points enqueue every stage back to back without host round trips (replayed as a CUDA
-// graph), then check the device status once; an output that overflowed the arena is grown to the
+// entry points enqueue every stage back to back without host round trips (as one CUDA graph from
+// a run's third repetition on), then check the device status once; an output that overflowed the arena is grown to the
 // reported requirement and the run repeated.
 #include <cuda_runtime.h>
 
@@ -699,6 +699,10 @@ RunKey run_key(const itsu_context *ctx)
 itsu_status launch_all(itsu_context *ctx)
 {
   constexpr int kRunsBeforeGraph = 2;
+  // a graph of the library's own can be neither made nor launched there, so no run is taken
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  ITSU_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone) return fail(ctx, ITSU_ERR_CUDA, "the context's stream is being captured");
   const RunKey key = run_key(ctx);
   if (!(ctx->graph && key == ctx->graph_key)) {
     ctx->last_key_runs = key == ctx->last_key ? ctx->last_key_runs + 1 : 1;
