@@ -231,8 +231,8 @@ itsu_status itsu_batch_run_host_compact(itsu_context *ctx, const itsu_cluster_in
 itsu_status itsu_batch_run_host_tracks(itsu_context *ctx, const itsu_cluster_track *clusters, const int32_t *layer_offsets,
                                        const float *vertices, int32_t n_events, itsu_road *roads, int64_t roads_capacity,
                                        int32_t *road_offsets);
-/* Launches every stage of the batch on the context stream without waiting (CUDA-graph
- * replay after the first call with the same shape); itsu_batch_status waits and reports. */
+/* Launches every stage of the batch on the context stream without waiting (a CUDA-graph
+ * replay from the third call in a row with the same inputs on); itsu_batch_status waits and reports. */
 itsu_status itsu_batch_launch(itsu_context *ctx, const itsu_batch *batch);
 itsu_status itsu_batch_status(itsu_context *ctx);
 /* Device pointer to the roads of the last batch (event-major) and to road_offsets[n_events+1]. */
@@ -302,7 +302,7 @@ itsu_status itsu_roads_report(itsu_context *ctx, const itsu_road *roads, const i
  * Runs are grouped in multiplicity bands: band = floor(log2(mean clusters per event)). For the
  * band of the last run, itsu_autotune times every candidate launch shape (threads per block of
  * the per-item kernels 64/128/256/512, resident blocks per SM of the grid-stride kernels 4/8/16,
- * the tracklet candidate index off/on/staged, event groups of 0/8/16/32 events) on the inputs
+ * tracklet candidate pruning off/on, event groups of 0/8/16/32 events) on the inputs
  * already resident, `repeats` times each, and
  * keeps the fastest for that band; later runs in the band use it. Results never depend on the
  * launch shape. itsu_get_tune / itsu_set_tune read and restore a band's entry (to persist a

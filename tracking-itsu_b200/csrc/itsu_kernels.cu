@@ -3,12 +3,12 @@
 // Every stage is a deterministic count -> exclusive scan -> write sequence over flat,
 // event-major arrays, so the output order is the reference's emission order (where a count pass
 // uses atomics, to reserve scratch or fill neighbour rows, the write pass restores the order):
-//   clustering   one CTA per (event, layer): vertex-relative transform, stable counting sort by
-//                bin (per-warp histograms, warp-match ranks), index table, z-sorted bin lists
-//                for the tracklet pruning (PVC.cxx:31-142)
-//   tracklets    count: one thread per inner cluster walking the reference's bin window,
-//                z-pruned (Tracker.cxx:45-117); tail: lookup, owners, crowded clusters; write:
-//                a map over tracklets (slope and correctly rounded azimuth)
+//   clustering   a CTA or a cluster of CTAs per (event, layer): vertex-relative transform, stable
+//                counting sort by bin (per-warp histograms, warp-match ranks), index table, a
+//                4-byte key per cluster for the tracklet pruning (PVC.cxx:31-142)
+//   tracklets    count: one thread per inner cluster walking the reference's bin window through a
+//                fixed-point window on the keys (Tracker.cxx:45-117); write: a map over tracklets
+//                (slope and correctly rounded azimuth), with the lookup table
 //   cells        count: the tracklet pairs inside a fixed-point window queued, then the exact cuts
 //                and the geometry, a lane per queued pair, one 40-byte entry per found cell
 //                (Tracker.cxx:120-235); learned form: the prefilter scores the entries; write: the
@@ -16,8 +16,8 @@
 //   neighbours   one thread per cell walking the next-layer cells of its outer tracklet; rows
 //                keyed by the next-layer cell, sorted ascending (Tracker.cxx:417-474)
 //   levels       layer-ordered longest-chain DP plus the number of level-decreasing chains
-//   roads        one thread per level-5 cell: depth-first enumeration in the reference's order,
-//                Moore-vote labels (Tracker.cxx:477-652)
+//   roads        one lane per road: the root's k-th chain in the reference's order, Moore-vote
+//                labels (Tracker.cxx:477-652)
 // Capacity overflow never writes out of bounds: the passes check the scanned totals and scratch
 // reservations against the arena capacities, record the requirement and skip; the host grows
 // and re-runs.
