@@ -137,6 +137,7 @@ struct itsu_context {
           *road_off = nullptr;
   int64_t *paths = nullptr;
   unsigned long long *nb_mask = nullptr;  // per cell, its passing candidates (neighbour count pass)
+  int32_t *nb_first = nullptr;
   // neighbour and road classes
   int32_t *nb = nullptr;
   itsu_road *roads = nullptr;
@@ -402,6 +403,7 @@ Arena arena_of(const itsu_context *ctx)
   a.nb_count = ctx->nb_count;
   a.nb_off = ctx->nb_off;
   a.nb_mask = ctx->nb_mask;
+  a.nb_first = ctx->nb_first;
   a.nb = ctx->nb;
   a.paths = ctx->paths;
   a.road_count = ctx->road_count;
@@ -544,6 +546,7 @@ itsu_status ensure_cell_outputs(itsu_context *ctx, int64_t need)
     ITSU_CUDA(ctx, alloc(ctx, ctx->nb_count, cap + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->nb_off, cap + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->nb_mask, cap));
+    ITSU_CUDA(ctx, alloc(ctx, ctx->nb_first, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->paths, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->road_count, cap + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->road_off, cap + 1));
@@ -1080,7 +1083,7 @@ void itsu_context_destroy(itsu_context *ctx)
   release(ctx->road_seg); release(ctx->vtx);
   release(ctx->tracklets); release(ctx->trk_key); release(ctx->trk_seg32); release(ctx->cell_span); release(ctx->cell_span_count); release(ctx->cell_span_off); release(ctx->cell_lookup);
   release(ctx->cells); release(ctx->cell_entries); release(ctx->cell_dca); release(ctx->cell_seg_id); release(ctx->nb_count); release(ctx->nb_off);
-  release(ctx->nb_mask);
+  release(ctx->nb_mask); release(ctx->nb_first);
   release(ctx->road_count); release(ctx->road_off); release(ctx->paths);
   release(ctx->nb); release(ctx->roads); release(ctx->scan_partials); release(ctx->d_status);
   release(ctx->d_master); release(ctx->d_mlp);

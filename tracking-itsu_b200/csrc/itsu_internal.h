@@ -131,6 +131,7 @@ struct Arena {
   int32_t *nb_count;
   int32_t *nb_off;
   unsigned long long *nb_mask;  // per cell of layers 0-3: its candidates that pass the cut (up to 64)
+  int32_t *nb_first;  // and the first candidate
   int32_t *nb;
   int64_t *paths;  // per cell: its chain count and level (chain_word)
   int32_t *road_count;

@@ -1789,12 +1789,6 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbour_reset(Arena a)
   }
 }
 
-// Tracker.cxx:416-474 (findCellsNeighbours): a cell of layer L and the cells of layer L + 1 built
-// on its second tracklet (from its cells lookup entry on, as long as they are built on it). The
-// count pass evaluates the cut, counts each passing pair in its row and keeps the passing candidates
-// as a mask (of up to kMaskedRun candidates; a longer run is marked in the top bit); the write pass,
-// after the scan of the counts, fills the rows from the mask (re-evaluating the cut only for the
-// marked cells), counting the counts down to zero. Row order is restored by k_levels' sort.
 // Adds count to the tile sum of item `at`: one atomic for the lanes that are here together and whose
 // items lie in one tile.
 __device__ __forceinline__ void add_to_tile(int64_t *partials, int64_t at, int count)
@@ -1807,6 +1801,14 @@ __device__ __forceinline__ void add_to_tile(int64_t *partials, int64_t at, int c
   }
 }
 
+// Tracker.cxx:416-474 (findCellsNeighbours): a cell of layer L and the cells of layer L + 1 built
+// on its second tracklet (from its cells lookup entry on, as long as they are built on it). The
+// count pass evaluates the cut, counts each passing pair in its row and keeps the first candidate and
+// the passing ones as a mask (of up to kMaskedRun candidates; a longer run is marked in the top bit);
+// the write pass, after the scan of the counts, fills the rows from these (re-evaluating the cut only
+// for the marked cells), counting the counts down to zero. Row order is restored by k_levels' sort.
+// Bound by the latency of the gathers: 0.118 and 0.065 ms per 128 central events; the write pass took
+// 0.095 when it looked the first candidate up again through the cell's record.
 constexpr int kMaskedRun = 63;
 constexpr unsigned long long kLongRun = 1ull << kMaskedRun;
 
@@ -1826,22 +1828,23 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbours(Arena a)
     if (layer >= ITSU_NEIGHBOUR_LAYERS) {
       continue;
     }
-    unsigned long long mask = 0ull;
-    if (kWrite && (mask = a.nb_mask[c]) == 0ull) {
-      continue;
+    const int32_t c_local = (int32_t)(c - a.cell_seg[sid]);
+    if (kWrite) {
+      unsigned long long mask = a.nb_mask[c];
+      const int32_t j0 = a.nb_first[c];
+      if (!(mask & kLongRun)) {
+        for (; mask; mask &= mask - 1ull) {
+          const int32_t j = j0 + __ffsll((long long)mask) - 1;
+          const int slot = atomicSub(&a.nb_count[j], 1) - 1;
+          a.nb[a.nb_off[j] + slot] = c_local;
+        }
+        continue;
+      }
     }
+    unsigned long long mask = 0ull;
     const int32_t second = a.cells[c].second_tracklet;
     const int32_t found = a.cell_lookup[a.trk_seg[e * ITSU_TRACKLET_LAYERS + layer + 1] + second];
     const int32_t j0 = a.cell_seg[sid + 1] + found, j1 = found < 0 ? j0 : a.cell_seg[sid + 2];
-    const int32_t c_local = (int32_t)(c - a.cell_seg[sid]);
-    if (kWrite && !(mask & kLongRun)) {
-      for (; mask; mask &= mask - 1ull) {
-        const int32_t j = j0 + __ffsll((long long)mask) - 1;
-        const int slot = atomicSub(&a.nb_count[j], 1) - 1;
-        a.nb[a.nb_off[j] + slot] = c_local;
-      }
-      continue;
-    }
     const itsu_cell cell = a.cells[c];
     const float3 n1 = make_float3(cell.nx, cell.ny, cell.nz);
     int links = 0;  // to cells of j0's scan tile
@@ -1874,6 +1877,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbours(Arena a)
     }
     if (!kWrite) {
       a.nb_mask[c] = mask;
+      a.nb_first[c] = j0;
       if (links > 0) {
         add_to_tile(a.scan_partials, j0, links);
       }
