@@ -130,6 +130,27 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T *warp_totals, T &block_
   return res;
 }
 
+// The sum of v over the lanes of mask, in 64 bits: counts go up to INT_MAX each (chains of cells, outer
+// clusters in one window), so a warp's sum can pass 2^32. Two 32-bit reductions, of the low and the high
+// halves, whose sums stay below 2^21.
+__device__ __forceinline__ unsigned long long warp_sum(unsigned mask, unsigned v)
+{
+  const unsigned long long low = __reduce_add_sync(mask, v & 0xffffu), high = __reduce_add_sync(mask, v >> 16);
+  return low + (high << 16);
+}
+
+// Adds count (not negative) to the tile sum of item `at`: one atomic for the lanes that are here together
+// and whose items lie in one tile.
+__device__ __forceinline__ void add_to_tile(int64_t *partials, int64_t at, int count)
+{
+  const unsigned tile = (unsigned)(at / kScanTile);
+  const unsigned peers = __match_any_sync(__activemask(), tile);
+  const unsigned long long sum = warp_sum(peers, (unsigned)count);
+  if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) {
+    atomicAdd(reinterpret_cast<unsigned long long *>(&partials[tile]), sum);
+  }
+}
+
 // One kernel per scan: the count passes have added each tile's counts up (partials), and a block
 // sums the tile sums before its tiles itself (at most a few thousand of them, from L2) instead of
 // taking them from a kernel of its own. The last tile's block checks the total. own_flag: the
@@ -938,9 +959,9 @@ __global__ void __launch_bounds__(kCountThreads, kGate ? 5 : 6) k_tracklets_coun
     });
   }
   // the warp's 32 clusters lie in one scan tile: their tracklets go to its sum
-  const int warp_count = (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
+  const unsigned long long warp_count = warp_sum(0xffffffffu, (unsigned)count);
   if ((threadIdx.x & 31) == 0 && warp_count != 0) {
-    atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[i / kScanTile]), (unsigned long long)warp_count);
+    atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[i / kScanTile]), warp_count);
   }
   if (!valid) {
     return;
@@ -1786,18 +1807,6 @@ __global__ void __launch_bounds__(kMaxThreads) k_neighbour_reset(Arena a)
   const int64_t n = a.status->total[kCells];
   for (int64_t c = global_thread(); c < n; c += grid_threads()) {
     reset_cell(a, c);
-  }
-}
-
-// Adds count to the tile sum of item `at`: one atomic for the lanes that are here together and whose
-// items lie in one tile.
-__device__ __forceinline__ void add_to_tile(int64_t *partials, int64_t at, int count)
-{
-  const unsigned tile = (unsigned)(at / kScanTile);
-  const unsigned peers = __match_any_sync(__activemask(), tile);
-  count = (int)__reduce_add_sync(peers, (unsigned)count);
-  if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) {
-    atomicAdd(reinterpret_cast<unsigned long long *>(&partials[tile]), (unsigned long long)count);
   }
 }
 
