@@ -127,7 +127,7 @@ struct itsu_context {
   itsu_tracklet *tracklets = nullptr;
   uint32_t *trk_key = nullptr;  // (tanL, phi) of each tracklet in fixed point, beside the records
   int32_t *trk_seg32 = nullptr, *cell_lookup = nullptr, *cell_span_count = nullptr, *cell_span_off = nullptr;
-  int2 *cell_span = nullptr;
+  uint2 *cell_span = nullptr;
   // cell class
   itsu_cell *cells = nullptr;
   itsu::CellEntry *cell_entries = nullptr;
@@ -525,7 +525,10 @@ itsu_status ensure_cell_entries(itsu_context *ctx, int64_t need)
   if (need > ctx->cap_cell_entries) {
     itsu_status st = growth_allowed(ctx, "cell entries", need, ctx->cap_cell_entries);
     if (st != ITSU_OK) return st;
-    const int64_t cap = grow_to(need);
+    if (need > itsu::kMaxCellEntries) {
+      return fail(ctx, ITSU_ERR_CAPACITY, "cell entries: %lld needed, %lld can be indexed", (long long)need, (long long)itsu::kMaxCellEntries);
+    }
+    const int64_t cap = std::min(grow_to(need), itsu::kMaxCellEntries);
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_entries, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_dca, cap));
     ctx->cap_cell_entries = cap;

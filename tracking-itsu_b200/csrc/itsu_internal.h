@@ -70,6 +70,9 @@ struct __align__(8) CellEntry {
   int32_t segment;
 };
 static_assert(sizeof(CellEntry) == 40 && sizeof(CellEntry) == sizeof(itsu_cell), "cell entry layout");
+// Entries the scratch may hold: 32 unsigned bits name one (44 bytes each, 189 GB), with room for a
+// warp's last 32 when the later passes count through them.
+constexpr int64_t kMaxCellEntries = 0xffffffffll - 63;
 constexpr int32_t kEntryUnscored = 1 << 30;  // flag on segment: the prefilter keeps the entry as it is
 constexpr int32_t kEntryDropped = -1;        // in place of segment: not a cell
 
@@ -117,7 +120,7 @@ struct Arena {
   int4 *cell_seginfo;  // per tracklet segment, two records: {first cluster of L (-1: no cells), of L+1, of L+2,
                        // first tracklet of L}, {first tracklet of L+1, vertex x, y, z (float bits)}
   // cells
-  int2 *cell_span;  // per span of first tracklets: its first cell entry and their number
+  uint2 *cell_span;  // per span of first tracklets: its first cell entry and their number
   int32_t *cell_span_count, *cell_span_off;  // per span: its cells (entries the prefilter kept), and their scan
   int32_t *cell_seg_count;    // per segment: its cells
   int32_t *cell_lookup;

@@ -975,13 +975,14 @@ __global__ void __launch_bounds__(kCountThreads, kGate ? 5 : 6) k_tracklets_coun
   }
 }
 
-__device__ __forceinline__ int warp_exclusive_sum(int v, int &total)
+template <typename T>
+__device__ __forceinline__ T warp_exclusive_sum(T v, T &total)
 {
   const int lane = threadIdx.x & 31;
-  int inc = v;
+  T inc = v;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, inc, d);
+    const T t = __shfl_up_sync(0xffffffffu, inc, d);
     if (lane >= d) {
       inc += t;
     }
@@ -992,12 +993,13 @@ __device__ __forceinline__ int warp_exclusive_sum(int v, int &total)
 
 // Owner lane of flattened item t given the lanes' exclusive prefix sums: the last lane whose
 // prefix is <= t (for t < total this lane holds item t). All lanes must call it together.
-__device__ __forceinline__ int owner_of(int excl, int t)
+template <typename T>
+__device__ __forceinline__ int owner_of(T excl, T t)
 {
   int owner = 0;
 #pragma unroll
   for (int step = 16; step > 0; step >>= 1) {
-    const int v = __shfl_sync(0xffffffffu, excl, owner + step);
+    const T v = __shfl_sync(0xffffffffu, excl, owner + step);
     if (v <= t) {
       owner += step;
     }
@@ -1367,7 +1369,7 @@ struct CellWarp {
   int2 state[kMaxSpan];        // first outgoing tracklet; segment (kCrowded: more than kMaxMaskedOut outgoing tracklets)
   union {
     uint16_t queue[kCellQueue];  // (first tracklet in the span) | (outgoing tracklet) << 7
-    uint32_t ring[kCellRing];    // the same, for any number of outgoing tracklets
+    uint2 ring[kCellRing];       // the same two, for any number of outgoing tracklets
   };
 };
 constexpr int kCrowded = 1 << 30;
@@ -1462,7 +1464,8 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
     }
     const uint32_t base = s * span;
     int total = 0;
-    bool queued = true;  // the span's pairs are all in the queue
+    unsigned long long many = 0;  // pairs behind crowded outer clusters, beside total (their sum can pass 2^32)
+    bool queued = true;           // the span's pairs are all in the queue
     for (uint32_t g = 0; g < span; g += 32) {
       const uint32_t at = g + lane, k = base + at;
       CellLane p;
@@ -1475,9 +1478,10 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
       w.state[at] = make_int2(p.j0, crowded ? p.sid | kCrowded : p.sid);
       unsigned long long mask = 0ull;
       int count = 0;
+      unsigned behind = 0;
       if (crowded) {
         for (int q = 0; q < p.n_out; ++q) {
-          count += key_window_pass(p.w.keys, a.trk_key[p.j0 + q]);
+          behind += key_window_pass(p.w.keys, a.trk_key[p.j0 + q]);
         }
       } else if (p.n_out > 0) {
         mask = cell_precut_mask(a, p);
@@ -1486,7 +1490,11 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
       int group_total;
       int to = total + warp_exclusive_sum(count, group_total);
       total += group_total;
-      queued = queued && total <= kCellQueue && !__any_sync(0xffffffffu, crowded);
+      queued = queued && total <= kCellQueue;
+      if (__any_sync(0xffffffffu, crowded)) {
+        many += warp_sum(0xffffffffu, behind);
+        queued = false;
+      }
       if (queued) {
         for (unsigned m = (unsigned)mask; m != 0; m &= m - 1u) {
           w.queue[to++] = (uint16_t)(at | (uint32_t)(__ffs(m) - 1) << 7);
@@ -1496,22 +1504,23 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
         }
       }
     }
-    int cells = 0;
+    unsigned cells = 0;
     unsigned long long first = 0;
-    if (total > 0) {
+    const unsigned long long pairs = many + (unsigned)total;
+    if (pairs > 0) {
       if (lane == 0) {
-        first = atomicAdd(reinterpret_cast<unsigned long long *>(&a.status->cell_entries), (unsigned long long)total);
-        if ((int64_t)first + total > a.cap_cell_entries) {
+        first = atomicAdd(reinterpret_cast<unsigned long long *>(&a.status->cell_entries), pairs);
+        if (first + pairs > (unsigned long long)a.cap_cell_entries) {
           atomicOr(&a.status->flags, kFlagCapScratch);  // nothing after this pass runs
         }
       }
       first = __shfl_sync(0xffffffffu, first, 0);
     }
-    if (total > 0 && (int64_t)first + total <= a.cap_cell_entries) {
+    if (pairs > 0 && first + pairs <= (unsigned long long)a.cap_cell_entries) {
       __syncwarp();
-      int head = 0, tail = queued ? total : 0;
+      unsigned head = 0, tail = queued ? total : 0;
       uint32_t next = queued ? span : 0;  // not queued (a crowded outer cluster, or more pairs than the queue holds):
-      int next_out = 0;                   // the first tracklets' keys are walked again, 32 of one tracklet at a time
+      uint32_t next_out = 0;              // the first tracklets' keys are walked again, 32 of one tracklet at a time
       for (;;) {
         if (next < span && tail - head < 32) {
           const uint32_t k = base + next;
@@ -1520,22 +1529,22 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
           if (k < n) {
             p = cell_lane(a, k);
           }
-          const int q = next_out + lane;
-          const bool listed = q < p.n_out && key_window_pass(p.w.keys, a.trk_key[p.j0 + q]);
+          const uint32_t q = next_out + lane;
+          const bool listed = q < (uint32_t)p.n_out && key_window_pass(p.w.keys, a.trk_key[p.j0 + q]);
           const unsigned m = __ballot_sync(0xffffffffu, listed);
           if (listed) {
-            w.ring[(tail + __popc(m & ((1u << lane) - 1u))) & (kCellRing - 1)] = next | (uint32_t)q << 7;
+            w.ring[(tail + __popc(m & ((1u << lane) - 1u))) & (kCellRing - 1)] = make_uint2(next, q);
           }
           tail += __popc(m);
           next_out += 32;
-          if (next_out >= p.n_out) {
+          if (next_out >= (uint32_t)p.n_out) {
             next_out = 0;
             ++next;
           }
           __syncwarp();
           continue;
         }
-        const int m = min(tail - head, 32);
+        const unsigned m = min(tail - head, 32u);
         if (m == 0) {
           break;
         }
@@ -1546,13 +1555,20 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
         int4 A, B;
         float3 normal;
         float curvature, dca;
-        if (lane < m) {
-          const uint32_t item = queued ? w.queue[head + lane] : w.ring[(head + lane) & (kCellRing - 1)], at = item & 127u;
+        if (lane < (int)m) {
+          uint2 item;  // place of the first tracklet in the span, and which outgoing tracklet
+          if (queued) {
+            const uint32_t packed = w.queue[head + lane];
+            item = make_uint2(packed & 127u, packed >> 7);
+          } else {
+            item = w.ring[(head + lane) & (kCellRing - 1)];
+          }
+          const uint32_t at = item.x;
           const int2 state = w.state[at];
           crowded = (state.y & kCrowded) != 0;
           sid = state.y & ~kCrowded;
           k = base + at;
-          j = (uint32_t)state.x + (item >> 7);
+          j = (uint32_t)state.x + item.y;
           A = a.cell_seginfo[2 * sid];
           B = a.cell_seginfo[2 * sid + 1];
           f = load_tracklet(a, k);
@@ -1589,14 +1605,26 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
       }
     }
     if (lane == 0) {
-      a.cell_span[s] = make_int2((int)first, cells);
-      a.cell_span_count[s] = cells;
+      a.cell_span[s] = make_uint2((unsigned)first, cells);  // within cap_cell_entries (kMaxCellEntries at most)
+      a.cell_span_count[s] = (int32_t)cells;
+      if (cells > INT_MAX) {
+        atomicOr(&a.status->flags, kFlagCountOverflow);
+      }
       if (cells > 0) {
         atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[s / kScanTile]), (unsigned long long)cells);
       }
     }
     __syncwarp();  // the span's state is refilled next
   }
+}
+
+// The place of the p-th entry of a warp's spans (each lane has one: its first entry and the prefix sum of
+// the lanes' entries before it), and the lane whose span it is of. All lanes call it together. Entries are
+// counted in 32 unsigned bits: the scratch holds kMaxCellEntries of them at most.
+__device__ __forceinline__ int64_t span_entry(unsigned first, unsigned excl, unsigned p, int &owner)
+{
+  owner = owner_of(excl, p);
+  return (int64_t)__shfl_sync(0xffffffffu, first, owner) + p - __shfl_sync(0xffffffffu, excl, owner);
 }
 
 // Learned prefilter: scores the cell entries, 32 per warp on the tensor cores, and drops those whose
@@ -1627,13 +1655,13 @@ __global__ void __launch_bounds__(kPrefilterThreads, kPrefilterBlocks) k_cells_p
   const int take = (int)min((int64_t)32, (spans + turns - 1) / turns);  // spans at a time
   for (int64_t s0 = ((int64_t)blockIdx.x * (kPrefilterThreads / 32) + warp) * take; s0 < spans;
        s0 += (int64_t)gridDim.x * (kPrefilterThreads / 32) * take) {
-    const int2 in = lane < take && s0 + lane < spans ? a.cell_span[s0 + lane] : make_int2(0, 0);  // first entry, entries
-    int total;
-    const int excl = warp_exclusive_sum(in.y, total);
-    for (int p0 = 0; p0 < total; p0 += 32) {
-      const int p = p0 + lane;
-      const int owner = owner_of(excl, p);
-      const int64_t i = (int64_t)__shfl_sync(0xffffffffu, in.x, owner) + p - __shfl_sync(0xffffffffu, excl, owner);
+    const uint2 in = lane < take && s0 + lane < spans ? a.cell_span[s0 + lane] : make_uint2(0, 0);  // first entry, entries
+    unsigned total;
+    const unsigned excl = warp_exclusive_sum(in.y, total);
+    for (unsigned p0 = 0; p0 < total; p0 += 32) {
+      const unsigned p = p0 + lane;
+      int owner;
+      const int64_t i = span_entry(in.x, excl, p, owner);
       int segment = kEntryUnscored;
       int2 h0, h1, h2;
       if (p < total) {
@@ -1712,15 +1740,15 @@ __global__ void __launch_bounds__(kScatterThreads) k_cells_scatter(Arena a)
   const int take = (int)min((int64_t)32, max((int64_t)1, spans / kScatterTurns));  // spans at a time
   for (int64_t s0 = ((int64_t)blockIdx.x * (kScatterThreads / 32) + (threadIdx.x >> 5)) * take; s0 < spans;
        s0 += (int64_t)gridDim.x * (kScatterThreads / 32) * take) {
-    const int2 in = lane < take && s0 + lane < spans ? a.cell_span[s0 + lane] : make_int2(0, 0);  // first entry, entries
-    int total;
-    const int excl = warp_exclusive_sum(in.y, total);
+    const uint2 in = lane < take && s0 + lane < spans ? a.cell_span[s0 + lane] : make_uint2(0, 0);  // first entry, entries
+    unsigned total;
+    const unsigned excl = warp_exclusive_sum(in.y, total);
     int out0 = a.cell_span_off[s0];
     int last_t1 = -1, last_segment = -1;  // of the cell before
-    for (int p0 = 0; p0 < total; p0 += 32) {
-      const int p = p0 + lane;
-      const int owner = owner_of(excl, p);
-      const int64_t i = (int64_t)__shfl_sync(0xffffffffu, in.x, owner) + p - __shfl_sync(0xffffffffu, excl, owner);
+    for (unsigned p0 = 0; p0 < total; p0 += 32) {
+      const unsigned p = p0 + lane;
+      int owner;
+      const int64_t i = span_entry(in.x, excl, p, owner);
       int2 h[5];
       h[1].y = 0;
       h[4].y = kEntryDropped;
