@@ -1,0 +1,57 @@
+"""A fixed arena (ITSU_FLAG_NO_GROW) whose five capacities are exactly what the results need runs them,
+however many tracklet pairs pass the cell stage's precut. Narrow bundles that miss the vertex have up
+to seventy such pairs per tracklet and few cells; their spans take the warp queue, overflow it, or stand
+behind outer clusters with more outgoing tracklets than a mask holds."""
+import numpy as np
+import pytest
+
+from itsu import capi, gen
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _bundle(seed, n, spread):
+    """n clusters on each of layers 0 to 2, on lines that pass 3 mm beside the vertex; one elsewhere."""
+    rng = np.random.default_rng(seed)
+    layers, first = [], 0
+    for layer, r in enumerate(gen.RADII_CM):
+        k = n if layer < 3 else 1
+        phi = 2.0 + np.arcsin(0.3 / r) + rng.uniform(-spread, spread, k)
+        c = np.zeros(k, gen.CLUSTER_DTYPE)
+        c["x"], c["y"], c["z"] = r * np.cos(phi), r * np.sin(phi), 0.3 * r + rng.uniform(-0.02, 0.02, k)
+        c["alpha"], c["mc"], c["id"] = phi, rng.integers(0, 99, k), np.arange(first, first + k)
+        first += k
+        layers.append(c)
+    return gen.Event(vertices=np.zeros((1, 3), np.float32), layers=layers, labels=np.zeros(0, gen.LABEL_DTYPE))
+
+
+@pytest.mark.parametrize("pair_prefilter", [False, True])
+@pytest.mark.parametrize("n, n_events, spread", [(20, 64, 0.002), (60, 8, 0.002), (300, 1, 0.002), (300, 2, 0.01)])
+def test_exact_capacities_suffice(n, n_events, spread, pair_prefilter):
+    events = [_bundle(100 * n + k, n, spread) for k in range(n_events)]
+    clusters, offsets, vertices = gen.pack_batch(events)
+    model = capi.prefilter_init(5)
+    growing = capi.Context()
+    fixed = None
+    try:
+        growing.prefilter_set_model(model)
+        growing.prefilter_enable(pair_prefilter)
+        roads, road_offsets = growing.batch_run_host(clusters, offsets, vertices)
+        want = [growing.results(e) for e in range(n_events)]
+        if not pair_prefilter:
+            for e in (0, n_events - 1):
+                assert oracle.diff(want[e], oracle.run_vertex(events[e].layers, events[e].vertices[0])) == []
+        caps = {"max_" + name: max(int(used), 1) for name, used in growing.memory_usage()["used"].items()}
+        fixed = capi.Context(flags=capi.FLAG_NO_GROW, max_clusters=len(clusters), max_events=n_events, **caps)
+        fixed.prefilter_set_model(model)
+        fixed.prefilter_enable(pair_prefilter)
+        got, got_offsets = fixed.batch_run_host(clusters, offsets, vertices, roads_capacity=caps["max_roads"])
+        assert np.array_equal(got_offsets, road_offsets) and got.tobytes() == roads.tobytes()
+        for e in range(n_events):
+            assert oracle.diff(fixed.results(e), want[e]) == [], e
+        assert oracle.diff(fixed.run_vertex(events[0].layers, events[0].vertices[0]), want[0]) == []
+    finally:
+        growing.close()
+        if fixed is not None:
+            fixed.close()

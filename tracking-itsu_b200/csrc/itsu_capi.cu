@@ -132,7 +132,7 @@ struct itsu_context {
   itsu_cell *cells = nullptr;
   itsu::CellEntry *cell_entries = nullptr;
   float *cell_dca = nullptr;
-  int64_t cap_cell_entries = 0;
+  int64_t cap_cell_pairs = 0, cap_cell_entries = 0;
   int32_t *cell_seg_id = nullptr, *nb_count = nullptr, *nb_off = nullptr, *road_count = nullptr,
           *road_off = nullptr;
   int64_t *paths = nullptr;
@@ -399,6 +399,7 @@ Arena arena_of(const itsu_context *ctx)
   a.cell_seg_id = ctx->cell_seg_id;
   a.cell_entries = ctx->cell_entries;
   a.cell_dca = ctx->cell_dca;
+  a.cap_cell_pairs = ctx->cap_cell_pairs;
   a.cap_cell_entries = ctx->cap_cell_entries;
   a.nb_count = ctx->nb_count;
   a.nb_off = ctx->nb_off;
@@ -510,31 +511,62 @@ itsu_status ensure_tracklets(itsu_context *ctx, int64_t need)
   return ensure_partials(ctx);
 }
 
-// Entry scratch for an arena of these capacities: the cell count pass reserves a place per pair that
-// its precut lets through (0.54 per tracklet in central events, up to one in pile-up frames) and
-// reports what did not fit. A fixed arena cannot grow it, so it gets room for twice its tracklets,
-// the pairs of crowded events' cells and every short run.
-int64_t cell_places(const itsu_context *ctx)
+// Entry scratch for an arena of these capacities. The cell count pass reserves a place per pair that its
+// precut lets through (0.54 per tracklet in central events, up to one in pile-up frames, a hundred in
+// narrow jets) and reports what did not fit. Pairs bound no result, so a fixed arena has a second part,
+// where cells that are counted first take exactly their places: as many as it holds cells, twice (the
+// pair prefilter drops some after them), and kExactPlaces.
+struct CellPlaces {
+  int64_t pairs, exact;
+};
+constexpr int64_t kExactPlaces = int64_t(5) << 19;
+int64_t exact_places(const itsu_context *ctx) { return 2 * ctx->cap_cells + kExactPlaces; }
+CellPlaces cell_places(const itsu_context *ctx)
 {
   const bool fixed = (ctx->flags & ITSU_FLAG_NO_GROW) != 0;
-  return fixed ? 2 * ctx->cap_tracklets + 8 * ctx->cap_cells + (int64_t(5) << 19) : ctx->cap_tracklets / 2 + ctx->cap_cells + (1 << 14);
+  return fixed ? CellPlaces{2 * ctx->cap_tracklets + ctx->cap_cells, exact_places(ctx)}
+               : CellPlaces{ctx->cap_tracklets / 2 + ctx->cap_cells + (1 << 14), 0};
 }
 
-itsu_status ensure_cell_entries(itsu_context *ctx, int64_t need)
+cudaError_t alloc_cell_entries(itsu_context *ctx, CellPlaces want)
 {
-  if (need > ctx->cap_cell_entries) {
-    itsu_status st = growth_allowed(ctx, "cell entries", need, ctx->cap_cell_entries);
-    if (st != ITSU_OK) return st;
-    if (need > itsu::kMaxCellEntries) {
-      return fail(ctx, ITSU_ERR_CAPACITY, "cell entries: %lld needed, %lld can be indexed", (long long)need, (long long)itsu::kMaxCellEntries);
-    }
-    const int64_t cap = std::min(grow_to(need), itsu::kMaxCellEntries);
-    ITSU_CUDA(ctx, alloc(ctx, ctx->cell_entries, cap));
-    ITSU_CUDA(ctx, alloc(ctx, ctx->cell_dca, cap));
+  ctx->cap_cell_pairs = ctx->cap_cell_entries = 0;
+  ctx->generation++;
+  const int64_t cap = want.pairs + want.exact;
+  if (cap > itsu::kMaxCellEntries) return cudaErrorMemoryAllocation;
+  cudaError_t err = alloc(ctx, ctx->cell_entries, cap);
+  if (err == cudaSuccess) err = alloc(ctx, ctx->cell_dca, cap);
+  if (err == cudaSuccess) {
+    ctx->cap_cell_pairs = want.pairs;
     ctx->cap_cell_entries = cap;
-    ctx->generation++;
   }
+  return err;
+}
+
+// At least these places of each part. Where places for all pairs are more than the memory or their
+// indexes allow, the arena's ordinary number of them and, as in a fixed one, exact places.
+itsu_status ensure_cell_entries(itsu_context *ctx, CellPlaces need)
+{
+  CellPlaces want{ctx->cap_cell_pairs, ctx->cap_cell_entries - ctx->cap_cell_pairs};
+  if (need.pairs <= want.pairs && need.exact <= want.exact) return ITSU_OK;
+  itsu_status st = growth_allowed(ctx, "cell entries", need.pairs + need.exact, ctx->cap_cell_entries);
+  if (st != ITSU_OK) return st;
+  if (need.pairs > want.pairs) want.pairs = grow_to(need.pairs);
+  if (need.exact > want.exact) want.exact = grow_to(need.exact);
+  cudaError_t err = alloc_cell_entries(ctx, want);
+  if (err == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    err = alloc_cell_entries(ctx, CellPlaces{std::min(want.pairs, cell_places(ctx).pairs), std::max(want.exact, exact_places(ctx))});
+  }
+  ITSU_CUDA(ctx, err);
   return ITSU_OK;
+}
+
+// Room for a run's entries that did not fit: for all its pairs, or for the cells counted in their place.
+itsu_status grow_cell_entries(itsu_context *ctx, const DevStatus &s)
+{
+  const int64_t exact = ctx->cap_cell_entries - ctx->cap_cell_pairs;
+  return ensure_cell_entries(ctx, exact > 0 ? CellPlaces{ctx->cap_cell_pairs, s.cell_exact} : CellPlaces{s.cell_entries, 0});
 }
 
 // The cell stage's outputs. Not its scratch: after the count pass, growing it would lose the entries.
@@ -756,9 +788,12 @@ itsu_status run_all(itsu_context *ctx)
     }
     if (s.flags & itsu::kFlagCountOverflow) return count_overflow(ctx);
     if (ctx->flags & ITSU_FLAG_NO_GROW) {
-      return fail(ctx, ITSU_ERR_CAPACITY, "result exceeds the arena (tracklets %lld/%lld cells %lld/%lld neighbours %lld/%lld roads %lld/%lld)",
+      return fail(ctx, ITSU_ERR_CAPACITY,
+                  "result exceeds the arena (tracklets %lld/%lld cells %lld/%lld neighbours %lld/%lld roads %lld/%lld, "
+                  "counted cell entries %lld/%lld)",
                   (long long)s.total[0], (long long)ctx->cap_tracklets, (long long)s.total[1], (long long)ctx->cap_cells,
-                  (long long)s.total[2], (long long)ctx->cap_neighbours, (long long)s.total[3], (long long)ctx->cap_roads);
+                  (long long)s.total[2], (long long)ctx->cap_neighbours, (long long)s.total[3], (long long)ctx->cap_roads,
+                  (long long)s.cell_exact, (long long)(ctx->cap_cell_entries - ctx->cap_cell_pairs));
     }
     if (s.flags & itsu::kFlagCapTracklets) {
       // cells, neighbours and roads scale with the tracklets: grow them in proportion too
@@ -769,7 +804,7 @@ itsu_status run_all(itsu_context *ctx)
       if ((st = ensure_roads(ctx, (int64_t)(ctx->cap_roads * f))) != ITSU_OK) return st;
     }
     if ((s.flags & itsu::kFlagCapCells) && (st = ensure_cells(ctx, s.total[1])) != ITSU_OK) return st;
-    if ((s.flags & itsu::kFlagCapScratch) && (st = ensure_cell_entries(ctx, s.cell_entries)) != ITSU_OK) {
+    if ((s.flags & itsu::kFlagCapScratch) && (st = grow_cell_entries(ctx, s)) != ITSU_OK) {
       return st;
     }
     if ((s.flags & itsu::kFlagCapNeighbours) && (st = ensure_neighbours(ctx, s.total[2])) != ITSU_OK) return st;
@@ -787,7 +822,7 @@ itsu_status stage_count_then_write(itsu_context *ctx, void (*count)(const Arena 
     if ((st = clear_flags(ctx)) != ITSU_OK) return st;
     // the entry reservation, the crowded list, the tile sums of the tracklet and cell scans and the
     // segments' cell counts (the count passes add to them) start empty for every count, also a retry
-    ITSU_CUDA(ctx, cudaMemsetAsync(&ctx->d_status->cell_entries, 0, 4 * sizeof(int64_t), ctx->stream));
+    ITSU_CUDA(ctx, cudaMemsetAsync(&ctx->d_status->cell_entries, 0, itsu::kStatusCounters * sizeof(int64_t), ctx->stream));
     ITSU_CUDA(ctx, cudaMemsetAsync(ctx->scan_partials, 0, sizeof(int64_t) * ctx->cap_partials, ctx->stream));
     ITSU_CUDA(ctx, cudaMemsetAsync(ctx->cell_seg_count, 0, sizeof(int32_t) * ITSU_CELL_LAYERS * ctx->n_events, ctx->stream));
     Launch l = launch_of(ctx);
@@ -799,7 +834,7 @@ itsu_status stage_count_then_write(itsu_context *ctx, void (*count)(const Arena 
     // grow it and count again
     if (!(ctx->h_status->flags & itsu::kFlagCapScratch) || (ctx->h_status->flags & itsu::kFlagCountOverflow)) break;
     if (attempt == 4) return fail(ctx, ITSU_ERR_CAPACITY, "cell entry scratch growth did not converge");
-    if ((st = ensure_cell_entries(ctx, ctx->h_status->cell_entries)) != ITSU_OK) return st;
+    if ((st = grow_cell_entries(ctx, *ctx->h_status)) != ITSU_OK) return st;
   }
   const DevStatus &s = *ctx->h_status;
   if (s.flags & itsu::kFlagCountOverflow) return count_overflow(ctx);
@@ -1837,7 +1872,7 @@ itsu_status run_host_streamed(itsu_context *ctx, const HostClusters &clusters, c
     const DevStatus &s = ctx->h_chunk_status[fail_chunk];
     itsu_status g = ITSU_OK;
     if (g == ITSU_OK && (s.flags & itsu::kFlagCapTracklets)) g = ensure_tracklets(x, s.total[itsu::kTracklets]);
-    if (g == ITSU_OK && (s.flags & itsu::kFlagCapScratch)) g = ensure_cell_entries(x, s.cell_entries);
+    if (g == ITSU_OK && (s.flags & itsu::kFlagCapScratch)) g = grow_cell_entries(x, s);
     if (g == ITSU_OK && (s.flags & itsu::kFlagCapCells)) g = ensure_cells(x, s.total[itsu::kCells]);
     if (g == ITSU_OK && (s.flags & itsu::kFlagCapNeighbours)) g = ensure_neighbours(x, s.total[itsu::kNeighbours]);
     if (g == ITSU_OK && (s.flags & itsu::kFlagCapRoads)) g = ensure_roads(x, s.total[itsu::kRoads]);

@@ -47,15 +47,18 @@ struct DevStatus {
   int32_t invalid_event;  // first event with a malformed vertex, INT32_MAX if none
   int32_t pad_;
   int64_t total[4];       // tracklets, cells, neighbours, roads
-  int64_t cell_entries;   // places reserved by the cell count pass (may exceed the scratch)
+  int64_t cell_entries;   // places the cell count pass's pairs ask for (may exceed the scratch)
   int64_t cell_spans;     // spans of first tracklets of the cell count pass
   int64_t trk_crowded;    // inner clusters the tracklet count pass listed in clu_crowded
   int64_t cell_next;      // spans handed out by the cell count pass's counter
+  int64_t cell_exact;     // places reserved for counted cells, behind those for pairs (may exceed them)
 };
-// The four counters are reset together before each count pass (one 32-byte memset).
+// The five counters are reset together before each count pass (one memset).
+constexpr int kStatusCounters = 5;
 static_assert(offsetof(DevStatus, cell_spans) == offsetof(DevStatus, cell_entries) + 8 &&
                   offsetof(DevStatus, trk_crowded) == offsetof(DevStatus, cell_entries) + 16 &&
-                  offsetof(DevStatus, cell_next) == offsetof(DevStatus, cell_entries) + 24,
+                  offsetof(DevStatus, cell_next) == offsetof(DevStatus, cell_entries) + 24 &&
+                  offsetof(DevStatus, cell_exact) == offsetof(DevStatus, cell_entries) + 32,
               "status counters");
 
 // A cell as the count pass finds it: the cell record (its three clusters, local to layers L, L+1,
@@ -129,7 +132,7 @@ struct Arena {
   int32_t *cell_seg_id;
   CellEntry *cell_entries;  // scratch of the cell count pass
   float *cell_dca;  // per entry, its DCA (written in the learned form only: a prefilter feature)
-  int64_t cap_cell_entries;
+  int64_t cap_cell_pairs, cap_cell_entries;  // places reserved per pair; from those on, per counted cell
   // neighbours, levels, roads
   int32_t *nb_count;
   int32_t *nb_off;

@@ -78,6 +78,7 @@ __global__ void k_status_init(Arena a)
   s->cell_entries = 0;
   s->cell_spans = 0;
   s->cell_next = 0;
+  s->cell_exact = 0;
   s->trk_crowded = 0;
 }
 
@@ -1345,7 +1346,9 @@ __global__ void __launch_bounds__(kCountThreads) k_tracklet_segments(Arena a, bo
 //  2. Geometry, a lane per queued pair, in rounds of 32 in the queue's order (a round per group of 32
 //     first tracklets would hold 17 pairs on average): the exact cheap cuts (Tracker.cxx:161-173) on
 //     the records, then the circle geometry. The passing pairs become the span's cell entries, in
-//     order, from the place reserved for the span on (room for all its pairs).
+//     order, from the place reserved for the span on (room for all its pairs). Where the scratch is
+//     short of that, and has a part for it (cap_cell_pairs), the rounds run twice: the first time they
+//     count the cells, which then get exactly their places.
 // The cells are counted per span (whose scan places them) and per segment (cell_seg): there is no
 // mask, count or offset per tracklet, and the write pass copies entries in order.
 // Bound by the gathers (half of the issue slots and of the L1 data pipe busy). Spans of 128 leave
@@ -1507,16 +1510,19 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
     unsigned cells = 0;
     unsigned long long first = 0;
     const unsigned long long pairs = many + (unsigned)total;
+    bool placed = false, counting = false;
     if (pairs > 0) {
       if (lane == 0) {
         first = atomicAdd(reinterpret_cast<unsigned long long *>(&a.status->cell_entries), pairs);
-        if (first + pairs > (unsigned long long)a.cap_cell_entries) {
-          atomicOr(&a.status->flags, kFlagCapScratch);  // nothing after this pass runs
-        }
       }
       first = __shfl_sync(0xffffffffu, first, 0);
+      placed = first + pairs <= (unsigned long long)a.cap_cell_pairs;
+      counting = !placed && a.cap_cell_pairs < a.cap_cell_entries;
+      if (lane == 0 && !placed && !counting) {
+        atomicOr(&a.status->flags, kFlagCapScratch);  // nothing after this pass runs
+      }
     }
-    if (pairs > 0 && first + pairs <= (unsigned long long)a.cap_cell_entries) {
+    while (placed || counting) {
       __syncwarp();
       unsigned head = 0, tail = queued ? total : 0;
       uint32_t next = queued ? span : 0;  // not queued (a crowded outer cluster, or more pairs than the queue holds):
@@ -1584,7 +1590,7 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
         head += m;
         const unsigned passed = __ballot_sync(0xffffffffu, pass);
         const unsigned same = __match_any_sync(0xffffffffu, pass ? segment : -1);
-        if (pass) {
+        if (pass && !counting) {
           const unsigned before = (1u << lane) - 1u;
           if ((same & before) == 0) {
             atomicAdd(&a.cell_seg_count[segment], __popc(same));
@@ -1602,6 +1608,21 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
         }
         cells += __popc(passed);
         __syncwarp();  // the queue's freed places are refilled
+      }
+      if (!counting) {
+        break;
+      }
+      counting = false;
+      if (cells > 0) {
+        if (lane == 0) {
+          first = a.cap_cell_pairs + atomicAdd(reinterpret_cast<unsigned long long *>(&a.status->cell_exact), (unsigned long long)cells);
+        }
+        first = __shfl_sync(0xffffffffu, first, 0);
+        placed = first + cells <= (unsigned long long)a.cap_cell_entries;
+        if (lane == 0 && !placed) {
+          atomicOr(&a.status->flags, kFlagCapScratch);
+        }
+        cells = 0;
       }
     }
     if (lane == 0) {
