@@ -71,7 +71,8 @@ int band_of(int64_t n_clusters, int32_t n_events)
 }
 }  // namespace
 
-// All that the launches of a whole run depend on.
+// All that the launches of a whole run depend on (the groups' cluster ranges are launch arguments, cut on
+// the host from the layer offsets, which the same buffers may hold anew).
 struct RunKey {
   const void *inputs[6] = {};
   int64_t n_clusters = -1;
@@ -81,13 +82,14 @@ struct RunKey {
   bool prefilter = false, gate = false;
   itsu::SortShape sort{};
   itsu::LevelShape levels{};
+  std::vector<int64_t> groups;
 
   bool operator==(const RunKey &k) const
   {
     return std::equal(inputs, inputs + 6, k.inputs) && n_clusters == k.n_clusters && n_events == k.n_events &&
            generation == k.generation && std::equal(tune, tune + 4, k.tune) && prefilter == k.prefilter && gate == k.gate &&
            sort.threads == k.sort.threads && sort.ctas == k.sort.ctas && levels.threads == k.levels.threads &&
-           levels.ctas == k.levels.ctas;
+           levels.ctas == k.levels.ctas && groups == k.groups;
   }
 };
 
@@ -700,8 +702,6 @@ void enqueue_run(const Arena &a, const Launch &l)
   itsu::launch_roads_write(a, l);
 }
 
-void enqueue_all(itsu_context *ctx) { enqueue_run(arena_of(ctx), whole_run_launch(ctx)); }
-
 void drop_graph(itsu_context *ctx)
 {
   if (ctx->graph) {
@@ -710,6 +710,7 @@ void drop_graph(itsu_context *ctx)
   }
 }
 
+// For the launch that whole_run_launch returned last.
 RunKey run_key(const itsu_context *ctx)
 {
   const Tune tune = current_tune(ctx);
@@ -727,6 +728,7 @@ RunKey run_key(const itsu_context *ctx)
   k.gate = ctx->gate;
   k.sort = itsu::sort_shape(ctx->n_events, ctx->n_clusters, ctx->max_segment);
   k.levels = itsu::level_shape(ctx->max_segment);
+  k.groups = ctx->group_bounds;
   return k;
 }
 
@@ -741,19 +743,20 @@ itsu_status launch_all(itsu_context *ctx)
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   ITSU_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
   if (capture != cudaStreamCaptureStatusNone) return fail(ctx, ITSU_ERR_CUDA, "the context's stream is being captured");
+  const Launch launch = whole_run_launch(ctx);
   const RunKey key = run_key(ctx);
   if (!(ctx->graph && key == ctx->graph_key)) {
     ctx->last_key_runs = key == ctx->last_key ? ctx->last_key_runs + 1 : 1;
     ctx->last_key = key;
     if (ctx->last_key_runs <= kRunsBeforeGraph) {
-      enqueue_all(ctx);
+      enqueue_run(arena_of(ctx), launch);
       ITSU_CUDA(ctx, cudaGetLastError());
       return ITSU_OK;
     }
     drop_graph(ctx);
     cudaGraph_t g = nullptr;
     ITSU_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    enqueue_all(ctx);
+    enqueue_run(arena_of(ctx), launch);
     const cudaError_t launch_err = cudaGetLastError();
     const cudaError_t end_err = cudaStreamEndCapture(ctx->stream, &g);
     if (launch_err != cudaSuccess || end_err != cudaSuccess) {
