@@ -51,6 +51,10 @@ struct Tune {
 };
 constexpr int kBands = 32;
 
+// The capacity of a class of buffers that is not allocated: below that of an empty run, whose passes
+// write offsets and totals too.
+constexpr int kNoBuffers = -1;
+
 // Before the raw clusters' buffer: a vertex's 8 layer offsets and its coordinates.
 constexpr int64_t kRawHead = 64;
 static_assert(sizeof(int32_t) * (ITSU_LAYERS + 1) + sizeof(float) * 3 <= kRawHead, "a vertex's head");
@@ -101,9 +105,9 @@ struct itsu_context {
   int num_sms = 148;
 
   // capacities
-  int64_t cap_clusters = 0;
-  int32_t cap_events = 0;
-  int64_t cap_tracklets = 0, cap_cells = 0, cap_neighbours = 0, cap_roads = 0, cap_partials = 0;
+  int64_t cap_clusters = kNoBuffers;
+  int32_t cap_events = kNoBuffers;
+  int64_t cap_tracklets = kNoBuffers, cap_cells = kNoBuffers, cap_neighbours = kNoBuffers, cap_roads = kNoBuffers, cap_partials = 0;
   int64_t init_tracklets = 0, init_cells = 0, init_neighbours = 0, init_roads = 0;
 
   // device buffers: cluster class
@@ -282,9 +286,32 @@ cudaError_t alloc(itsu_context *ctx, T *&p, int64_t count)
   if (err == cudaSuccess) {
     ctx->arena_sizes[(const void *)p] = bytes;
     ctx->arena_bytes += (int64_t)bytes;
+  } else {
+    cudaGetLastError();  // reported here, not by the next launch's check
   }
   return err;
 }
+
+// A class of buffers while it is replaced: it has no capacity and, where an allocation fails, the context
+// no results.
+template <typename Capacity>
+struct Growth {
+  itsu_context *ctx;
+  Capacity &cap;
+  const int stage;
+
+  Growth(itsu_context *c, Capacity &class_cap) : ctx(c), cap(class_cap), stage(c->stage)
+  {
+    cap = kNoBuffers;
+    ctx->stage = std::min(stage, (int)kNone);
+    ctx->generation++;
+  }
+  void done(Capacity class_cap)
+  {
+    cap = class_cap;
+    ctx->stage = stage;
+  }
+};
 
 Tune current_tune(const itsu_context *ctx)
 {
@@ -441,9 +468,9 @@ itsu_status ensure_partials(itsu_context *ctx)
 {
   const int64_t need = std::max({ctx->cap_clusters, ctx->cap_tracklets, ctx->cap_cells}) / 2048 + 2;
   if (need > ctx->cap_partials) {
+    Growth<int64_t> growth(ctx, ctx->cap_partials);
     ITSU_CUDA(ctx, alloc(ctx, ctx->scan_partials, 2 * need));
-    ctx->cap_partials = need;
-    ctx->generation++;
+    growth.done(need);
   }
   return ITSU_OK;
 }
@@ -453,7 +480,8 @@ itsu_status ensure_clusters(itsu_context *ctx, int64_t n_clusters, int32_t n_eve
   if (n_clusters > ctx->cap_clusters) {
     itsu_status st = growth_allowed(ctx, "clusters", n_clusters, ctx->cap_clusters);
     if (st != ITSU_OK) return st;
-    const int64_t cap = grow_to(n_clusters);
+    const int64_t cap = n_clusters > 0 ? grow_to(n_clusters) : 0;
+    Growth<int64_t> growth(ctx, ctx->cap_clusters);
     ITSU_CUDA(ctx, alloc(ctx, ctx->raw_head, kRawHead + (int64_t)sizeof(itsu_cluster) * cap));
     ctx->raw = reinterpret_cast<itsu_cluster *>(ctx->raw_head + kRawHead);
     ITSU_CUDA(ctx, alloc(ctx, ctx->sorted, cap));
@@ -470,13 +498,13 @@ itsu_status ensure_clusters(itsu_context *ctx, int64_t n_clusters, int32_t n_eve
     ITSU_CUDA(ctx, alloc(ctx, ctx->clu_aux, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->clu_crowded, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_slots, cap * itsu::kTrackletSlotsPerCluster));
-    ctx->cap_clusters = cap;
-    ctx->generation++;
+    growth.done(cap);
   }
   if (n_events > ctx->cap_events) {
     itsu_status st = growth_allowed(ctx, "events", n_events, ctx->cap_events);
     if (st != ITSU_OK) return st;
-    const int32_t cap = n_events + n_events / 4 + 4;
+    const int32_t cap = n_events > 0 ? n_events + n_events / 4 + 4 : 0;
+    Growth<int32_t> growth(ctx, ctx->cap_events);
     ITSU_CUDA(ctx, alloc(ctx, ctx->layer_off, (int64_t)cap * ITSU_LAYERS + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->vtx, (int64_t)cap * 3));
     ITSU_CUDA(ctx, alloc(ctx, ctx->index_tables, (int64_t)cap * ITSU_TRACKLET_LAYERS * ITSU_INDEX_TABLE_SIZE));
@@ -488,8 +516,7 @@ itsu_status ensure_clusters(itsu_context *ctx, int64_t n_clusters, int32_t n_eve
     ITSU_CUDA(ctx, alloc(ctx, ctx->seg_rrange, (int64_t)cap * ITSU_LAYERS));
     ITSU_CUDA(ctx, alloc(ctx, ctx->seg_regular, (int64_t)cap * ITSU_LAYERS));
     ITSU_CUDA(ctx, alloc(ctx, ctx->raw_off, (int64_t)cap * ITSU_LAYERS));
-    ctx->cap_events = cap;
-    ctx->generation++;
+    growth.done(cap);
   }
   return ensure_partials(ctx);
 }
@@ -500,6 +527,7 @@ itsu_status ensure_tracklets(itsu_context *ctx, int64_t need)
     itsu_status st = growth_allowed(ctx, "tracklets", need, ctx->cap_tracklets);
     if (st != ITSU_OK) return st;
     const int64_t cap = grow_to(need);
+    Growth<int64_t> growth(ctx, ctx->cap_tracklets);
     ITSU_CUDA(ctx, alloc(ctx, ctx->tracklets, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_key, cap + 4));  // read in aligned groups of four
     ITSU_CUDA(ctx, alloc(ctx, ctx->trk_seg32, cap / 32 + 1));
@@ -507,8 +535,7 @@ itsu_status ensure_tracklets(itsu_context *ctx, int64_t need)
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_span_count, cap / 32 + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_span_off, cap / 32 + 2));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_lookup, cap));
-    ctx->cap_tracklets = cap;
-    ctx->generation++;
+    growth.done(cap);
   }
   return ensure_partials(ctx);
 }
@@ -532,15 +559,15 @@ CellPlaces cell_places(const itsu_context *ctx)
 
 cudaError_t alloc_cell_entries(itsu_context *ctx, CellPlaces want)
 {
-  ctx->cap_cell_pairs = ctx->cap_cell_entries = 0;
-  ctx->generation++;
   const int64_t cap = want.pairs + want.exact;
+  Growth<int64_t> growth(ctx, ctx->cap_cell_entries);
+  ctx->cap_cell_pairs = ctx->cap_cell_entries = 0;
   if (cap > itsu::kMaxCellEntries) return cudaErrorMemoryAllocation;
   cudaError_t err = alloc(ctx, ctx->cell_entries, cap);
   if (err == cudaSuccess) err = alloc(ctx, ctx->cell_dca, cap);
   if (err == cudaSuccess) {
     ctx->cap_cell_pairs = want.pairs;
-    ctx->cap_cell_entries = cap;
+    growth.done(cap);
   }
   return err;
 }
@@ -555,9 +582,10 @@ itsu_status ensure_cell_entries(itsu_context *ctx, CellPlaces need)
   if (st != ITSU_OK) return st;
   if (need.pairs > want.pairs) want.pairs = grow_to(need.pairs);
   if (need.exact > want.exact) want.exact = grow_to(need.exact);
+  const int stage = ctx->stage;
   cudaError_t err = alloc_cell_entries(ctx, want);
   if (err == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
+    ctx->stage = stage;
     err = alloc_cell_entries(ctx, CellPlaces{std::min(want.pairs, cell_places(ctx).pairs), std::max(want.exact, exact_places(ctx))});
   }
   ITSU_CUDA(ctx, err);
@@ -578,6 +606,7 @@ itsu_status ensure_cell_outputs(itsu_context *ctx, int64_t need)
     itsu_status st = growth_allowed(ctx, "cells", need, ctx->cap_cells);
     if (st != ITSU_OK) return st;
     const int64_t cap = grow_to(need);
+    Growth<int64_t> growth(ctx, ctx->cap_cells);
     ITSU_CUDA(ctx, alloc(ctx, ctx->cells, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->cell_seg_id, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->nb_count, cap + 1));
@@ -587,8 +616,7 @@ itsu_status ensure_cell_outputs(itsu_context *ctx, int64_t need)
     ITSU_CUDA(ctx, alloc(ctx, ctx->paths, cap));
     ITSU_CUDA(ctx, alloc(ctx, ctx->road_count, cap + 1));
     ITSU_CUDA(ctx, alloc(ctx, ctx->road_off, cap + 1));
-    ctx->cap_cells = cap;
-    ctx->generation++;
+    growth.done(cap);
   }
   return ensure_partials(ctx);
 }
@@ -606,9 +634,9 @@ itsu_status ensure_neighbours(itsu_context *ctx, int64_t need)
     itsu_status st = growth_allowed(ctx, "neighbours", need, ctx->cap_neighbours);
     if (st != ITSU_OK) return st;
     const int64_t cap = grow_to(need);
+    Growth<int64_t> growth(ctx, ctx->cap_neighbours);
     ITSU_CUDA(ctx, alloc(ctx, ctx->nb, cap));
-    ctx->cap_neighbours = cap;
-    ctx->generation++;
+    growth.done(cap);
   }
   return ITSU_OK;
 }
@@ -619,9 +647,9 @@ itsu_status ensure_roads(itsu_context *ctx, int64_t need)
     itsu_status st = growth_allowed(ctx, "roads", need, ctx->cap_roads);
     if (st != ITSU_OK) return st;
     const int64_t cap = grow_to(need);
+    Growth<int64_t> growth(ctx, ctx->cap_roads);
     ITSU_CUDA(ctx, alloc(ctx, ctx->roads, cap));
-    ctx->cap_roads = cap;
-    ctx->generation++;
+    growth.done(cap);
   }
   return ITSU_OK;
 }
@@ -1360,6 +1388,7 @@ static itsu_status set_batch(itsu_context *ctx, const itsu_batch *batch)
   if (batch->n_events < 0 || batch->n_clusters < 0 || batch->n_clusters > INT32_MAX) {
     return fail(ctx, ITSU_ERR_INVALID, "bad batch size (%d events, %lld clusters)", batch->n_events, (long long)batch->n_clusters);
   }
+  if (batch->n_events == 0 && batch->n_clusters > 0) return fail(ctx, ITSU_ERR_INVALID, "%lld clusters of no event", (long long)batch->n_clusters);
   if (batch->n_events > 0 && (!batch->layer_offsets || !batch->vertices || (batch->n_clusters > 0 && !batch->clusters))) {
     return fail(ctx, ITSU_ERR_INVALID, "null batch pointer");
   }
@@ -1442,12 +1471,12 @@ itsu_status itsu_memory_usage_get(itsu_context *ctx, itsu_memory_usage *out)
   if (!ctx || !out) return fail(ctx, ITSU_ERR_INVALID, "itsu_memory_usage_get: null argument");
   std::memset(out, 0, sizeof *out);
   out->device_bytes = ctx->arena_bytes + (ctx->twin ? ctx->twin->arena_bytes : 0);
-  out->clusters_capacity = ctx->cap_clusters;
-  out->events_capacity = ctx->cap_events;
-  out->capacity[0] = ctx->cap_tracklets;
-  out->capacity[1] = ctx->cap_cells;
-  out->capacity[2] = ctx->cap_neighbours;
-  out->capacity[3] = ctx->cap_roads;
+  out->clusters_capacity = std::max(ctx->cap_clusters, decltype(ctx->cap_clusters)(0));
+  out->events_capacity = std::max(ctx->cap_events, decltype(ctx->cap_events)(0));
+  out->capacity[0] = std::max<int64_t>(ctx->cap_tracklets, 0);
+  out->capacity[1] = std::max<int64_t>(ctx->cap_cells, 0);
+  out->capacity[2] = std::max<int64_t>(ctx->cap_neighbours, 0);
+  out->capacity[3] = std::max<int64_t>(ctx->cap_roads, 0);
   for (int k = 0; k < 4; ++k) out->used[k] = ctx->h_status ? ctx->h_status->total[k] : 0;
   out->cell_entries_capacity = ctx->cap_cell_entries;
   return ITSU_OK;
@@ -1548,6 +1577,7 @@ itsu_status itsu_roads_report(itsu_context *ctx, const itsu_road *roads, const i
   const size_t total = o_cnt + align(sizeof(itsu_report_counts) * (size_t)n_events);
   // the scratch stays with the context (grown when a call needs more)
   if ((int64_t)total > ctx->cap_report_scratch) {
+    ctx->cap_report_scratch = 0;
     ITSU_CUDA(ctx, alloc(ctx, ctx->report_scratch, grow_to((int64_t)total)));
     ctx->cap_report_scratch = grow_to((int64_t)total);
   }
@@ -1610,6 +1640,7 @@ itsu_status grow_buffer(itsu_context *ctx, T *&p, int64_t &cap, int64_t need)
 {
   if (need > cap) {
     const int64_t c = grow_to(need);
+    cap = 0;
     ITSU_CUDA(ctx, alloc(ctx, p, c));
     cap = c;
   }
@@ -1891,9 +1922,11 @@ itsu_status batch_run_host(itsu_context *ctx, const HostClusters &clusters, cons
   if (!ctx) return fail(nullptr, ITSU_ERR_INVALID, "null context");
   if (n_events < 0 || (n_events > 0 && (!layer_offsets || !vertices))) return fail(ctx, ITSU_ERR_INVALID, "bad batch arguments");
   ITSU_CUDA(ctx, cudaSetDevice(ctx->device));
+  static const int32_t kNoOffsets[1] = {0};
+  if (!layer_offsets) layer_offsets = kNoOffsets;  // no events
   const int64_t n_clusters = n_events > 0 ? layer_offsets[(int64_t)n_events * ITSU_LAYERS] : 0;
   if (n_clusters > 0 && !clusters.any()) return fail(ctx, ITSU_ERR_INVALID, "null clusters");
-  if (layer_offsets && layer_offsets[0] != 0) return fail(ctx, ITSU_ERR_INVALID, "layer offsets must start at 0");
+  if (layer_offsets[0] != 0) return fail(ctx, ITSU_ERR_INVALID, "layer offsets must start at 0");
   for (int64_t k = 1; n_events > 0 && k <= (int64_t)n_events * ITSU_LAYERS; ++k) {
     if (layer_offsets[k] < layer_offsets[k - 1]) return fail(ctx, ITSU_ERR_INVALID, "layer offsets decrease at %lld", (long long)k);
   }
@@ -1912,7 +1945,9 @@ itsu_status batch_run_host(itsu_context *ctx, const HostClusters &clusters, cons
   if ((st = upload_clusters(ctx, clusters, 0, n_clusters, ctx->stream)) != ITSU_OK) return st;
   ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->layer_off, layer_offsets, sizeof(int32_t) * ((int64_t)n_events * ITSU_LAYERS + 1),
                                  cudaMemcpyHostToDevice, ctx->stream));
-  ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->vtx, vertices, sizeof(float) * 3 * (int64_t)n_events, cudaMemcpyHostToDevice, ctx->stream));
+  if (n_events > 0) {
+    ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->vtx, vertices, sizeof(float) * 3 * (int64_t)n_events, cudaMemcpyHostToDevice, ctx->stream));
+  }
   if ((st = ensure_outputs_for(ctx, n_clusters)) != ITSU_OK) return st;
   ctx->n_events = n_events;
   ctx->n_clusters = n_clusters;
