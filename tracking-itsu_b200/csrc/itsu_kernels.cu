@@ -1370,6 +1370,7 @@ __device__ __forceinline__ uint32_t span_of(uint32_t n) { return n >= (1u << 22)
 
 struct CellWarp {
   int2 state[kMaxSpan];        // first outgoing tracklet; segment (kCrowded: more than kMaxMaskedOut outgoing tracklets)
+  unsigned long long many;
   union {
     uint16_t queue[kCellQueue];  // (first tracklet in the span) | (outgoing tracklet) << 7
     uint2 ring[kCellRing];       // the same two, for any number of outgoing tracklets
@@ -1424,6 +1425,9 @@ __device__ __forceinline__ unsigned long long cell_precut_mask(const Arena &a, c
 
 // Runs over the spans that end among the tracklets of events below e1 and not below e0 (last: to the
 // end of the run): every span is taken once its tracklets are written.
+// kExact: the scratch has a part for cells that are counted first (cap_cell_pairs); without one the rounds
+// only run once (1.03 ms per 128 central events, 1.06 with the check for it in every span).
+template <bool kExact>
 __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena a, int32_t e0, int32_t e1, bool last)
 {
   __shared__ CellWarp shared[kCellThreads / 32];
@@ -1433,6 +1437,7 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
   }
   const int lane = threadIdx.x & 31;
   CellWarp &w = shared[threadIdx.x >> 5];
+  w.many = 0;
   // tracklet indices stay below 2^31 (the scan flags larger totals), a span's end below 2^32
   const uint32_t n = (uint32_t)a.status->total[kTracklets];
   const uint32_t span = span_of(n), spans = (n + span - 1) / span;
@@ -1467,7 +1472,6 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
     }
     const uint32_t base = s * span;
     int total = 0;
-    unsigned long long many = 0;  // pairs behind crowded outer clusters, beside total (their sum can pass 2^32)
     bool queued = true;           // the span's pairs are all in the queue
     for (uint32_t g = 0; g < span; g += 32) {
       const uint32_t at = g + lane, k = base + at;
@@ -1481,12 +1485,7 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
       w.state[at] = make_int2(p.j0, crowded ? p.sid | kCrowded : p.sid);
       unsigned long long mask = 0ull;
       int count = 0;
-      unsigned behind = 0;
-      if (crowded) {
-        for (int q = 0; q < p.n_out; ++q) {
-          behind += key_window_pass(p.w.keys, a.trk_key[p.j0 + q]);
-        }
-      } else if (p.n_out > 0) {
+      if (!crowded && p.n_out > 0) {
         mask = cell_precut_mask(a, p);
         count = __popcll(mask);
       }
@@ -1495,7 +1494,14 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
       total += group_total;
       queued = queued && total <= kCellQueue;
       if (__any_sync(0xffffffffu, crowded)) {
-        many += warp_sum(0xffffffffu, behind);
+        unsigned behind = 0;
+        for (int q = 0; crowded && q < p.n_out; ++q) {
+          behind += key_window_pass(p.w.keys, a.trk_key[p.j0 + q]);
+        }
+        const unsigned long long sum = warp_sum(0xffffffffu, behind);
+        if (lane == 0) {
+          w.many += sum;
+        }
         queued = false;
       }
       if (queued) {
@@ -1509,7 +1515,8 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
     }
     unsigned cells = 0;
     unsigned long long first = 0;
-    const unsigned long long pairs = many + (unsigned)total;
+    __syncwarp();
+    const unsigned long long pairs = queued ? (unsigned long long)total : w.many + (unsigned)total;
     bool placed = false, counting = false;
     if (pairs > 0) {
       if (lane == 0) {
@@ -1517,12 +1524,12 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
       }
       first = __shfl_sync(0xffffffffu, first, 0);
       placed = first + pairs <= (unsigned long long)a.cap_cell_pairs;
-      counting = !placed && a.cap_cell_pairs < a.cap_cell_entries;
+      counting = kExact && !placed;
       if (lane == 0 && !placed && !counting) {
         atomicOr(&a.status->flags, kFlagCapScratch);  // nothing after this pass runs
       }
     }
-    while (placed || counting) {
+    while (placed || (kExact && counting)) {
       __syncwarp();
       unsigned head = 0, tail = queued ? total : 0;
       uint32_t next = queued ? span : 0;  // not queued (a crowded outer cluster, or more pairs than the queue holds):
@@ -1590,7 +1597,7 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
         head += m;
         const unsigned passed = __ballot_sync(0xffffffffu, pass);
         const unsigned same = __match_any_sync(0xffffffffu, pass ? segment : -1);
-        if (pass && !counting) {
+        if (pass && !(kExact && counting)) {
           const unsigned before = (1u << lane) - 1u;
           if ((same & before) == 0) {
             atomicAdd(&a.cell_seg_count[segment], __popc(same));
@@ -1609,7 +1616,7 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
         cells += __popc(passed);
         __syncwarp();  // the queue's freed places are refilled
       }
-      if (!counting) {
+      if (!kExact || !counting) {
         break;
       }
       counting = false;
@@ -1634,6 +1641,9 @@ __global__ void __launch_bounds__(kCellThreads, kCellBlocks) k_cells_count(Arena
       if (cells > 0) {
         atomicAdd(reinterpret_cast<unsigned long long *>(&a.scan_partials[s / kScanTile]), (unsigned long long)cells);
       }
+    }
+    if (lane == 0 && !queued) {
+      w.many = 0;
     }
     __syncwarp();  // the span's state is refilled next
   }
@@ -2311,7 +2321,12 @@ void step_tracklet_segments(const Arena &a, const Launch &l)
 
 void launch_cells_range(const Arena &a, const Launch &l, int32_t e0, int32_t e1, bool last)
 {
-  k_cells_count<<<blocks_for(l.num_sms * kCellBlocks, likely_tracklets(a), kCellThreads), kCellThreads, 0, l.stream>>>(a, e0, e1, last);
+  const unsigned blocks = blocks_for(l.num_sms * kCellBlocks, likely_tracklets(a), kCellThreads);
+  if (a.cap_cell_pairs < a.cap_cell_entries) {
+    k_cells_count<true><<<blocks, kCellThreads, 0, l.stream>>>(a, e0, e1, last);
+  } else {
+    k_cells_count<false><<<blocks, kCellThreads, 0, l.stream>>>(a, e0, e1, last);
+  }
 }
 
 void step_cells_count(const Arena &a, const Launch &l)
