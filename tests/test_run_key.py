@@ -8,7 +8,8 @@ import subprocess
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-SOURCE = open(os.path.join(ROOT, "tracking-itsu_b200", "csrc", "itsu_capi.cu")).read()
+CSRC = os.path.join(ROOT, "tracking-itsu_b200", "csrc")
+SOURCE = open(os.path.join(CSRC, "itsu_capi.cu")).read()
 
 PROGRAM = r"""
 #include <algorithm>
@@ -16,7 +17,9 @@ PROGRAM = r"""
 #include <cstdio>
 #include <vector>
 #define ITSU_LAYERS 7
-namespace itsu { struct SortShape { int threads, ctas; }; struct LevelShape { int threads, ctas; }; }
+namespace itsu {
+%s
+}
 %s
 %s
 static RunKey key(const std::vector<int> &sizes, int group)
@@ -38,9 +41,10 @@ int main()
 
 
 def test_key_of_another_event_order(tmp_path):
+    shapes = "\n".join(re.findall(r"^struct (?:Sort|Level)Shape \{.*?^\};", open(os.path.join(CSRC, "itsu_internal.h")).read(), re.M | re.S))
     struct = re.search(r"^struct RunKey \{.*?^\};", SOURCE, re.M | re.S).group(0)
     bounds = re.search(r"^void group_bounds\(.*?^\}", SOURCE, re.M | re.S).group(0)
-    (tmp_path / "key.cpp").write_text(PROGRAM % (struct, bounds))
+    (tmp_path / "key.cpp").write_text(PROGRAM % (shapes, struct, bounds))
     subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-o", str(tmp_path / "key"), str(tmp_path / "key.cpp")], check=True)
     out = subprocess.run([str(tmp_path / "key")], check=True, capture_output=True, text=True).stdout
     assert out.split() == ["1", "0", "1", "1"]  # without groups nothing of the offsets is in the launches

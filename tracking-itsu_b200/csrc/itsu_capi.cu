@@ -93,7 +93,7 @@ struct RunKey {
     return std::equal(inputs, inputs + 6, k.inputs) && n_clusters == k.n_clusters && n_events == k.n_events &&
            generation == k.generation && std::equal(tune, tune + 4, k.tune) && prefilter == k.prefilter && gate == k.gate &&
            sort.threads == k.sort.threads && sort.ctas == k.sort.ctas && levels.threads == k.levels.threads &&
-           levels.ctas == k.levels.ctas && groups == k.groups;
+           levels.ctas == k.levels.ctas && levels.wide == k.levels.wide && groups == k.groups;
   }
 };
 
@@ -755,7 +755,7 @@ RunKey run_key(const itsu_context *ctx)
   k.prefilter = ctx->prefilter;
   k.gate = ctx->gate;
   k.sort = itsu::sort_shape(ctx->n_events, ctx->n_clusters, ctx->max_segment);
-  k.levels = itsu::level_shape(ctx->max_segment);
+  k.levels = itsu::level_shape(ctx->n_events, ctx->max_segment, ctx->num_sms);
   k.groups = ctx->group_bounds;
   return k;
 }

@@ -202,11 +202,12 @@ struct SortShape {
 };
 SortShape sort_shape(int32_t n_events, int64_t n_clusters, int64_t max_segment);
 
-// How the level pass is launched.
+// How the level pass is launched: clusters of ctas CTAs per event, or a wide launch per layer.
 struct LevelShape {
   int threads, ctas;
+  bool wide;
 };
-LevelShape level_shape(int64_t max_segment);
+LevelShape level_shape(int32_t n_events, int64_t max_segment, int num_sms);
 
 // Stage launchers (asynchronous on l.stream).
 void launch_status_init(const Arena &a, const Launch &l);

@@ -2033,6 +2033,22 @@ __global__ void __launch_bounds__(kThreads_) k_levels(Arena a)
   }
 }
 
+// One layer of the level pass over the whole chip (the blocks of grid row y take events y, y + gridDim.y,
+// ...): for few events whose layers are more than a cluster of CTAs takes in a few rounds (level_shape).
+__global__ void __launch_bounds__(kMaxThreads) k_levels_layer(Arena a, int layer)
+{
+  if (capacity_failed(a.status)) {
+    return;
+  }
+  for (int e = blockIdx.y; e < a.n_events; e += gridDim.y) {
+    const int32_t *cs = a.cell_seg + e * ITSU_CELL_LAYERS;
+    const int64_t prev_base = cs[layer - 1];
+    for (int64_t c = cs[layer] + global_thread(); c < cs[layer + 1]; c += grid_threads()) {
+      level_of(a, c, prev_base, layer);
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------
 // (e) roads: Tracker<IsGPU>::findTracks / traverseCellsTree / computeMontecarloLabels
 
@@ -2380,8 +2396,12 @@ void step_levels(const Arena &a, const Launch &l)
   if (a.n_events <= 0) {
     return;
   }
-  const LevelShape shape = level_shape(l.max_segment);
-  if (shape.threads == 128) {
+  const LevelShape shape = level_shape(a.n_events, l.max_segment, l.num_sms);
+  if (shape.wide) {
+    for (int layer = 1; layer < ITSU_CELL_LAYERS; ++layer) {
+      k_levels_layer<<<event_grid(a, l), l.block, 0, l.stream>>>(a, layer);
+    }
+  } else if (shape.threads == 128) {
     launch_clusters(k_levels<128>, a.n_events, 1, 128, 0, l.stream, a);
   } else {
     launch_clusters(k_levels<512>, a.n_events, shape.ctas, 512, 0, l.stream, a);
@@ -2449,8 +2469,13 @@ SortShape sort_shape(int32_t n_events, int64_t n_clusters, int64_t max_segment)
   return s;
 }
 
-// The level pass's launch for a run whose largest layer has max_segment clusters.
-LevelShape level_shape(int64_t max_segment)
+// The level pass's launch for a run whose largest layer has max_segment clusters. A cluster of 8 CTAs has
+// 4096 threads for an event's layer, and the cells of a layer grow with the square of its clusters: few
+// events with large layers take a wide launch per layer instead. One event with layers of 9,450 clusters:
+// 34 us in clusters, 28 wide; of 26,250: 126 and 38; of 52,500: 478 and 55. Four of 9,450: 37 and 38;
+// eight of 12,600: 49 and 41; 16: 54 and 50; 32: 74 and 77.
+constexpr int64_t kWideLevels = 10000;
+LevelShape level_shape(int32_t n_events, int64_t max_segment, int num_sms)
 {
   LevelShape s;
   s.threads = max_segment > 192 ? 512 : 128;
@@ -2458,6 +2483,7 @@ LevelShape level_shape(int64_t max_segment)
   while (s.threads == 512 && s.ctas < 8 && 3 * max_segment > 4 * 512 * s.ctas) {
     s.ctas *= 2;
   }
+  s.wide = max_segment > kWideLevels && 2 * (int64_t)n_events * s.ctas < 3 * num_sms;
   return s;
 }
 
