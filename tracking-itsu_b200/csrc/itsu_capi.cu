@@ -86,6 +86,7 @@ struct RunKey {
   bool prefilter = false, gate = false;
   itsu::SortShape sort{};
   itsu::LevelShape levels{};
+  int64_t tracklets = 0, cells = 0;
   std::vector<int64_t> groups;
 
   bool operator==(const RunKey &k) const
@@ -93,7 +94,8 @@ struct RunKey {
     return std::equal(inputs, inputs + 6, k.inputs) && n_clusters == k.n_clusters && n_events == k.n_events &&
            generation == k.generation && std::equal(tune, tune + 4, k.tune) && prefilter == k.prefilter && gate == k.gate &&
            sort.threads == k.sort.threads && sort.ctas == k.sort.ctas && levels.threads == k.levels.threads &&
-           levels.ctas == k.levels.ctas && levels.wide == k.levels.wide && groups == k.groups;
+           levels.ctas == k.levels.ctas && levels.wide == k.levels.wide && tracklets == k.tracklets && cells == k.cells &&
+           groups == k.groups;
   }
 };
 
@@ -164,6 +166,9 @@ struct itsu_context {
   int64_t n_clusters = 0;
   std::vector<int32_t> h_layer_off;
   int64_t max_segment = 0;  // clusters of the current run's largest layer
+  int64_t most_tracklets = 0;  // pairs of clusters of the current run's adjacent layers
+  // how often the last run's counts double the ordinary 10 tracklets and 2 cells per cluster
+  int dense_tracklets = 0, dense_cells = 0;
   std::vector<int64_t> group_bounds;  // event groups of the current whole run (whole_run_launch)
   const itsu_cluster *in_raw = nullptr;
   const itsu_cluster_in *in_raw_in = nullptr;  // the 24-byte input records instead of in_raw (compact host calls)
@@ -322,6 +327,29 @@ Tune current_tune(const itsu_context *ctx)
   return t.set ? t : Tune{};
 }
 
+// What grids go by, before the counts of a run are known on the host: ten tracklets and two cells per
+// cluster (above what any workload here has), times the last run's density beyond that, so that a narrow
+// jet's hundreds per cluster find a full grid from its second run on; and, so that its first run finds
+// some blocks, as many tracklets as its layers' pairs allow, up to three blocks per SM (a full grid costs
+// an ordinary small event 1 us in each kernel). One event of three layers of 300 clusters on one line has
+// 181 thousand tracklets: 4.2 ms by its clusters alone.
+constexpr int64_t kUsualTracklets = 10, kUsualCells = 2;
+
+int doublings(int64_t count, int64_t usual)
+{
+  int d = 0;
+  while (d < 24 && count > usual << d) ++d;
+  return d;
+}
+
+// After a run of n_clusters clusters, or the stages of it that have run (zero counts: not yet).
+void note_density(itsu_context *ctx, int64_t n_clusters, const DevStatus &s)
+{
+  n_clusters = std::max<int64_t>(n_clusters, 1);
+  if (s.total[itsu::kTracklets] > 0) ctx->dense_tracklets = doublings(s.total[itsu::kTracklets], kUsualTracklets * n_clusters);
+  if (s.total[itsu::kCells] > 0) ctx->dense_cells = doublings(s.total[itsu::kCells], kUsualCells * n_clusters);
+}
+
 Launch launch_of(const itsu_context *ctx)
 {
   const Tune t = current_tune(ctx);
@@ -331,17 +359,29 @@ Launch launch_of(const itsu_context *ctx)
   l.block = t.block;
   l.blocks_per_sm = t.blocks_per_sm;
   l.max_segment = ctx->max_segment;
+  l.tracklets = std::max((kUsualTracklets * ctx->n_clusters) << ctx->dense_tracklets, std::min<int64_t>(ctx->most_tracklets, 3 * 128 * ctx->num_sms));
+  l.cells = std::max((kUsualCells * ctx->n_clusters) << ctx->dense_cells, std::min<int64_t>(ctx->most_tracklets, 256 * ctx->num_sms));
+  l.level_size = ctx->max_segment;
+  if (ctx->dense_cells > 0 && ctx->n_events > 0) {
+    // five layers of cells, four for three clusters of an ordinary one
+    l.level_size = std::max(l.level_size, 3 * ((kUsualCells * ctx->n_clusters) << ctx->dense_cells) / (20 * (int64_t)ctx->n_events));
+  }
   return l;
 }
 
-// Clusters of the largest of the segments whose offsets are off[0 .. n_segments].
-int64_t largest_segment(const int32_t *off, int64_t n_segments)
+// The sizes that launches go by, from the layer offsets of n_events events.
+void note_segments(itsu_context *ctx, const int32_t *off, int32_t n_events)
 {
-  int64_t largest = 0;
-  for (int64_t k = 0; k < n_segments; ++k) {
-    largest = std::max<int64_t>(largest, off[k + 1] - off[k]);
+  ctx->max_segment = ctx->most_tracklets = 0;
+  for (int64_t e = 0; e < n_events; ++e) {
+    int64_t before = 0;
+    for (int l = 0; l < ITSU_LAYERS; ++l, ++off) {
+      const int64_t n = off[1] - off[0];
+      ctx->max_segment = std::max(ctx->max_segment, n);
+      ctx->most_tracklets += before * n;
+      before = n;
+    }
   }
-  return largest;
 }
 
 // Event groups of a run of n_events events with host layer offsets off[n_events * 7 + 1]: group g
@@ -683,6 +723,7 @@ itsu_status sync_status(itsu_context *ctx)
   ITSU_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(DevStatus), cudaMemcpyDeviceToHost, ctx->stream));
   ITSU_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->pinned_busy = false;
+  note_density(ctx, ctx->n_clusters, *ctx->h_status);
   if (ctx->h_status->flags & itsu::kFlagLaunchShape) {
     return fail(ctx, ITSU_ERR_INVALID, "launch shape: the per-item passes need a block size that is a multiple of 32");
   }
@@ -738,8 +779,7 @@ void drop_graph(itsu_context *ctx)
   }
 }
 
-// For the launch that whole_run_launch returned last.
-RunKey run_key(const itsu_context *ctx)
+RunKey run_key(const itsu_context *ctx, const Launch &l)
 {
   const Tune tune = current_tune(ctx);
   RunKey k;
@@ -754,9 +794,11 @@ RunKey run_key(const itsu_context *ctx)
   k.tune[3] = tune.group;
   k.prefilter = ctx->prefilter;
   k.gate = ctx->gate;
-  k.sort = itsu::sort_shape(ctx->n_events, ctx->n_clusters, ctx->max_segment);
-  k.levels = itsu::level_shape(ctx->n_events, ctx->max_segment, ctx->num_sms);
-  k.groups = ctx->group_bounds;
+  k.sort = itsu::sort_shape(ctx->n_events, ctx->n_clusters, l.max_segment);
+  k.levels = itsu::level_shape(ctx->n_events, l.level_size, l.num_sms);
+  k.tracklets = l.tracklets;
+  k.cells = l.cells;
+  k.groups.assign(l.groups, l.groups + (l.n_groups > 0 ? l.n_groups + 1 : 0));
   return k;
 }
 
@@ -772,7 +814,7 @@ itsu_status launch_all(itsu_context *ctx)
   ITSU_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
   if (capture != cudaStreamCaptureStatusNone) return fail(ctx, ITSU_ERR_CUDA, "the context's stream is being captured");
   const Launch launch = whole_run_launch(ctx);
-  const RunKey key = run_key(ctx);
+  const RunKey key = run_key(ctx, launch);
   if (!(ctx->graph && key == ctx->graph_key)) {
     ctx->last_key_runs = key == ctx->last_key ? ctx->last_key_runs + 1 : 1;
     ctx->last_key = key;
@@ -961,7 +1003,7 @@ itsu_status upload_vertex(itsu_context *ctx, const itsu_cluster *const layers[IT
   ctx->n_events = 1;
   ctx->n_clusters = off[ITSU_LAYERS];
   ctx->h_layer_off = off;
-  ctx->max_segment = *std::max_element(counts, counts + ITSU_LAYERS);
+  note_segments(ctx, off.data(), 1);
   ctx->in_raw = ctx->raw;
   ctx->in_raw_in = nullptr;
   ctx->in_raw_track = nullptr;
@@ -1415,7 +1457,7 @@ static itsu_status set_batch(itsu_context *ctx, const itsu_batch *batch)
       if (ctx->h_layer_off[k] < ctx->h_layer_off[k - 1]) return fail(ctx, ITSU_ERR_INVALID, "layer offsets decrease at %zu", k);
     }
   }
-  ctx->max_segment = largest_segment(ctx->h_layer_off.data(), (int64_t)batch->n_events * ITSU_LAYERS);
+  note_segments(ctx, ctx->h_layer_off.data(), batch->n_events);
   ctx->stage = kNone;
   return ITSU_OK;
 }
@@ -1813,7 +1855,7 @@ itsu_status run_host_streamed(itsu_context *ctx, const HostClusters &clusters, c
     Arena arena = arena_of(x);
     arena.mlp = ctx->prefilter ? ctx->d_mlp : nullptr;  // the context's models serve both arenas
     arena.gate = ctx->gate ? ctx->d_gate : nullptr;
-    x->max_segment = largest_segment(layer_offsets + (int64_t)ev[c] * ITSU_LAYERS, (int64_t)x->n_events * ITSU_LAYERS);
+    note_segments(x, layer_offsets + (int64_t)ev[c] * ITSU_LAYERS, x->n_events);
     Launch l = launch_of(x);
     std::vector<int64_t> bounds;  // the chunk's event groups (read while its launches are enqueued)
     const int group = current_tune(x).group;
@@ -1844,6 +1886,7 @@ itsu_status run_host_streamed(itsu_context *ctx, const HostClusters &clusters, c
       break;
     }
     const DevStatus &s = ctx->h_chunk_status[c];
+    note_density(twin && (c & 1) ? twin : ctx, layer_offsets[(int64_t)ev[c + 1] * ITSU_LAYERS] - layer_offsets[(int64_t)ev[c] * ITSU_LAYERS], s);
     if (s.flags & itsu::kFlagInvalid) {
       if (s.invalid_event != INT32_MAX) {
         st = fail(ctx, ITSU_ERR_INVALID, "primary vertex of event %d is not finite or beyond 1e6 cm", ev[c] + s.invalid_event);
@@ -1956,7 +1999,7 @@ itsu_status batch_run_host(itsu_context *ctx, const HostClusters &clusters, cons
   ctx->in_layer_off = ctx->layer_off;
   ctx->in_vtx = ctx->vtx;
   ctx->h_layer_off.assign(layer_offsets, layer_offsets + (int64_t)n_events * ITSU_LAYERS + 1);
-  ctx->max_segment = largest_segment(layer_offsets, (int64_t)n_events * ITSU_LAYERS);
+  note_segments(ctx, layer_offsets, n_events);
   if ((st = run_all(ctx)) != ITSU_OK) return st;
   const int64_t total = ctx->h_status->total[itsu::kRoads];
   if (road_offsets) {
@@ -2055,7 +2098,7 @@ itsu_status itsu_frames_run_host(itsu_context *ctx, const itsu_frames *frames, i
   ctx->in_layer_off = ctx->layer_off;
   ctx->in_vtx = ctx->vtx;
   ctx->h_layer_off = run_off;
-  ctx->max_segment = largest_segment(run_off.data(), (int64_t)nv * ITSU_LAYERS);
+  note_segments(ctx, run_off.data(), nv);
   if ((st = run_all(ctx)) != ITSU_OK) return st;
   const int64_t n_roads = ctx->h_status->total[itsu::kRoads];
   if (road_offsets) {

@@ -193,6 +193,9 @@ struct Launch {
   int group_events = 0;
   const int64_t *groups = nullptr;
   int64_t max_segment = 0;  // clusters of the run's largest layer
+  // what the host expects of the run (grids go by it; any value gives the same results): its tracklets and
+  // cells, and the clusters of a layer that ordinarily have as many cells as its largest layer will
+  int64_t tracklets = 0, cells = 0, level_size = 0;
   bool staged = false;      // a stage call, whose outputs may have to grow between its count and its write
 };
 
@@ -207,7 +210,7 @@ struct LevelShape {
   int threads, ctas;
   bool wide;
 };
-LevelShape level_shape(int32_t n_events, int64_t max_segment, int num_sms);
+LevelShape level_shape(int32_t n_events, int64_t size, int num_sms);
 
 // Stage launchers (asynchronous on l.stream).
 void launch_status_init(const Arena &a, const Launch &l);

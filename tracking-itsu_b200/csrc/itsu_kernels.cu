@@ -238,16 +238,13 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(Arena a, const int32_t *_
   }
 }
 
-// Blocks of a grid-stride kernel: those of a full grid, or what about `items` items need. The counts
-// are on the device; the host goes by the clusters (10 tracklets and 2 cells each are the arena's first
-// sizes, above what any workload here has), and any grid gives the same results. A pp event's kernels
-// took 5.5 us each with full grids of idle blocks.
+// Blocks of a grid-stride kernel: those of a full grid, or what about `items` items need (Launch::tracklets
+// and ::cells; any grid gives the same results). A pp event's kernels took 5.5 us each with full grids of
+// idle blocks, 4.3 with its own.
 unsigned blocks_for(int64_t full, int64_t items, int64_t per_block)
 {
   return (unsigned)std::max<int64_t>(1, std::min(full, (items + per_block - 1) / per_block));
 }
-int64_t likely_tracklets(const Arena &a) { return 10 * a.n_clusters; }
-int64_t likely_cells(const Arena &a) { return 2 * a.n_clusters; }
 
 // The four scans of a run: tracklets per cluster, cells per span of tracklets, neighbours per cell,
 // roads per cell. The first leaves the check of its capacity to the segment pass.
@@ -260,15 +257,15 @@ void step_scan(const Arena &a, const Launch &l)
                                                                 &a.status->total[kTracklets], INT64_MAX, 0);
     break;
   case 1:
-    k_scan<true><<<blocks_for(l.num_sms * 4, likely_tracklets(a) / 32, kScanTile) + 1, kScanThreads, 0, l.stream>>>(a, a.cell_span_count, a.cell_span_off, &a.status->cell_spans, 0, a.scan_partials,
+    k_scan<true><<<blocks_for(l.num_sms * 4, l.tracklets / 32, kScanTile) + 1, kScanThreads, 0, l.stream>>>(a, a.cell_span_count, a.cell_span_off, &a.status->cell_spans, 0, a.scan_partials,
                                                                &a.status->total[kCells], a.cap_cells, kFlagCapCells);
     break;
   case 2:
-    k_scan<false><<<blocks_for(l.num_sms * 4, likely_cells(a), kScanTile), kScanThreads, 0, l.stream>>>(a, a.nb_count, a.nb_off, &a.status->total[kCells], 0, a.scan_partials,
+    k_scan<false><<<blocks_for(l.num_sms * 4, l.cells, kScanTile), kScanThreads, 0, l.stream>>>(a, a.nb_count, a.nb_off, &a.status->total[kCells], 0, a.scan_partials,
                                                                 &a.status->total[kNeighbours], a.cap_neighbours, kFlagCapNeighbours);
     break;
   default:
-    k_scan<false><<<blocks_for(l.num_sms * 4, likely_cells(a), kScanTile), kScanThreads, 0, l.stream>>>(a, a.road_count, a.road_off, &a.status->total[kCells], 0, a.road_partials,
+    k_scan<false><<<blocks_for(l.num_sms * 4, l.cells, kScanTile), kScanThreads, 0, l.stream>>>(a, a.road_count, a.road_off, &a.status->total[kCells], 0, a.road_partials,
                                                                 &a.status->total[kRoads], a.cap_roads, kFlagCapRoads);
   }
 }
@@ -2201,7 +2198,7 @@ dim3 event_grid(const Arena &a, const Launch &l)
 {
   const int rows = std::min(a.n_events, 65535);
   const int64_t full = std::max(1, (fixed_grid(l) + rows - 1) / rows);
-  return dim3(blocks_for(full, likely_cells(a) / std::max(rows, 1), l.block), (unsigned)rows);
+  return dim3(blocks_for(full, l.cells / std::max(rows, 1), l.block), (unsigned)rows);
 }
 
 void step_status_init(const Arena &a, const Launch &l)
@@ -2323,8 +2320,8 @@ void step_tracklets_crowded(const Arena &a, const Launch &l)
   }
 }
 
-// Blocks for the segments, and for the crowded clusters of larger runs.
-unsigned segment_blocks(const Arena &a, const Launch &l) { return blocks_for(l.num_sms, a.n_events * ITSU_TRACKLET_LAYERS + a.n_clusters / 32, 128); }
+// Blocks for the segments, and a thread per cluster, any of which may be crowded.
+unsigned segment_blocks(const Arena &a, const Launch &l) { return blocks_for(l.num_sms, a.n_events * ITSU_TRACKLET_LAYERS + a.n_clusters, 128); }
 
 void step_tracklet_segments(const Arena &a, const Launch &l)
 {
@@ -2337,7 +2334,7 @@ void step_tracklet_segments(const Arena &a, const Launch &l)
 
 void launch_cells_range(const Arena &a, const Launch &l, int32_t e0, int32_t e1, bool last)
 {
-  const unsigned blocks = blocks_for(l.num_sms * kCellBlocks, likely_tracklets(a), kCellThreads);
+  const unsigned blocks = blocks_for(l.num_sms * kCellBlocks, l.tracklets, kCellThreads);
   if (a.cap_cell_pairs < a.cap_cell_entries) {
     k_cells_count<true><<<blocks, kCellThreads, 0, l.stream>>>(a, e0, e1, last);
   } else {
@@ -2377,7 +2374,7 @@ void step_cells_prefilter(const Arena &a, const Launch &l)
   }
 }
 
-void step_cells_scatter(const Arena &a, const Launch &l) { k_cells_scatter<<<blocks_for(l.num_sms * 8, likely_tracklets(a) / 32, kScatterThreads / 32), kScatterThreads, 0, l.stream>>>(a); }
+void step_cells_scatter(const Arena &a, const Launch &l) { k_cells_scatter<<<blocks_for(l.num_sms * 8, l.tracklets / 32, kScatterThreads / 32), kScatterThreads, 0, l.stream>>>(a); }
 
 void step_neighbour_reset(const Arena &a, const Launch &l)
 {
@@ -2387,7 +2384,7 @@ void step_neighbour_reset(const Arena &a, const Launch &l)
 }
 
 template <bool kWrite>
-void step_neighbours(const Arena &a, const Launch &l) { k_neighbours<kWrite><<<blocks_for(fixed_grid(l), likely_cells(a), l.block), l.block, 0, l.stream>>>(a); }
+void step_neighbours(const Arena &a, const Launch &l) { k_neighbours<kWrite><<<blocks_for(fixed_grid(l), l.cells, l.block), l.block, 0, l.stream>>>(a); }
 
 // Threads for about half of the cells of the largest event's largest layer (a layer of hits has about
 // 1.3 cells per hit), so that a layer takes one or two rounds.
@@ -2396,7 +2393,7 @@ void step_levels(const Arena &a, const Launch &l)
   if (a.n_events <= 0) {
     return;
   }
-  const LevelShape shape = level_shape(a.n_events, l.max_segment, l.num_sms);
+  const LevelShape shape = level_shape(a.n_events, l.level_size, l.num_sms);
   if (shape.wide) {
     for (int layer = 1; layer < ITSU_CELL_LAYERS; ++layer) {
       k_levels_layer<<<event_grid(a, l), l.block, 0, l.stream>>>(a, layer);
@@ -2469,21 +2466,22 @@ SortShape sort_shape(int32_t n_events, int64_t n_clusters, int64_t max_segment)
   return s;
 }
 
-// The level pass's launch for a run whose largest layer has max_segment clusters. A cluster of 8 CTAs has
+// The level pass's launch for a run whose largest layer has as many cells as `size` clusters ordinarily
+// give (Launch::level_size). A cluster of 8 CTAs has
 // 4096 threads for an event's layer, and the cells of a layer grow with the square of its clusters: few
 // events with large layers take a wide launch per layer instead. One event with layers of 9,450 clusters:
 // 34 us in clusters, 28 wide; of 26,250: 126 and 38; of 52,500: 478 and 55. Four of 9,450: 37 and 38;
 // eight of 12,600: 49 and 41; 16: 54 and 50; 32: 74 and 77.
 constexpr int64_t kWideLevels = 10000;
-LevelShape level_shape(int32_t n_events, int64_t max_segment, int num_sms)
+LevelShape level_shape(int32_t n_events, int64_t size, int num_sms)
 {
   LevelShape s;
-  s.threads = max_segment > 192 ? 512 : 128;
+  s.threads = size > 192 ? 512 : 128;
   s.ctas = 1;
-  while (s.threads == 512 && s.ctas < 8 && 3 * max_segment > 4 * 512 * s.ctas) {
+  while (s.threads == 512 && s.ctas < 8 && 3 * size > 4 * 512 * s.ctas) {
     s.ctas *= 2;
   }
-  s.wide = max_segment > kWideLevels && 2 * (int64_t)n_events * s.ctas < 3 * num_sms;
+  s.wide = size > kWideLevels && 2 * (int64_t)n_events * s.ctas < 3 * num_sms;
   return s;
 }
 
