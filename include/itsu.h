@@ -93,14 +93,17 @@ typedef enum itsu_status {
   ITSU_OK = 0,
   ITSU_ERR_INVALID = 1,  /* malformed input or argument (rejected before any kernel runs) */
   ITSU_ERR_CAPACITY = 2, /* a result did not fit and the arena could not grow */
-  ITSU_ERR_TIMEOUT = 3,  /* a bounded device wait gave up */
+  ITSU_ERR_TIMEOUT = 3,  /* reserved: no device code waits */
   ITSU_ERR_CUDA = 4,     /* a CUDA runtime call failed */
   ITSU_ERR_NOMEM = 5,    /* device or host allocation failed */
   ITSU_ERR_STATE = 6     /* call out of order (e.g. stage before initialize) */
 } itsu_status;
 
 /* Flags of itsu_config.flags */
-#define ITSU_FLAG_NO_GROW 1u /* report ITSU_ERR_CAPACITY instead of growing and re-running */
+/* Report ITSU_ERR_CAPACITY instead of growing and re-running: the arena keeps what it was created with,
+ * and takes every run whose tracklets, cells, neighbours and roads it holds (with the pair prefilter,
+ * where the cells before it are at most twice as many as it holds and 2.6 million). */
+#define ITSU_FLAG_NO_GROW 1u
 /* itsu_batch_run_host streams: the batch runs as consecutive chunks of events, each chunk's
  * upload overlapping the work on the one before; only the roads and road offsets are kept
  * (the per-event results API then reports ITSU_ERR_STATE until the next run). */
@@ -232,7 +235,9 @@ itsu_status itsu_batch_run_host_tracks(itsu_context *ctx, const itsu_cluster_tra
                                        const float *vertices, int32_t n_events, itsu_road *roads, int64_t roads_capacity,
                                        int32_t *road_offsets);
 /* Launches every stage of the batch on the context stream without waiting (a CUDA-graph
- * replay from the third call in a row with the same inputs on); itsu_batch_status waits and reports. */
+ * replay from the third call in a row with the same inputs on); itsu_batch_status waits and reports. A
+ * batch with the pointers and sizes of the last run is taken to have its layer offsets too (checked then);
+ * its clusters and vertices may be others. */
 itsu_status itsu_batch_launch(itsu_context *ctx, const itsu_batch *batch);
 itsu_status itsu_batch_status(itsu_context *ctx);
 /* Device pointer to the roads of the last batch (event-major) and to road_offsets[n_events+1]. */
@@ -506,7 +511,8 @@ typedef struct itsu_memory_usage {
   int64_t events_capacity;
   int64_t capacity[4];           /* tracklets, cells, neighbours, roads the arena holds */
   int64_t used[4];               /* the last synchronised run's totals (0 before any) */
-  int64_t cell_entries_capacity; /* the cell count pass's entry scratch */
+  int64_t cell_entries_capacity; /* the cell count pass's entry scratch (places for tracklet pairs; in a fixed
+                                    arena also for cells that are counted first) */
 } itsu_memory_usage;
 itsu_status itsu_memory_usage_get(itsu_context *ctx, itsu_memory_usage *out);
 

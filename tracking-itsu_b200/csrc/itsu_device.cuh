@@ -105,15 +105,6 @@ __device__ __forceinline__ int4 bins_rect(float phi, int layer, float dir_z)
                    min(kZBins - 1, z_bin_index(layer + 1, z_max)), phi_bin_index(normalized_phi(phi_max)));
 }
 
-// Tracker.cxx:93-100: the tracklet cut for candidate (r2, z2, phi2) of inner cluster (r1, z1, phi1).
-__device__ __forceinline__ bool tracklet_cut(int layer, float tan_lambda, float r1, float z1, float phi1, float r2, float z2,
-                                             float phi2)
-{
-  const float delta_z = fabsf(tan_lambda * (r2 - r1) + z1 - z2);
-  const float delta_phi = fabsf(phi1 - phi2);
-  return delta_z < kC.trk_max_dz[layer] && (delta_phi < kPhiCoordinateCut || delta_phi > kPhiWrapTracklet);
-}
-
 // Tracker.cxx:161-173: the cheap cell cuts, which need only the two tracklets and the first
 // cluster (c = (x, y, z, r)); most pairs stop here. Every term is evaluated (no early exit: the
 // terms are pure, so the result is the reference's short-circuit one) so that a loop over

@@ -276,7 +276,7 @@ struct KernelStep {
                      // runs with event groups (kGroupedStep) or without (kUngroupedStep), stage calls (kStagedStep)
 };
 const KernelStep *pipeline_steps(int *count);
-int kernels_per_run();  // kernels one plain run launches (the learned form adds the learned_only steps)
+int kernels_per_run();  // kernels one plain run launches, a wide level pass's four counted as one (the learned form adds the learned_only steps)
 
 // Learned networks (itsu_prefilter.cu), all asynchronous on `stream`; each call has an
 // overload for the pair prefilter (itsu_prefilter_model, MlpDevice) and one for the tracklet gate

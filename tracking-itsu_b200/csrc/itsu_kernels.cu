@@ -15,7 +15,8 @@
 //                entries copied to their scanned places, with the lookup table
 //   neighbours   one thread per cell walking the next-layer cells of its outer tracklet; rows
 //                keyed by the next-layer cell, sorted ascending (Tracker.cxx:417-474)
-//   levels       layer-ordered longest-chain DP plus the number of level-decreasing chains
+//   levels       layer-ordered longest-chain DP plus the number of level-decreasing chains; one launch
+//                of a CTA cluster per event, or wide ones per layer for few large events
 //   roads        one lane per road: the root's k-th chain in the reference's order, Moore-vote
 //                labels (Tracker.cxx:477-652)
 // Capacity overflow never writes out of bounds: the passes check the scanned totals and scratch
@@ -723,7 +724,7 @@ __device__ __forceinline__ void write_tracklet(const Arena &a, int out, int64_t 
 }
 
 constexpr int kTrackletSlots = kTrackletSlotsPerCluster;
-constexpr int kMaskKeys = 32;  // keys of the walk's window a mask holds (of 64: 0.72 in place of 0.66 ms per 128 central events)
+constexpr int kMaskKeys = 32;  // keys of the walk's window a mask holds (with 64 the pass took 0.72 ms per 128 central events when with 32 it took 0.66; it takes 0.59 now)
 constexpr int kMaxMaskedOut = 64;  // out-degrees up to this are evaluated pair-parallel with a pass mask
 
 // The reference's candidate sequence of one inner cluster (Tracker.cxx:73-113), calling
@@ -1173,7 +1174,7 @@ constexpr int kWriteThreads = 256;
 constexpr int kWriteBlocks = 5;  // resident blocks per SM
 // A block prefetches the lines of the block a wave later: coordinates, offsets, segments and the first
 // slots (0.499 ms without; 12 slots and 16 cost more than they bring, 0.490 and 0.496, two waves 0.509).
-constexpr int kWriteAhead = 148 * kWriteBlocks;
+constexpr int kWriteAhead = 148 * kWriteBlocks;  // of the 148 SMs of a B200
 constexpr int kWriteAheadSlots = 8;
 static_assert(kWriteAheadSlots <= kTrackletSlots && 6 + kWriteAheadSlots <= 32, "a line per lane");
 
@@ -1362,7 +1363,9 @@ constexpr int kCellQueue = 512;  // queued pairs of a warp (a span of 128 has 68
 constexpr int kCellRing = 64;
 static_assert(kMaxSpan <= 128 && kMaxMaskedOut <= 64, "a queue item is 7 bits of span and 6 of outgoing tracklets");
 
-// First tracklets in a span, of a run of n (there are 4736 warps: from 2^21 on each has 3 spans of 128 or more).
+// First tracklets in a span, of a run of n. A full grid has 5328 warps (9 blocks of 4 on 148 SMs): from
+// 2^20 tracklets on each of them has three spans of 64 or more, from 2^22 six of 128; shorter runs take
+// the shortest spans, for as many warps as there are.
 __device__ __forceinline__ uint32_t span_of(uint32_t n) { return n >= (1u << 22) ? 128 : (n >= (1u << 20) ? 64 : 32); }
 
 struct CellWarp {
@@ -2462,9 +2465,10 @@ void run_steps(int first, int last, const Arena &a, const Launch &l)
 
 // The clustering's launch for a run whose largest layer has max_segment clusters (any shape gives the
 // same results). Small layers take small CTAs: the tables' set-up is most of their work. Layers of
-// even size are split over clusters of 2 to 8 CTAs while that makes no more than 1024 of them (about
-// three waves), so that the last wave is not nearly empty; where the sizes differ widely, the large
-// ones only while the chip has room for all of them at once.
+// even size are split over clusters of 2 to 8 CTAs while that makes no more than 1024 of them (two to
+// three waves at three CTAs on each of 148 SMs), so that the last wave is not nearly empty; where the
+// sizes differ widely, the large ones only while the chip has room for all of them at once (296: two per
+// SM).
 SortShape sort_shape(int32_t n_events, int64_t n_clusters, int64_t max_segment)
 {
   const int64_t segments = (int64_t)n_events * ITSU_LAYERS;

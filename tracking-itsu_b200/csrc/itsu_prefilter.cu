@@ -24,7 +24,7 @@ namespace {
 
 constexpr int kTrainWarps = 4;
 constexpr int kTrainSamples = 16 * kTrainWarps;  // a block's tile
-constexpr int kMaxGradBlocks = 2 * 148;          // two per SM; each leaves a gradient partial
+constexpr int kMaxGradBlocks = 2 * 148;          // two per SM of a B200; each leaves a gradient partial
 
 __device__ __forceinline__ uint64_t splitmix64(uint64_t x)
 {
