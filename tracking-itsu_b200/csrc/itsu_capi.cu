@@ -581,8 +581,8 @@ itsu_status ensure_tracklets(itsu_context *ctx, int64_t need)
 }
 
 // Entry scratch for an arena of these capacities. The cell count pass reserves a place per pair that its
-// precut lets through (0.54 per tracklet in central events, up to one in pile-up frames, a hundred in
-// narrow jets) and reports what did not fit. Pairs bound no result, so a fixed arena has a second part,
+// precut lets through (0.54 per tracklet in central events, up to one in pile-up frames, 74 in a bundle
+// of 300 lines) and reports what did not fit. Pairs bound no result, so a fixed arena has a second part,
 // where cells that are counted first take exactly their places: as many as it holds cells, twice (the
 // pair prefilter drops some after them), and kExactPlaces.
 struct CellPlaces {
