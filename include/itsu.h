@@ -511,8 +511,8 @@ typedef struct itsu_memory_usage {
   int64_t events_capacity;
   int64_t capacity[4];           /* tracklets, cells, neighbours, roads the arena holds */
   int64_t used[4];               /* the last synchronised run's totals (0 before any) */
-  int64_t cell_entries_capacity; /* the cell count pass's entry scratch (places for tracklet pairs; in a fixed
-                                    arena also for cells that are counted first) */
+  int64_t cell_entries_capacity; /* the cell count pass's entry scratch (places for tracklet pairs; in fixed
+                                    and very large arenas also for cells that are counted first) */
 } itsu_memory_usage;
 itsu_status itsu_memory_usage_get(itsu_context *ctx, itsu_memory_usage *out);
 

@@ -55,3 +55,26 @@ def test_exact_capacities_suffice(n, n_events, spread, pair_prefilter):
         growing.close()
         if fixed is not None:
             fixed.close()
+
+
+def test_pairs_beyond_a_quarter_of_the_memory():
+    """1.36e9 pairs of 4 million tracklets: a growing arena keeps places for some of them and counts the
+    cells of the other spans, a fixed one counts nearly all; tracklets, cells and lookups are the same."""
+    ev = _bundle(1, 1400, 0.002)
+    growing, fixed = capi.Context(), None
+    try:
+        want = growing.run_vertex(ev.layers, ev.vertices[0])
+        assert sum(map(len, want["cells"])) > 1000
+        usage = growing.memory_usage()
+        assert usage["device_bytes"] < 60e9
+        roads = growing.clusters_to_tracks(ev.layers, ev.vertices[0])
+        assert oracle.diff(growing.results(0), want) == []
+        caps = {"max_" + name: max(int(used), 1) for name, used in usage["used"].items()}
+        fixed = capi.Context(flags=capi.FLAG_NO_GROW, max_clusters=sum(map(len, ev.layers)), max_events=1, **caps)
+        assert fixed.memory_usage()["device_bytes"] < 2e9
+        assert fixed.clusters_to_tracks(ev.layers, ev.vertices[0]).tobytes() == roads.tobytes()
+        assert oracle.diff(fixed.results(0), want) == []
+    finally:
+        growing.close()
+        if fixed is not None:
+            fixed.close()

@@ -105,6 +105,7 @@ struct itsu_context {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   int num_sms = 148;
+  int64_t device_bytes = 0;  // memory of the device
 
   // capacities
   int64_t cap_clusters = kNoBuffers;
@@ -582,19 +583,23 @@ itsu_status ensure_tracklets(itsu_context *ctx, int64_t need)
 
 // Entry scratch for an arena of these capacities. The cell count pass reserves a place per pair that its
 // precut lets through (0.54 per tracklet in central events, up to one in pile-up frames, 74 in a bundle
-// of 300 lines) and reports what did not fit. Pairs bound no result, so a fixed arena has a second part,
-// where cells that are counted first take exactly their places: as many as it holds cells, twice (the
-// pair prefilter drops some after them), and kExactPlaces.
+// of 300 lines) and reports what did not fit. Pairs bound no result, so there is a second part, where
+// cells that are counted first take exactly their places, in fixed arenas, which cannot grow, and in
+// others where a run's pairs would take more than a quarter of the device's memory: as many places as the
+// arena holds cells, twice (the pair prefilter drops some after them), and kExactPlaces. Counting first
+// costs more than half of such spans' time again: an event of 800 lines, 255 million pairs, 5.1 ms in
+// places by pairs, 7.8 with most of them counted.
 struct CellPlaces {
   int64_t pairs, exact;
 };
 constexpr int64_t kExactPlaces = int64_t(5) << 19;
+int64_t most_pairs(const itsu_context *ctx) { return ctx->device_bytes / 4 / (int64_t)(sizeof(itsu::CellEntry) + sizeof(float)); }
 int64_t exact_places(const itsu_context *ctx) { return 2 * ctx->cap_cells + kExactPlaces; }
 CellPlaces cell_places(const itsu_context *ctx)
 {
-  const bool fixed = (ctx->flags & ITSU_FLAG_NO_GROW) != 0;
-  return fixed ? CellPlaces{2 * ctx->cap_tracklets + ctx->cap_cells, exact_places(ctx)}
-               : CellPlaces{ctx->cap_tracklets / 2 + ctx->cap_cells + (1 << 14), 0};
+  if (ctx->flags & ITSU_FLAG_NO_GROW) return CellPlaces{2 * ctx->cap_tracklets + ctx->cap_cells, exact_places(ctx)};
+  return CellPlaces{ctx->cap_tracklets / 2 + ctx->cap_cells + (1 << 14),
+                    ctx->cap_cell_pairs < ctx->cap_cell_entries ? exact_places(ctx) : 0};
 }
 
 cudaError_t alloc_cell_entries(itsu_context *ctx, CellPlaces want)
@@ -612,19 +617,18 @@ cudaError_t alloc_cell_entries(itsu_context *ctx, CellPlaces want)
   return err;
 }
 
-// At least these places of each part. Where places for all pairs are more than the memory or their
-// indexes allow, the arena's ordinary number of them and, as in a fixed one, exact places.
+// At least these places of each part.
 itsu_status ensure_cell_entries(itsu_context *ctx, CellPlaces need)
 {
   CellPlaces want{ctx->cap_cell_pairs, ctx->cap_cell_entries - ctx->cap_cell_pairs};
   if (need.pairs <= want.pairs && need.exact <= want.exact) return ITSU_OK;
   itsu_status st = growth_allowed(ctx, "cell entries", need.pairs + need.exact, ctx->cap_cell_entries);
   if (st != ITSU_OK) return st;
-  if (need.pairs > want.pairs) want.pairs = grow_to(need.pairs);
+  if (need.pairs > want.pairs) want.pairs = std::max(need.pairs, std::min(grow_to(need.pairs), most_pairs(ctx)));
   if (need.exact > want.exact) want.exact = grow_to(need.exact);
   const int stage = ctx->stage;
   cudaError_t err = alloc_cell_entries(ctx, want);
-  if (err == cudaErrorMemoryAllocation) {
+  if (err == cudaErrorMemoryAllocation) {  // more pairs than the memory or their indexes allow: the ordinary number of them
     ctx->stage = stage;
     err = alloc_cell_entries(ctx, CellPlaces{std::min(want.pairs, cell_places(ctx).pairs), std::max(want.exact, exact_places(ctx))});
   }
@@ -632,11 +636,16 @@ itsu_status ensure_cell_entries(itsu_context *ctx, CellPlaces need)
   return ITSU_OK;
 }
 
-// Room for a run's entries that did not fit: for all its pairs, or for the cells counted in their place.
+// Room for a run's entries that did not fit: for all its pairs, or, where those are many, for some of them
+// and for counted cells.
 itsu_status grow_cell_entries(itsu_context *ctx, const DevStatus &s)
 {
-  const int64_t exact = ctx->cap_cell_entries - ctx->cap_cell_pairs;
-  return ensure_cell_entries(ctx, exact > 0 ? CellPlaces{ctx->cap_cell_pairs, s.cell_exact} : CellPlaces{s.cell_entries, 0});
+  CellPlaces need{s.cell_entries, 0};
+  if (ctx->cap_cell_pairs < ctx->cap_cell_entries || s.cell_entries > most_pairs(ctx)) {
+    need.pairs = std::min(s.cell_entries, most_pairs(ctx));
+    need.exact = std::max(s.cell_exact, exact_places(ctx));
+  }
+  return ensure_cell_entries(ctx, need);
 }
 
 // The cell stage's outputs. Not its scratch: after the count pass, growing it would lose the entries.
@@ -1153,6 +1162,9 @@ itsu_status itsu_context_create(const itsu_config *cfg, itsu_context **out)
       break;
     }
     cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, c.device);
+    size_t free_bytes = 0, all_bytes = 0;
+    if ((err = cudaMemGetInfo(&free_bytes, &all_bytes)) != cudaSuccess) break;
+    ctx->device_bytes = (int64_t)all_bytes;
     if ((err = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess) break;
     ctx->own_stream = true;
     if ((err = cudaMalloc((void **)&ctx->d_status, sizeof(DevStatus))) != cudaSuccess) break;
