@@ -78,3 +78,27 @@ def test_pairs_beyond_a_quarter_of_the_memory():
         growing.close()
         if fixed is not None:
             fixed.close()
+
+
+@pytest.mark.parametrize("group", [1, 2])
+@pytest.mark.parametrize("flags", [0, capi.FLAG_STREAM_HOST])
+def test_scratch_overflow_with_event_groups(group, flags):
+    """The first group's pairs do not fit the entry scratch of a new arena: the groups after it are
+    written and counted all the same, for what the run needs, and the repeated run gives the oracle's
+    results."""
+    events = [_bundle(7, 180, 0.002)] + [gen.pbpb_event(60 + k) for k in range(3)]
+    want = [oracle.run_vertex(ev.layers, ev.vertices[0]) for ev in events]
+    clusters, offsets, vertices = gen.pack_batch(events)
+    ctx = capi.Context(flags=flags, stream_chunk_clusters=60000)
+    try:
+        for band in range(32):
+            ctx.set_tune(band, 256, 8, 1, group)
+        for _ in range(2):
+            roads, road_offsets = ctx.batch_run_host(clusters, offsets, vertices)
+            for e, w in enumerate(want):
+                assert roads[road_offsets[e]:road_offsets[e + 1]].tobytes() == w["roads"].tobytes(), e
+        if flags == 0:
+            for e, w in enumerate(want):
+                assert oracle.diff(ctx.results(e), w) == [], e
+    finally:
+        ctx.close()

@@ -1187,7 +1187,9 @@ struct WriteWarp {
 __global__ void __launch_bounds__(kWriteThreads, kWriteBlocks) k_tracklets_write(Arena a, int64_t c0, int64_t c1)
 {
   __shared__ WriteWarp shared[kWriteThreads / 32];
-  if (capacity_failed(a.status)) {
+  // not stopped by the scratch flag: with event groups the count pass of an earlier group may have raised
+  // it, and this group's goes on to add up what the run needs, on tracklets that have to be there
+  if ((*(volatile const int32_t *)&a.status->flags & kCapacityMask & ~kFlagCapScratch) != 0) {
     return;
   }
   WriteWarp &w = shared[threadIdx.x >> 5];
