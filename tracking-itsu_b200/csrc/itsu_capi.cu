@@ -331,9 +331,9 @@ Tune current_tune(const itsu_context *ctx)
 // What grids go by, before the counts of a run are known on the host: ten tracklets and two cells per
 // cluster (above what any workload here has), times the last run's density beyond that, so that a narrow
 // jet's hundreds per cluster find a full grid from its second run on; and, so that its first run finds
-// some blocks, as many tracklets as its layers' pairs allow, up to three blocks per SM (a full grid costs
-// an ordinary small event 1 us in each kernel). One event of three layers of 300 clusters on one line has
-// 181 thousand tracklets: 4.2 ms by its clusters alone.
+// some blocks, one in three of its layers' pairs, up to three blocks per SM (a full grid costs an ordinary
+// small event 1 us in each kernel; all pairs in place of a third cost it 1 to 2 us in all). One event of
+// three layers of 300 clusters on one line has 181 thousand tracklets: 4.2 ms by its clusters alone.
 constexpr int64_t kUsualTracklets = 10, kUsualCells = 2;
 
 int doublings(int64_t count, int64_t usual)
@@ -360,8 +360,8 @@ Launch launch_of(const itsu_context *ctx)
   l.block = t.block;
   l.blocks_per_sm = t.blocks_per_sm;
   l.max_segment = ctx->max_segment;
-  l.tracklets = std::max((kUsualTracklets * ctx->n_clusters) << ctx->dense_tracklets, std::min<int64_t>(ctx->most_tracklets, 3 * 128 * ctx->num_sms));
-  l.cells = std::max((kUsualCells * ctx->n_clusters) << ctx->dense_cells, std::min<int64_t>(ctx->most_tracklets, 256 * ctx->num_sms));
+  l.tracklets = std::max((kUsualTracklets * ctx->n_clusters) << ctx->dense_tracklets, std::min<int64_t>(ctx->most_tracklets / 3, 3 * 128 * ctx->num_sms));
+  l.cells = std::max((kUsualCells * ctx->n_clusters) << ctx->dense_cells, std::min<int64_t>(ctx->most_tracklets / 3, 256 * ctx->num_sms));
   l.level_size = ctx->max_segment;
   if (ctx->dense_cells > 0 && ctx->n_events > 0) {
     // five layers of cells, four for three clusters of an ordinary one
